@@ -1,0 +1,517 @@
+"""Performance cases: the work that users of this framework have it do.
+
+Each case is one kind of call through the public Python API (lmff_gb300.capi, the ctypes
+binding of the C ABI) on a seeded layered system:
+
+  eval     lmff_compute on host arrays, as the LAMMPS pair styles call it each step
+  device   lmff_compute_device on CUDA tensors, as an in-process GPU program calls it
+  noalloc  lmff_compute_device_noalloc, the allocation-free call for small systems
+  rank     lmff_compute_ghost, one MPI rank of a domain decomposition
+  md       lmff_run_nve on a resident system, then a frame read back
+  minimize lmff_upload + lmff_minimize
+  batch    lmff_batch_set + lmff_batch_compute on many independent systems
+
+FP64 is the precision every entry point and the LAMMPS styles have by default; mixed is
+the large-scale MD precision.
+"""
+import math
+import os
+import sys
+
+import numpy as np
+import torch
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PKG = os.path.join(ROOT, "lammps-lmff_gb300")
+if PKG not in sys.path:
+    sys.path.insert(0, PKG)
+
+from lmff_gb300 import capi  # noqa: E402
+from lmff_gb300 import structures as S  # noqa: E402
+
+POT = os.path.join(PKG, "potentials")
+BNC, ILP_FILE, KC_FILE = (os.path.join(POT, f) for f in ("BNC.tersoff", "BNCH.ILP", "CC.KC-full"))
+CUT = 16.0          # pair_style ... ilp/graphene/hbn 16.0 1
+
+
+def _case(name, kind, system, nx, ny, layers, prec, **more):
+    """system: "graphite" (layers AB-stacked, ids 1,2,1,2: odd separations interact), "stack"
+    (the same with an id per layer: every separation interacts), "hbn" / "graphene" (a
+    twisted top layer on graphene); nx x ny 4-atom cells per layer; prec "fp64" or "mixed"."""
+    c = {"kind": kind, "system": system, "nx": nx, "ny": ny, "layers": layers, "prec": prec, "skin": 2.0,
+         "style": "ilp", "steps": 0, "count": 1, "theta": 0.0, "vatom": False}
+    c.update(more)
+    return c if name is None else dict(c, name=name)
+
+
+def listed():
+    return [
+        # the smallest call: a small bilayer evaluated inside another GPU program, device
+        # buffers in and out, energies and virial; launches and latency are its time
+        _case("noalloc_1152_fp64", "noalloc", "graphite", 16, 9, 2, "fp64"),
+        # a LAMMPS user's own case size (six layers, 5,016 atoms): four consecutive time
+        # steps of a pair style, forces only, host arrays, the first one reneighbouring
+        _case("steps_5016_fp64", "eval", "stack", 19, 11, 6, "fp64", count=4),
+        # the plain FP64 drop-in's parity workload advanced on the device
+        _case("md_7200_fp64", "md", "graphite", 30, 30, 2, "fp64", steps=40),
+        # the same bilayer in mixed precision at the autotuned skin: launch-bound MD
+        _case("md_7200_mixed", "md", "graphite", 30, 30, 2, "mixed", steps=200, skin=1.5),
+        # production MD of a twisted graphene/hBN heterostructure, several elements
+        _case("md_twisted_490k_mixed", "md", "hbn", 329, 190, 2, "mixed", steps=40, theta=0.6),
+        # the largest: the 2.7M-atom ten-layer graphite slab of the benchmark
+        _case("md_graphite_2p7m_mixed", "md", "graphite", 342, 197, 10, "mixed", steps=50, skin=1.0),
+        # single point with energies and virial of a large slab at full precision, device
+        # buffers
+        _case("point_331k_fp64", "device", "graphite", 120, 69, 10, "fp64"),
+        # a thermo / compute stress/atom step: per-atom energy and per-atom virial too
+        _case("stress_36800_fp64", "eval", "graphite", 40, 23, 10, "fp64", vatom=True),
+        _case("stress_331k_mixed", "eval", "graphite", 120, 69, 10, "mixed", vatom=True),
+        # a screening job: 64 independent replicas of ragged sizes (500 to 20,000 atoms),
+        # loaded and evaluated as one batch
+        _case("batch_64_mixed", "batch", "replicas", 500, 20000, 2, "mixed", count=64),
+        # relaxation of a thermally displaced stack of six layers
+        _case("minimize_5016_fp64", "minimize", "stack", 19, 11, 6, "fp64", steps=20),
+        # one of four MPI ranks of a slab: owned atoms and the ghost shell
+        _case("rank_twisted_61k_fp64", "rank", "hbn", 117, 67, 2, "fp64", theta=1.1),
+    ]
+
+
+# atoms of the largest drawn system per kind: what keeps a drawn case below the largest
+# listed one (50 steps of the 2.7M-atom slab)
+_MOST = {"noalloc": 2048, "eval": 300_000, "device": 300_000, "rank": 100_000, "md": 1_000_000, "minimize": 25_000,
+         "batch": 0}
+
+
+def draw(rng):
+    kind = rng.choice(["noalloc", "eval", "eval", "device", "rank", "md", "md", "minimize", "batch"])
+    prec = rng.choice(["fp64", "mixed"])
+    if kind == "batch":
+        nmin = rng.randrange(500, 3000)
+        return _case(None, kind, "replicas", nmin, nmin + rng.randrange(200, 17000), 2, prec,
+                     count=rng.randrange(3, 49))
+    system = rng.choice(["graphite", "stack", "hbn", "graphene"])
+    layers = 2 if system in ("hbn", "graphene") else rng.choice([2, 3] if kind == "noalloc" else [2, 3, 5, 6, 8])
+    most = _MOST[kind] if prec == "mixed" or kind != "md" else 30_000
+    lo = 400.0 if kind == "noalloc" else 1000.0
+    atoms = math.exp(rng.uniform(math.log(lo), math.log(most * 0.9)))
+    cells = max(40.0, atoms / (4 * layers))
+    shape = math.sqrt(3.0) * math.exp(rng.uniform(-0.3, 0.3))
+    nx, ny = max(4, round(math.sqrt(cells * shape))), max(3, round(math.sqrt(cells / shape)))
+    if kind == "noalloc":
+        while 4 * nx * ny * layers > 1900:   # the entry point's limit is 2,048 atoms
+            nx -= 1
+    style = "kc" if system in ("graphite", "stack", "graphene") and kind in ("eval", "device", "md") and \
+        rng.random() < 0.25 else "ilp"
+    c = _case(None, kind, system, nx, ny, layers, prec, style=style, skin=rng.choice([1.0, 1.5, 2.0]),
+              theta=round(rng.uniform(0.3, 5.0), 2) if system in ("hbn", "graphene") else 0.0)
+    if kind == "eval":
+        c["vatom"] = rng.random() < 0.3 and nx * ny * layers * 4 < 60_000
+        c["count"] = 1 if c["vatom"] else rng.randrange(1, 5)
+    elif kind == "md":
+        c["steps"] = rng.randrange(5, 60)
+    elif kind == "minimize":
+        c["steps"] = rng.randrange(5, 25)
+    return c
+
+
+# ------------------------------------------------------------------------------- inputs
+
+def _lattice(c):
+    if c["system"] in ("hbn", "graphene"):
+        return S.twisted_bilayer(c["nx"], c["ny"], c["theta"], top=c["system"], spacing=3.35)
+    return S.graphite_slab(c["layers"], c["nx"], c["ny"],
+                           mol_mode="unique" if c["system"] == "stack" else "alternate")
+
+
+def _systems(c, seed):
+    """The seeded system(s) of a case: thermal displacements (as at 300 K) and velocities."""
+    if c["kind"] == "batch":
+        return [S.displace(s, 0.03, seed + k) for k, s in
+                enumerate(S.replica_set(c["count"], c["nx"], c["ny"]))]
+    s = S.thermalize(_lattice(c), 300.0, seed)
+    return [s if c["kind"] == "md" else S.displace(s, 0.03, seed + 1)]
+
+
+def _frames(c, s):
+    """Consecutive 1 fs steps of the system's own motion."""
+    return [s.x + (0.001 * k) * s.v for k in range(c["count"])]
+
+
+def _engine(c):
+    prec = capi.MIXED if c["prec"] == "mixed" else capi.FP64
+    if c["style"] == "kc":
+        return capi.Engine(BNC, None, kc_file=KC_FILE, ilp_elements=("C", "NULL", "NULL"), cut_global=CUT,
+                           skin=c["skin"], precision=prec)
+    return capi.Engine(BNC, ILP_FILE, cut_global=CUT, skin=c["skin"], precision=prec)
+
+
+def _rank_atoms(c, s):
+    """Owned atoms of the lower-left quarter of the box and their ghost shell: every
+    periodic image within the neighbour cutoff of the quarter (comm_brick's rule).  Drawn
+    on the lattice, with room for the displacements, so that the counts are the case's."""
+    L, cg = s.box_hi - s.box_lo, CUT + c["skin"] + 0.5
+    lo, hi = s.box_lo.copy(), s.box_hi.copy()
+    hi[:2] = lo[:2] + 0.5 * L[:2]
+    lat = _lattice(c).x
+    x = s.x
+    own = np.nonzero(((lat >= lo) & (lat < hi))[:, :2].all(axis=1))[0]
+    is_own = np.zeros(s.n, bool)
+    is_own[own] = True
+    idx, gx = [own], [x[own]]
+    reach = [int(math.ceil(cg / L[d])) for d in range(2)]
+    for sx in range(-reach[0], reach[0] + 1):
+        for sy in range(-reach[1], reach[1] + 1):
+            shift = np.array([sx * L[0], sy * L[1], 0.0])
+            near = ((lat + shift >= lo - cg) & (lat + shift < hi + cg))[:, :2].all(axis=1)
+            if sx == 0 and sy == 0:
+                near &= ~is_own
+            k = np.nonzero(near)[0]
+            idx.append(k)
+            gx.append(x[k] + shift)
+    idx = np.concatenate(idx)
+    return len(own), np.concatenate(gx), idx
+
+
+def prepare(case, seed):
+    c = dict(case)
+    eng = _engine(c)
+    ss = _systems(c, seed)
+    s = ss[0]
+    st = {"case": c, "eng": eng, "sys": s}
+    kind = c["kind"]
+    if kind in ("device", "noalloc"):
+        eng.set_box(s.box_lo, s.box_hi, s.periodic)
+        st.update(x=torch.tensor(s.x, device="cuda"), t=torch.tensor(s.type, device="cuda"),
+                  m=torch.tensor(s.mol, device="cuda"), g=torch.tensor(s.tag, device="cuda"),
+                  f=torch.zeros(s.n, 3, dtype=torch.float64, device="cuda"))
+    elif kind == "eval":
+        eng.set_box(s.box_lo, s.box_hi, s.periodic)
+        st["frames"] = _frames(c, s)
+    elif kind == "rank":
+        nlocal, x, idx = _rank_atoms(c, s)
+        st.update(nlocal=nlocal, x=x, t=np.ascontiguousarray(s.type[idx]), m=np.ascontiguousarray(s.mol[idx]),
+                  g=np.ascontiguousarray(s.tag[idx]))
+    elif kind == "md":
+        eng.upload(s)
+    elif kind == "batch":
+        st["systems"] = ss
+    return st
+
+
+def _scalars(r):
+    return {"pvector": r["pvector"], "e": np.array([r["e_tersoff"], r["e_ilp"]]), "virial_tersoff": r["virial_tersoff"],
+            "virial_ilp": r["virial_ilp"]}
+
+
+def run(state):
+    c, eng, kind = state["case"], state["eng"], state["case"]["kind"]
+    s = state["sys"]
+    if kind == "noalloc":
+        r = eng.compute_device_noalloc(state["x"], state["t"], state["m"], state["f"])
+        return dict(_scalars(r), f=state["f"])
+    if kind == "device":
+        r = eng.compute_device(state["x"], state["t"], state["m"], state["g"], state["f"])
+        return dict(_scalars(r), f=state["f"])
+    if kind == "eval":
+        if c["vatom"]:
+            r = eng.compute(state["frames"][0], s.type, s.mol, s.tag, eatom=True, vatom=True)
+            return dict(_scalars(r), f=r["f"], eatom=r["eatom"], vatom_tersoff=r["vatom_tersoff"],
+                        vatom_ilp=r["vatom_ilp"])
+        return {"f": [eng.compute(x, s.type, s.mol, s.tag, eflag=False, vflag=False, same_atoms=k > 0)["f"]
+                      for k, x in enumerate(state["frames"])]}
+    if kind == "rank":
+        r = eng.compute_ghost(state["nlocal"], state["x"], state["t"], state["m"], state["g"])
+        return dict(_scalars(r), f=r["f"])
+    if kind == "md":
+        th = eng.run_nve(c["steps"], 0.001, thermo_every=c["steps"])
+        x, v, f = eng.download()
+        return {"x": x, "v": v, "f": f, "pe": th[-1]["pe"], "ke": th[-1]["ke"], "virial": th[-1]["virial"]}
+    if kind == "minimize":
+        eng.upload(s)
+        r = eng.minimize(1e-12, 1e-12, c["steps"], 100 * c["steps"])
+        x, _, f = eng.download()
+        return {"x": x, "f": f, "einitial": r["einitial"], "efinal": r["efinal"], "neval": r["neval"]}
+    eng.batch_set(state["systems"])
+    r = eng.batch_compute()
+    return {"f": np.concatenate([q["f"] for q in r]),
+            **{k: np.array([_scalars(q)[k] for q in r]) for k in ("pvector", "e", "virial_tersoff", "virial_ilp")}}
+
+
+# --------------------------------------------------------------------------------- work
+
+def work(case):
+    """Flops: the reference's arithmetic, 122.5 per directed interlayer pair inside the
+    cutoff and about 900 per atom for three Tersoff bonds and the normals.  Bytes: each
+    evaluation's positions in and forces out."""
+    c = case
+    sigma = 4.0 / (3.0 * math.sqrt(3.0) * S.A_CC_GRAPHENE ** 2)   # atoms per A^2 of a layer
+    if c["kind"] == "batch":
+        atoms, layers = c["count"] * (c["ny"] - c["nx"]) / math.log(c["ny"] / c["nx"]), 2
+    else:
+        atoms, layers = 4.0 * c["nx"] * c["ny"] * c["layers"], c["layers"]
+    pairs = 0.0
+    for sep in range(1, layers):
+        if c["system"] == "graphite" and sep % 2 == 0:
+            continue
+        pairs += 2.0 * (layers - sep) / layers * sigma * math.pi * max(0.0, CUT * CUT - (3.35 * sep) ** 2)
+    evals = {"md": c["steps"], "minimize": 2 * c["steps"]}.get(c["kind"], max(1, c["count"]))
+    if c["kind"] == "batch":
+        evals = 1
+    if c["kind"] == "rank":
+        atoms *= 0.25
+    extra = 13 * 8 if c["vatom"] else 0
+    return {"bytes": atoms * evals * (24 + 24 + extra), "flops": atoms * evals * (122.5 * pairs + 900.0)}
+
+
+# -------------------------------------------------------------------------------- exact
+# The two potentials in FP64 torch, from the published functional forms: energies by direct
+# sums over explicit periodic images, forces and virials by automatic differentiation.
+
+_ELEM = ("C", "B", "N")
+
+
+def _read(path, words):
+    out, tok = {}, []
+    for line in open(path):
+        tok += line.split("#")[0].split()
+        while len(tok) >= words:
+            n = 3 if words == 17 else 2
+            out[tuple(tok[:n])] = [float(w) for w in tok[n:words]]
+            tok = tok[words:]
+    return out
+
+
+def _tables(style, dev):
+    def tab(rows):
+        return torch.tensor(rows, dtype=torch.float64, device=dev)
+    t = _read(BNC, 17)
+    ters = tab([[[t[(a, b, d)] for d in _ELEM] for b in _ELEM] for a in _ELEM])
+    if style == "kc":
+        k = _read(KC_FILE, 12)[("C", "C")]
+        return ters, tab([[k] * 3] * 3)
+    p = _read(ILP_FILE, 13)
+    return ters, tab([[p[(a, b)] for b in _ELEM] for a in _ELEM])
+
+
+def _neighbours(x, mol, L, per, rc, dev, lo=0, hi=None, most=30_000_000, sub=None):
+    """Blocks (i, j, shift) of all directed pairs (images included) with r < rc."""
+    n = x.shape[0]
+    reach = [int(math.ceil(rc / L[d])) if per[d] else 0 for d in range(3)]
+    xs, js, sh = [], [], []
+    xmin, xmax = x.min(dim=0).values, x.max(dim=0).values
+    ids = torch.arange(n, device=dev)
+    for sx in range(-reach[0], reach[0] + 1):
+        for sy in range(-reach[1], reach[1] + 1):
+            for sz in range(-reach[2], reach[2] + 1):
+                t = torch.tensor([sx * L[0], sy * L[1], sz * L[2]], dtype=torch.float64, device=dev)
+                y = x + t
+                k = ((y > xmin - rc) & (y < xmax + rc)).all(dim=1).nonzero().squeeze(1)
+                xs.append(y[k])
+                js.append(ids[k])
+                sh.append(t.expand(len(k), 3))
+    xs, js, sh = torch.cat(xs), torch.cat(js), torch.cat(sh)
+    order = torch.argsort(xs[:, 0])
+    xs, js, sh = xs[order], js[order], sh[order]
+    oi = torch.argsort(x[:, 0])
+    if sub is not None:
+        oi = oi[sub[oi]]
+    xi = x[oi]
+    key = xs[:, 0].contiguous()
+    at = 0
+    while at < len(oi):
+        a = int(torch.searchsorted(key, xi[at, 0] - rc))
+        size = 4096
+        while True:
+            end = min(len(oi), at + size)
+            b = int(torch.searchsorted(key, xi[end - 1, 0] + rc, right=True))
+            if size <= 64 or (end - at) * (b - a) <= most:
+                break
+            size //= 2
+        d2 = ((xi[at:end, None, :] - xs[None, a:b, :]) ** 2).sum(-1)
+        d2 = torch.where((js[None, a:b] == oi[at:end, None]) & (d2 < 1e-12), torch.full_like(d2, 1e30), d2)
+        p, q = (d2 < rc * rc).nonzero(as_tuple=True)
+        yield oi[at:end][p], js[a:b][q], sh[a:b][q]
+        at = end
+
+
+def _tersoff(x, e, P, bonds):
+    """Energy per directed bond and centre: 1/2 sum fc (A e^-l1 r) + 1/2 sum b_ij (-B e^-l2 r) fc."""
+    i, j, sh = bonds
+    d = x[j] + sh - x[i]
+    r = d.norm(dim=1)
+
+    def fc(r, p):
+        R, D = p[..., 10], p[..., 11]
+        mid = 0.5 * (1.0 - torch.sin(0.5 * math.pi * (r - R) / D))
+        return torch.where(r < R - D, torch.ones_like(r), torch.where(r > R + D, torch.zeros_like(r), mid))
+    pij = P[e[i], e[j], e[j]]
+    # triplets: bonds sharing a centre
+    order = torch.argsort(i, stable=True)
+    i, j, d, r, pij = i[order], j[order], d[order], r[order], pij[order]
+    n = x.shape[0]
+    cnt = torch.bincount(i, minlength=n)
+    start = torch.cumsum(cnt, 0) - cnt
+    b = torch.arange(len(i), device=x.device)
+    most = int(cnt.max()) if len(i) else 0
+    zeta = torch.zeros_like(r)
+    for q in range(most):
+        k = start[i] + q
+        ok = (q < cnt[i]) & (k != b)
+        bb, kk = b[ok], k[ok]
+        pk = P[e[i[bb]], e[j[bb]], e[j[kk]]]
+        cs = (d[bb] * d[kk]).sum(-1) / (r[bb] * r[kk])
+        u2 = (pk[:, 5] - cs) ** 2
+        c2, d2 = pk[:, 3] ** 2, pk[:, 4] ** 2
+        g = pk[:, 1] * (1.0 + c2 / d2 - c2 / (d2 + u2))
+        arg = pk[:, 2] * (r[bb] - r[kk])
+        arg = torch.where(pk[:, 0] == 3.0, arg ** 3, arg)
+        zeta = zeta.index_add(0, bb, fc(r[kk], pk) * g * torch.exp(arg))
+    nn, t = pij[:, 6], pij[:, 7] * zeta
+    ts = torch.where(t > 0, t, torch.ones_like(t))
+    tn = ts ** nn
+    bij = (1.0 + tn) ** (-0.5 / nn)
+    c1, c2 = (2.0 * nn * 1e-16) ** (-1.0 / nn), (2.0 * nn * 1e-8) ** (-1.0 / nn)
+    bij = torch.where(t < 1.0 / c2, 1.0 - tn / (2.0 * nn), bij)
+    bij = torch.where(t < 1.0 / c1, torch.ones_like(t), bij)
+    bij = torch.where(t > c2, (1.0 - ts ** -nn / (2.0 * nn)) / ts.sqrt(), bij)
+    bij = torch.where(t > c1, 1.0 / ts.sqrt(), bij)
+    f = fc(r, pij)
+    eb = 0.5 * f * pij[:, 13] * torch.exp(-pij[:, 12] * r) \
+        - 0.5 * bij * pij[:, 9] * torch.exp(-pij[:, 8] * r) * f
+    return eb.sum()
+
+
+def _normals(x, bonds):
+    """Unit normals: the bond cross products of two or three intralayer neighbours, else z."""
+    i, j, sh = bonds
+    order = torch.argsort(i, stable=True)
+    i, j, sh = i[order], j[order], sh[order]
+    n = x.shape[0]
+    cnt = torch.bincount(i, minlength=n)
+    start = torch.cumsum(cnt, 0) - cnt
+    d = torch.cat([x[j] + sh - x[i], torch.zeros(3, 3, dtype=x.dtype, device=x.device)])
+    v0, v1, v2 = (d[torch.clamp(start + q, max=d.shape[0] - 1)] for q in range(3))
+    three = (cnt == 3)[:, None]
+    a = torch.where(three, v1 - v0, v0)
+    b = torch.where(three, v2 - v0, v1)
+    c = torch.linalg.cross(a, b)
+    z = torch.zeros_like(c)
+    z[:, 2] = 1.0
+    c = torch.where((cnt >= 2)[:, None], c, z)
+    return c / c.norm(dim=1, keepdim=True)
+
+
+def _inter(style, x, nrm, e, P, pairs):
+    """(vdW, repulsion) energies of directed interlayer pairs inside the cutoff."""
+    i, j, sh = pairs
+    d = x[i] - x[j] - sh
+    r2 = (d * d).sum(-1)
+    r = r2.sqrt()
+    t = r / CUT
+    tap = 1.0 + t ** 4 * (((20.0 * t - 70.0) * t + 84.0) * t - 35.0)
+    rho2 = r2 - (nrm[i] * d).sum(-1) ** 2
+    p = P[e[i], e[j]]
+    if style == "kc":
+        z0, C0, C2, C4, C, delta, lam, A, sc = (p[:, k] for k in range(9))
+        mev = 1e-3 * sc
+        y = rho2 / delta ** 2
+        rep = torch.exp(-lam * (r - z0)) * (0.5 * C * mev + torch.exp(-y) * (C0 + C2 * y + C4 * y * y) * mev)
+        vdw = -0.5 * A * mev * (z0 / r) ** 6
+    else:
+        z0, alpha, delta, eps, C, dd, sR, reff, C6, sc = (p[:, k] for k in range(10))
+        mev = 1e-3 * sc
+        rep = torch.exp(-alpha / z0 * (r - z0)) * (0.5 * eps * mev + C * mev * torch.exp(-rho2 / delta ** 2))
+        vdw = -0.5 * C6 * mev / r2 ** 3 / (1.0 + torch.exp(-dd * (r / (sR * reff) - 1.0)))
+    return (tap * vdw).sum(), (tap * rep).sum()
+
+
+def _exact_eval(c, x, typ, mol, L, per, dev="cuda"):
+    """Energies (Tersoff, vdW, repulsion), forces and virials (xx yy zz xy xz yz) per style."""
+    ters, inter = _tables(c["style"], dev)
+    e = torch.as_tensor(typ, device=dev).long() - 1
+    mol = torch.as_tensor(mol, device=dev)
+    x = torch.as_tensor(x, dtype=torch.float64, device=dev)
+    # short bonds first
+    sb = [torch.cat(t) for t in zip(*_neighbours(x, mol, L, per, 2.11, dev))]
+    rs = (x[sb[1]] + sb[2] - x[sb[0]]).norm(dim=1)
+    bt = rs < ters[e[sb[0]], e[sb[1]], e[sb[1]]][:, 10:12].sum(-1)
+    rcut = inter[..., -1][e[sb[0]], e[sb[1]]]
+    bn = (rs < rcut) & (mol[sb[0]] == mol[sb[1]])
+    tb, nb = [t[bt] for t in sb], [t[bn] for t in sb]
+
+    def strained(x0):
+        eps = torch.zeros(3, 3, dtype=torch.float64, device=dev, requires_grad=True)
+        return eps, (lambda v: v + v @ eps.T)
+
+    def voigt(g):   # W_ab = sum r_a f_b = -dE/d eps_ba
+        w = -g
+        return torch.stack([w[0, 0], w[1, 1], w[2, 2], w[1, 0], w[2, 0], w[2, 1]])
+    xt = x.clone().requires_grad_(True)
+    eps, st = strained(x)
+    et = _tersoff(st(xt), e, ters, (tb[0], tb[1], st(tb[2])))
+    gt, wt = torch.autograd.grad(et, (xt, eps))
+    xn = x.clone().requires_grad_(True)
+    epn, stn = strained(x)
+    nrm = _normals(stn(xn), (nb[0], nb[1], stn(nb[2])))
+    nl = nrm.detach().clone()
+    gx, gn, gw = torch.zeros_like(x), torch.zeros_like(x), torch.zeros(3, 3, dtype=torch.float64, device=dev)
+    ev = er = 0.0
+    for i, j, sh in _neighbours(x, mol, L, per, CUT, dev):
+        k = (mol[i] != mol[j])
+        if c["style"] == "kc":
+            k &= (e[i] == 0) & (e[j] == 0)
+        i, j, sh = i[k], j[k], sh[k]
+        for a in range(0, len(i), 4_000_000):
+            b = slice(a, a + 4_000_000)
+            xa, na = x.clone().requires_grad_(True), nl.clone().requires_grad_(True)
+            ep, sx = strained(x)
+            v, r = _inter(c["style"], sx(xa), na, e, inter, (i[b], j[b], sx(sh[b])))
+            g = torch.autograd.grad(v + r, (xa, na, ep))
+            gx += g[0]
+            gn += g[1]
+            gw += g[2]
+            ev, er = ev + float(v.detach()), er + float(r.detach())
+    g = torch.autograd.grad(nrm, (xn, epn), grad_outputs=gn)
+    gx, gw = gx + g[0], gw + g[1]
+    return {"pvector": np.array([ev, er]), "e": np.array([float(et.detach()), ev + er]),
+            "virial_tersoff": voigt(wt).cpu().numpy(), "virial_ilp": voigt(gw).cpu().numpy(),
+            "f": (-gt - gx).cpu().numpy()}
+
+
+def exact(case, seed):
+    """What run returns, in 64 bits.  None where it has no value of its own: how per-atom
+    energies and virials are split over atoms and which periodic image a position is given
+    in are conventions, a minimiser's path hangs on its stopping tests, and a rank's ghost
+    shares are partial sums."""
+    c = dict(case)
+    kind = c["kind"]
+    evals = 4 * c["nx"] * c["ny"] * c["layers"] * (c["steps"] if kind == "md" else c["count"])
+    if kind in ("minimize", "rank") or (kind != "batch" and evals > (1_500_000 if kind == "md" else 500_000)):
+        return None
+    ss = _systems(c, seed)
+    if kind == "batch":
+        if sum(s.n for s in ss) > 400_000:
+            return None
+        r = [_exact_eval(c, s.x, s.type, s.mol, s.box_hi - s.box_lo, s.periodic) for s in ss]
+        return {"f": np.concatenate([q["f"] for q in r]),
+                **{k: np.array([q[k] for q in r]) for k in ("pvector", "e", "virial_tersoff", "virial_ilp")}}
+    s = ss[0]
+    L = s.box_hi - s.box_lo
+    if kind == "md":
+        m = s.masses()[:, None]
+        acc, dt = 1.0 / (S.MVV2E_METAL * m), 0.001
+        x, v = s.x.copy(), s.v.copy()
+        r = _exact_eval(c, x, s.type, s.mol, L, s.periodic)
+        for _ in range(c["steps"]):
+            v = v + 0.5 * dt * acc * r["f"]
+            x = x + dt * v
+            r = _exact_eval(c, x, s.type, s.mol, L, s.periodic)
+            v = v + 0.5 * dt * acc * r["f"]
+        return {"x": None, "v": v, "f": r["f"], "pe": float(r["e"].sum()),
+                "ke": float(0.5 * S.MVV2E_METAL * (m * v * v).sum()), "virial": r["virial_tersoff"] + r["virial_ilp"]}
+    if kind == "eval" and not c["vatom"]:
+        return {"f": [_exact_eval(c, x, s.type, s.mol, L, s.periodic)["f"] for x in _frames(c, s)]}
+    r = _exact_eval(c, s.x, s.type, s.mol, L, s.periodic)
+    if kind == "eval":
+        return dict(r, eatom=None, vatom_tersoff=None, vatom_ilp=None)
+    return r
