@@ -138,11 +138,12 @@ def _frames(c, s):
 
 
 def _engine(c):
+    """The pair_coeff elements are those of the system's atom types: C alone for graphite."""
     prec = capi.MIXED if c["prec"] == "mixed" else capi.FP64
-    if c["style"] == "kc":
-        return capi.Engine(BNC, None, kc_file=KC_FILE, ilp_elements=("C", "NULL", "NULL"), cut_global=CUT,
-                           skin=c["skin"], precision=prec)
-    return capi.Engine(BNC, ILP_FILE, cut_global=CUT, skin=c["skin"], precision=prec)
+    elements = ("C", "B", "N") if c["system"] in ("hbn", "replicas") else ("C",)
+    kc = {"kc_file": KC_FILE, "ilp_elements": elements} if c["style"] == "kc" else {}
+    return capi.Engine(BNC, None if kc else ILP_FILE, elements=elements, cut_global=CUT, skin=c["skin"],
+                       precision=prec, **kc)
 
 
 def _rank_atoms(c, s):
