@@ -1,0 +1,211 @@
+// Double-float arithmetic: a value held as the unevaluated sum of two FP32 numbers, about
+// 48 significand bits, in FP32 instructions only.  GB300 issues FP64 at 1/75 of its FP32
+// rate (measured: 0.52 against 39 T lane operations per second), and a double-float
+// product costs 4 FP32 instructions and a sum 8, so the FP64 mode's heavy arithmetic runs
+// here several times faster than on the FP64 pipe.
+//
+// Everything is built from error-free transformations (T. J. Dekker, Numer. Math. 18, 1971;
+// D. E. Knuth, TAOCP vol. 2): two_sum and the FMA product error.  The types are templates
+// over V = float or V = float2; float2 holds two independent values and uses the packed
+// FP32x2 instructions, which take half the issue slots at the same arithmetic rate (the
+// negation of an operand is free in both).
+//
+// Results are left unnormalised (|l| of a few ulp of h): products and sums accept that, and
+// renorm is called where a chain would let it grow.
+#pragma once
+
+#include <cuda_runtime.h>
+
+namespace lmff {
+namespace df {
+
+#define LMFF_DF static __device__ __forceinline__
+LMFF_DF float vset(float a, float) { return a; }
+LMFF_DF float vneg(float a) { return -a; }
+LMFF_DF float vadd(float a, float b) { return __fadd_rn(a, b); }
+LMFF_DF float vsub(float a, float b) { return __fsub_rn(a, b); }
+LMFF_DF float vmul(float a, float b) { return __fmul_rn(a, b); }
+LMFF_DF float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+LMFF_DF float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
+LMFF_DF float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+LMFF_DF float2 vsub(float2 a, float2 b) { return __fadd2_rn(a, vneg(b)); }
+LMFF_DF float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+LMFF_DF float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+template <class V>
+LMFF_DF V vall(float a);   // the same value in every component
+template <>
+__device__ __forceinline__ float vall<float>(float a) { return a; }
+template <>
+__device__ __forceinline__ float2 vall<float2>(float a) { return make_float2(a, a); }
+// f applied to each component (MUFU estimates, table addresses)
+template <class F>
+LMFF_DF float vmap(F f, float a) { return f(a); }
+template <class F>
+LMFF_DF float2 vmap(F f, float2 a) { return make_float2(f(a.x), f(a.y)); }
+
+template <class V>
+struct D {
+  V h, l;
+};
+template <class V>
+LMFF_DF D<V> mk(V h, V l) {
+  D<V> r;
+  r.h = h;
+  r.l = l;
+  return r;
+}
+template <class V>
+LMFF_DF D<V> neg(D<V> a) { return mk(vneg(a.h), vneg(a.l)); }
+
+// s + e = a + b exactly
+template <class V>
+LMFF_DF D<V> two_sum(V a, V b) {
+  const V s = vadd(a, b), bb = vsub(s, a);
+  return mk(s, vadd(vsub(a, vsub(s, bb)), vsub(b, bb)));
+}
+// the same for |a| >= |b| or a = 0
+template <class V>
+LMFF_DF D<V> fast_two_sum(V a, V b) {
+  const V s = vadd(a, b);
+  return mk(s, vsub(b, vsub(s, a)));
+}
+template <class V>
+LMFF_DF D<V> renorm(D<V> a) { return fast_two_sum(a.h, a.l); }
+
+template <class V>
+LMFF_DF D<V> mul(D<V> a, D<V> b) {
+  const V p = vmul(a.h, b.h);
+  V e = vfma(a.h, b.h, vneg(p));
+  e = vfma(a.h, b.l, e);
+  return mk(p, vfma(a.l, b.h, e));
+}
+template <class V>
+LMFF_DF D<V> sqr(D<V> a) {
+  const V p = vmul(a.h, a.h);
+  const V e = vfma(a.h, a.h, vneg(p));
+  return mk(p, vfma(vadd(a.h, a.h), a.l, e));
+}
+template <class V>
+LMFF_DF D<V> add(D<V> a, D<V> b) {
+  const D<V> s = two_sum(a.h, b.h);
+  return mk(s.h, vadd(s.l, vadd(a.l, b.l)));
+}
+// |a| >= |b|
+template <class V>
+LMFF_DF D<V> add_ordered(D<V> a, D<V> b) {
+  const D<V> s = fast_two_sum(a.h, b.h);
+  return mk(s.h, vadd(s.l, vadd(a.l, b.l)));
+}
+// a + b, b in single precision
+template <class V>
+LMFF_DF D<V> add1(D<V> a, V b) {
+  const D<V> s = two_sum(a.h, b);
+  return mk(s.h, vadd(s.l, a.l));
+}
+// running sum: acc += a
+template <class V>
+LMFF_DF void acc(D<V> &s, D<V> a) { s = add(s, a); }
+// running sum of products: s += a b, s -= a b
+template <class V>
+LMFF_DF void acc_mul(D<V> &s, D<V> a, D<V> b) { acc(s, mul(a, b)); }
+
+// a . b of three-vectors
+template <class V>
+LMFF_DF D<V> dot3(const D<V> *a, const D<V> *b) {
+  const D<V> x = mul(a[0], b[0]), y = mul(a[1], b[1]), z = mul(a[2], b[2]);
+  const D<V> s = two_sum(x.h, y.h), t = two_sum(s.h, z.h);
+  const V lo = vadd(vadd(vadd(x.l, y.l), z.l), vadd(s.l, t.l));
+  return fast_two_sum(t.h, lo);
+}
+
+LMFF_DF float rsqrt_est(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+LMFF_DF float rcp_est(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// r = sqrt(q) and ri = 1 / sqrt(q), q > 0: the FP32 estimate y (relative error 2^-22.9) is
+// brought to FP32 rounding by one Newton step, so that the final Newton corrections, whose
+// error is the square of y's, stay below 2^-47
+template <class V>
+LMFF_DF void sqrt_rsqrt(D<V> q, D<V> &r, D<V> &ri) {
+  V y = vmap([](float x) { return rsqrt_est(x); }, q.h);
+  const V half = vall<V>(0.5f), one = vall<V>(1.f);
+  y = vfma(vmul(half, y), vfma(vneg(vmul(q.h, y)), y, one), y);
+  const V r0 = vmul(q.h, y), hy = vmul(half, y);
+  const V res = vadd(vfma(vneg(r0), r0, q.h), q.l);
+  r = fast_two_sum(r0, vmul(res, hy));
+  const V t = vfma(vneg(r.l), y, vfma(vneg(r.h), y, one));
+  ri = mk(y, vmul(y, vfma(t, t, t)));
+}
+
+// 1 / a
+template <class V>
+LMFF_DF D<V> rcp(D<V> a) {
+  const V y = vmap([](float x) { return rcp_est(x); }, a.h);
+  const V t = vfma(vneg(a.l), y, vfma(vneg(a.h), y, vall<V>(1.f)));
+  return mk(y, vmul(y, vfma(t, t, t)));   // 1/(1 - t) = 1 + t + t^2, |t| < 2^-22
+}
+
+// 2^a by Tang's table-driven method (P. T. P. Tang, ACM TOMS 15, 1989): a = k/64 + f,
+// |f| <= 1/128, 2^a = 2^(k>>6) T[k & 63] e^g with g = f ln 2 as a double-float and
+// e^g - 1 = g + g^2/2 + g^3 (1/6 + g/24 + g^2/120), the last bracket in FP32 (truncation
+// below 2^-54).  tab holds T as double-floats (EXP2_TAB entries, filled by exp2_entry).
+// a.h is clamped to [-125, 127]: results below 2^-125 come out as about 2^-125.
+constexpr int EXP2_TAB = 64;
+LMFF_DF float2 exp2_entry(int j) {
+  const double t = exp2((double)j / EXP2_TAB);
+  const float h = (float)t;
+  return make_float2(h, (float)(t - (double)h));
+}
+LMFF_DF float clamp_exp(float x) { return fminf(fmaxf(x, -125.f), 127.f); }
+LMFF_DF void exp2_parts(float t, const float2 *tab, float &th, float &tl, float &sc) {
+  const int k = __float_as_int(t) - 0x4b400000;   // t = 1.5 2^23 + k
+  const float2 T = tab[k & (EXP2_TAB - 1)];
+  th = T.x;
+  tl = T.y;
+  sc = __int_as_float(((k >> 6) + 127) << 23);
+}
+LMFF_DF void exp2_parts(float2 t, const float2 *tab, float2 &th, float2 &tl, float2 &sc) {
+  exp2_parts(t.x, tab, th.x, tl.x, sc.x);
+  exp2_parts(t.y, tab, th.y, tl.y, sc.y);
+}
+template <class V>
+LMFF_DF D<V> exp2(D<V> a, const float2 *tab) {
+  const V magic = vall<V>(12582912.f);   // 1.5 2^23
+  const V ah = vmap([](float x) { return clamp_exp(x); }, a.h);
+  const V t = vfma(ah, vall<V>((float)EXP2_TAB), magic);
+  const V k = vsub(t, magic);
+  // ah - k/64 is exact and a multiple of ulp(ah), so zero or larger than a.l
+  const D<V> f = fast_two_sum(vfma(vneg(k), vall<V>(1.f / EXP2_TAB), ah), a.l);
+  const V L = vall<V>(0.693147182464599609375f), Ll = vall<V>(-1.90465429995776804525e-9f);   // ln 2
+  const V p = vmul(f.h, L);
+  V e = vfma(f.h, L, vneg(p));
+  e = vfma(f.h, Ll, e);
+  e = vfma(f.l, L, e);
+  const V c = vfma(vfma(p, vall<V>(1.f / 60.f), vall<V>(1.f / 12.f)), p, vall<V>(1.f / 3.f));
+  const V hp = vmul(vall<V>(0.5f), p);
+  const V q = vmul(hp, p);
+  V qe = vfma(hp, p, vneg(q));
+  qe = vfma(p, e, qe);
+  qe = vfma(vmul(q, p), c, qe);
+  const D<V> s = fast_two_sum(p, q);
+  const V sl = vadd(s.l, vadd(e, qe));
+  V th, tl, sc;
+  exp2_parts(t, tab, th, tl, sc);
+  const V m = vmul(th, s.h);
+  V me = vfma(th, s.h, vneg(m));
+  me = vfma(th, sl, me);
+  me = vfma(tl, s.h, me);
+  const D<V> r = fast_two_sum(th, m);
+  return mk(vmul(r.h, sc), vmul(vadd(r.l, vadd(me, tl)), sc));
+}
+#undef LMFF_DF
+
+}  // namespace df
+}  // namespace lmff

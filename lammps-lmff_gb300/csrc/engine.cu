@@ -505,6 +505,24 @@ static void sys_geometry(SysDesc &sd, const double lo[3], const double L[3], con
   double e = 4.0 * std::ldexp(2.0 * sd.base, -23);
   double r = cutneigh_max + 2.0 * e;
   sd.prefilt_sq = (float)(r * r * (1.0 + 1e-5));
+  // three-part positions: the coarse grid leaves 24 bits for four times the largest
+  // coordinate in or near the box (differences of h are then exact in FP32), the fine grid
+  // is 2^-21 of it (differences of m, up to several image shifts included, stay within 24
+  // bits); beyond dfmax, four times what the coarse grid holds, m would need more
+  double big = 0.0;
+  for (int k = 0; k < 3; k++)
+    big = std::max(big, std::max(std::fabs(sd.lo[k]), std::fabs(sd.lo[k] + sd.L[k])) + sd.L[k] + 64.0);
+  const int ex = (int)std::ceil(std::log2(4.0 * big));
+  const double g1 = std::ldexp(1.0, ex - 24), g2 = std::ldexp(g1, -21);
+  sd.dfmax = (float)std::ldexp(1.0, ex + 1);
+  sd.dfM1 = std::ldexp(1.5, 52) * g1;
+  sd.dfM2 = std::ldexp(1.5, 52) * g2;
+  for (int k = 0; k < 3; k++) {
+    const double h = std::rint(sd.L[k] / g1) * g1, m = std::rint((sd.L[k] - h) / g2) * g2;
+    sd.dfL[0][k] = (float)h;
+    sd.dfL[1][k] = (float)m;
+    sd.dfL[2][k] = (float)(sd.L[k] - h - m);
+  }
 }
 
 struct Engine {
@@ -930,9 +948,34 @@ struct Engine {
     }
   }
 
+  // whether the FP64 mode's pair kernel runs in double-float arithmetic (the number of ILP
+  // elements, else 0): ilp/graphene/hbn with every element pair's constants equal to the
+  // swapped pair's (one constant set serves both repulsion terms and the vdW pair), and of
+  // a size that keeps every factor of a pair beyond 0.5 A inside the FP32 exponent range
+  // (e^80 < 2^116; 2^48 of the lo part's digits fit below the smallest factor that counts)
+  int pair_df_elements() const {
+    if (!i_on || pot64.kc || !pot64.vdw_sym) return 0;
+    auto in = [](double v, double lo, double hi) { return v == 0.0 || (std::fabs(v) >= lo && std::fabs(v) <= hi); };
+    if (!(cut_global >= 1.0 && cut_global <= 1e3)) return 0;
+    for (int a = 0; a < pot64.i_ne; a++)
+      for (int b = 0; b < pot64.i_ne; b++) {
+        const IlpP<double> &q = pot64.ilp[a * MAXELEM + b];
+        if (!q.same_as_swapped) return 0;
+        if (!(std::fabs(q.lambda * q.z0) <= 40.0 && std::fabs(q.d) <= 40.0 && std::fabs(q.d_over_seff) <= 1e3 &&
+              std::fabs(q.lambda) <= 1e3 && std::fabs(q.delta2inv) <= 1e3))
+          return 0;
+        if (!(in(q.C, 1e-12, 1e6) && in(q.eps_half, 1e-12, 1e6) && in(q.C6, 1e-6, 1e8) && q.lambda >= 0.0 &&
+              q.d_over_seff >= 0.0 && q.delta2inv >= 0.0))
+          return 0;
+      }
+    return pot64.i_ne;
+  }
+  int pair_df = 0;
+
   int build_consts() {
     fill_pot(pot64);
     fill_pot(pot32);
+    pair_df = pair_df_elements();
     memset(&nbc, 0, sizeof nbc);
     cutneigh_max = 0.0;
     double rmaxilp = 0.0;
@@ -1504,6 +1547,7 @@ struct Engine {
     a.pair_tile = pair_tile;
     a.no_small = !small_variants;
     a.kc = i_on && hi.model == LMFF_INTERLAYER_KC;
+    a.pair_df = pair_df;
     // not while kernels are timed one by one (events between the launches)
     if (!ktiming && n <= PDL_MAX_ATOMS) a.pdl = pdl_short ? pdl_mask : (pdl_mask & ~PDL_SHORT);
     return a;
@@ -3049,7 +3093,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
   Carve cv{(unsigned char *)basev, (unsigned char *)basev + NOALLOC_BYTES};
   d4 *xq = cv.take<d4>(c), *xq2 = cv.take<d4>(c), *nrm64 = cv.take<d4>(c), *ilp_g = cv.take<d4>(c);
   float4 *xh = cv.take<float4>(c), *xl = cv.take<float4>(c), *nrm32 = cv.take<float4>(c);
-  float4 *jrec = cv.take<float4>(3 * (size_t)c), *jrec2 = cv.take<float4>(2 * (size_t)c);
+  float4 *jrec = cv.take<float4>(5 * (size_t)c), *jrec2 = jrec + 3 * (size_t)c;
   double *v = cv.take<double>(3 * c), *v2 = cv.take<double>(3 * c), *mass = cv.take<double>(c),
          *mass2 = cv.take<double>(c);
   int64_t *tag = cv.take<int64_t>(c), *tag2 = cv.take<int64_t>(c);
@@ -3161,6 +3205,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     a.do_ilp = g.i_on && (which & LMFF_ILP);
     a.list_full = g.list_full;
     a.kc = g.i_on && g.hi.model == LMFF_INTERLAYER_KC;
+    a.pair_df = g.pair_df;
   };
   const bool ev = true;
   if (g.precision == LMFF_FP64) {

@@ -104,6 +104,12 @@ struct SysDesc {
   double binv[3];             // 1 / bin size
   double base;                // double-float offset (x - lo + 32 + base in [base, 2 base))
   float Lhi[3], Llo[3];       // L split into two floats
+  // three-part FP32 positions (FP64 mode's pair kernel): x = h + m + l with h a multiple of
+  // the coarse grid and m of the fine one; adding and subtracting dfM1 / dfM2 in FP64
+  // rounds to the grids.  dfL: L in the same three parts
+  double dfM1, dfM2;
+  float dfL[3][3];
+  float dfmax;                // atoms with a coordinate beyond it take the FP64 pair form
   float prefilt_sq;           // list build: a candidate whose hi-part distance squared
                               // exceeds this is beyond every cutoff (rounding margin in)
 };

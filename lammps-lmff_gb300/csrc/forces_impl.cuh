@@ -8,6 +8,7 @@
 #include <type_traits>
 
 #include "forces.cuh"
+#include "ilp_df.cuh"
 
 namespace lmff {
 namespace LMFF_NS {
@@ -63,6 +64,33 @@ __device__ __forceinline__ bool lt_exact(R rsq, R thr, const d4 *xq, const SysDe
     return rsq_rn(dx, dy, dz) < thr64;
   }
 }
+
+#ifndef LMFF_PACKED_X2
+// Record of the double-float pair kernel, four float4 per atom (ForceArgs::jrec): the
+// position as h + m + l, h on the system's coarse grid and m on its fine one (SysDesc::
+// dfM1, dfM2), so that differences of h and of m are exact in FP32 and l carries the rest
+// of the FP64 value; the unit normal as hi and lo; the ILP element.  Layout: (h, m_x),
+// (m_y, m_z, nh_x, nh_y), (nh_z, nl), (l, element).
+__device__ __forceinline__ void df_split(double x, double M1, double M2, float &h, float &m, float &l) {
+  h = (float)__dsub_rn(__dadd_rn(x, M1), M1);
+  const double r = __dsub_rn(x, (double)h);
+  m = (float)__dsub_rn(__dadd_rn(r, M2), M2);
+  l = (float)__dsub_rn(r, (double)m);
+}
+__device__ __forceinline__ void df_record(const ForceArgs<double> &a, const SysDesc &sd, int i, double x, double y,
+                                          double z, double nx, double ny, double nz, int ie) {
+  float hx, hy, hz, mx, my, mz, lx, ly, lz;
+  df_split(x, sd.dfM1, sd.dfM2, hx, mx, lx);
+  df_split(y, sd.dfM1, sd.dfM2, hy, my, ly);
+  df_split(z, sd.dfM1, sd.dfM2, hz, mz, lz);
+  const float nhx = (float)nx, nhy = (float)ny, nhz = (float)nz;
+  float4 *q = a.jrec + 4 * (size_t)i;
+  q[0] = make_float4(hx, hy, hz, mx);
+  q[1] = make_float4(my, mz, nhx, nhy);
+  q[2] = make_float4(nhz, (float)(nx - (double)nhx), (float)(ny - (double)nhy), (float)(nz - (double)nhz));
+  q[3] = make_float4(lx, ly, lz, __int_as_float(ie));
+}
+#endif
 
 // ============================================================== k_short ==========
 // Per atom: the current-step ILP intralayer list (ILP_neigh, pair_ilp_graphene_hbn.cpp:
@@ -202,6 +230,7 @@ __global__ void k_short(ForceArgs<R> a, const double *cutILPsq64, double tcutmax
       nx, ny, nz, __uint_as_float((h2_bits(__floats2half2_rn(ai.lz, 0.f)) & 0xffffu) | ((unsigned)(ie & 0xffff) << 16)));
 #else
   a.nrm64[i] = make_d4(nx, ny, nz, 0.0);
+  if (a.pair_df) df_record(a, sd, i, ai.x, ai.y, ai.z, nx, ny, nz, ie);
 #endif
 }
 
@@ -1981,6 +2010,335 @@ __global__ void __launch_bounds__(256, (ilp_min_blocks<TPA, EV, EATOM, ONE, GH, 
   }
 }
 
+#ifndef LMFF_PACKED_X2
+// ============================================================ k_ilp_df ===========
+// The FP64 mode's interlayer pair kernel in double-float arithmetic: the sums of k_ilp
+// (force on i, dE/dn_i, energies, virial) from pair terms that carry ~48 bits, formed in
+// FP32 instructions.  The FP64 form of a pair is ~120 FP64 instructions, and the FP64
+// pipe (1/75 of the FP32 rate) bound k_ilp<double> completely; here a pair is ~700 FP32
+// instructions, packed two list entries per lane in FP32x2, with no FP64 instruction in
+// the loop (331,200-atom slab, energies and virial: 79.3 -> 9.3 ms; 7,200-atom bilayer,
+// forces: 786 -> 98 us; FMA pipe 64 % busy).  Displacements come from three-part positions whose leading parts subtract
+// exactly.
+// The error of a pair's force against 64-bit arithmetic is below the FP64 form's, whose
+// 1/sqrt and 1/x are one FP64 Newton step from an FP32 estimate (CPU emulation against
+// 113-bit arithmetic, rms over 200,000 pairs of BNCH.ILP's element pairs: 3-9e-14 of the
+// rms pair force here, 1-9e-13 there).
+// The virial: half of del (x) f_ij at each end of a pair, which sums to the whole of the
+// pair's; the n_i part of f_ij is applied to the sums after the loop (f -= tpi n_i,
+// W -= g (x) n_i).
+// Pairs closer than 0.5 A, whose powers of 1/r leave the FP32 range, are left to ilp_pair
+// (FP64) in a second walk over the lane's entries; so is every pair of an atom so far
+// outside its box that the position grids do not hold it (SysDesc::dfmax).
+// Blocks of up to 128 threads, 4 per SM (128 registers, no spills); with energies and
+// virial 3 (168 registers).  A launch_bounds of 3 / 5 blocks for the force-only form
+// measured 5 % faster / 9 % slower on 5,016 atoms and 1 % faster / 13 % slower on 7,200.
+constexpr int DF_THREADS = 128;
+constexpr float DF_CLOSE = 0.25f;   // A^2
+constexpr int DF_ROWS = MAXELEM * MAXELEM * MAXELEM;
+__constant__ float2 c_dfk[df::K_N];          // element 0's constants, each duplicated
+__constant__ df::PairG c_dfg;
+__device__ float2 g_dfk[DF_ROWS * df::K_N];  // (ie, jeA, jeB) rows: (X[ie][jeA], X[ie][jeB]), ne^3 of them
+__device__ float2 g_exp2_df[df::EXP2_TAB];
+
+__global__ void k_fill_exp2_df() {
+  const int j = threadIdx.x;
+  if (j < df::EXP2_TAB) g_exp2_df[j] = df::exp2_entry(j);
+}
+
+// an atom's record
+struct DfAtom {
+  float h[3], m[3], l[3];
+  float nh[3], nl[3];
+  int el;
+  __device__ __forceinline__ void load(const float4 *jrec, int i) {
+    const float4 *q = jrec + 4 * (size_t)i;
+    const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
+    h[0] = q0.x; h[1] = q0.y; h[2] = q0.z;
+    m[0] = q0.w; m[1] = q1.x; m[2] = q1.y;
+    nh[0] = q1.z; nh[1] = q1.w; nh[2] = q2.x;
+    nl[0] = q2.y; nl[1] = q2.z; nl[2] = q2.w;
+    l[0] = q3.x; l[1] = q3.y; l[2] = q3.z;
+    el = __float_as_int(q3.w);
+  }
+};
+// x_i - (x_j + s L): the h and m differences are exact and |h difference| is zero or at
+// least the m difference's, up to values whose sum is exact anyway
+template <bool IMG>
+__device__ __forceinline__ void df_disp(const DfAtom &I, const DfAtom &A, const SysDesc &sd, int sx, int sy, int sz, int c,
+                                        float &dh, float &dm, float &dl) {
+  dh = __fsub_rn(I.h[c], A.h[c]);
+  dm = __fsub_rn(I.m[c], A.m[c]);
+  dl = __fsub_rn(I.l[c], A.l[c]);
+  if constexpr (IMG) {
+    const float s = (float)(c == 0 ? sx : c == 1 ? sy : sz);
+    dh = __fmaf_rn(-s, sd.dfL[0][c], dh);
+    dm = __fmaf_rn(-s, sd.dfL[1][c], dm);
+    dl = __fmaf_rn(-s, sd.dfL[2][c], dl);
+  }
+}
+
+// the pairs closer than DF_CLOSE (with all, every pair) of one lane's entries, in FP64
+template <bool EV, bool ONE, bool GH>
+__device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int lane, int tpa, int ie, bool iown,
+                                            bool all, IlpAcc &acc) {
+  const SysDesc &sd = a.A.sys[a.A.sysid[i]];
+  AtomI<R> ai;
+  ai.load(a.A, i);
+  const d4 ni = a.nrm64[i];
+  const long long itag = a.tag[i];
+  DfAtom I;
+  I.load(a.jrec, i);
+  const int64_t b = a.list_off[i];
+  const int cnt = (int)(a.list_off[i + 1] - b);
+  for (int k = lane; k < cnt; k += tpa) {
+    const uint32_t e = a.list[b + k];
+    int j, sx, sy, sz;
+    decode_entry(e, a.lc, j, sx, sy, sz);
+    DfAtom A;
+    A.load(a.jrec, j);
+    df::D<float> d[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      float dh, dm, dl;
+      df_disp<true>(I, A, sd, sx, sy, sz, c, dh, dm, dl);
+      d[c] = df::fast_two_sum(dh, dm);
+      d[c].l = __fadd_rn(d[c].l, dl);
+    }
+    if (!all && !(df::dot3(d, d).h < DF_CLOSE)) continue;
+    ilp_pair<EV, ONE, false, true, GH>(a, ai, sd, e, ai.fetch(a.A, j), NrmJ<R>::load(a, j), ni.x, ni.y, ni.z, ie,
+                                       info_mol(ai.info), itag, false, iown, acc);
+  }
+}
+
+template <bool EV, bool ONE, bool GH>
+__global__ void __launch_bounds__(DF_THREADS, EV ? 3 : 4) k_ilp_df(ForceArgs<R> a, int tpa, int eatom, int ne) {
+  pdl_enter(a.pdl);
+  using namespace df;
+  typedef float2 V;
+  __shared__ float2 s_tab[EXP2_TAB];
+  __shared__ float2 s_dfk[ONE ? 1 : DF_ROWS * K_N];
+  for (int w = threadIdx.x; w < EXP2_TAB; w += blockDim.x) s_tab[w] = g_exp2_df[w];
+  if constexpr (!ONE) {
+    for (int w = threadIdx.x; w < ne * ne * ne * K_N; w += blockDim.x) s_dfk[w] = g_dfk[w];
+    const int words = (int)(sizeof(c_pot.ilp) / sizeof(int));
+    const int *src = reinterpret_cast<const int *>(c_pot.ilp);
+    int *dst = reinterpret_cast<int *>(s_ilp);
+    for (int w = threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
+  }
+  __syncthreads();
+  const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = gtid / tpa;
+  const int lane = threadIdx.x & (tpa - 1);
+  const bool valid = i < a.n;
+  const int ii = valid ? i : a.n - 1;
+  const SysDesc &sd = a.A.sys[a.A.sysid[ii]];
+  DfAtom I;
+  I.load(a.jrec, ii);
+  const int ie = I.el;
+  const long long itag = GH ? a.tag[ii] : 0;
+  const bool iown = !GH || owned(a, ii);
+  D<V> f[3], g[3], tpi, ev, er, w[6];
+  const V zero = vall<V>(0.f);
+#pragma unroll
+  for (int c = 0; c < 3; c++) f[c] = g[c] = mk(zero, zero);
+  tpi = ev = er = mk(zero, zero);
+#pragma unroll
+  for (int c = 0; c < 6; c++) w[c] = mk(zero, zero);
+  const bool out = fabsf(I.h[0]) > sd.dfmax || fabsf(I.h[1]) > sd.dfmax || fabsf(I.h[2]) > sd.dfmax;
+  bool close = valid && ie >= 0 && out;
+  if (valid && ie >= 0 && !out) {
+    const int64_t b = a.list_off[i];
+    const uint32_t *lst = a.list + b;
+    const int cnt = (int)(a.list_off[i + 1] - b);
+    auto run = [&](auto img_t) {
+      constexpr bool IMG = decltype(img_t)::value;
+      for (int k = lane; k < cnt; k += 2 * tpa) {
+        const uint32_t ea = __ldg(&lst[k]);
+        const bool bval = k + tpa < cnt;
+        const uint32_t eb = bval ? __ldg(&lst[k + tpa]) : ea;
+        int ja, jb, ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
+        if constexpr (IMG) {
+          decode_entry(ea, a.lc, ja, ax, ay, az);
+          decode_entry(eb, a.lc, jb, bx, by, bz);
+        } else {
+          ja = (int)(ea & a.lc.imask);
+          jb = (int)(eb & a.lc.imask);
+        }
+        DfAtom A, B;
+        A.load(a.jrec, ja);
+        B.load(a.jrec, jb);
+        D<V> d[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          V dh, dm, dl;
+          df_disp<IMG>(I, A, sd, ax, ay, az, c, dh.x, dm.x, dl.x);
+          df_disp<IMG>(I, B, sd, bx, by, bz, c, dh.y, dm.y, dl.y);
+          d[c] = fast_two_sum(dh, dm);
+          d[c].l = vadd(d[c].l, dl);
+        }
+        D<V> q = dot3(d, d);
+        const bool inA = __fadd_rn(__fsub_rn(q.h.x, c_dfg.cut_h), __fsub_rn(q.l.x, c_dfg.cut_l)) < 0.f;
+        const bool inB = bval && __fadd_rn(__fsub_rn(q.h.y, c_dfg.cut_h), __fsub_rn(q.l.y, c_dfg.cut_l)) < 0.f;
+        if (!(inA || inB)) continue;
+        V on = make_float2(inA ? 1.f : 0.f, inB ? 1.f : 0.f);
+        if (q.h.x < DF_CLOSE || q.h.y < DF_CLOSE) {   // rare
+          close = true;
+          if (q.h.x < DF_CLOSE) { q.h.x = 4.f; on.x = 0.f; }
+          if (q.h.y < DF_CLOSE) { q.h.y = 4.f; on.y = 0.f; }
+        }
+        D<V> nj[3], ni[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          nj[c] = mk(make_float2(A.nh[c], B.nh[c]), make_float2(A.nl[c], B.nl[c]));
+          ni[c] = mk(vall<V>(I.nh[c]), vall<V>(I.nl[c]));
+        }
+        V wv = on, wi = on, wj = on;
+        if constexpr (GH) {
+          auto wt = [&](int j, float dx, float dy, float dz, float &v, float &wi_, float &wj_) {
+            const bool jown = owned(a, j);
+            const bool keep = keep_half_r(itag, (long long)a.tag[j], -dx, -dy, -dz);
+            v = (keep ? iown : jown) ? 1.f : 0.f;
+            wi_ = iown ? 1.f : 0.f;
+            wj_ = jown ? 1.f : 0.f;
+          };
+          wt(ja, d[0].h.x + d[0].l.x, d[1].h.x + d[1].l.x, d[2].h.x + d[2].l.x, wv.x, wi.x, wj.x);
+          wt(jb, d[0].h.y + d[0].l.y, d[1].h.y + d[1].l.y, d[2].h.y + d[2].l.y, wv.y, wi.y, wj.y);
+        }
+        PairOut<V> o;
+        if constexpr (ONE) {
+          pair_terms<EV, GH>(c_dfg, [&](int k2) { return c_dfk[k2]; }, s_tab, q, dot3(ni, d), dot3(nj, d), on, wv, wi,
+                             wj, o);
+        } else {
+          const float2 *row = s_dfk + ((ie * ne + A.el) * ne + B.el) * K_N;
+          pair_terms<EV, GH>(c_dfg, [&](int k2) { return row[k2]; }, s_tab, q, dot3(ni, d), dot3(nj, d), on, wv, wi, wj,
+                             o);
+        }
+        const D<V> ntq = neg(o.tq);
+        acc(tpi, o.tp);
+#pragma unroll
+        for (int c = 0; c < 3; c++) acc_mul(g[c], o.tp, d[c]);
+        D<V> t[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          t[c] = add(mul(o.crad, d[c]), mul(ntq, nj[c]));
+          acc(f[c], t[c]);
+        }
+        if constexpr (EV) {
+          acc(ev, o.evdw);
+          acc(er, o.erep);
+          acc_mul(w[0], d[0], t[0]); acc_mul(w[1], d[1], t[1]); acc_mul(w[2], d[2], t[2]);
+          acc_mul(w[3], d[0], t[1]); acc_mul(w[4], d[0], t[2]); acc_mul(w[5], d[1], t[2]);
+        }
+      }
+    };
+    if (a.list_img[i]) run(std::true_type{});
+    else run(std::false_type{});
+  }
+  // ---- the lane's two halves, then the atom's lanes, in double-float; FP64 from there
+  auto total = [&](const D<V> &v) {
+    D<float> s = add(mk(v.h.x, v.l.x), mk(v.h.y, v.l.y));
+    s = renorm(s);
+    for (int o = tpa / 2; o > 0; o >>= 1) {
+      const D<float> p = mk(__shfl_xor_sync(0xffffffffu, s.h, o), __shfl_xor_sync(0xffffffffu, s.l, o));
+      s = renorm(add(s, p));
+    }
+    return (double)s.h + (double)s.l;
+  };
+  IlpAcc x;
+  double sf[3], sg[3], sw[6], se = 0, sr = 0;
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    sf[c] = total(f[c]);
+    sg[c] = total(g[c]);
+  }
+  const double st = total(tpi);
+  if constexpr (EV) {
+    se = total(ev);
+    sr = total(er);
+#pragma unroll
+    for (int c = 0; c < 6; c++) sw[c] = total(w[c]);
+  }
+  const bool any = __any_sync(0xffffffffu, close);
+  if (any) {
+    if (close) df_close_pairs<EV, ONE, GH>(a, i, lane, tpa, ie, iown, out, x);
+    double *v[14] = {&x.fx, &x.fy, &x.fz, &x.gxa, &x.gya, &x.gza, &x.evdw, &x.erep, &x.w0, &x.w1, &x.w2, &x.w3, &x.w4,
+                     &x.w5};
+#pragma unroll
+    for (int c = 0; c < (EV ? 14 : 6); c++)
+      for (int o = tpa / 2; o > 0; o >>= 1) *v[c] += __shfl_xor_sync(0xffffffffu, *v[c], o);
+  }
+  if (!valid || lane != 0) return;
+  const double n[3] = {(double)I.nh[0] + (double)I.nl[0], (double)I.nh[1] + (double)I.nl[1],
+                       (double)I.nh[2] + (double)I.nl[2]};
+  a.ilp_f[i] = fma(-st, n[0], sf[0]) + x.fx;
+  a.ilp_f[a.n + i] = fma(-st, n[1], sf[1]) + x.fy;
+  a.ilp_f[2 * a.n + i] = fma(-st, n[2], sf[2]) + x.fz;
+  a.ilp_g[i] = make_d4(sg[0] + x.gxa, sg[1] + x.gya, sg[2] + x.gza, 0.0);
+  if constexpr (EV) {
+    double *q = a.stat_ilp;
+    const double evdw = 0.5 * se + x.evdw, erep = 0.5 * sr + x.erep;
+    q[i] = evdw;
+    q[(size_t)a.n + i] = erep;
+    q[(size_t)2 * a.n + i] = 0.5 * fma(-sg[0], n[0], sw[0]) + x.w0;
+    q[(size_t)3 * a.n + i] = 0.5 * fma(-sg[1], n[1], sw[1]) + x.w1;
+    q[(size_t)4 * a.n + i] = 0.5 * fma(-sg[2], n[2], sw[2]) + x.w2;
+    q[(size_t)5 * a.n + i] = 0.5 * fma(-sg[0], n[1], sw[3]) + x.w3;
+    q[(size_t)6 * a.n + i] = 0.5 * fma(-sg[0], n[2], sw[4]) + x.w4;
+    q[(size_t)7 * a.n + i] = 0.5 * fma(-sg[1], n[2], sw[5]) + x.w5;
+    if (eatom) a.eatom_ilp[i] = evdw + erep;
+  }
+}
+
+// constants of the double-float kernel from the FP64 ones
+static void upload_pair_df(const PotConst<R> &p, cudaStream_t s) {
+  static float2 one[df::K_N], rows[DF_ROWS * df::K_N];   // static: the asynchronous copies read them after return
+  static df::PairG g;
+  auto split = [](double v, float &h, float &l) {
+    h = (float)v;
+    l = (float)(v - (double)h);
+  };
+  const double cut = 1.0 / p.i_inv_rcut;
+  split(p.i_inv_rcut, g.irc_h, g.irc_l);
+  split(-140.0 / cut, g.dt_h, g.dt_l);
+  split(p.i_cutsq, g.cut_h, g.cut_l);
+  g.tap = p.tap;
+  auto consts = [&](const IlpP<R> &q, float *h, float *l) {
+    const double v[df::K_N / 2] = {q.nd2_l2e, q.C, 2.0 * q.eps_half, 2.0 * q.C * q.delta2inv, q.lambda, q.lam_l2e, q.z0,
+                                   q.ts_a, q.seff, q.C6, q.d_over_seff};
+    for (int k = 0; k < df::K_N / 2; k++) split(v[k], h[k], l[k]);
+  };
+  const int ne = p.i_ne;
+  float h[MAXELEM * MAXELEM][df::K_N / 2], l[MAXELEM * MAXELEM][df::K_N / 2];
+  for (int a = 0; a < ne; a++)
+    for (int b = 0; b < ne; b++) consts(p.ilp[a * MAXELEM + b], h[a * ne + b], l[a * ne + b]);
+  for (int k = 0; k < df::K_N / 2; k++) {
+    one[2 * k] = make_float2(h[0][k], h[0][k]);
+    one[2 * k + 1] = make_float2(l[0][k], l[0][k]);
+    for (int a = 0; a < ne; a++)
+      for (int b = 0; b < ne; b++)
+        for (int c = 0; c < ne; c++) {
+          float2 *r = rows + ((a * ne + b) * ne + c) * df::K_N + 2 * k;
+          r[0] = make_float2(h[a * ne + b][k], h[a * ne + c][k]);
+          r[1] = make_float2(l[a * ne + b][k], l[a * ne + c][k]);
+        }
+  }
+  cudaMemcpyToSymbolAsync(c_dfk, one, sizeof one, 0, cudaMemcpyHostToDevice, s);
+  cudaMemcpyToSymbolAsync(c_dfg, &g, sizeof g, 0, cudaMemcpyHostToDevice, s);
+  cudaMemcpyToSymbolAsync(g_dfk, rows, sizeof rows, 0, cudaMemcpyHostToDevice, s);
+  k_fill_exp2_df<<<1, df::EXP2_TAB, 0, s>>>();
+}
+
+template <bool ONE, bool GH>
+static void launch_ilp_df(const ForceArgs<R> &a, bool ev, bool eatom, int tpa, int block, cudaStream_t s) {
+  block = block < DF_THREADS ? block : DF_THREADS;
+  const int g = (int)(((long long)a.n * tpa + block - 1) / block);
+  const bool p = (a.pdl & PDL_ILP) != 0;
+  if (ev) launch_pdl(p, k_ilp_df<true, ONE, GH>, g, block, s, a, tpa, (int)eatom, a.pair_df);
+  else launch_pdl(p, k_ilp_df<false, ONE, GH>, g, block, s, a, tpa, (int)eatom, a.pair_df);
+}
+#endif  // !LMFF_PACKED_X2
+
 // ============================================================== k_nderiv =========
 // Normal-derivative assembly in FP64, one thread per atom i (calc_normal's dnormdri and
 // dnormal, pair_ilp_graphene_hbn.cpp:893-926 / :1043-1067, applied to the reverse-
@@ -2800,7 +3158,10 @@ __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
 
 void upload_pot(const PotConst<R> &p, cudaStream_t s) {
   cudaMemcpyToSymbolAsync(c_pot, &p, sizeof(p), 0, cudaMemcpyHostToDevice, s);
-  if (sizeof(R) == 8) k_fill_exp2_f64<<<1, EXP2_F64_N, 0, s>>>();
+#ifndef LMFF_PACKED_X2
+  k_fill_exp2_f64<<<1, EXP2_F64_N, 0, s>>>();
+  if (p.i_enabled && !p.kc) upload_pair_df(p, s);
+#endif
 #ifdef LMFF_PACKED_X2
   {
     static PairX2Const x2;   // static: the asynchronous copy reads it after return
@@ -2954,6 +3315,19 @@ static void launch_ilp_ghost(const ForceArgs<R> &a, bool ev, bool eatom, int blo
 
 void launch_ilp(const ForceArgs<R> &a, bool ev, bool eatom, int tpa, int block, bool one_element, cudaStream_t s) {
   if (a.n == 0) return;
+#ifndef LMFF_PACKED_X2
+  if (a.pair_df && !a.list_full) {
+    if (a.own_perm) {
+      if (one_element) launch_ilp_df<true, true>(a, ev, eatom, tpa, block, s);
+      else launch_ilp_df<false, true>(a, ev, eatom, tpa, block, s);
+    } else if (one_element) {
+      launch_ilp_df<true, false>(a, ev, eatom, tpa, block, s);
+    } else {
+      launch_ilp_df<false, false>(a, ev, eatom, tpa, block, s);
+    }
+    return;
+  }
+#endif
   if (a.own_perm) {
     if (one_element) launch_ilp_ghost<true>(a, ev, eatom, block, s);
     else launch_ilp_ghost<false>(a, ev, eatom, block, s);
