@@ -45,7 +45,7 @@ namespace lmff {
 LMFF_FORCE_API(f64, double)
 LMFF_FORCE_API(f32, float)
 namespace f64 {
-void launch_vatom_terms(const ForceArgs<double> &a, bool ilp, cudaStream_t s);
+void launch_vatom_terms(const ForceArgs<double> &a, bool ilp, bool one_element, cudaStream_t s);
 void launch_vatom_gather(const ForceArgs<double> &a, double *out, cudaStream_t s);
 }
 namespace f32 {
@@ -602,7 +602,7 @@ struct Engine {
   // per-atom virial pass (lmff_compute_vatom): own shares, slots, the sorted result, the
   // result in the caller's order and the mixed pass's frame tensors (7 float4), VA_DOUBLES
   // per atom of capacity va_cap
-  static constexpr int VA_DOUBLES = 6 * (2 + MAXTERS + MAXILP + 2) + 14;
+  static constexpr int VA_DOUBLES = 6 * (2 + MAXTERS + MAXILP + 2) + 28;
   double *d_va = nullptr;
   int va_cap = 0;
   // device calls on this engine (counted by DeviceCall) and the one whose evaluation
@@ -2068,7 +2068,7 @@ struct Engine {
     // the interlayer shares in the precision of the evaluation: FP64, or the mixed
     // engines' FP32 pair form with FP64 sums
     const bool mixed_ilp = precision == LMFF_MIXED && a.do_ilp;
-    f64::launch_vatom_terms(a, !mixed_ilp, stream);
+    f64::launch_vatom_terms(a, !mixed_ilp, i_one, stream);
     if (mixed_ilp) {
       ForceArgs<float> b = args<float>();
       b.do_ters = a.do_ters;

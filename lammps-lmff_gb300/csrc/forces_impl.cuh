@@ -2078,6 +2078,18 @@ __device__ __forceinline__ void df_disp(const DfAtom &I, const DfAtom &A, const 
   }
 }
 
+template <bool IMG>
+__device__ __forceinline__ void df_del(const DfAtom &I, const DfAtom &A, const SysDesc &sd, int sx, int sy, int sz,
+                                       df::D<float> d[3]) {
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    float dh, dm, dl;
+    df_disp<IMG>(I, A, sd, sx, sy, sz, c, dh, dm, dl);
+    d[c] = df::fast_two_sum(dh, dm);
+    d[c].l = __fadd_rn(d[c].l, dl);
+  }
+}
+
 // the pairs closer than DF_CLOSE (with all, every pair) of one lane's entries, in FP64
 template <bool EV, bool ONE, bool GH>
 __device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int lane, int tpa, int ie, bool iown,
@@ -2098,13 +2110,7 @@ __device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int la
     DfAtom A;
     A.load(a.jrec, j);
     df::D<float> d[3];
-#pragma unroll
-    for (int c = 0; c < 3; c++) {
-      float dh, dm, dl;
-      df_disp<true>(I, A, sd, sx, sy, sz, c, dh, dm, dl);
-      d[c] = df::fast_two_sum(dh, dm);
-      d[c].l = __fadd_rn(d[c].l, dl);
-    }
+    df_del<true>(I, A, sd, sx, sy, sz, d);
     if (!all && !(df::dot3(d, d).h < DF_CLOSE)) continue;
     ilp_pair<EV, ONE, false, true, GH>(a, ai, sd, e, ai.fetch(a.A, j), NrmJ<R>::load(a, j), ni.x, ni.y, ni.z, ie,
                                        info_mol(ai.info), itag, false, iown, acc);
@@ -2864,6 +2870,83 @@ __device__ __forceinline__ void va_add_xyz(double v[6], double s, double dx, dou
   v[3] += s * (dx * f[1]); v[4] += s * (dx * f[2]); v[5] += s * (dy * f[2]);
 }
 
+// one entry e of atom i's list: its shares into w, and the sums g, G of the term i owns
+template <bool GH, bool KC>
+__device__ __forceinline__ void va_pair64(const ForceArgs<R> &a, int i, uint32_t e, int ie, long long mi, long long itag,
+                                          bool iown, double nix, double niy, double niz, double w[6], double &gx,
+                                          double &gy, double &gz, double G[6]) {
+  const SysDesc &sd = a.A.sys[a.A.sysid[i]];
+  const double cutsq = c_pot.i_cutsq;
+  int j, sx, sy, sz;
+  decode_entry(e, a.lc, j, sx, sy, sz);
+  const long long jinfo = __double_as_longlong(a.A.xq[j].w);
+  if (info_mol(jinfo) == mi) return;
+  const int je = c_pot.i_map[info_type(jinfo)];
+  if (je < 0) return;
+  double dx, dy, dz;
+  disp64(a.A.xq, sd, i, j, sx, sy, sz, dx, dy, dz);
+  const double rsq = rsq_rn(dx, dy, dz);
+  if (!(rsq < cutsq)) return;
+  const double r = sqrt(rsq);
+  double Tap = 1.0, dTap = 0.0;
+  if (c_pot.tap) {
+    // Tap = 20x^7 - 70x^6 + 84x^5 - 35x^4 + 1, dTap/dr = 140 x^3 (x - 1)^3 / Rcut
+    const double xr = r * c_pot.i_inv_rcut, x2 = xr * xr;
+    Tap = (((20.0 * xr - 70.0) * xr + 84.0) * xr - 35.0) * (x2 * x2) + 1.0;
+    const double y = x2 - xr;
+    dTap = (y * y) * (y * (140.0 * c_pot.i_inv_rcut));
+  }
+  const bool jown = !GH || owned(a, j);
+  const long long jtag = a.tag[j];
+  const bool keep = GH ? keep_half_r(itag, jtag, -dx, -dy, -dz) : keep_half(itag, jtag, sx, sy, sz);
+  // ---- vdW (calc_FvdW :506-540), the kept end's parameters
+  if (!GH || (keep ? iown : jown)) {
+    const IlpP<double> &pv = c_pot.ilp[(keep || c_pot.vdw_sym) ? ie * MAXELEM + je : je * MAXELEM + ie];
+    const double r2inv = 1.0 / rsq, r6inv = r2inv * r2inv * r2inv, r8inv = r6inv * r2inv;
+    double Vv, fpv;
+    if constexpr (KC) {
+      Vv = -pv.kc_Az06 * r6inv;
+      fpv = -6.0 * pv.kc_Az06 * r8inv;
+    } else {
+      const double TS = 1.0 + exp(-pv.d * (r / pv.seff - 1.0));
+      const double TS2inv = 1.0 / (TS * TS);
+      Vv = -pv.C6 * r6inv / TS;
+      fpv = -6.0 * pv.C6 * r8inv / TS + pv.C6 * pv.d / pv.seff * (TS - 1.0) * TS2inv * r8inv * r;
+    }
+    const double fs = fpv * Tap - Vv * dTap / r;
+    const double f3[3] = {fs * dx, fs * dy, fs * dz};
+    va_add_xyz(w, 0.5, dx, dy, dz, f3);
+  }
+  // ---- the term with i's normal
+  if (iown) {
+    double fkc[3], c;
+    va_rep<KC>(c_pot.ilp[ie * MAXELEM + je], nix, niy, niz, dx, dy, dz, rsq, r, Tap, dTap, fkc, c);
+    va_add_xyz(w, 0.5, dx, dy, dz, fkc);
+    gx += c * dx; gy += c * dy; gz += c * dz;
+    G[0] += c * (dx * dx); G[1] += c * (dy * dy); G[2] += c * (dz * dz);
+    G[3] += c * (dx * dy); G[4] += c * (dx * dz); G[5] += c * (dy * dz);
+  }
+  // ---- the term with j's normal, i its partner: del' = x_j - x_i
+  if (jown) {
+    NFrame frj;
+    double njx, njy, njz;
+    va_frame(a, j, frj, njx, njy, njz);
+    const double ex = -dx, ey = -dy, ez = -dz;
+    double fkc[3], c;
+    va_rep<KC>(c_pot.ilp[je * MAXELEM + ie], njx, njy, njz, ex, ey, ez, rsq, r, Tap, dTap, fkc, c);
+    va_add_xyz(w, 0.5, ex, ey, ez, fkc);
+    if (frj.ok) {
+      NDeriv o;
+      nderiv_apply<true>(frj, make_d4(c * ex, c * ey, c * ez, 0.0), o);
+      const double sc[3] = {o.c[0][0] + o.c[1][0] + o.c[2][0], o.c[0][1] + o.c[1][1] + o.c[2][1],
+                            o.c[0][2] + o.c[1][2] + o.c[2][2]};
+#pragma unroll
+      for (int k = 0; k < 6; k++) w[k] += 0.5 * o.W[k];
+      va_add_xyz(w, 0.5, ex, ey, ez, sc);
+    }
+  }
+}
+
 template <bool GH, bool KC>
 __global__ void __launch_bounds__(128) k_va_ilp(ForceArgs<R> a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2878,85 +2961,231 @@ __global__ void __launch_bounds__(128) k_va_ilp(ForceArgs<R> a) {
   double nix, niy, niz;
   va_frame(a, i, fri, nix, niy, niz);
   if (ie >= 0) {
-    const SysDesc &sd = a.A.sys[a.A.sysid[i]];
     const long long mi = info_mol(iinfo);
     const long long itag = a.tag[i];
-    const double cutsq = c_pot.i_cutsq;
     const int64_t q1 = a.list_off[i + 1];
-    for (int64_t q = a.list_off[i]; q < q1; q++) {
-      int j, sx, sy, sz;
-      decode_entry(a.list[q], a.lc, j, sx, sy, sz);
-      const long long jinfo = __double_as_longlong(a.A.xq[j].w);
-      if (info_mol(jinfo) == mi) continue;
-      const int je = c_pot.i_map[info_type(jinfo)];
-      if (je < 0) continue;
-      double dx, dy, dz;
-      disp64(a.A.xq, sd, i, j, sx, sy, sz, dx, dy, dz);
-      const double rsq = rsq_rn(dx, dy, dz);
-      if (!(rsq < cutsq)) continue;
-      const double r = sqrt(rsq);
-      double Tap = 1.0, dTap = 0.0;
-      if (c_pot.tap) {
-        // Tap = 20x^7 - 70x^6 + 84x^5 - 35x^4 + 1, dTap/dr = 140 x^3 (x - 1)^3 / Rcut
-        const double xr = r * c_pot.i_inv_rcut, x2 = xr * xr;
-        Tap = (((20.0 * xr - 70.0) * xr + 84.0) * xr - 35.0) * (x2 * x2) + 1.0;
-        const double y = x2 - xr;
-        dTap = (y * y) * (y * (140.0 * c_pot.i_inv_rcut));
-      }
-      const bool jown = !GH || owned(a, j);
-      const long long jtag = a.tag[j];
-      const bool keep = GH ? keep_half_r(itag, jtag, -dx, -dy, -dz) : keep_half(itag, jtag, sx, sy, sz);
-      // ---- vdW (calc_FvdW :506-540), the kept end's parameters
-      if (!GH || (keep ? iown : jown)) {
-        const IlpP<double> &pv = c_pot.ilp[(keep || c_pot.vdw_sym) ? ie * MAXELEM + je : je * MAXELEM + ie];
-        const double r2inv = 1.0 / rsq, r6inv = r2inv * r2inv * r2inv, r8inv = r6inv * r2inv;
-        double Vv, fpv;
-        if constexpr (KC) {
-          Vv = -pv.kc_Az06 * r6inv;
-          fpv = -6.0 * pv.kc_Az06 * r8inv;
-        } else {
-          const double TS = 1.0 + exp(-pv.d * (r / pv.seff - 1.0));
-          const double TS2inv = 1.0 / (TS * TS);
-          Vv = -pv.C6 * r6inv / TS;
-          fpv = -6.0 * pv.C6 * r8inv / TS + pv.C6 * pv.d / pv.seff * (TS - 1.0) * TS2inv * r8inv * r;
-        }
-        const double fs = fpv * Tap - Vv * dTap / r;
-        const double f3[3] = {fs * dx, fs * dy, fs * dz};
-        va_add_xyz(w, 0.5, dx, dy, dz, f3);
-      }
-      // ---- the term with i's normal
-      if (iown) {
-        double fkc[3], c;
-        va_rep<KC>(c_pot.ilp[ie * MAXELEM + je], nix, niy, niz, dx, dy, dz, rsq, r, Tap, dTap, fkc, c);
-        va_add_xyz(w, 0.5, dx, dy, dz, fkc);
-        gx += c * dx; gy += c * dy; gz += c * dz;
-        G[0] += c * (dx * dx); G[1] += c * (dy * dy); G[2] += c * (dz * dz);
-        G[3] += c * (dx * dy); G[4] += c * (dx * dz); G[5] += c * (dy * dz);
-      }
-      // ---- the term with j's normal, i its partner: del' = x_j - x_i
-      if (jown) {
-        NFrame frj;
-        double njx, njy, njz;
-        va_frame(a, j, frj, njx, njy, njz);
-        const double ex = -dx, ey = -dy, ez = -dz;
-        double fkc[3], c;
-        va_rep<KC>(c_pot.ilp[je * MAXELEM + ie], njx, njy, njz, ex, ey, ez, rsq, r, Tap, dTap, fkc, c);
-        va_add_xyz(w, 0.5, ex, ey, ez, fkc);
-        if (frj.ok) {
-          NDeriv o;
-          nderiv_apply<true>(frj, make_d4(c * ex, c * ey, c * ez, 0.0), o);
-          const double sc[3] = {o.c[0][0] + o.c[1][0] + o.c[2][0], o.c[0][1] + o.c[1][1] + o.c[2][1],
-                                o.c[0][2] + o.c[1][2] + o.c[2][2]};
-#pragma unroll
-          for (int k = 0; k < 6; k++) w[k] += 0.5 * o.W[k];
-          va_add_xyz(w, 0.5, ex, ey, ez, sc);
-        }
-      }
-    }
+    for (int64_t q = a.list_off[i]; q < q1; q++)
+      va_pair64<GH, KC>(a, i, a.list[q], ie, mi, itag, iown, nix, niy, niz, w, gx, gy, gz, G);
   }
 #pragma unroll
   for (int k = 0; k < 6; k++) a.va_i[6 * (size_t)i + k] = w[k];
   va_write_slots(a, i, ie >= 0 && iown, fri, gx, gy, gz, G);
+}
+
+// ---- the same shares in double-float arithmetic (k_ilp_df's pair terms), where that
+// kernel takes the potential.  As in the mixed pass, the own share is half of del (x) f_ij
+// and the partner's normal-derivative share comes from the 27 numbers of the partner's
+// frame, here as double-floats.  VA_LANES lanes per atom share its list; the atom's g_i and
+// G_i go to its slot storage, from which k_va_slots forms the slots with full warps.
+// k_va_ilp's ~500 FP64 instructions per pair at 1/75 of the FP32 rate become ~1,100 FP32
+// ones (36,800-atom slab: 30 -> 1.5 ms for the pass's pair kernel).
+constexpr int VA_LANES = 8;
+
+// per atom: A (18, row-major k, a) then B (9, row-major a, b) of k_va_ilp_df as (hi, lo)
+// pairs, 14 float4
+__global__ void __launch_bounds__(128) k_va_tens_df(ForceArgs<R> a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  NFrame fr;
+  double nx, ny, nz;
+  va_frame(a, i, fr, nx, ny, nz);
+  double t[28];
+#pragma unroll
+  for (int k = 0; k < 28; k++) t[k] = 0.0;
+  if (fr.ok) {
+#pragma unroll
+    for (int e = 0; e < 3; e++) {
+      NDeriv o;
+      nderiv_apply<true>(fr, make_d4(e == 0 ? 1.0 : 0.0, e == 1 ? 1.0 : 0.0, e == 2 ? 1.0 : 0.0, 0.0), o);
+#pragma unroll
+      for (int k = 0; k < 6; k++) t[3 * k + e] = o.W[k];
+#pragma unroll
+      for (int b = 0; b < 3; b++) t[18 + 3 * e + b] = o.c[0][b] + o.c[1][b] + o.c[2][b];
+    }
+  }
+  float4 *q = a.va_tens + 14 * (size_t)i;
+#pragma unroll
+  for (int k = 0; k < 14; k++) {
+    const float h0 = (float)t[2 * k], h1 = (float)t[2 * k + 1];
+    q[k] = make_float4(h0, (float)(t[2 * k] - (double)h0), h1, (float)(t[2 * k + 1] - (double)h1));
+  }
+}
+
+// the pairs closer than DF_CLOSE (with all, every pair) of one lane's entries, in FP64:
+// v = w[6], g[3], G[6]
+template <bool GH>
+__device__ __noinline__ void va_close_pairs(const ForceArgs<R> &a, int i, int lane, int ie, bool iown, bool all,
+                                            double *v) {
+  const SysDesc &sd = a.A.sys[a.A.sysid[i]];
+  const long long mi = info_mol(__double_as_longlong(a.A.xq[i].w));
+  const long long itag = a.tag[i];
+  const d4 ni = a.nrm64[i];
+  DfAtom I;
+  I.load(a.jrec, i);
+  const int64_t q1 = a.list_off[i + 1];
+  for (int64_t q = a.list_off[i] + lane; q < q1; q += VA_LANES) {
+    const uint32_t e = a.list[q];
+    int j, sx, sy, sz;
+    decode_entry(e, a.lc, j, sx, sy, sz);
+    DfAtom A;
+    A.load(a.jrec, j);
+    df::D<float> d[3];
+    df_del<true>(I, A, sd, sx, sy, sz, d);
+    if (!all && !(df::dot3(d, d).h < DF_CLOSE)) continue;
+    va_pair64<GH, false>(a, i, e, ie, mi, itag, iown, ni.x, ni.y, ni.z, v, v[6], v[7], v[8], v + 9);
+  }
+}
+
+template <bool ONE, bool GH>
+__global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
+  using namespace df;
+  typedef float V;
+  __shared__ float2 s_tab[EXP2_TAB];
+  for (int w = threadIdx.x; w < EXP2_TAB; w += blockDim.x) s_tab[w] = g_exp2_df[w];
+  __syncthreads();
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / VA_LANES;
+  const int lane = threadIdx.x & (VA_LANES - 1);
+  if (i >= a.n) return;   // whole groups
+  const unsigned gmask = ((1u << VA_LANES) - 1) << ((threadIdx.x & 31) & ~(VA_LANES - 1));
+  const SysDesc &sd = a.A.sys[a.A.sysid[i]];
+  DfAtom I;
+  I.load(a.jrec, i);
+  const int ie = I.el;
+  const long long itag = GH ? a.tag[i] : 0;
+  const bool iown = !GH || owned(a, i);
+  D<V> s[15];   // w[6], g[3], G[6]
+#pragma unroll
+  for (int c = 0; c < 15; c++) s[c] = mk(0.f, 0.f);
+  const bool out = fabsf(I.h[0]) > sd.dfmax || fabsf(I.h[1]) > sd.dfmax || fabsf(I.h[2]) > sd.dfmax;
+  bool close = ie >= 0 && out;
+  if (ie >= 0 && !out) {
+    D<V> ni[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) ni[c] = mk(I.nh[c], I.nl[c]);
+    const int64_t q1 = a.list_off[i + 1];
+    for (int64_t k = a.list_off[i] + lane; k < q1; k += VA_LANES) {
+      const uint32_t e = __ldg(&a.list[k]);
+      int j, sx, sy, sz;
+      decode_entry(e, a.lc, j, sx, sy, sz);
+      DfAtom A;
+      A.load(a.jrec, j);
+      D<V> d[3], nj[3];
+      df_del<true>(I, A, sd, sx, sy, sz, d);
+      const D<V> q = dot3(d, d);
+      if (!(__fadd_rn(__fsub_rn(q.h, c_dfg.cut_h), __fsub_rn(q.l, c_dfg.cut_l)) < 0.f)) continue;
+      if (q.h < DF_CLOSE) {
+        close = true;
+        continue;
+      }
+#pragma unroll
+      for (int c = 0; c < 3; c++) nj[c] = mk(A.nh[c], A.nl[c]);
+      float wv = 1.f, wi = 1.f, wj = 1.f;
+      if constexpr (GH) {
+        const bool jown = owned(a, j);
+        const bool keep = keep_half_r(itag, (long long)a.tag[j], -(d[0].h + d[0].l), -(d[1].h + d[1].l), -(d[2].h + d[2].l));
+        wv = (keep ? iown : jown) ? 1.f : 0.f;
+        wi = iown ? 1.f : 0.f;
+        wj = jown ? 1.f : 0.f;
+      }
+      PairOut<V> o;
+      if constexpr (ONE) {
+        pair_terms<false, GH>(c_dfg, [&](int k2) { return c_dfk[k2].x; }, s_tab, q, dot3(ni, d), dot3(nj, d), 1.f, wv,
+                              wi, wj, o);
+      } else {
+        const float2 *row = g_dfk + ((ie * ne + A.el) * ne + A.el) * K_N;
+        pair_terms<false, GH>(c_dfg, [&](int k2) { return __ldg(&row[k2]).x; }, s_tab, q, dot3(ni, d), dot3(nj, d), 1.f,
+                              wv, wi, wj, o);
+      }
+      const D<V> ntq = neg(o.tq);
+      D<V> t[3], h[3];
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        t[c] = add(mul(o.crad, d[c]), mul(ntq, nj[c]));
+        h[c] = mul(o.tp, d[c]);
+        acc(s[6 + c], h[c]);
+      }
+      constexpr int P[6] = {0, 1, 2, 0, 0, 1}, Q[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+      for (int c = 0; c < 6; c++) {
+        acc_mul(s[c], d[P[c]], t[Q[c]]);
+        acc_mul(s[9 + c], h[P[c]], d[Q[c]]);
+      }
+      if (o.tq.h != 0.f) {
+        // the partner's normal-derivative share, g = tq del
+        D<V> g[3], b[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) g[c] = mul(o.tq, d[c]);
+        const float4 *tt = a.va_tens + 14 * (size_t)j;
+        float4 T[14];
+#pragma unroll
+        for (int c = 0; c < 14; c++) T[c] = __ldg(tt + c);
+        auto num = [&](int c) { return (c & 1) ? mk(T[c / 2].z, T[c / 2].w) : mk(T[c / 2].x, T[c / 2].y); };
+        bool any = false;   // B = 0 for atoms with three intralayer neighbours
+#pragma unroll
+        for (int c = 18; c < 27; c++) any = any || num(c).h != 0.f;
+        if (any) {
+#pragma unroll
+          for (int c = 0; c < 3; c++) {   // - sum_e B[e][c] g_e
+            b[c] = mul(num(18 + c), g[0]);
+            acc_mul(b[c], num(21 + c), g[1]);
+            acc_mul(b[c], num(24 + c), g[2]);
+            b[c] = neg(renorm(b[c]));
+          }
+#pragma unroll
+          for (int c = 0; c < 6; c++) acc_mul(s[c], d[P[c]], b[Q[c]]);
+        }
+#pragma unroll
+        for (int c = 0; c < 6; c++) {
+          acc_mul(s[c], num(3 * c), g[0]);
+          acc_mul(s[c], num(3 * c + 1), g[1]);
+          acc_mul(s[c], num(3 * c + 2), g[2]);
+        }
+      }
+    }
+  }
+  double v[15];
+#pragma unroll
+  for (int c = 0; c < 15; c++) {
+    D<V> x = renorm(s[c]);
+    for (int o = VA_LANES / 2; o > 0; o >>= 1)
+      x = renorm(add(x, mk(__shfl_xor_sync(gmask, x.h, o), __shfl_xor_sync(gmask, x.l, o))));
+    v[c] = (double)x.h + (double)x.l;
+  }
+  const double n[3] = {(double)I.nh[0] + (double)I.nl[0], (double)I.nh[1] + (double)I.nl[1],
+                       (double)I.nh[2] + (double)I.nl[2]};
+  // the n_i part of the pair forces, and the halves
+  v[0] = 0.5 * fma(-v[6], n[0], v[0]); v[1] = 0.5 * fma(-v[7], n[1], v[1]); v[2] = 0.5 * fma(-v[8], n[2], v[2]);
+  v[3] = 0.5 * fma(-v[6], n[1], v[3]); v[4] = 0.5 * fma(-v[6], n[2], v[4]); v[5] = 0.5 * fma(-v[7], n[2], v[5]);
+  if (__any_sync(gmask, close)) {
+    double x[15];
+#pragma unroll
+    for (int c = 0; c < 15; c++) x[c] = 0.0;
+    if (close) va_close_pairs<GH>(a, i, lane, ie, iown, out, x);
+#pragma unroll
+    for (int c = 0; c < 15; c++) {
+      for (int o = VA_LANES / 2; o > 0; o >>= 1) x[c] += __shfl_xor_sync(gmask, x[c], o);
+      v[c] += x[c];
+    }
+  }
+  if (lane != 0) return;
+#pragma unroll
+  for (int c = 0; c < 6; c++) a.va_i[6 * (size_t)i + c] = v[c];
+  double *q = a.va_is + 6 * MAXILP * (size_t)i;
+#pragma unroll
+  for (int c = 0; c < 9; c++) q[c] = v[6 + c];
+}
+
+// the intralayer slots of the atoms from the sums g_i, G_i left in their slot storage
+__global__ void __launch_bounds__(128) k_va_slots(ForceArgs<R> a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  NFrame fr;
+  double nx, ny, nz, v[9];
+  va_frame(a, i, fr, nx, ny, nz);
+  const double *q = a.va_is + 6 * MAXILP * (size_t)i;
+#pragma unroll
+  for (int c = 0; c < 9; c++) v[c] = q[c];
+  va_write_slots(a, i, true, fr, v[0], v[1], v[2], v + 3);
 }
 
 // Per atom: its own shares plus the slots its Tersoff bond partners and the atoms whose
@@ -3021,7 +3250,11 @@ __global__ void __launch_bounds__(128) k_va_gather(ForceArgs<R> a, double *out) 
 //    g = c_ji del_ji = Tap q fpair1(j) del, is linear in g: with the 27 numbers of
 //    k_va_tens per atom (A[k][a] = W_j(e_a)[k], B[a][b] = sum_m c_m(e_a)[b]) it is
 //    sum_a A[k][a] g_a - del_p(k) sum_a B[a][b(k)] g_a;
-//  * g_i, G_i and the shares are summed in FP64, and the slots come from the FP64 frame.
+//  * g_i, G_i and the shares are sums of FP32 terms held as double-floats (error below
+//    2^-47 of the largest partial sum; as FP64 sums, 21 FP64 additions per pair at 1/75 of
+//    the FP32 rate, they were most of the pass), and the slots come from the FP64 frame.
+// VA_LANES lanes per atom share its list; the lanes' sums meet in double-float.
+constexpr int VA_LANES = 8;
 
 // per atom: A (18, row-major k, a) then B (9, row-major a, b), from three applications
 // of the FP64 frame to the unit vectors, stored as FP32 in 7 float4
@@ -3051,11 +3284,13 @@ __global__ void __launch_bounds__(128) k_va_tens(ForceArgs<R> a) {
 
 template <bool GH, bool KC>
 __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  double w[6] = {0, 0, 0, 0, 0, 0};
-  double gx = 0, gy = 0, gz = 0;
-  double G[6] = {0, 0, 0, 0, 0, 0};   // xx yy zz xy xz yz
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / VA_LANES;
+  const int lane = threadIdx.x & (VA_LANES - 1);
+  if (i >= a.n) return;   // whole groups
+  const unsigned gmask = ((1u << VA_LANES) - 1) << ((threadIdx.x & 31) & ~(VA_LANES - 1));
+  df::D<float> s[15];   // w[6] (without the halves), g[3], G[6] (xx yy zz xy xz yz)
+#pragma unroll
+  for (int k = 0; k < 15; k++) s[k] = df::mk(0.f, 0.f);
   AtomI<R> ai;
   ai.load(a.A, i);
   const int ie = c_pot.i_map[info_type(ai.info)];
@@ -3066,7 +3301,7 @@ __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
     const long long itag = a.tag[i];
     const float4 ni = a.nrm32[i];
     const int64_t q1 = a.list_off[i + 1];
-    for (int64_t q = a.list_off[i]; q < q1; q++) {
+    for (int64_t q = a.list_off[i] + lane; q < q1; q += VA_LANES) {
       int j, sx, sy, sz;
       decode_entry(a.list[q], a.lc, j, sx, sy, sz);
       R dx, dy, dz;
@@ -3120,11 +3355,11 @@ __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
       const R fx = crad * dx - tp1 * ni.x - tq1 * nj.x;
       const R fy = crad * dy - tp1 * ni.y - tq1 * nj.y;
       const R fz = crad * dz - tp1 * ni.z - tq1 * nj.z;
-      w[0] += 0.5 * (double)(dx * fx); w[1] += 0.5 * (double)(dy * fy); w[2] += 0.5 * (double)(dz * fz);
-      w[3] += 0.5 * (double)(dx * fy); w[4] += 0.5 * (double)(dx * fz); w[5] += 0.5 * (double)(dy * fz);
-      gx += (double)(tp1 * dx); gy += (double)(tp1 * dy); gz += (double)(tp1 * dz);
-      G[0] += (double)(tp1 * (dx * dx)); G[1] += (double)(tp1 * (dy * dy)); G[2] += (double)(tp1 * (dz * dz));
-      G[3] += (double)(tp1 * (dx * dy)); G[4] += (double)(tp1 * (dx * dz)); G[5] += (double)(tp1 * (dy * dz));
+      const R t15[15] = {dx * fx, dy * fy, dz * fz, dx * fy, dx * fz, dy * fz, tp1 * dx, tp1 * dy, tp1 * dz,
+                         tp1 * (dx * dx), tp1 * (dy * dy), tp1 * (dz * dz), tp1 * (dx * dy), tp1 * (dx * dz),
+                         tp1 * (dy * dz)};
+#pragma unroll
+      for (int k = 0; k < 15; k++) s[k] = df::add1(s[k], t15[k]);
       if (tq1 != R(0)) {
         // the partner's normal-derivative share, g = tq1 del
         const R g0 = tq1 * dx, g1 = tq1 * dy, g2 = tq1 * dz;
@@ -3140,17 +3375,40 @@ __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
         const R s0 = t4.z * g0 + t5.y * g1 + t6.x * g2;   // sum_e B[e][0] g_e
         const R s1 = t4.w * g0 + t5.z * g1 + t6.y * g2;   // b = 1
         const R s2 = t5.x * g0 + t5.w * g1 + t6.z * g2;   // b = 2
-        w[0] += 0.5 * (double)(A0 - dx * s0); w[1] += 0.5 * (double)(A1 - dy * s1);
-        w[2] += 0.5 * (double)(A2 - dz * s2); w[3] += 0.5 * (double)(A3 - dx * s1);
-        w[4] += 0.5 * (double)(A4 - dx * s2); w[5] += 0.5 * (double)(A5 - dy * s2);
+        const R b6[6] = {A0 - dx * s0, A1 - dy * s1, A2 - dz * s2, A3 - dx * s1, A4 - dx * s2, A5 - dy * s2};
+#pragma unroll
+        for (int k = 0; k < 6; k++) s[k] = df::add1(s[k], b6[k]);
       }
     }
   }
+  double v[15];
 #pragma unroll
-  for (int k = 0; k < 6; k++) a.va_i[6 * (size_t)i + k] = w[k];
-  NFrame fri;
-  nframe_eval(a, i, fri);
-  va_write_slots(a, i, ie >= 0 && iown, fri, gx, gy, gz, G);
+  for (int k = 0; k < 15; k++) {
+    df::D<float> x = df::renorm(s[k]);
+    for (int o = VA_LANES / 2; o > 0; o >>= 1)
+      x = df::renorm(df::add(x, df::mk(__shfl_xor_sync(gmask, x.h, o), __shfl_xor_sync(gmask, x.l, o))));
+    v[k] = (double)x.h + (double)x.l;
+  }
+  if (lane != 0) return;
+#pragma unroll
+  for (int k = 0; k < 6; k++) a.va_i[6 * (size_t)i + k] = 0.5 * v[k];
+  double *q = a.va_is + 6 * MAXILP * (size_t)i;
+#pragma unroll
+  for (int k = 0; k < 9; k++) q[k] = v[6 + k];
+}
+
+// the intralayer slots of the atoms from the sums g_i, G_i left in their slot storage
+// (zero where i owns no term)
+__global__ void __launch_bounds__(128) k_va_slots(ForceArgs<R> a) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  NFrame fr;
+  nframe_eval(a, i, fr);
+  double v[9];
+  const double *q = a.va_is + 6 * MAXILP * (size_t)i;
+#pragma unroll
+  for (int c = 0; c < 9; c++) v[c] = q[c];
+  va_write_slots(a, i, true, fr, v[0], v[1], v[2], v + 3);
 }
 #endif  // LMFF_PACKED_X2
 
@@ -3381,7 +3639,7 @@ void launch_finish(const ForceArgs<R> &a, bool eatom, const KickArgs *kick, cuda
 // the gather into out[6 n] (sorted order).  a.do_ters / a.do_ilp select the styles.
 // ilp = false leaves the interlayer shares to the mixed pass (launch_vatom_ilp of the
 // FP32 unit), which runs between this and launch_vatom_gather.
-void launch_vatom_terms(const ForceArgs<R> &a, bool ilp, cudaStream_t s) {
+void launch_vatom_terms(const ForceArgs<R> &a, bool ilp, bool one_element, cudaStream_t s) {
   if (a.n == 0) return;
   const int g = (a.n + 127) / 128;
   const bool gh = a.own_perm != nullptr;
@@ -3391,7 +3649,15 @@ void launch_vatom_terms(const ForceArgs<R> &a, bool ilp, cudaStream_t s) {
   }
   if (a.do_ilp && ilp) {
     k_nframe<<<g, 128, 0, s>>>(a);
-    if (gh && a.kc) k_va_ilp<true, true><<<g, 128, 0, s>>>(a);
+    if (a.pair_df && !a.list_full) {
+      const int gl = (int)(((long long)a.n * VA_LANES + 127) / 128);
+      k_va_tens_df<<<g, 128, 0, s>>>(a);
+      if (gh && one_element) k_va_ilp_df<true, true><<<gl, 128, 0, s>>>(a, a.pair_df);
+      else if (gh) k_va_ilp_df<false, true><<<gl, 128, 0, s>>>(a, a.pair_df);
+      else if (one_element) k_va_ilp_df<true, false><<<gl, 128, 0, s>>>(a, a.pair_df);
+      else k_va_ilp_df<false, false><<<gl, 128, 0, s>>>(a, a.pair_df);
+      k_va_slots<<<g, 128, 0, s>>>(a);
+    } else if (gh && a.kc) k_va_ilp<true, true><<<g, 128, 0, s>>>(a);
     else if (gh) k_va_ilp<true, false><<<g, 128, 0, s>>>(a);
     else if (a.kc) k_va_ilp<false, true><<<g, 128, 0, s>>>(a);
     else k_va_ilp<false, false><<<g, 128, 0, s>>>(a);
@@ -3409,11 +3675,13 @@ void launch_vatom_ilp(const ForceArgs<R> &a, cudaStream_t s) {
   if (a.n == 0 || !a.do_ilp) return;
   const int g = (a.n + 127) / 128;
   const bool gh = a.own_perm != nullptr;
+  const int gl = (int)(((long long)a.n * VA_LANES + 127) / 128);
   k_va_tens<<<g, 128, 0, s>>>(a);
-  if (gh && a.kc) k_va_ilp32<true, true><<<g, 128, 0, s>>>(a);
-  else if (gh) k_va_ilp32<true, false><<<g, 128, 0, s>>>(a);
-  else if (a.kc) k_va_ilp32<false, true><<<g, 128, 0, s>>>(a);
-  else k_va_ilp32<false, false><<<g, 128, 0, s>>>(a);
+  if (gh && a.kc) k_va_ilp32<true, true><<<gl, 128, 0, s>>>(a);
+  else if (gh) k_va_ilp32<true, false><<<gl, 128, 0, s>>>(a);
+  else if (a.kc) k_va_ilp32<false, true><<<gl, 128, 0, s>>>(a);
+  else k_va_ilp32<false, false><<<gl, 128, 0, s>>>(a);
+  k_va_slots<<<g, 128, 0, s>>>(a);
 }
 #endif
 

@@ -99,6 +99,18 @@ def test_close_pairs_and_free_atoms():
         assert np.abs(a["f"] - b["f"])[rest].max() <= 10.0 * TOL
 
 
+def test_per_atom_virial():
+    """The per-atom virial's double-float pass against the FP64 one: several elements and
+    images, free edges with zero to three intralayer neighbours, a close pair."""
+    t = S.displace(S.graphite_slab(2, 5, 3), 0.02, seed=4)
+    t.x[-1] = t.x[0] + 0.3 * np.array([0.6, 0.0, 0.8])
+    for s in (S.displace(S.twisted_bilayer(11, 7, 3.0, top="hbn", spacing=3.3), 0.05, seed=5),
+              S.displace(S.graphite_slab(3, 1, 1, mol_mode="unique"), 0.05, seed=1),
+              S.displace(S.flake_edges(6, 4), 0.03, seed=3), t):
+        a, b = _pair(s, vatom=True)
+        assert np.abs(a["vatom_ilp"] - b["vatom_ilp"]).max() <= TOL * np.abs(b["vatom_ilp"]).max()
+
+
 @pytest.mark.parametrize("ev", [False, True])
 def test_subdomain_form(ev):
     s = S.displace(S.twisted_bilayer(14, 8, 2.0, top="hbn", spacing=3.3), 0.03, seed=7)
@@ -111,10 +123,12 @@ def test_subdomain_form(ev):
                 gx.append(s.x + np.array([sx * L[0], sy * L[1], 0.0]))
     idx, x = np.concatenate(idx), np.concatenate(gx)
     r = []
+    va = dict(vatom=ev)
     for full in (0, 1):
         eng = capi.Engine(TERSOFF, ILP)
         eng.set_option("list_full", full)
-        r.append(eng.compute_ghost(s.n, x, s.type[idx], s.mol[idx], s.tag[idx], which=capi.ILP, eflag=ev, vflag=ev))
+        r.append(eng.compute_ghost(s.n, x, s.type[idx], s.mol[idx], s.tag[idx], which=capi.ILP, eflag=ev, vflag=ev, **va))
     _close(*r)
     if ev:
         _scalars(*r)
+        assert np.abs(r[0]["vatom_ilp"] - r[1]["vatom_ilp"]).max() <= TOL * np.abs(r[1]["vatom_ilp"]).max()
