@@ -102,6 +102,15 @@ LMFF_DF D<V> add1(D<V> a, V b) {
   const D<V> s = two_sum(a.h, b);
   return mk(s.h, vadd(s.l, a.l));
 }
+// c + a, c a constant that is a multiple of ulp(a.h) (an integer, |a| < 2^23): fast_two_sum
+// is exact for that too, whichever of the two is larger
+template <class V>
+LMFF_DF D<V> addc(float c, D<V> a) {
+  const D<V> s = fast_two_sum(vall<V>(c), a.h);
+  return mk(s.h, vadd(s.l, a.l));
+}
+template <class V>
+LMFF_DF D<V> scale(D<V> a, V m) { return mk(vmul(a.h, m), vmul(a.l, m)); }   // m a power of two or zero
 // running sum: acc += a
 template <class V>
 LMFF_DF void acc(D<V> &s, D<V> a) { s = add(s, a); }
@@ -156,14 +165,14 @@ LMFF_DF D<V> rcp(D<V> a) {
 // |f| <= 1/128, 2^a = 2^(k>>6) T[k & 63] e^g with g = f ln 2 as a double-float and
 // e^g - 1 = g + g^2/2 + g^3 (1/6 + g/24 + g^2/120), the last bracket in FP32 (truncation
 // below 2^-54).  tab holds T as double-floats (EXP2_TAB entries, filled by exp2_entry).
-// a.h is clamped to [-125, 127]: results below 2^-125 come out as about 2^-125.
+// For a <= 0 (a.h is clamped to [-125, 1]: results below 2^-125 come out as about 2^-125).
 constexpr int EXP2_TAB = 64;
 LMFF_DF float2 exp2_entry(int j) {
   const double t = exp2((double)j / EXP2_TAB);
   const float h = (float)t;
   return make_float2(h, (float)(t - (double)h));
 }
-LMFF_DF float clamp_exp(float x) { return fminf(fmaxf(x, -125.f), 127.f); }
+LMFF_DF float clamp_exp(float x) { return fminf(fmaxf(x, -125.f), 1.f); }
 LMFF_DF void exp2_parts(float t, const float2 *tab, float &th, float &tl, float &sc) {
   const int k = __float_as_int(t) - 0x4b400000;   // t = 1.5 2^23 + k
   const float2 T = tab[k & (EXP2_TAB - 1)];

@@ -25,6 +25,7 @@
 
 #include "engine.cuh"
 #include "forces.cuh"
+#include "ilp_df.cuh"
 #include "lmff_gb300.h"
 #include "neighbor.cuh"
 #include "potentials.h"
@@ -950,23 +951,21 @@ struct Engine {
 
   // whether the FP64 mode's pair kernel runs in double-float arithmetic (the number of ILP
   // elements, else 0): ilp/graphene/hbn with every element pair's constants equal to the
-  // swapped pair's (one constant set serves both repulsion terms and the vdW pair), and of
-  // a size that keeps every factor of a pair beyond 0.5 A inside the FP32 exponent range
-  // (e^80 < 2^116; 2^48 of the lo part's digits fit below the smallest factor that counts)
+  // swapped pair's (one set of tables serves both repulsion terms and the vdW pair), the
+  // cutoff inside the tables' range, and constants of a size that keeps every factor of a
+  // pair beyond 0.5 A inside the FP32 exponent range with room for a lo part
   int pair_df_elements() const {
     if (!i_on || pot64.kc || !pot64.vdw_sym) return 0;
     auto in = [](double v, double lo, double hi) { return v == 0.0 || (std::fabs(v) >= lo && std::fabs(v) <= hi); };
-    if (!(cut_global >= 1.0 && cut_global <= 1e3)) return 0;
+    if (!(cut_global >= 1.0 && cut_global * cut_global <= 0.99 * df::Q_MAX)) return 0;
     for (int a = 0; a < pot64.i_ne; a++)
       for (int b = 0; b < pot64.i_ne; b++) {
         const IlpP<double> &q = pot64.ilp[a * MAXELEM + b];
         if (!q.same_as_swapped) return 0;
-        if (!(std::fabs(q.lambda * q.z0) <= 40.0 && std::fabs(q.d) <= 40.0 && std::fabs(q.d_over_seff) <= 1e3 &&
-              std::fabs(q.lambda) <= 1e3 && std::fabs(q.delta2inv) <= 1e3))
+        if (!(q.lambda >= 0.0 && q.lambda <= 20.0 && q.lambda * q.z0 <= 40.0 && q.d >= 0.0 && q.d <= 40.0 &&
+              q.seff > 0.0 && q.d_over_seff <= 40.0 && q.delta2inv >= 0.0 && q.delta2inv <= 1e3))
           return 0;
-        if (!(in(q.C, 1e-12, 1e6) && in(q.eps_half, 1e-12, 1e6) && in(q.C6, 1e-6, 1e8) && q.lambda >= 0.0 &&
-              q.d_over_seff >= 0.0 && q.delta2inv >= 0.0))
-          return 0;
+        if (!(in(q.C, 1e-12, 1e6) && in(q.eps_half, 1e-12, 1e6) && in(q.C6, 1e-6, 1e8))) return 0;
       }
     return pot64.i_ne;
   }
@@ -1548,6 +1547,7 @@ struct Engine {
     a.no_small = !small_variants;
     a.kc = i_on && hi.model == LMFF_INTERLAYER_KC;
     a.pair_df = pair_df;
+    a.jstride = cap_n;
     // not while kernels are timed one by one (events between the launches)
     if (!ktiming && n <= PDL_MAX_ATOMS) a.pdl = pdl_short ? pdl_mask : (pdl_mask & ~PDL_SHORT);
     return a;
@@ -3206,6 +3206,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     a.list_full = g.list_full;
     a.kc = g.i_on && g.hi.model == LMFF_INTERLAYER_KC;
     a.pair_df = g.pair_df;
+    a.jstride = c;
   };
   const bool ev = true;
   if (g.precision == LMFF_FP64) {

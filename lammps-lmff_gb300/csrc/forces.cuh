@@ -329,6 +329,7 @@ struct ForceArgs {
   // FP64 mode: the number of ILP elements when the double-float pair kernel takes the
   // potential (Engine::pair_df), 0: k_ilp.  jrec then holds its records
   int pair_df;
+  int jstride;         // atoms per array of the records
   // programmatic dependent launch (PDL) of the step's chain kernels, a PDL_* mask: which
   // kernels are launched early behind the kernel before them on the stream (the pair
   // kernel, the normal-derivative kernel, the gather, and inside a step graph the

@@ -66,11 +66,14 @@ __device__ __forceinline__ bool lt_exact(R rsq, R thr, const d4 *xq, const SysDe
 }
 
 #ifndef LMFF_PACKED_X2
-// Record of the double-float pair kernel, four float4 per atom (ForceArgs::jrec): the
+// Record of the double-float pair kernel, four float4 per atom in four arrays of jstride
+// (ForceArgs::jrec; neighbours in a list are mostly consecutive atoms, whose 16-byte pieces
+// then share cache lines: with the 64 bytes of an atom in one place every load touched
+// four times as many): the
 // position as h + m + l, h on the system's coarse grid and m on its fine one (SysDesc::
 // dfM1, dfM2), so that differences of h and of m are exact in FP32 and l carries the rest
 // of the FP64 value; the unit normal as hi and lo; the ILP element.  Layout: (h, m_x),
-// (m_y, m_z, nh_x, nh_y), (nh_z, nl), (l, element).
+// (m_y, m_z, l_x, l_y), (l_z, nh), (nl, element).
 __device__ __forceinline__ void df_split(double x, double M1, double M2, float &h, float &m, float &l) {
   h = (float)__dsub_rn(__dadd_rn(x, M1), M1);
   const double r = __dsub_rn(x, (double)h);
@@ -84,11 +87,12 @@ __device__ __forceinline__ void df_record(const ForceArgs<double> &a, const SysD
   df_split(y, sd.dfM1, sd.dfM2, hy, my, ly);
   df_split(z, sd.dfM1, sd.dfM2, hz, mz, lz);
   const float nhx = (float)nx, nhy = (float)ny, nhz = (float)nz;
-  float4 *q = a.jrec + 4 * (size_t)i;
+  float4 *q = a.jrec + i;
+  const size_t s = a.jstride;
   q[0] = make_float4(hx, hy, hz, mx);
-  q[1] = make_float4(my, mz, nhx, nhy);
-  q[2] = make_float4(nhz, (float)(nx - (double)nhx), (float)(ny - (double)nhy), (float)(nz - (double)nhz));
-  q[3] = make_float4(lx, ly, lz, __int_as_float(ie));
+  q[s] = make_float4(my, mz, lx, ly);
+  q[2 * s] = make_float4(lz, nhx, nhy, nhz);
+  q[3 * s] = make_float4((float)(nx - (double)nhx), (float)(ny - (double)nhy), (float)(nz - (double)nhz), __int_as_float(ie));
 }
 #endif
 
@@ -2012,34 +2016,66 @@ __global__ void __launch_bounds__(256, (ilp_min_blocks<TPA, EV, EATOM, ONE, GH, 
 
 #ifndef LMFF_PACKED_X2
 // ============================================================ k_ilp_df ===========
-// The FP64 mode's interlayer pair kernel in double-float arithmetic: the sums of k_ilp
-// (force on i, dE/dn_i, energies, virial) from pair terms that carry ~48 bits, formed in
-// FP32 instructions.  The FP64 form of a pair is ~120 FP64 instructions, and the FP64
-// pipe (1/75 of the FP32 rate) bound k_ilp<double> completely; here a pair is ~700 FP32
-// instructions, packed two list entries per lane in FP32x2, with no FP64 instruction in
-// the loop (331,200-atom slab, energies and virial: 79.3 -> 9.3 ms; 7,200-atom bilayer,
-// forces: 786 -> 98 us; FMA pipe 64 % busy).  Displacements come from three-part positions whose leading parts subtract
-// exactly.
+// The FP64 mode's interlayer pair kernel: the sums of k_ilp (force on i, dE/dn_i, energies,
+// virial) from pair terms in double-float arithmetic (ilp_df.cuh), ~48 bits in FP32
+// instructions.  The FP64 form of a pair is ~120 FP64 instructions, and the FP64 pipe
+// (1/75 of the FP32 rate) bound k_ilp<double> completely.  Here the functions of r^2 come
+// from tables, the exponentials of the normals' terms and all products are double-floats,
+// and there is no FP64 instruction in the loop; displacements come from three-part
+// positions whose leading parts subtract exactly.
+// (Pair kernel against the FP64 form: 331,200-atom slab with energies and virial 79.3 ->
+// 8.0 ms, 7,200-atom bilayer, forces, 786 -> 68 us, 5,016 atoms in six layers 2,010 -> 149 us.)
 // The error of a pair's force against 64-bit arithmetic is below the FP64 form's, whose
 // 1/sqrt and 1/x are one FP64 Newton step from an FP32 estimate (CPU emulation against
-// 113-bit arithmetic, rms over 200,000 pairs of BNCH.ILP's element pairs: 3-9e-14 of the
+// 113-bit arithmetic, rms over 200,000 pairs of BNCH.ILP's element pairs: 2-5e-14 of the
 // rms pair force here, 1-9e-13 there).
 // The virial: half of del (x) f_ij at each end of a pair, which sums to the whole of the
 // pair's; the n_i part of f_ij is applied to the sums after the loop (f -= tpi n_i,
 // W -= g (x) n_i).
-// Pairs closer than 0.5 A, whose powers of 1/r leave the FP32 range, are left to ilp_pair
-// (FP64) in a second walk over the lane's entries; so is every pair of an atom so far
-// outside its box that the position grids do not hold it (SysDesc::dfmax).
-// Blocks of up to 128 threads, 4 per SM (128 registers, no spills); with energies and
-// virial 3 (168 registers).  A launch_bounds of 3 / 5 blocks for the force-only form
-// measured 5 % faster / 9 % slower on 5,016 atoms and 1 % faster / 13 % slower on 7,200.
+// Pairs closer than 0.5 A (below the tables) are left to ilp_pair (FP64) in a second walk
+// over the lane's entries; so is every pair of an atom so far outside its box that the
+// position grids do not hold it (SysDesc::dfmax).
+//
+// An atom's lanes walk its list tpa entries at a time.  The parts the normals enter are
+// ~350 instructions for a third of the pairs (carbon), scattered through the list: entries
+// that need them go to a queue per atom, and the lanes take tpa queued entries at once
+// (331,200-atom slab, forces: 23 of 32 lanes active and 6.5 ms when each lane evaluated
+// its own in place with direct radial functions; 31 of 32 and 5.2 ms with queue and
+// tables).  What bounds it now is the gathers: L1 wavefronts 75 %, issue 51 %.
+// Blocks of up to 128 threads, 5 per SM (96 registers), with energies and virial 4 (128):
+// one block more or less per SM measured 3-10 % slower on the 331,200-atom slab.
 constexpr int DF_THREADS = 128;
-constexpr float DF_CLOSE = 0.25f;   // A^2
-constexpr int DF_ROWS = MAXELEM * MAXELEM * MAXELEM;
-__constant__ float2 c_dfk[df::K_N];          // element 0's constants, each duplicated
-__constant__ df::PairG c_dfg;
-__device__ float2 g_dfk[DF_ROWS * df::K_N];  // (ie, jeA, jeB) rows: (X[ie][jeA], X[ie][jeB]), ne^3 of them
+constexpr int DF_BLOCKS = 5, DF_BLOCKS_EV = 4;
+constexpr float DF_CLOSE = df::Q_MIN;   // A^2
+struct DfCut {
+  float h, l;   // r_cut^2
+};
+__constant__ DfCut c_dfcut;
+__constant__ float c_dfk[df::K_N];                    // element pair (0, 0)'s constants
+__device__ float g_dfk[MAXELEM * MAXELEM * df::K_N];  // element pair (a, b)'s at (a * ne + b) * K_N
 __device__ float2 g_exp2_df[df::EXP2_TAB];
+// tables (ilp_df.cuh), per interval of element pair a * ne + b: the coefficients of A and of
+// M in two float4 each, U and TE at the centre
+__device__ float4 g_dfA[MAXELEM * MAXELEM * df::TAB_N * 2];
+__device__ float4 g_dfM[MAXELEM * MAXELEM * df::TAB_N * 2];
+__device__ float2 g_dfU[MAXELEM * MAXELEM * df::TAB_N];
+__device__ float2 g_dfTE[MAXELEM * MAXELEM * df::TAB_N];
+
+__global__ void k_fill_df_tables(int ne) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= ne * ne * df::TAB_N) return;
+  const int p = k / df::TAB_N, a = p / ne, b = p % ne;
+  const IlpP<R> &q = c_pot.ilp[a * MAXELEM + b];
+  const df::TabP t = {q.z0, q.lambda, 2.0 * q.eps_half, q.d, q.seff, q.C6, 1.0 / c_pot.i_inv_rcut, c_pot.tap};
+  float ca[8], cm[8], u[2], te[2];
+  df::tab_fill(t, k % df::TAB_N, ca, cm, u, te);
+  for (int m = 0; m < 2; m++) {
+    g_dfA[2 * (size_t)k + m] = make_float4(ca[4 * m], ca[4 * m + 1], ca[4 * m + 2], ca[4 * m + 3]);
+    g_dfM[2 * (size_t)k + m] = make_float4(cm[4 * m], cm[4 * m + 1], cm[4 * m + 2], cm[4 * m + 3]);
+  }
+  g_dfU[k] = make_float2(u[0], u[1]);
+  g_dfTE[k] = make_float2(te[0], te[1]);
+}
 
 __global__ void k_fill_exp2_df() {
   const int j = threadIdx.x;
@@ -2051,14 +2087,14 @@ struct DfAtom {
   float h[3], m[3], l[3];
   float nh[3], nl[3];
   int el;
-  __device__ __forceinline__ void load(const float4 *jrec, int i) {
-    const float4 *q = jrec + 4 * (size_t)i;
-    const float4 q0 = __ldg(q), q1 = __ldg(q + 1), q2 = __ldg(q + 2), q3 = __ldg(q + 3);
+  __device__ __forceinline__ void load(const float4 *jrec, int s, int i) {
+    const float4 *q = jrec + i;
+    const float4 q0 = __ldg(q), q1 = __ldg(q + s), q2 = __ldg(q + 2 * (size_t)s), q3 = __ldg(q + 3 * (size_t)s);
     h[0] = q0.x; h[1] = q0.y; h[2] = q0.z;
     m[0] = q0.w; m[1] = q1.x; m[2] = q1.y;
-    nh[0] = q1.z; nh[1] = q1.w; nh[2] = q2.x;
-    nl[0] = q2.y; nl[1] = q2.z; nl[2] = q2.w;
-    l[0] = q3.x; l[1] = q3.y; l[2] = q3.z;
+    l[0] = q1.z; l[1] = q1.w; l[2] = q2.x;
+    nh[0] = q2.y; nh[1] = q2.z; nh[2] = q2.w;
+    nl[0] = q3.x; nl[1] = q3.y; nl[2] = q3.z;
     el = __float_as_int(q3.w);
   }
 };
@@ -2100,7 +2136,7 @@ __device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int la
   const d4 ni = a.nrm64[i];
   const long long itag = a.tag[i];
   DfAtom I;
-  I.load(a.jrec, i);
+  I.load(a.jrec, a.jstride, i);
   const int64_t b = a.list_off[i];
   const int cnt = (int)(a.list_off[i + 1] - b);
   for (int k = lane; k < cnt; k += tpa) {
@@ -2108,7 +2144,7 @@ __device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int la
     int j, sx, sy, sz;
     decode_entry(e, a.lc, j, sx, sy, sz);
     DfAtom A;
-    A.load(a.jrec, j);
+    A.load(a.jrec, a.jstride, j);
     df::D<float> d[3];
     df_del<true>(I, A, sd, sx, sy, sz, d);
     if (!all && !(df::dot3(d, d).h < DF_CLOSE)) continue;
@@ -2118,135 +2154,197 @@ __device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int la
 }
 
 template <bool EV, bool ONE, bool GH>
-__global__ void __launch_bounds__(DF_THREADS, EV ? 3 : 4) k_ilp_df(ForceArgs<R> a, int tpa, int eatom, int ne) {
+__global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_ilp_df(ForceArgs<R> a, int tpa, int eatom, int ne) {
   pdl_enter(a.pdl);
   using namespace df;
-  typedef float2 V;
+  typedef float V;
   __shared__ float2 s_tab[EXP2_TAB];
-  __shared__ float2 s_dfk[ONE ? 1 : DF_ROWS * K_N];
+  __shared__ float s_dfk[ONE ? 1 : MAXELEM * MAXELEM * K_N];
+  __shared__ uint32_t s_queue[DF_THREADS * 4];   // 4 tpa entries per atom
   for (int w = threadIdx.x; w < EXP2_TAB; w += blockDim.x) s_tab[w] = g_exp2_df[w];
   if constexpr (!ONE) {
-    for (int w = threadIdx.x; w < ne * ne * ne * K_N; w += blockDim.x) s_dfk[w] = g_dfk[w];
+    for (int w = threadIdx.x; w < ne * ne * K_N; w += blockDim.x) s_dfk[w] = g_dfk[w];
     const int words = (int)(sizeof(c_pot.ilp) / sizeof(int));
     const int *src = reinterpret_cast<const int *>(c_pot.ilp);
     int *dst = reinterpret_cast<int *>(s_ilp);
     for (int w = threadIdx.x; w < words; w += blockDim.x) dst[w] = src[w];
   }
   __syncthreads();
+  const unsigned FULL = 0xffffffffu;
   const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
   const int i = gtid / tpa;
   const int lane = threadIdx.x & (tpa - 1);
+  const unsigned gmask = (tpa == 32 ? FULL : ((1u << tpa) - 1u) << ((threadIdx.x & 31) & ~(tpa - 1)));
+  const unsigned below = gmask & ((1u << (threadIdx.x & 31)) - 1u);
+  uint32_t *const queue = s_queue + 4 * (threadIdx.x & ~(tpa - 1));
   const bool valid = i < a.n;
   const int ii = valid ? i : a.n - 1;
   const SysDesc &sd = a.A.sys[a.A.sysid[ii]];
   DfAtom I;
-  I.load(a.jrec, ii);
+  I.load(a.jrec, a.jstride, ii);
   const int ie = I.el;
   const long long itag = GH ? a.tag[ii] : 0;
   const bool iown = !GH || owned(a, ii);
   D<V> f[3], g[3], tpi, ev, er, w[6];
-  const V zero = vall<V>(0.f);
 #pragma unroll
-  for (int c = 0; c < 3; c++) f[c] = g[c] = mk(zero, zero);
-  tpi = ev = er = mk(zero, zero);
+  for (int c = 0; c < 3; c++) f[c] = g[c] = mk(0.f, 0.f);
+  tpi = ev = er = mk(0.f, 0.f);
 #pragma unroll
-  for (int c = 0; c < 6; c++) w[c] = mk(zero, zero);
+  for (int c = 0; c < 6; c++) w[c] = mk(0.f, 0.f);
   const bool out = fabsf(I.h[0]) > sd.dfmax || fabsf(I.h[1]) > sd.dfmax || fabsf(I.h[2]) > sd.dfmax;
   bool close = valid && ie >= 0 && out;
-  if (valid && ie >= 0 && !out) {
-    const int64_t b = a.list_off[i];
-    const uint32_t *lst = a.list + b;
-    const int cnt = (int)(a.list_off[i + 1] - b);
-    auto run = [&](auto img_t) {
-      constexpr bool IMG = decltype(img_t)::value;
-      for (int k = lane; k < cnt; k += 2 * tpa) {
-        const uint32_t ea = __ldg(&lst[k]);
-        const bool bval = k + tpa < cnt;
-        const uint32_t eb = bval ? __ldg(&lst[k + tpa]) : ea;
-        int ja, jb, ax = 0, ay = 0, az = 0, bx = 0, by = 0, bz = 0;
-        if constexpr (IMG) {
-          decode_entry(ea, a.lc, ja, ax, ay, az);
-          decode_entry(eb, a.lc, jb, bx, by, bz);
-        } else {
-          ja = (int)(ea & a.lc.imask);
-          jb = (int)(eb & a.lc.imask);
-        }
-        DfAtom A, B;
-        A.load(a.jrec, ja);
-        B.load(a.jrec, jb);
-        D<V> d[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          V dh, dm, dl;
-          df_disp<IMG>(I, A, sd, ax, ay, az, c, dh.x, dm.x, dl.x);
-          df_disp<IMG>(I, B, sd, bx, by, bz, c, dh.y, dm.y, dl.y);
-          d[c] = fast_two_sum(dh, dm);
-          d[c].l = vadd(d[c].l, dl);
-        }
-        D<V> q = dot3(d, d);
-        const bool inA = __fadd_rn(__fsub_rn(q.h.x, c_dfg.cut_h), __fsub_rn(q.l.x, c_dfg.cut_l)) < 0.f;
-        const bool inB = bval && __fadd_rn(__fsub_rn(q.h.y, c_dfg.cut_h), __fsub_rn(q.l.y, c_dfg.cut_l)) < 0.f;
-        if (!(inA || inB)) continue;
-        V on = make_float2(inA ? 1.f : 0.f, inB ? 1.f : 0.f);
-        if (q.h.x < DF_CLOSE || q.h.y < DF_CLOSE) {   // rare
-          close = true;
-          if (q.h.x < DF_CLOSE) { q.h.x = 4.f; on.x = 0.f; }
-          if (q.h.y < DF_CLOSE) { q.h.y = 4.f; on.y = 0.f; }
-        }
-        D<V> nj[3], ni[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          nj[c] = mk(make_float2(A.nh[c], B.nh[c]), make_float2(A.nl[c], B.nl[c]));
-          ni[c] = mk(vall<V>(I.nh[c]), vall<V>(I.nl[c]));
-        }
-        V wv = on, wi = on, wj = on;
-        if constexpr (GH) {
-          auto wt = [&](int j, float dx, float dy, float dz, float &v, float &wi_, float &wj_) {
-            const bool jown = owned(a, j);
-            const bool keep = keep_half_r(itag, (long long)a.tag[j], -dx, -dy, -dz);
-            v = (keep ? iown : jown) ? 1.f : 0.f;
-            wi_ = iown ? 1.f : 0.f;
-            wj_ = jown ? 1.f : 0.f;
-          };
-          wt(ja, d[0].h.x + d[0].l.x, d[1].h.x + d[1].l.x, d[2].h.x + d[2].l.x, wv.x, wi.x, wj.x);
-          wt(jb, d[0].h.y + d[0].l.y, d[1].h.y + d[1].l.y, d[2].h.y + d[2].l.y, wv.y, wi.y, wj.y);
-        }
-        PairOut<V> o;
-        if constexpr (ONE) {
-          pair_terms<EV, GH>(c_dfg, [&](int k2) { return c_dfk[k2]; }, s_tab, q, dot3(ni, d), dot3(nj, d), on, wv, wi,
-                             wj, o);
-        } else {
-          const float2 *row = s_dfk + ((ie * ne + A.el) * ne + B.el) * K_N;
-          pair_terms<EV, GH>(c_dfg, [&](int k2) { return row[k2]; }, s_tab, q, dot3(ni, d), dot3(nj, d), on, wv, wi, wj,
-                             o);
-        }
-        const D<V> ntq = neg(o.tq);
-        acc(tpi, o.tp);
-#pragma unroll
-        for (int c = 0; c < 3; c++) acc_mul(g[c], o.tp, d[c]);
-        D<V> t[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) {
-          t[c] = add(mul(o.crad, d[c]), mul(ntq, nj[c]));
-          acc(f[c], t[c]);
-        }
-        if constexpr (EV) {
-          acc(ev, o.evdw);
-          acc(er, o.erep);
-          acc_mul(w[0], d[0], t[0]); acc_mul(w[1], d[1], t[1]); acc_mul(w[2], d[2], t[2]);
-          acc_mul(w[3], d[0], t[1]); acc_mul(w[4], d[0], t[2]); acc_mul(w[5], d[1], t[2]);
-        }
+  const int64_t b = a.list_off[ii];
+  const uint32_t *const lst = a.list + b;
+  const int cnt = valid && ie >= 0 && !out ? (int)(a.list_off[ii + 1] - b) : 0;
+  const int most = __reduce_max_sync(FULL, cnt);
+  auto run = [&](auto img_t) {
+    constexpr bool IMG = decltype(img_t)::value;
+    auto pair_of = [&](uint32_t e, DfAtom &A, int &j, D<V> d[3]) {
+      int sx = 0, sy = 0, sz = 0;
+      if constexpr (IMG) decode_entry(e, a.lc, j, sx, sy, sz);
+      else j = (int)(e & a.lc.imask);
+      A.load(a.jrec, a.jstride, j);
+      df_del<IMG>(I, A, sd, sx, sy, sz, d);
+    };
+    // weights of the subdomain mode: the vdW pair, the terms with n_i and with n_j
+    auto weights = [&](int j, const D<V> d[3], float &wv, float &wi, float &wj) {
+      if constexpr (GH) {
+        const bool jown = owned(a, j);
+        const bool keep =
+            keep_half_r(itag, (long long)a.tag[j], -(d[0].h + d[0].l), -(d[1].h + d[1].l), -(d[2].h + d[2].l));
+        wv = (keep ? iown : jown) ? 1.f : 0.f;
+        wi = iown ? 1.f : 0.f;
+        wj = jown ? 1.f : 0.f;
       }
     };
-    if (a.list_img[i]) run(std::true_type{});
-    else run(std::false_type{});
-  }
-  // ---- the lane's two halves, then the atom's lanes, in double-float; FP64 from there
+    auto consts = [&](int je) {
+      return [&, je](int k) {
+        if constexpr (ONE) return c_dfk[k];
+        else return s_dfk[(ie * ne + je) * K_N + k];
+      };
+    };
+    auto virial = [&](const D<V> d[3], const D<V> t[3]) {
+      acc_mul(w[0], d[0], t[0]); acc_mul(w[1], d[1], t[1]); acc_mul(w[2], d[2], t[2]);
+      acc_mul(w[3], d[0], t[1]); acc_mul(w[4], d[0], t[2]); acc_mul(w[5], d[1], t[2]);
+    };
+    // the parts the normals enter, of the first entries in the queue
+    int qh = 0, qn = 0;   // taken and put so far, the same in every lane of the atom
+    auto near_batch = [&](bool on) {
+      __syncwarp();
+      if (on && qh + lane < qn) {
+        DfAtom A;
+        int j;
+        D<V> d[3], ni[3], nj[3], tp, tq, S, crad = mk(0.f, 0.f);
+        pair_of(queue[(qh + lane) & (4 * tpa - 1)], A, j, d);
+        const D<V> q = dot3(d, d);
+        float th, wv = 1.f, wi = 1.f, wj = 1.f;
+        int k = tab_at(q.h, th);
+        if constexpr (!ONE) k += (ie * ne + A.el) * TAB_N;
+        const D<V> off = fast_two_sum(th, q.l);
+        Coef<V> c;
+        coef_set(c, g_dfM + 2 * k);
+        const float2 f0 = __ldg(g_dfTE + k);
+        weights(j, d, wv, wi, wj);
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+          ni[x] = mk(I.nh[x], I.nl[x]);
+          nj[x] = mk(A.nh[x], A.nl[x]);
+        }
+        const auto K = consts(A.el);
+        const D<V> TE = tab_integral(c, f0.x, f0.y, off);
+        pair_near<GH>(K, s_tab, q, TE, tab_poly(c, off), dot3(ni, d), dot3(nj, d), wi, wj, crad, tp, tq, S);
+        acc(tpi, tp);
+        const D<V> ntq = neg(tq);
+        D<V> t[3];
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+          acc_mul(g[x], tp, d[x]);
+          t[x] = add(mul(crad, d[x]), mul(ntq, nj[x]));
+          acc(f[x], t[x]);
+        }
+        if constexpr (EV) {
+          acc(er, mul(mul(TE, S), mk(K(K_C), K(K_C + 1))));
+          virial(d, t);
+        }
+      }
+      if (on) qh = min(qh + tpa, qn);
+      __syncwarp();
+    };
+    for (int k0 = 0, it = 1; k0 < most; k0 += tpa, it++) {
+      bool near = false;
+      uint32_t e = 0;
+      if (k0 + lane < cnt) {
+        e = __ldg(&lst[k0 + lane]);
+        DfAtom A;
+        int j;
+        D<V> d[3];
+        pair_of(e, A, j, d);
+        const D<V> q = dot3(d, d);
+        bool in = __fadd_rn(__fsub_rn(q.h, c_dfcut.h), __fsub_rn(q.l, c_dfcut.l)) < 0.f;
+        if (in && q.h < DF_CLOSE) {   // rare
+          close = true;
+          in = false;
+        }
+        if (in) {
+          float th;
+          int k = tab_at(q.h, th);
+          if constexpr (!ONE) k += (ie * ne + A.el) * TAB_N;
+          const D<V> off = fast_two_sum(th, q.l);
+          Coef<V> c;
+          coef_set(c, g_dfA + 2 * k);
+          D<V> crad = tab_poly(c, off);
+          const auto K = consts(A.el);
+          if constexpr (EV || GH) {
+            float wv = 1.f, wi = 1.f, wj = 1.f;
+            weights(j, d, wv, wi, wj);
+            const float wm = 0.5f * (wi + wj);
+            const D<V> eps = mk(K(K_EPS), K(K_EPS + 1));
+            Coef<V> cM;
+            coef_set(cM, g_dfM + 2 * k);
+            // A = vdW part + eps M: weights wv and (wi + wj) / 2
+            if constexpr (GH) crad = add(scale(crad, wv), scale(mul(tab_poly(cM, off), eps), wm - wv));
+            if constexpr (EV) {
+              const float2 u0 = __ldg(g_dfU + k), f0 = __ldg(g_dfTE + k);
+              const D<V> te = mul(tab_integral(cM, f0.x, f0.y, off), eps);
+              D<V> vdw = add(tab_integral(c, u0.x, u0.y, off), neg(te));
+              if constexpr (GH) {
+                vdw = scale(vdw, wv);
+                acc(er, scale(te, wm));
+              } else {
+                acc(er, te);
+              }
+              acc(ev, vdw);
+            }
+          }
+          near = near_one(K(K_ND2), q.h, I.nh[0] * d[0].h + I.nh[1] * d[1].h + I.nh[2] * d[2].h,
+                          A.nh[0] * d[0].h + A.nh[1] * d[1].h + A.nh[2] * d[2].h);
+          D<V> t[3];
+#pragma unroll
+          for (int x = 0; x < 3; x++) {
+            t[x] = mul(crad, d[x]);
+            acc(f[x], t[x]);
+          }
+          if constexpr (EV) virial(d, t);
+        }
+      }
+      const unsigned bits = __ballot_sync(FULL, near);
+      if (near) queue[(qn + __popc(bits & below)) & (4 * tpa - 1)] = e;
+      qn += __popc(bits & gmask);
+      // whole batches every third round (fewer than 4 tpa entries wait), so that when and on
+      // which lane an entry is evaluated depends on its atom's list alone: results are
+      // the same whatever atoms share the warp
+      if (it % 3 == 0)
+        while (__any_sync(FULL, qn - qh >= tpa)) near_batch(qn - qh >= tpa);
+    }
+    while (__any_sync(FULL, qh < qn)) near_batch(true);
+  };
+  if (__any_sync(FULL, cnt > 0 && a.list_img[ii] != 0)) run(std::true_type{});
+  else run(std::false_type{});
+  // ---- the atom's lanes in double-float; FP64 from there
   auto total = [&](const D<V> &v) {
-    D<float> s = add(mk(v.h.x, v.l.x), mk(v.h.y, v.l.y));
-    s = renorm(s);
+    D<float> s = renorm(v);
     for (int o = tpa / 2; o > 0; o >>= 1) {
-      const D<float> p = mk(__shfl_xor_sync(0xffffffffu, s.h, o), __shfl_xor_sync(0xffffffffu, s.l, o));
+      const D<float> p = mk(__shfl_xor_sync(FULL, s.h, o), __shfl_xor_sync(FULL, s.l, o));
       s = renorm(add(s, p));
     }
     return (double)s.h + (double)s.l;
@@ -2265,14 +2363,13 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? 3 : 4) k_ilp_df(ForceArgs<R> 
 #pragma unroll
     for (int c = 0; c < 6; c++) sw[c] = total(w[c]);
   }
-  const bool any = __any_sync(0xffffffffu, close);
-  if (any) {
+  if (__any_sync(FULL, close)) {
     if (close) df_close_pairs<EV, ONE, GH>(a, i, lane, tpa, ie, iown, out, x);
     double *v[14] = {&x.fx, &x.fy, &x.fz, &x.gxa, &x.gya, &x.gza, &x.evdw, &x.erep, &x.w0, &x.w1, &x.w2, &x.w3, &x.w4,
                      &x.w5};
 #pragma unroll
     for (int c = 0; c < (EV ? 14 : 6); c++)
-      for (int o = tpa / 2; o > 0; o >>= 1) *v[c] += __shfl_xor_sync(0xffffffffu, *v[c], o);
+      for (int o = tpa / 2; o > 0; o >>= 1) *v[c] += __shfl_xor_sync(FULL, *v[c], o);
   }
   if (!valid || lane != 0) return;
   const double n[3] = {(double)I.nh[0] + (double)I.nl[0], (double)I.nh[1] + (double)I.nl[1],
@@ -2296,43 +2393,29 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? 3 : 4) k_ilp_df(ForceArgs<R> 
   }
 }
 
-// constants of the double-float kernel from the FP64 ones
+// constants and tables of the double-float kernel from the FP64 ones (c_pot's copy is queued
+// on s before this)
 static void upload_pair_df(const PotConst<R> &p, cudaStream_t s) {
-  static float2 one[df::K_N], rows[DF_ROWS * df::K_N];   // static: the asynchronous copies read them after return
-  static df::PairG g;
+  static float rows[MAXELEM * MAXELEM * df::K_N];   // static: the asynchronous copies read them after return
+  static DfCut cut;
   auto split = [](double v, float &h, float &l) {
     h = (float)v;
     l = (float)(v - (double)h);
   };
-  const double cut = 1.0 / p.i_inv_rcut;
-  split(p.i_inv_rcut, g.irc_h, g.irc_l);
-  split(-140.0 / cut, g.dt_h, g.dt_l);
-  split(p.i_cutsq, g.cut_h, g.cut_l);
-  g.tap = p.tap;
-  auto consts = [&](const IlpP<R> &q, float *h, float *l) {
-    const double v[df::K_N / 2] = {q.nd2_l2e, q.C, 2.0 * q.eps_half, 2.0 * q.C * q.delta2inv, q.lambda, q.lam_l2e, q.z0,
-                                   q.ts_a, q.seff, q.C6, q.d_over_seff};
-    for (int k = 0; k < df::K_N / 2; k++) split(v[k], h[k], l[k]);
-  };
+  split(p.i_cutsq, cut.h, cut.l);
   const int ne = p.i_ne;
-  float h[MAXELEM * MAXELEM][df::K_N / 2], l[MAXELEM * MAXELEM][df::K_N / 2];
   for (int a = 0; a < ne; a++)
-    for (int b = 0; b < ne; b++) consts(p.ilp[a * MAXELEM + b], h[a * ne + b], l[a * ne + b]);
-  for (int k = 0; k < df::K_N / 2; k++) {
-    one[2 * k] = make_float2(h[0][k], h[0][k]);
-    one[2 * k + 1] = make_float2(l[0][k], l[0][k]);
-    for (int a = 0; a < ne; a++)
-      for (int b = 0; b < ne; b++)
-        for (int c = 0; c < ne; c++) {
-          float2 *r = rows + ((a * ne + b) * ne + c) * df::K_N + 2 * k;
-          r[0] = make_float2(h[a * ne + b][k], h[a * ne + c][k]);
-          r[1] = make_float2(l[a * ne + b][k], l[a * ne + c][k]);
-        }
-  }
-  cudaMemcpyToSymbolAsync(c_dfk, one, sizeof one, 0, cudaMemcpyHostToDevice, s);
-  cudaMemcpyToSymbolAsync(c_dfg, &g, sizeof g, 0, cudaMemcpyHostToDevice, s);
+    for (int b = 0; b < ne; b++) {
+      const IlpP<R> &q = p.ilp[a * MAXELEM + b];
+      const double v[df::K_N / 2] = {q.nd2_l2e, q.C, 2.0 * q.eps_half, 2.0 * q.C * q.delta2inv};
+      float *r = rows + (a * ne + b) * df::K_N;
+      for (int k = 0; k < df::K_N / 2; k++) split(v[k], r[2 * k], r[2 * k + 1]);
+    }
+  cudaMemcpyToSymbolAsync(c_dfk, rows, sizeof c_dfk, 0, cudaMemcpyHostToDevice, s);
+  cudaMemcpyToSymbolAsync(c_dfcut, &cut, sizeof cut, 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(g_dfk, rows, sizeof rows, 0, cudaMemcpyHostToDevice, s);
   k_fill_exp2_df<<<1, df::EXP2_TAB, 0, s>>>();
+  k_fill_df_tables<<<(ne * ne * df::TAB_N + 63) / 64, 64, 0, s>>>(ne);
 }
 
 template <bool ONE, bool GH>
@@ -3021,14 +3104,14 @@ __device__ __noinline__ void va_close_pairs(const ForceArgs<R> &a, int i, int la
   const long long itag = a.tag[i];
   const d4 ni = a.nrm64[i];
   DfAtom I;
-  I.load(a.jrec, i);
+  I.load(a.jrec, a.jstride, i);
   const int64_t q1 = a.list_off[i + 1];
   for (int64_t q = a.list_off[i] + lane; q < q1; q += VA_LANES) {
     const uint32_t e = a.list[q];
     int j, sx, sy, sz;
     decode_entry(e, a.lc, j, sx, sy, sz);
     DfAtom A;
-    A.load(a.jrec, j);
+    A.load(a.jrec, a.jstride, j);
     df::D<float> d[3];
     df_del<true>(I, A, sd, sx, sy, sz, d);
     if (!all && !(df::dot3(d, d).h < DF_CLOSE)) continue;
@@ -3049,7 +3132,7 @@ __global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
   const unsigned gmask = ((1u << VA_LANES) - 1) << ((threadIdx.x & 31) & ~(VA_LANES - 1));
   const SysDesc &sd = a.A.sys[a.A.sysid[i]];
   DfAtom I;
-  I.load(a.jrec, i);
+  I.load(a.jrec, a.jstride, i);
   const int ie = I.el;
   const long long itag = GH ? a.tag[i] : 0;
   const bool iown = !GH || owned(a, i);
@@ -3068,11 +3151,11 @@ __global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
       int j, sx, sy, sz;
       decode_entry(e, a.lc, j, sx, sy, sz);
       DfAtom A;
-      A.load(a.jrec, j);
+      A.load(a.jrec, a.jstride, j);
       D<V> d[3], nj[3];
       df_del<true>(I, A, sd, sx, sy, sz, d);
       const D<V> q = dot3(d, d);
-      if (!(__fadd_rn(__fsub_rn(q.h, c_dfg.cut_h), __fsub_rn(q.l, c_dfg.cut_l)) < 0.f)) continue;
+      if (!(__fadd_rn(__fsub_rn(q.h, c_dfcut.h), __fsub_rn(q.l, c_dfcut.l)) < 0.f)) continue;
       if (q.h < DF_CLOSE) {
         close = true;
         continue;
@@ -3087,21 +3170,39 @@ __global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
         wi = iown ? 1.f : 0.f;
         wj = jown ? 1.f : 0.f;
       }
-      PairOut<V> o;
-      if constexpr (ONE) {
-        pair_terms<false, GH>(c_dfg, [&](int k2) { return c_dfk[k2].x; }, s_tab, q, dot3(ni, d), dot3(nj, d), 1.f, wv,
-                              wi, wj, o);
-      } else {
-        const float2 *row = g_dfk + ((ie * ne + A.el) * ne + A.el) * K_N;
-        pair_terms<false, GH>(c_dfg, [&](int k2) { return __ldg(&row[k2]).x; }, s_tab, q, dot3(ni, d), dot3(nj, d), 1.f,
-                              wv, wi, wj, o);
+      const float *row = ONE ? nullptr : g_dfk + (ie * ne + A.el) * K_N;
+      auto K = [&](int k2) {
+        if constexpr (ONE) return c_dfk[k2];
+        else return __ldg(&row[k2]);
+      };
+      float th;
+      int ki = tab_at(q.h, th);
+      if constexpr (!ONE) ki += (ie * ne + A.el) * TAB_N;
+      const D<V> off = fast_two_sum(th, q.l);
+      Coef<V> cc;
+      coef_set(cc, g_dfA + 2 * ki);
+      D<V> crad = tab_poly(cc, off);
+      const bool near = near_one(K(K_ND2), q.h, I.nh[0] * d[0].h + I.nh[1] * d[1].h + I.nh[2] * d[2].h,
+                                 A.nh[0] * d[0].h + A.nh[1] * d[1].h + A.nh[2] * d[2].h);
+      D<V> M, tp = mk(0.f, 0.f), tq = tp;
+      if (GH || near) {
+        coef_set(cc, g_dfM + 2 * ki);
+        M = tab_poly(cc, off);
       }
-      const D<V> ntq = neg(o.tq);
+      if constexpr (GH)
+        crad = add(scale(crad, wv), scale(mul(M, mk(K(K_EPS), K(K_EPS + 1))), 0.5f * (wi + wj) - wv));
+      if (near) {
+        const float2 f0 = __ldg(g_dfTE + ki);
+        D<V> S;
+        pair_near<GH>(K, s_tab, q, tab_integral(cc, f0.x, f0.y, off), M, dot3(ni, d), dot3(nj, d), wi, wj, crad, tp,
+                      tq, S);
+      }
+      const D<V> ntq = neg(tq);
       D<V> t[3], h[3];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        t[c] = add(mul(o.crad, d[c]), mul(ntq, nj[c]));
-        h[c] = mul(o.tp, d[c]);
+        t[c] = add(mul(crad, d[c]), mul(ntq, nj[c]));
+        h[c] = mul(tp, d[c]);
         acc(s[6 + c], h[c]);
       }
       constexpr int P[6] = {0, 1, 2, 0, 0, 1}, Q[6] = {0, 1, 2, 1, 2, 2};
@@ -3110,11 +3211,11 @@ __global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
         acc_mul(s[c], d[P[c]], t[Q[c]]);
         acc_mul(s[9 + c], h[P[c]], d[Q[c]]);
       }
-      if (o.tq.h != 0.f) {
+      if (tq.h != 0.f) {
         // the partner's normal-derivative share, g = tq del
         D<V> g[3], b[3];
 #pragma unroll
-        for (int c = 0; c < 3; c++) g[c] = mul(o.tq, d[c]);
+        for (int c = 0; c < 3; c++) g[c] = mul(tq, d[c]);
         const float4 *tt = a.va_tens + 14 * (size_t)j;
         float4 T[14];
 #pragma unroll

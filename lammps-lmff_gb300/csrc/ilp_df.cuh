@@ -1,6 +1,27 @@
 // The FP64 mode's interlayer pair terms in double-float arithmetic (dfloat.cuh): what
 // calc_FvdW and calc_FRep (pair_ilp_graphene_hbn.cpp:449-675) form per pair, for two pairs
 // at a time (V = float2) or one (V = float).
+//
+// With q = r^2, Tap and dTap of r, E0 = e^{-lambda (r - z0)}, E = e^{-d (r/seff - 1)},
+// X = 1/(r^6 (1 + E)), G_n = e^{-rho_n^2/delta^2} of the two normals n, S = G_i + G_j:
+//   f on i = crad del - tp n_i - tq n_j
+//   crad = A + (C M + B) S, B = TE 2C/delta^2, tp = (n_i.del) B G_i, tq = (n_j.del) B G_j
+//   A  = [C6 X (Tap (d/seff E r^6 X - 6/r) + dTap) + (lambda Tap - dTap) E0 eps] / r
+//   TE = Tap E0,  M = (lambda Tap - dTap) E0 / r,  U = -C6 X Tap + eps TE
+//   energies: vdW U - eps TE, repulsion V_ij + V_ji = TE (eps + C S)
+// A, M, U and TE depend on q and the element pair alone, A = -2 dU/dq and M = -2 dTE/dq.
+// They are tabulated per potential: 2^TAB_BITS intervals per factor of two in q; on each,
+// A and M are polynomials of degree 4 in q about the interval's centre (Chebyshev
+// interpolation of FP64 values, the interpolation error below 2e-14 of the function where
+// it is steepest and 1e-15 over most of the range), U and TE their integrals from the FP64
+// values at the centre.  A takes 26 FP32 instructions, where square root, taper, two
+// exponentials and the divisions of it take about 290 in double-float arithmetic; two
+// 16-byte loads bring its coefficients, since the gathers of the tables load the L1 pipe
+// (degree 6 over half as many intervals, three loads: the pipe 76 % busy and the kernel
+// no faster than the direct evaluation).
+//
+// The part the normals enter is left out for lanes whose pairs lie so far sideways
+// (rho > 8 A for carbon) that G_n < 2^-64: S is then below a double's rounding of the rest.
 #pragma once
 
 #include "dfloat.cuh"
@@ -14,95 +35,136 @@ enum PairK {
   K_C = 2,        // C
   K_EPS = 4,      // epsilon (both repulsion terms' halves together)
   K_C2D = 6,      // 2 C / delta^2
-  K_LAM = 8,      // lambda
-  K_LAM2 = 10,    // lambda log2(e)
-  K_Z0 = 12,
-  K_TSA = 14,     // (d / seff) log2(e)
-  K_SEFF = 16,
-  K_C6 = 18,
-  K_DOS = 20,     // d / seff
-  K_N = 22
+  K_N = 8
 };
-// per potential constants
-struct PairG {
-  float irc_h, irc_l;        // 1 / r_cut
-  float dt_h, dt_l;          // -140 / r_cut
-  float cut_h, cut_l;        // r_cut^2
+
+constexpr float Q_MIN = 0.25f;          // A^2: the tables' range, [Q_MIN, Q_MAX)
+constexpr float Q_MAX = 1024.f;
+constexpr int TAB_BITS = 9;             // mantissa bits of q that select an interval
+constexpr int TAB_SHIFT = 23 - TAB_BITS;
+constexpr int TAB_BASE = (127 - 2) << TAB_BITS;          // of Q_MIN = 2^-2
+constexpr int TAB_N = 12 << TAB_BITS;                    // 12 octaves
+
+// the parameters of one element pair, for the tables
+struct TabP {
+  double z0, lambda, eps, d, seff, C6, cut;
   int tap;
 };
+// A, M, U and TE at q in FP64
+static __device__ inline void tab_functions(const TabP &p, double q, double &A, double &M, double &U, double &TE) {
+  const double r = sqrt(q), ri = 1.0 / r;
+  double Tap = 1.0, dTap = 0.0;
+  if (p.tap) {
+    const double x = r / p.cut, y = 1.0 - x, xy = x * y;
+    Tap = (y * y) * (y * y) * (1.0 + x * (4.0 + x * (10.0 + x * 20.0)));
+    dTap = -140.0 / p.cut * (xy * xy * xy);
+  }
+  const double E = exp(-p.d * (r / p.seff - 1.0)), E0 = exp(-p.lambda * (r - p.z0));
+  const double c = p.C6 / (q * q * q * (1.0 + E));
+  M = (p.lambda * Tap - dTap) * E0 * ri;
+  A = ri * (c * (Tap * (p.d / p.seff * (E / (1.0 + E)) - 6.0 * ri) + dTap)) + M * p.eps;
+  TE = Tap * E0;
+  U = p.eps * TE - c * Tap;
+}
+// interval k's coefficients: of A and M c0, c1, c2 (hi, lo), c3, c4, and U and TE at the centre
+static __device__ inline void tab_fill(const TabP &p, int k, float ca[8], float cm[8], float u[2], float te[2]) {
+  const double lo = ldexp(1.0 + (k & ((1 << TAB_BITS) - 1)) / (double)(1 << TAB_BITS), (k >> TAB_BITS) - 2);
+  const double half = 0.5 * ldexp(1.0, (k >> TAB_BITS) - 2 - TAB_BITS), mid = lo + half;
+  double v[2][5], U, TE;
+  for (int j = 0; j < 5; j++) tab_functions(p, mid + half * cos(M_PI * (2 * j + 1) / 10.0), v[0][j], v[1][j], U, TE);
+  for (int f = 0; f < 2; f++) {
+    double a[5];
+    for (int m = 0; m < 5; m++) {
+      double s = 0.0;
+      for (int j = 0; j < 5; j++) s += v[f][j] * cos(M_PI * (m * (2 * j + 1)) / 10.0);
+      a[m] = s * (m ? 0.4 : 0.2);
+    }
+    // Chebyshev to powers of (q - mid) / half, then of q - mid
+    const double c[5] = {a[0] - a[2] + a[4], a[1] - 3.0 * a[3], 2.0 * a[2] - 8.0 * a[4], 4.0 * a[3], 8.0 * a[4]};
+    float *o = f ? cm : ca;
+    double w = 1.0;
+    for (int m = 0; m < 5; m++, w /= half) {
+      const float h = (float)(c[m] * w);
+      if (m < 3) {
+        o[2 * m] = h;
+        o[2 * m + 1] = (float)(c[m] * w - (double)h);
+      } else {
+        o[3 + m] = h;
+      }
+    }
+  }
+  double a, m;
+  tab_functions(p, mid, a, m, U, TE);
+  u[0] = (float)U;
+  u[1] = (float)(U - (double)u[0]);
+  te[0] = (float)TE;
+  te[1] = (float)(TE - (double)te[0]);
+}
 
+// interval of q.h (in [Q_MIN, Q_MAX)) and q.h minus its centre (exact)
+static __device__ __forceinline__ int tab_at(float qh, float &t) {
+  const int u = __float_as_int(qh);
+  t = __fsub_rn(qh, __int_as_float((u & ~((1 << TAB_SHIFT) - 1)) | (1 << (TAB_SHIFT - 1))));
+  return (u >> TAB_SHIFT) - TAB_BASE;
+}
+// one interval's coefficients
 template <class V>
-struct PairOut {
-  D<V> crad;      // radial factor of the pair force: f = crad del - tp n_i - tq n_j
-  D<V> tp, tq;    // Tap (n . del) fpair1 of the two repulsion terms
-  D<V> evdw, erep;   // Tap V_vdw and Tap (V_ij + V_ji) (EV)
+struct Coef {
+  V c0h, c0l, c1h, c1l, c2h, c2l, c3, c4;
 };
+static __device__ __forceinline__ void coef_set(Coef<float> &o, const float4 *a) {
+  const float4 x = __ldg(a), y = __ldg(a + 1);
+  o.c0h = x.x; o.c0l = x.y; o.c1h = x.z; o.c1l = x.w;
+  o.c2h = y.x; o.c2l = y.y; o.c3 = y.z; o.c4 = y.w;
+}
+// the polynomial at t (normalised).  |t| is below 2^-TAB_BITS-1 of q, so the terms fall off
+// by ~2^-7 each and FP32 serves from the third power on
+template <class V>
+static __device__ __forceinline__ D<V> tab_poly(const Coef<V> &c, D<V> t) {
+  D<V> s = mul(mk(c.c2h, vfma(vfma(c.c4, t.h, c.c3), t.h, c.c2l)), t);
+  const D<V> s1 = two_sum(c.c1h, s.h);
+  s = mul(mk(s1.h, vadd(s1.l, vadd(s.l, c.c1l))), t);
+  const D<V> s0 = two_sum(c.c0h, s.h);
+  return mk(s0.h, vadd(s0.l, vadd(s.l, c.c0l)));
+}
+// f0 - 1/2 the integral of the polynomial from 0 to t
+template <class V>
+static __device__ __forceinline__ D<V> tab_integral(const Coef<V> &c, V f0h, V f0l, D<V> t) {
+  const V half = vall<V>(0.5f);
+  V u = vfma(vmul(c.c4, vall<V>(0.2f)), t.h, vmul(c.c3, vall<V>(0.25f)));
+  u = vfma(u, t.h, vmul(c.c2h, vall<V>(1.f / 3.f)));
+  D<V> s = mul(mk(vmul(half, c.c1h), vfma(u, t.h, vmul(half, c.c1l))), t);
+  const D<V> s1 = two_sum(c.c0h, s.h);
+  s = scale(mul(mk(s1.h, vadd(s1.l, vadd(s.l, c.c0l))), t), vall<V>(-0.5f));
+  const D<V> s0 = two_sum(f0h, s.h);
+  return mk(s0.h, vadd(s0.l, vadd(s.l, f0l)));
+}
 
-// del: x_i - x_j; q = |del|^2; pn = n_i . del, qn = n_j . del; on: 1 for a pair that counts
-// (0 zeroes every output); K(k): constant k; tab: the exp2 table.  W (subdomain mode):
-// weights wv of the vdW pair, wi and wj of the repulsion terms with n_i and n_j.
-template <bool EV, bool W, class V, class KF>
-static __device__ __forceinline__ void pair_terms(const PairG &g, KF K, const float2 *tab, D<V> q, D<V> pn, D<V> qn,
-                                                  V on, V wv, V wi, V wj, PairOut<V> &o) {
+// whether G_n of a pair can matter: log2 G_n above FAR_EXP for either normal, in FP32
+constexpr float FAR_EXP = -64.f;
+static __device__ __forceinline__ bool near_one(float nd2, float q, float p1, float p2) {
+  return nd2 * (q - p1 * p1) > FAR_EXP || nd2 * (q - p2 * p2) > FAR_EXP;
+}
+
+// The parts the normals enter: crad += (C M + B) S, tp, tq, and S (weighted).  pn = n_i .
+// del, qn = n_j . del; K(k): constant k; tab: the exp2 table.  W (subdomain mode): weights
+// wi and wj of the repulsion terms with n_i and n_j.
+template <bool W, class V, class KF>
+static __device__ __forceinline__ void pair_near(KF K, const float2 *tab, D<V> q, D<V> TE, D<V> M, D<V> pn, D<V> qn, V wi,
+                                                 V wj, D<V> &crad, D<V> &tp, D<V> &tq, D<V> &S) {
   auto KD = [&](int k) { return mk<V>(K(k), K(k + 1)); };
-  D<V> r, ri;
-  sqrt_rsqrt(q, r, ri);
-  // taper (pair_ilp_graphene_hbn.h:80-115) in y = 1 - x, x = r / r_cut: its degree-7
-  // polynomial is y^4 (1 + 4x + 10x^2 + 20x^3), all terms positive, and
-  // dTap/dr = -140 (x y)^3 / r_cut
-  D<V> Tap = mk(on, vall<V>(0.f)), dTap = mk(vall<V>(0.f), vall<V>(0.f));
-  if (g.tap) {
-    const D<V> x = mul(r, mk(vall<V>(g.irc_h), vall<V>(g.irc_l)));
-    const V one = vall<V>(1.f);
-    const V s = vsub(one, x.h);
-    const D<V> y = mk(s, vsub(vsub(vsub(one, s), x.h), x.l));
-    const V c20 = vall<V>(20.f);
-    const V u = vmul(c20, x.h);
-    D<V> p = add1(mk(u, vfma(c20, x.l, vfma(c20, x.h, vneg(u)))), vall<V>(10.f));
-    p = add1(mul(x, p), vall<V>(4.f));
-    p = renorm(add1(mul(x, p), one));
-    const D<V> y2 = sqr(y), xy = mul(x, y);
-    Tap = renorm(mul(sqr(renorm(y2)), p));
-    dTap = mul(renorm(mul(sqr(xy), xy)), mk(vall<V>(g.dt_h), vall<V>(g.dt_l)));
-    Tap = mk(vmul(Tap.h, on), vmul(Tap.l, on));
-    dTap = mk(vmul(dTap.h, on), vmul(dTap.l, on));
-  }
-  const D<V> DR = renorm(mul(dTap, ri));
-  // ---- vdW: -C6 r^-6 / TS, TS = 1 + E, E = exp(-d (r / seff - 1)); 1 - 1/TS = E / TS
-  const D<V> ri2 = sqr(ri);
-  const D<V> rm = neg(r);
-  const D<V> E = exp2(mul(add(KD(K_SEFF), rm), KD(K_TSA)), tab);
-  const D<V> TSi = rcp(renorm(add1(E, vall<V>(1.f))));
-  D<V> c6r6 = mul(renorm(mul(sqr(renorm(ri2)), ri2)), mul(TSi, KD(K_C6)));   // -V
-  c6r6 = renorm(c6r6);
-  if constexpr (W) c6r6 = mk(vmul(c6r6.h, wv), vmul(c6r6.l, wv));
-  const D<V> G = add1(mul(renorm(mul(E, TSi)), mul(r, KD(K_DOS))), vall<V>(-6.f));
-  // fpv Tap - V dTap / r = c6r6 (G Tap / r^2 + DR)
-  const D<V> TR2 = mul(Tap, ri2);
-  D<V> fv = mul(c6r6, renorm(add(mul(renorm(G), renorm(TR2)), DR)));
-  // ---- repulsion of the terms with n_i and n_j: E0 (eps/2 + C e^{-rho^2/delta^2})
-  const D<V> E0 = renorm(exp2(mul(add(KD(K_Z0), rm), KD(K_LAM2)), tab));
-  const D<V> rho1 = renorm(add_ordered(q, neg(sqr(pn)))), rho2 = renorm(add_ordered(q, neg(sqr(qn))));
-  D<V> F1 = mul(E0, exp2(mul(rho1, KD(K_ND2)), tab));
-  D<V> F2 = mul(E0, exp2(mul(rho2, KD(K_ND2)), tab));
-  D<V> Ee = mul(E0, KD(K_EPS));
+  const D<V> rho1 = add_ordered(q, neg(sqr(pn))), rho2 = add_ordered(q, neg(sqr(qn)));
+  D<V> G1 = exp2(mul(renorm(rho1), KD(K_ND2)), tab);
+  D<V> G2 = exp2(mul(renorm(rho2), KD(K_ND2)), tab);
   if constexpr (W) {
-    F1 = mk(vmul(F1.h, wi), vmul(F1.l, wi));
-    F2 = mk(vmul(F2.h, wj), vmul(F2.l, wj));
-    const V wm = vmul(vall<V>(0.5f), vadd(wi, wj));
-    Ee = mk(vmul(Ee.h, wm), vmul(Ee.l, wm));
+    G1 = scale(G1, wi);
+    G2 = scale(G2, wj);
   }
-  const D<V> S = renorm(add(F1, F2));
-  const D<V> VS = renorm(add(Ee, mul(S, KD(K_C))));
-  const D<V> TC = renorm(mul(Tap, KD(K_C2D)));   // Tap 2 C / delta^2
-  const D<V> LT = add(mul(mul(Tap, ri), KD(K_LAM)), neg(DR));
-  o.crad = renorm(add(fv, add(mul(S, TC), mul(VS, renorm(LT)))));
-  o.tp = renorm(mul(mul(pn, TC), F1));
-  o.tq = renorm(mul(mul(qn, TC), F2));
-  if constexpr (EV) {
-    o.evdw = neg(mul(c6r6, Tap));
-    o.erep = mul(VS, Tap);
-  }
+  S = renorm(add(G1, G2));
+  const D<V> B = renorm(mul(TE, KD(K_C2D)));
+  tp = mul(mul(pn, B), G1);
+  tq = mul(mul(qn, B), G2);
+  crad = add(crad, mul(S, renorm(add(mul(M, KD(K_C)), B))));
 }
 
 }  // namespace df
