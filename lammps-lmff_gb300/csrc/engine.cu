@@ -124,7 +124,8 @@ __device__ __forceinline__ void block_max_disp(double d2, unsigned long long *ma
 // hand unwrapped coordinates, or coordinates it just wrapped): the list's image codes
 // stay valid and an atom that crossed the box edge is not a displacement.
 __global__ void k_update_x(int n, const int *perm, const double *x, d4 *xq, const double *xhold,
-                           unsigned long long *maxdisp, const SysDesc *sys, const int *sysid) {
+                           unsigned long long *maxdisp, const SysDesc *sys, const int *sysid, float4 *xh,
+                           float4 *xl) {
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   double d2 = 0.0;
   if (q < n) {
@@ -136,6 +137,7 @@ __global__ void k_update_x(int n, const int *perm, const double *x, d4 *xq, cons
     if (sd.per[1]) b -= sd.L[1] * rint((b - xhold[3 * q + 1]) / sd.L[1]);
     if (sd.per[2]) c -= sd.L[2] * rint((c - xhold[3 * q + 2]) / sd.L[2]);
     xq[q] = make_d4(a, b, c, w.w);
+    hilo_split(q, a, b, c, sd, xh, xl);
     double dx = a - xhold[3 * q], dy = b - xhold[3 * q + 1], dz = c - xhold[3 * q + 2];
     d2 = dx * dx + dy * dy + dz * dz;
   }
@@ -261,7 +263,7 @@ struct Lookahead {
 // double-float split and tracks the displacement since the last build
 __global__ void k_nve1(int n, d4 *xq, double *v, const double *f, DtfmTab tab, double dtv,
                        const double *xhold, unsigned long long *maxdisp, const SysDesc *sys, const int *sysid,
-                       float4 *xh, float4 *xl, int do_hilo, cudaGraphConditionalHandle h = 0, double trig2 = 0.0,
+                       float4 *xh, float4 *xl, cudaGraphConditionalHandle h = 0, double trig2 = 0.0,
                        unsigned *ticket = nullptr, Lookahead la = Lookahead{}) {
   int q = blockIdx.x * blockDim.x + threadIdx.x;
   double d2 = 0.0, p2 = 0.0;
@@ -273,7 +275,7 @@ __global__ void k_nve1(int n, d4 *xq, double *v, const double *f, DtfmTab tab, d
     double vy = v[n + q] + dtfm * fy;
     double vz = v[2 * n + q] + dtfm * fz;
     v[q] = vx; v[n + q] = vy; v[2 * n + q] = vz;
-    d2 = nve_drift(q, vx, vy, vz, dtv, xq, xhold, xh, xl, sys, sysid, do_hilo);
+    d2 = nve_drift(q, vx, vy, vz, dtv, xq, xhold, xh, xl, sys, sysid);
     if (la.pred) {
       const double p = sqrt(d2) + la.hv * sqrt(vx * vx + vy * vy + vz * vz) +
                        la.ha * fabs(dtfm) * sqrt(fx * fx + fy * fy + fz * fz);
@@ -1412,6 +1414,7 @@ struct Engine {
     if (st) return status_error(st);
     update_stride(maxcnt);
     built = true;
+    hilo_fresh = true;   // of the wrapped, sorted positions
     forces_valid = false;
     rebuilds++;
     return LMFF_OK;
@@ -1564,14 +1567,18 @@ struct Engine {
     // kernels are timed one by one.
     const bool fork = a.do_ters && a.do_ilp && ters_concurrent && !ktiming && ensure_stream2() == LMFF_OK;
     a.ters_alone = !fork;
-    // the normal frames (the g-independent part of the normal-derivative assembly) on a
-    // third stream, beside both
+    // the normal frames (the g-independent part of the normal-derivative assembly): mixed on
+    // a third stream, beside both; FP64 ahead of the pair kernel, which takes its normals
+    // from them
+    constexpr bool FRAME_FIRST = sizeof(R) == 8;
     if (fork) {
       cudaEventRecord(ev_fork, stream);
       cudaStreamWaitEvent(stream2, ev_fork, 0);
-      cudaStreamWaitEvent(stream3, ev_fork, 0);
-      fr(a, stream3);
-      cudaEventRecord(ev_frame, stream3);
+      if constexpr (!FRAME_FIRST) {
+        cudaStreamWaitEvent(stream3, ev_fork, 0);
+        fr(a, stream3);
+        cudaEventRecord(ev_frame, stream3);
+      }
       ft(a, ev, eatom, stream2);
       cudaEventRecord(ev_join, stream2);
     } else if (a.do_ters) {
@@ -1580,9 +1587,9 @@ struct Engine {
       cudaMemsetAsync(stat_ters, 0, sizeof(double) * 8 * (size_t)n, stream);
     }
     if (a.do_ilp) {
-      if (!fork) timed(6, [&] { fr(a, stream); });
+      if (!fork || FRAME_FIRST) timed(6, [&] { fr(a, stream); });
       timed(0, [&] { fi(a, ev, eatom, tpa, block, i_one, stream); });
-      if (fork) cudaStreamWaitEvent(stream, ev_frame, 0);
+      if (fork && !FRAME_FIRST) cudaStreamWaitEvent(stream, ev_frame, 0);
       timed(6, [&] { fn(a, ev, stream); });
     }
     else if (ev) cudaMemsetAsync(stat_ilp, 0, sizeof(double) * 8 * (size_t)n, stream);
@@ -1607,7 +1614,7 @@ struct Engine {
     cudaEventCreate(&e1);
     cudaEventRecord(e0, stream);
     if (n > 0) {
-      if (precision == LMFF_MIXED && !hilo_fresh) hilo_all();
+      if (!hilo_fresh) hilo_all();
       const bool cap = use_graphs && !ktiming && !kick_on;
       std::vector<unsigned char> key;
       if (cap) {
@@ -1782,14 +1789,11 @@ struct Engine {
       return load_from_staging(nn, false, false);
     }
     if (nn > 0) {
-      k_update_x<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, d_xin, d.xq, d.xhold, d.maxdisp, d.sys, d.sysid);
+      k_update_x<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, d_xin, d.xq, d.xhold, d.maxdisp, d.sys, d.sysid, d.xh,
+                                                       d.xl);
       CK(cudaGetLastError());
     }
-    hilo_fresh = false;
-    if (precision == LMFF_MIXED) {
-      hilo_all();
-      hilo_fresh = true;
-    }
+    hilo_fresh = true;   // k_update_x made the split too
     return test ? maybe_rebuild() : LMFF_OK;
   }
 
@@ -2249,7 +2253,6 @@ struct Engine {
     DtfmTab t = dtfm_table(dtf);
     for (int k = 0; k <= MAXTYPE; k++) kick_args.dtfm[k] = t.v[k];
     kick_args.drift = 0;
-    kick_args.do_hilo = precision == LMFF_MIXED;
     kick_args.dtv = dt;
     kick_args.trig2 = 0.25 * skin * skin;
     kick_args.xq = d.xq;
@@ -2330,7 +2333,6 @@ struct Engine {
   // sets the condition of an IF node holding the rebuild) when check, the others steps
   // between checks, whose first half the previous step's gather makes (no k_nve1).
   int capture_steps(double dt, double dtf, int nsteps, bool check, cudaGraphExec_t *out) {
-    const bool mixed = precision == LMFF_MIXED;
     const double trig2 = 0.25 * skin * skin;
     cudaGraph_t g = nullptr;
     CK(cudaGraphCreate(&g, 0));
@@ -2341,7 +2343,7 @@ struct Engine {
       const bool chk = check && s == 0;
       if (s == 0)
         k_nve1<<<(n + per_atom_block(n) - 1) / per_atom_block(n), per_atom_block(n), 0, stream>>>(n, d.xq, d.v, d.f, dtfm_table(dtf), dt, d.xhold, d.maxdisp, d.sys,
-                                                    d.sysid, d.xh, d.xl, mixed ? 1 : 0, h, trig2,
+                                                    d.sysid, d.xh, d.xl, h, trig2,
                                                     chk ? d_cond_ticket : nullptr, lookahead_for(chk, true, dt));
       kick_args.drift = s + 1 < nsteps;
       if (chk) {
@@ -2432,7 +2434,7 @@ struct Engine {
     CK(cudaMemcpyAsync(&nrb, d_graph_rebuilds, sizeof nrb, cudaMemcpyDeviceToHost, stream));
     CK(cudaMemsetAsync(d_graph_rebuilds, 0, sizeof nrb, stream));
     CK(cudaStreamSynchronize(stream));
-    hilo_fresh = precision == LMFF_MIXED;
+    hilo_fresh = true;
     if (st & (ST_LIST_OVERFLOW | ST_SHORT_OVERFLOW | ST_SKIN_TRIP)) {
       // redo the chunk on the eager path, which grows the list as needed and rebuilds at
       // any step an atom moved more than skin/2
@@ -2461,15 +2463,14 @@ struct Engine {
   int run_steps_eager(int nsteps, double dt) {
     double dtf = 0.5 * dt * FTM2V;
     for (int s = 1; s <= nsteps; s++) {
-      bool mixed = precision == LMFF_MIXED;
       const bool chk = check_step(steps);
       timed(4, [&] {
         k_nve1<<<(n + per_atom_block(n) - 1) / per_atom_block(n), per_atom_block(n), 0, stream>>>(n, d.xq, d.v, d.f, dtfm_table(dtf), dt, d.xhold, d.maxdisp, d.sys,
-                                                    d.sysid, d.xh, d.xl, mixed ? 1 : 0, 0, 0.0, nullptr,
+                                                    d.sysid, d.xh, d.xl, 0, 0.0, nullptr,
                                                     lookahead_for(chk, false, dt));
       });
       CK(cudaGetLastError());
-      hilo_fresh = mixed;
+      hilo_fresh = true;
       int rc = maybe_rebuild(chk && ck > 1);
       if (rc) return rc;
       set_kick(dtf);   // after any rebuild: it may have moved d.v
@@ -2551,13 +2552,12 @@ struct Engine {
         if (rc) return rc;
       }
       if (th_at_end) {
-        bool mixed = precision == LMFF_MIXED;
         const bool chk = check_step(steps);
         k_nve1<<<(n + per_atom_block(n) - 1) / per_atom_block(n), per_atom_block(n), 0, stream>>>(n, d.xq, d.v, d.f, dtfm_table(dtf), dtv, d.xhold, d.maxdisp, d.sys,
-                                                    d.sysid, d.xh, d.xl, mixed ? 1 : 0, 0, 0.0, nullptr,
+                                                    d.sysid, d.xh, d.xl, 0, 0.0, nullptr,
                                                     lookahead_for(chk, false, dt));
         CK(cudaGetLastError());
-        hilo_fresh = mixed;
+        hilo_fresh = true;
         rc = maybe_rebuild(chk && ck > 1);
         if (rc) return rc;
         rc = forces(LMFF_TERSOFF | LMFF_ILP, true, false, &hr);
@@ -3216,6 +3216,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     if (a.do_ters) f64::launch_tersoff(a, ev, false, st);
     else CK2(cudaMemsetAsync(stat_ters, 0, sizeof(double) * 8 * (size_t)nn, st));
     if (a.do_ilp) {
+      f64::launch_nframe(a, st);
       f64::launch_ilp(a, ev, false, g.tpa, g.block, g.i_one, st);
       f64::launch_nderiv(a, ev, st);
     } else {

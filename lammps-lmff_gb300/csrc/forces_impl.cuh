@@ -50,18 +50,27 @@ __device__ __forceinline__ R rsqR(R dx, R dy, R dz) {
   else return dx * dx + dy * dy + dz * dz;
 }
 
-// rsq < thr decided exactly as FP64 would (mixed: FP32 first, FP64 when within 1e-5)
-__device__ __forceinline__ bool lt_exact(R rsq, R thr, const d4 *xq, const SysDesc &sd, int i, int j, int sx,
+// rsq < thr decided exactly as FP64 would (FP32 first, FP64 when within 1e-5)
+__device__ __forceinline__ bool lt_exact(float rsq, float thr, const d4 *xq, const SysDesc &sd, int i, int j, int sx,
                                          int sy, int sz, double thr64) {
+  float m = 1e-5f * thr;
+  if (rsq < thr - m) return true;
+  if (rsq > thr + m) return false;
+  double dx, dy, dz;
+  disp64(xq, sd, i, j, sx, sy, sz, dx, dy, dz);
+  return rsq_rn(dx, dy, dz) < thr64;
+}
+// rsq = 0 as the mode's own distance says it: the mixed mode's FP32 one, the FP64 mode's
+// FP64 one (taken only for pairs closer than 1e-3 A)
+__device__ __forceinline__ bool same_place(float rsq, const d4 *xq, const SysDesc &sd, int i, int j, int sx, int sy,
+                                           int sz) {
   if constexpr (sizeof(R) == 8) {
-    return rsq < thr;
-  } else {
-    float m = 1e-5f * thr;
-    if (rsq < thr - m) return true;
-    if (rsq > thr + m) return false;
+    if (rsq > 1e-6f) return false;
     double dx, dy, dz;
     disp64(xq, sd, i, j, sx, sy, sz, dx, dy, dz);
-    return rsq_rn(dx, dy, dz) < thr64;
+    return rsq_rn(dx, dy, dz) == 0.0;
+  } else {
+    return rsq == 0.f;
   }
 }
 
@@ -100,7 +109,11 @@ __device__ __forceinline__ void df_record(const ForceArgs<double> &a, const SysD
 // Per atom: the current-step ILP intralayer list (ILP_neigh, pair_ilp_graphene_hbn.cpp:
 // 723-743: same molecule, rsq != 0, rsq < cutILPsq) and the Tersoff short list
 // (pair_tersoff.cpp:132-147: rsq < cutmax^2), both taken in candidate order from the
-// short candidate list built with skin; then the unit normal (calc_normal :776-1074).
+// short candidate list built with skin; then, in the mixed mode, the unit normal
+// (calc_normal :776-1074).  The distances are FP32 ones of the double-float position
+// parts in both modes, decided in FP64 near a cutoff.  In FP64 the normal comes from
+// k_frame: here one lane of an atom's SG would issue its ~120 FP64 instructions for a
+// whole warp (7,200 atoms: 44 us with FP64 distances and normals, 9.5 us and 4 us for k_frame; 331,200 atoms: 540 -> 80 + 40 us).
 // SG lanes per atom share its short candidates.  Each round the lanes test one
 // candidate each; ballots over the atom's lanes give every accepted entry its position
 // in candidate order, so the lists equal a one-lane walk's, and the bond vectors of the
@@ -121,37 +134,39 @@ __global__ void k_short(ForceArgs<R> a, const double *cutILPsq64, double tcutmax
   const unsigned gmask = SG == 1 ? 0u : ((1u << SG) - 1) << (wl & ~(SG - 1));
   const unsigned below = gmask & ((1u << wl) - 1);
   const SysDesc &sd = a.A.sys[a.A.sysid[i]];
-  AtomI<R> ai;
+  AtomI<float> ai;
   ai.load(a.A, i);
   int ti = info_type(ai.info);
   long long mi = info_mol(ai.info);
   int ie = c_pot.i_enabled ? c_pot.i_map[ti] : -1;
   int te = c_pot.t_enabled ? c_pot.t_map[ti] : -1;
   int nilp = 0, nters = 0;   // the same in every lane of the atom
+#ifdef LMFF_PACKED_X2
   R vx[MAXILP], vy[MAXILP], vz[MAXILP];
+#endif
   const int cnt = a.short_cnt[i];
   for (int c0 = 0; c0 < cnt; c0 += SG) {
     const int c = c0 + (wl & (SG - 1));
     bool take_ilp = false, take_ters = false;
     uint32_t e = 0;
-    R dx = 0, dy = 0, dz = 0;
+    float dx = 0, dy = 0, dz = 0;
     if (c < cnt) {
       e = a.short_nb[(size_t)i * MAXSHORT + c];
       int j, sx, sy, sz;
       decode_entry(e, a.lc, j, sx, sy, sz);
       long long jinfo;
       ai.disp(a.A, sd, j, sx, sy, sz, dx, dy, dz, jinfo);
-      R rsq = rsqR(dx, dy, dz);
+      const float rsq = dx * dx + dy * dy + dz * dz;
       int tj = info_type(jinfo);
       if (ie >= 0 && info_mol(jinfo) == mi) {
         int je = c_pot.i_map[tj];
-        if (je >= 0 && rsq != R(0)) {
+        if (je >= 0 && !same_place(rsq, a.A.xq, sd, i, j, sx, sy, sz)) {
           int pe = ie * MAXELEM + je;
-          take_ilp = lt_exact(rsq, c_pot.i_cutILPsq[pe], a.A.xq, sd, i, j, sx, sy, sz, cutILPsq64[pe]);
+          take_ilp = lt_exact(rsq, (float)c_pot.i_cutILPsq[pe], a.A.xq, sd, i, j, sx, sy, sz, cutILPsq64[pe]);
         }
       }
       if (te >= 0 && c_pot.t_map[tj] >= 0)
-        take_ters = lt_exact(rsq, c_pot.t_cutmaxsq, a.A.xq, sd, i, j, sx, sy, sz, tcutmaxsq64);
+        take_ters = lt_exact(rsq, (float)c_pot.t_cutmaxsq, a.A.xq, sd, i, j, sx, sy, sz, tcutmaxsq64);
     }
     unsigned bi, bt;
     if constexpr (SG == 1) {
@@ -169,6 +184,7 @@ __global__ void k_short(ForceArgs<R> a, const double *cutILPsq64, double tcutmax
       const int pos = nters + __popc(bt & below);
       if (pos < MAXTERS) a.ters_nb[(size_t)i * MAXTERS + pos] = e;
     }
+#ifdef LMFF_PACKED_X2
     // constant indices keep the bond vectors in registers
 #pragma unroll
     for (int q = 0; q < MAXILP; q++) {
@@ -187,6 +203,7 @@ __global__ void k_short(ForceArgs<R> a, const double *cutILPsq64, double tcutmax
         }
       }
     }
+#endif
     nilp += __popc(bi);
     nters += __popc(bt);
   }
@@ -201,6 +218,7 @@ __global__ void k_short(ForceArgs<R> a, const double *cutILPsq64, double tcutmax
   }
   a.ilp_cnt[i] = nilp;
   a.ters_cnt[i] = nters;
+#ifdef LMFF_PACKED_X2   // FP64: k_frame
   // unit normal
   R nx = 0, ny = 0, nz = 1;
   if (nilp >= 2) {
@@ -224,7 +242,6 @@ __global__ void k_short(ForceArgs<R> a, const double *cutILPsq64, double tcutmax
       nx = n1x / nn; ny = n1y / nn; nz = n1z / nn;
     }
   }
-#ifdef LMFF_PACKED_X2
   a.nrm32[i] = make_float4(nx, ny, nz, 0.f);
   a.jrec[3 * (size_t)i] = make_float4(ai.hx, ai.hy, ai.hz, __int_as_float((int)ai.info));
   a.jrec[3 * (size_t)i + 1] = make_float4(ai.lx, ai.ly, ai.lz, 0.f);
@@ -232,9 +249,6 @@ __global__ void k_short(ForceArgs<R> a, const double *cutILPsq64, double tcutmax
   a.jrec2[2 * (size_t)i] = make_float4(ai.hx, ai.hy, ai.hz, __uint_as_float(h2_bits(__floats2half2_rn(ai.lx, ai.ly))));
   a.jrec2[2 * (size_t)i + 1] = make_float4(
       nx, ny, nz, __uint_as_float((h2_bits(__floats2half2_rn(ai.lz, 0.f)) & 0xffffu) | ((unsigned)(ie & 0xffff) << 16)));
-#else
-  a.nrm64[i] = make_d4(nx, ny, nz, 0.0);
-  if (a.pair_df) df_record(a, sd, i, ai.x, ai.y, ai.z, nx, ny, nz, ie);
 #endif
 }
 
@@ -2489,8 +2503,13 @@ __device__ __forceinline__ void nframe_eval(const ForceArgs<R> &a, int i, NFrame
     const double nn2 = n1x * n1x + n1y * n1y + n1z * n1z;
     if (nn2 > 0.0) {
       double inn;
-      if constexpr (sizeof(R) == 4) inn = nn2 > 1e-30 ? rsqrt_nr(nn2) : 1.0 / sqrt(nn2);
-      else inn = 1.0 / sqrt(nn2);
+      if (nn2 > 1e-30 && nn2 < 1e30) {
+        inn = rsqrt_nr(nn2);
+        // FP64 mode: a second Newton step, to the rounding of a double
+        if constexpr (sizeof(R) == 8) inn = fma(0.5 * inn, fma(-(nn2 * inn), inn, 1.0), inn);
+      } else {
+        inn = 1.0 / sqrt(nn2);
+      }
       fr.ok = true;
       fr.inn = inn;
       fr.nx = n1x * inn; fr.ny = n1y * inn; fr.nz = n1z * inn;
@@ -2571,6 +2590,36 @@ __device__ __forceinline__ void nderiv_eval(const ForceArgs<R> &a, int i, NDeriv
   nderiv_apply<EV>(fr, a.ilp_g[i], o);
 }
 
+#ifndef LMFF_PACKED_X2
+// FP64 mode: the frame with the unit normal it carries (calc_normal :776-1074: (0, 0, 1) for
+// fewer than two intralayer neighbours) and the double-float pair kernel's record, one
+// thread per atom on full warps
+__global__ void __launch_bounds__(128) k_frame(ForceArgs<R> a) {
+  pdl_enter(a.pdl);
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.n) return;
+  NFrame fr;
+  nframe_eval(a, i, fr);
+  if (fr.cont >= 2 && !fr.ok) raise_status(a.status, ST_ZERO_NORMAL);
+  if (a.nframe) {
+    d4 *q = a.nframe + 4 * (size_t)i;
+    q[0] = make_d4(fr.nx, fr.ny, fr.nz, fr.inn);
+    q[1] = make_d4(fr.v[0][0], fr.v[0][1], fr.v[0][2], (double)fr.cont);
+    q[2] = make_d4(fr.v[1][0], fr.v[1][1], fr.v[1][2], fr.ok ? 1.0 : 0.0);
+    q[3] = make_d4(fr.v[2][0], fr.v[2][1], fr.v[2][2], 0.0);
+  }
+  if (!fr.ok) {
+    fr.nx = fr.ny = 0.0;
+    fr.nz = 1.0;
+  }
+  a.nrm64[i] = make_d4(fr.nx, fr.ny, fr.nz, 0.0);
+  if (a.pair_df) {
+    const d4 x = a.A.xq[i];
+    df_record(a, a.A.sys[a.A.sysid[i]], i, x.x, x.y, x.z, fr.nx, fr.ny, fr.nz,
+              c_pot.i_map[info_type(__double_as_longlong(x.w))]);
+  }
+}
+#else
 __global__ void k_nframe(ForceArgs<R> a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
@@ -2582,6 +2631,7 @@ __global__ void k_nframe(ForceArgs<R> a) {
   q[2] = make_d4(fr.v[1][0], fr.v[1][1], fr.v[1][2], fr.ok ? 1.0 : 0.0);
   q[3] = make_d4(fr.v[2][0], fr.v[2][1], fr.v[2][2], 0.0);
 }
+#endif
 
 template <bool EV>
 __global__ void k_nderiv(ForceArgs<R> a) {
@@ -2622,8 +2672,7 @@ __device__ __forceinline__ void kick_atom(const KickArgs &kick, const ForceArgs<
   kick.v[a.n + i] = vy;
   kick.v[2 * a.n + i] = vz;
   if (kick.drift) {
-    const double d2 = nve_drift(i, vx, vy, vz, kick.dtv, kick.xq, kick.xhold, kick.xh, kick.xl, kick.sys, kick.sysid,
-                                kick.do_hilo);
+    const double d2 = nve_drift(i, vx, vy, vz, kick.dtv, kick.xq, kick.xhold, kick.xh, kick.xl, kick.sys, kick.sysid);
     if (d2 > kick.trig2) atomicOr(kick.status, ST_SKIN_TRIP);
   }
 }
@@ -3697,9 +3746,13 @@ void launch_ilp(const ForceArgs<R> &a, bool ev, bool eatom, int tpa, int block, 
 }
 
 void launch_nframe(const ForceArgs<R> &a, cudaStream_t s) {
-  if (a.n == 0 || !a.nframe) return;
+  if (a.n == 0) return;
   const int b = per_atom_block(a.n);
-  k_nframe<<<(a.n + b - 1) / b, b, 0, s>>>(a);
+#ifdef LMFF_PACKED_X2
+  if (a.nframe) k_nframe<<<(a.n + b - 1) / b, b, 0, s>>>(a);
+#else
+  launch_pdl((a.pdl & PDL_NDERIV) != 0, k_frame, (a.n + b - 1) / b, b, s, a);   // k_short is ahead on s
+#endif
 }
 
 void launch_nderiv(const ForceArgs<R> &a, bool ev, cudaStream_t s) {
@@ -3749,7 +3802,7 @@ void launch_vatom_terms(const ForceArgs<R> &a, bool ilp, bool one_element, cudaS
     else k_tersoff<false, false, false, true><<<g, 128, 0, s>>>(a);
   }
   if (a.do_ilp && ilp) {
-    k_nframe<<<g, 128, 0, s>>>(a);
+    k_frame<<<g, 128, 0, s>>>(a);
     if (a.pair_df && !a.list_full) {
       const int gl = (int)(((long long)a.n * VA_LANES + 127) / 128);
       k_va_tens_df<<<g, 128, 0, s>>>(a);
