@@ -973,10 +973,31 @@ struct Engine {
   }
   int pair_df = 0;
 
+  // the square of the smallest R - D where every Tersoff entry has lambda3 = 0, symmetric
+  // repulsion and constants whose functions stay in the FP32 exponent range (the estimates
+  // the FP64 forms start from), else 0: then only the general routine runs
+  double ters_fast_rlosq() const {
+    if (!t_on || !pot64.rep_sym) return 0.0;
+    double lo = 1e30;
+    for (int a = 0; a < pot64.t_ne; a++)
+      for (int b = 0; b < pot64.t_ne; b++)
+        for (int c = 0; c < pot64.t_ne; c++) {
+          const TersP<double> &q = pot64.ters[(a * MAXELEM + b) * MAXELEM + c];
+          if (q.lam3 != 0.0 || !(q.rlo64 > 0.1 && q.rlo64 < 10.0)) return 0.0;
+          if (!(q.d2 >= 1e-12 && q.d2 <= 1e12 && q.cd2 <= 1e15 && q.powern >= 0.3 && q.powern <= 50.0 && q.beta <= 1e6 &&
+                q.lam1 * q.rlo64 <= 300.0 && q.lam2 * q.rlo64 <= 300.0 && q.gamma <= 1e12))
+            return 0.0;
+          lo = std::min(lo, q.rlo64);
+        }
+    return lo < 1e30 ? lo * lo : 0.0;
+  }
+  double ters_rlosq = 0.0;
+
   int build_consts() {
     fill_pot(pot64);
     fill_pot(pot32);
     pair_df = pair_df_elements();
+    ters_rlosq = ters_fast_rlosq();
     memset(&nbc, 0, sizeof nbc);
     cutneigh_max = 0.0;
     double rmaxilp = 0.0;
@@ -1551,6 +1572,7 @@ struct Engine {
     a.kc = i_on && hi.model == LMFF_INTERLAYER_KC;
     a.pair_df = pair_df;
     a.jstride = cap_n;
+    a.ters_rlosq = ters_rlosq;
     // not while kernels are timed one by one (events between the launches)
     if (!ktiming && n <= PDL_MAX_ATOMS) a.pdl = pdl_short ? pdl_mask : (pdl_mask & ~PDL_SHORT);
     return a;
@@ -3207,6 +3229,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     a.kc = g.i_on && g.hi.model == LMFF_INTERLAYER_KC;
     a.pair_df = g.pair_df;
     a.jstride = c;
+    a.ters_rlosq = g.ters_rlosq;
   };
   const bool ev = true;
   if (g.precision == LMFF_FP64) {

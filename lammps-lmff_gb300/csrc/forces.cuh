@@ -331,6 +331,9 @@ struct ForceArgs {
   // potential (Engine::pair_df), 0: k_ilp.  jrec then holds its records
   int pair_df;
   int jstride;         // atoms per array of the records
+  // FP64 mode: the square of the smallest R - D of the Tersoff triplets where tersoff_fast
+  // takes the potential (Engine::ters_rlosq), else 0
+  double ters_rlosq;
   // programmatic dependent launch (PDL) of the step's chain kernels, a PDL_* mask: which
   // kernels are launched early behind the kernel before them on the stream (the pair
   // kernel, the normal-derivative kernel, the gather, and inside a step graph the

@@ -814,6 +814,226 @@ __device__ __forceinline__ void tersoff_atom(const ForceArgs<R> &a, int i, int i
   }
 }
 
+// ---- FP64 arithmetic of the plain form: the FP64 pipe runs at 1/75 of the FP32 rate, so the
+// exponentials, logarithms, square roots and divisions are written
+// with fewer FP64 instructions at full double accuracy (results within a few ulp of the
+// library functions, far inside the 1e-10 parity bar).
+//
+// e^x by Tang's table-driven method (P. T. P. Tang, ACM TOMS 15, 1989): n = rint(256 x /
+// ln2), r = x - n ln2/256 (|r| <= ln2/512; one FMA with ln2/256 rounded to double costs
+// at most |n| 2^-62 absolute in r, hence in the relative error of e^x: |n| < 2^18, so
+// below 6e-14 for |x| < 700 and below 4e-15 for |x| < 40), e^x = 2^(n>>8)
+// 2^((n&255)/256) (1 + p(r)), p the degree-4 Taylor polynomial of e^r - 1 (truncation
+// below 4e-17 relative: the 256-entry table keeps |r| small enough for degree 4, two FP64
+// FMAs fewer than degree 6 over 64 entries).  Outside |x| < 700 the library exp.
+constexpr int EXP2_F64_N = 256;
+__device__ double g_exp2_f64[EXP2_F64_N];
+
+__global__ void k_fill_exp2_f64() {
+  const int j = threadIdx.x;
+  if (j < EXP2_F64_N) g_exp2_f64[j] = exp2((double)j / EXP2_F64_N);
+}
+
+__device__ __forceinline__ double exp_t64(double x) {
+  if (!(fabs(x) < 700.0)) return exp(x);
+  const double magic = 6755399441055744.0;   // 1.5 * 2^52
+  const double tn = __dadd_rn(x * 369.3299304675746, magic);   // 256 / ln2
+  const int n = __double2loint(tn);
+  const double nd = __dsub_rn(tn, magic);
+  const double r = fma(-nd, 0.0027076061740622863, x);          // ln2 / 256
+  double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
+  p = fma(p, r, 0.5);
+  p = fma(p, r, 1.0);
+  p = p * r;
+  const double T = __ldg(&g_exp2_f64[n & (EXP2_F64_N - 1)]);
+  const double v = fma(T, p, T);
+  return __hiloint2double(__double2hiint(v) + (int)((unsigned)(n >> 8) << 20), __double2loint(v));
+}
+
+// 1/sqrt(x), 1/x: FP32 estimates (relative error ~2^-22) and one FP64 Newton step
+// (~1e-13 relative, the error squared)
+__device__ __forceinline__ double rsqrt_nr1(double x) {
+  const double y = (double)rsqrt_ftz((float)x);
+  return fma(0.5 * y, fma(-(x * y), y, 1.0), y);
+}
+__device__ __forceinline__ double rcp_nr1(double x) {
+  const double y = (double)rcp_ftz((float)x);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+#ifndef LMFF_PACKED_X2
+// 1/x, 1/sqrt(x) to the rounding of a double: an FP32 estimate (relative error e0 ~ 2^-22)
+// and one third-order step, e0^3 below 2^-64
+__device__ __forceinline__ double rcp3(double x) {
+  const double y = (double)rcp_ftz((float)x);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+__device__ __forceinline__ double rsqrt3(double x) {
+  const double y = (double)rsqrt_ftz((float)x);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y, e * fma(e, 0.375, 0.5), y);
+}
+// ln x for x in the FP32 normal range: with L the FP32 estimate, ln x = L + ln(1 + e),
+// e = x exp(-L) - 1 of ~1e-6
+__device__ __forceinline__ double ln_t64(double x) {
+  const double L = (double)__log2f((float)x) * 0.693147180559945309417;
+  const double e = fma(x, exp_t64(-L), -1.0);
+  return L + e * fma(e, fma(e, 1.0 / 3.0, -0.5), 1.0);
+}
+
+// FP64 mode: a centre atom with two or three bonds, all of them inside every triplet's
+// R - D (fc = 1) and lambda3 = 0 throughout (ForceArgs::ters_rlosq > 0) -- the atoms of an
+// intact sp2 layer.  The bonds' functions and forces of tersoff_atom in ~500 FP64
+// instructions instead of ~1,800: library exponentials, powers, divisions and square roots
+// replaced by the forms above, each angle evaluated once for both of its bonds (the
+// three-body force of bonds s and k on atom k points along e_s - cos e_k, whichever of
+// the two is the term's own bond, and on s along e_k - cos e_s), and g(theta) without the
+// cancellation of two ~1e8 terms (c^2/d^2 - c^2/(d^2 + u^2) = c^2 u^2/(d^2 (d^2 + u^2))).
+// Bound by the FP64 pipe: with energies and virial 1,267 -> 377 us on 331k atoms, 26 us of
+// latency at 5k.  Against 80-bit arithmetic the forces' error is 0.9e-14 where the general
+// routine's is 1.2e-14.
+// Returns false, nothing written, for an atom it does not take.
+template <bool EV, bool GH>
+__device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int ie, int cnt) {
+  if (cnt < 2 || cnt > 3 || !(a.ters_rlosq > 0.0)) return false;
+  const SysDesc &sd = a.A.sys[a.A.sysid[i]];
+  double d[3][3], r[3], ri[3], e[3][3];
+  int el[3];
+  uint32_t en[3];
+  bool ok = true;
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    el[s] = 0;
+    en[s] = 0;
+    if (s < cnt) {
+      en[s] = a.ters_nb[(size_t)i * MAXTERS + s];
+      int j, sx, sy, sz;
+      decode_entry(en[s], a.lc, j, sx, sy, sz);
+      double x, y, z;
+      disp64(a.A.xq, sd, i, j, sx, sy, sz, x, y, z);
+      d[s][0] = -x; d[s][1] = -y; d[s][2] = -z;   // x_j - x_i
+      const double rs = x * x + y * y + z * z;
+      ok = ok && rs < a.ters_rlosq && rs > 1e-12;
+      ri[s] = rsqrt3(rs);
+      r[s] = rs * ri[s];
+      e[s][0] = d[s][0] * ri[s]; e[s][1] = d[s][1] * ri[s]; e[s][2] = d[s][2] * ri[s];
+      el[s] = c_pot.t_map[info_type(__double_as_longlong(a.A.xq[j].w))];
+    }
+  }
+  if (!ok) return false;
+  const bool iown = !GH || owned(a, i);
+  // ---- angles: cos(theta), g and dg/dcos of each ordered bond pair, zeta
+  double cs[3][3], gd[3][3], zeta[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+#pragma unroll
+    for (int k = s + 1; k < 3; k++) {
+      if (k < cnt) {
+        const double c = e[s][0] * e[k][0] + e[s][1] * e[k][1] + e[s][2] * e[k][2];
+        cs[s][k] = c;
+        auto ang = [&](const TersP<R> &p, double &g, double &g1) {
+          const double u = p.h - c, U = u * u, inv = rcp3(p.d2 + U);
+          g = p.gamma * fma(p.cd2 * U, inv, 1.0);
+          g1 = (p.gamma * p.c2) * (-2.0 * u) * (inv * inv);
+        };
+        double gs, gk;
+        ang(c_pot.ters[(ie * MAXELEM + el[s]) * MAXELEM + el[k]], gs, gd[s][k]);
+        gk = gs;
+        gd[k][s] = gd[s][k];
+        if (el[s] != el[k]) ang(c_pot.ters[(ie * MAXELEM + el[k]) * MAXELEM + el[s]], gk, gd[k][s]);
+        zeta[s] += gs;
+        zeta[k] += gk;
+      }
+    }
+  }
+  // ---- the bonds: repulsion from this end, attraction with b_ij
+  double cr[3], fp2[3], eb[3], pref[3], hw[3], eng = 0.0;   // cr: force on i along d; hw: half of the repulsion's fpair
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    if (s < cnt) {
+      const TersP<R> &p = c_pot.ters[(ie * MAXELEM + el[s]) * MAXELEM + el[s]];
+      const double e1 = exp_t64(-p.lam1_64 * r[s]);
+      double rep = p.Al1_64 * e1 * ri[s], on = 1.0;
+      if constexpr (GH) {
+        int j, sx, sy, sz;
+        decode_entry(en[s], a.lc, j, sx, sy, sz);
+        on = (keep_half_r(a.tag[i], a.tag[j], d[s][0], d[s][1], d[s][2]) ? iown : owned(a, j)) ? 1.0 : 0.0;
+        rep *= on;
+      }
+      if (EV) eng += 0.5 * on * p.A64 * e1;
+      hw[s] = 0.5 * rep;
+      fp2[s] = eb[s] = pref[s] = 0.0;
+      if (iown) {
+        const double tmp = p.beta * zeta[s];
+        if (!(tmp > p.c3 && tmp <= p.c2t)) return false;
+        const double T = exp_t64(p.powern * ln_t64(tmp)), W = 1.0 + T;
+        const double bij = exp_t64(-p.inv2n * ln_t64(W));
+        const double bd = -0.5 * (bij * T) * rcp3(W * zeta[s]);
+        const double e2 = exp_t64(-p.lam2_64 * r[s]), fa = -p.B64 * e2;
+        fp2[s] = 0.5 * bij * (p.Bl2_64 * e2) * ri[s];
+        eb[s] = 0.5 * bij * fa;
+        pref[s] = -0.5 * fa * bd;
+        if (EV) eng += eb[s];
+      }
+      cr[s] = fp2[s] - rep;
+    }
+  }
+  // ---- forces on the partners: radial, then three-body
+  double t[3][3];
+#pragma unroll
+  for (int s = 0; s < 3; s++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) t[s][c] = 0.0;
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+#pragma unroll
+    for (int k = s + 1; k < 3; k++) {
+      if (k < cnt) {
+        const double q = fma(pref[s], gd[s][k], pref[k] * gd[k][s]), qs = q * ri[s], qk = q * ri[k], c = cs[s][k];
+#pragma unroll
+        for (int x = 0; x < 3; x++) {
+          t[k][x] = fma(qk, fma(-c, e[k][x], e[s][x]), t[k][x]);
+          t[s][x] = fma(qs, fma(-c, e[s][x], e[k][x]), t[s][x]);
+        }
+      }
+    }
+  }
+  double f[3] = {0.0, 0.0, 0.0}, v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    if (s < cnt) {
+      double g[3];
+#pragma unroll
+      for (int x = 0; x < 3; x++) {
+        f[x] = fma(cr[s], d[s][x], f[x] - t[s][x]);
+        g[x] = fma(-fp2[s], d[s][x], t[s][x]);
+      }
+      a.ters_g[(size_t)i * MAXTERS + s] = make_d4(g[0], g[1], g[2], eb[s]);
+      if (EV) {
+        // the forces on the partner, and half of the repulsion, against d
+        double h[3];
+#pragma unroll
+        for (int x = 0; x < 3; x++) h[x] = fma(hw[s], d[s][x], g[x]);
+        v[0] = fma(d[s][0], h[0], v[0]); v[1] = fma(d[s][1], h[1], v[1]); v[2] = fma(d[s][2], h[2], v[2]);
+        v[3] = fma(d[s][0], h[1], v[3]); v[4] = fma(d[s][0], h[2], v[4]); v[5] = fma(d[s][1], h[2], v[5]);
+      }
+    }
+  }
+  a.ters_f[i] = f[0];
+  a.ters_f[a.n + i] = f[1];
+  a.ters_f[2 * a.n + i] = f[2];
+  if (EV) {
+    double *st = a.stat_ters;
+    st[i] = eng;
+    st[(size_t)a.n + i] = 0.0;
+#pragma unroll
+    for (int c = 0; c < 6; c++) st[(size_t)(2 + c) * a.n + i] = v[c];
+  }
+  return true;
+}
+#endif
+
 // sp2 layers give 3 bonds per atom: those atoms run with their bonds in registers
 template <bool EV, bool EATOM, bool GH, bool VA = false>
 __global__ void __launch_bounds__(128) k_tersoff(ForceArgs<R> a) {
@@ -822,6 +1042,10 @@ __global__ void __launch_bounds__(128) k_tersoff(ForceArgs<R> a) {
   const long long iinfo = __double_as_longlong(a.A.xq[i].w);
   const int ie = c_pot.t_map[info_type(iinfo)];
   const int cnt = ie < 0 ? 0 : a.ters_cnt[i];
+#ifndef LMFF_PACKED_X2
+  if constexpr (!VA)
+    if (tersoff_fast<EV, GH>(a, i, ie, cnt)) return;
+#endif
   if (cnt <= 3) tersoff_atom<3, EV, GH, VA>(a, i, ie, cnt);
   else tersoff_atom<MAXTERS, EV, GH, VA>(a, i, ie, cnt);
 }
@@ -1302,53 +1526,6 @@ __device__ __forceinline__ void rep_term(const IlpP<R> &p, R exp0, R exp1, R rho
 }
 
 // One list entry (i, j, image) with j's position and normal already loaded.
-// ---- FP64 pair-kernel arithmetic (the plain form): the FP64 pipe runs at 1/64 of the FP32
-// rate, so the exponentials, the square root and the divisions of a pair are written
-// with fewer FP64 instructions at full double accuracy (results within a few ulp of the
-// library functions, far inside the 1e-10 parity bar).
-//
-// e^x by Tang's table-driven method (P. T. P. Tang, ACM TOMS 15, 1989): n = rint(256 x /
-// ln2), r = x - n ln2/256 (|r| <= ln2/512; one FMA with ln2/256 rounded to double costs
-// at most |n| 2^-62 absolute in r, hence in the relative error of e^x: |n| < 2^18, so
-// below 6e-14 for |x| < 700 and below 4e-15 for |x| < 40), e^x = 2^(n>>8)
-// 2^((n&255)/256) (1 + p(r)), p the degree-4 Taylor polynomial of e^r - 1 (truncation
-// below 4e-17 relative: the 256-entry table keeps |r| small enough for degree 4, two FP64
-// FMAs fewer than degree 6 over 64 entries).  Outside |x| < 700 the library exp.
-constexpr int EXP2_F64_N = 256;
-__device__ double g_exp2_f64[EXP2_F64_N];
-
-__global__ void k_fill_exp2_f64() {
-  const int j = threadIdx.x;
-  if (j < EXP2_F64_N) g_exp2_f64[j] = exp2((double)j / EXP2_F64_N);
-}
-
-__device__ __forceinline__ double exp_t64(double x) {
-  if (!(fabs(x) < 700.0)) return exp(x);
-  const double magic = 6755399441055744.0;   // 1.5 * 2^52
-  const double tn = __dadd_rn(x * 369.3299304675746, magic);   // 256 / ln2
-  const int n = __double2loint(tn);
-  const double nd = __dsub_rn(tn, magic);
-  const double r = fma(-nd, 0.0027076061740622863, x);          // ln2 / 256
-  double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
-  p = fma(p, r, 0.5);
-  p = fma(p, r, 1.0);
-  p = p * r;
-  const double T = __ldg(&g_exp2_f64[n & (EXP2_F64_N - 1)]);
-  const double v = fma(T, p, T);
-  return __hiloint2double(__double2hiint(v) + (int)((unsigned)(n >> 8) << 20), __double2loint(v));
-}
-
-// 1/sqrt(x), 1/x: FP32 estimates (relative error ~2^-22) and one FP64 Newton step
-// (~1e-13 relative, the error squared)
-__device__ __forceinline__ double rsqrt_nr1(double x) {
-  const double y = (double)rsqrt_ftz((float)x);
-  return fma(0.5 * y, fma(-(x * y), y, 1.0), y);
-}
-__device__ __forceinline__ double rcp_nr1(double x) {
-  const double y = (double)rcp_ftz((float)x);
-  return fma(y, fma(-x, y, 1.0), y);
-}
-
 // Multi-element pair parameters, copied into shared memory by each block of k_ilp: lanes
 // index them by their own element pair, which in constant memory would serialise (one
 // constant-cache access per distinct address in a warp).
@@ -2347,8 +2524,23 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
       // whole batches every third round (fewer than 4 tpa entries wait), so that when and on
       // which lane an entry is evaluated depends on its atom's list alone: results are
       // the same whatever atoms share the warp
-      if (it % 3 == 0)
+      if (it % 3 == 0) {
         while (__any_sync(FULL, qn - qh >= tpa)) near_batch(qn - qh >= tpa);
+        // the sums' lo parts gather one rounding of the hi part per term: brought back below
+        // it before their own rounding shows
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          f[c] = renorm(f[c]);
+          g[c] = renorm(g[c]);
+        }
+        tpi = renorm(tpi);
+        if constexpr (EV) {
+          ev = renorm(ev);
+          er = renorm(er);
+#pragma unroll
+          for (int c = 0; c < 6; c++) w[c] = renorm(w[c]);
+        }
+      }
     }
     while (__any_sync(FULL, qh < qn)) near_batch(true);
   };
@@ -3666,7 +3858,7 @@ void launch_tersoff(const ForceArgs<R> &a, bool ev, bool eatom, cudaStream_t s) 
     else k_tersoff<false, false, true><<<g, b, 0, s>>>(a);
   } else if (ev) {
     k_tersoff<true, false, false><<<g, b, 0, s>>>(a);
-  } else if (a.ters_alone && a.n <= TERS_LANES_MAX_ATOMS && !a.no_small) {
+  } else if (a.ters_alone && a.n <= TERS_LANES_MAX_ATOMS && !a.no_small && !(sizeof(R) == 8 && a.ters_rlosq > 0.0)) {
     k_tersoff_lanes<<<(int)(((long long)a.n * TERS_LANES + 127) / 128), 128, 0, s>>>(a);
   } else {
     k_tersoff<false, false, false><<<g, b, 0, s>>>(a);
