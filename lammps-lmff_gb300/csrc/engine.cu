@@ -603,9 +603,9 @@ struct Engine {
   double **d_karrs = nullptr;
   double *d_kout = nullptr;
   // per-atom virial pass (lmff_compute_vatom): own shares, slots, the sorted result, the
-  // result in the caller's order and the mixed pass's frame tensors (7 float4), VA_DOUBLES
-  // per atom of capacity va_cap
-  static constexpr int VA_DOUBLES = 6 * (2 + MAXTERS + MAXILP + 2) + 28;
+  // result in the caller's order and the frame tensors (7 float4 in the mixed pass, 28
+  // doubles and 14 float4 in the FP64 one), VA_DOUBLES per atom of capacity va_cap
+  static constexpr int VA_DOUBLES = 6 * (2 + MAXTERS + MAXILP + 2) + 56;
   double *d_va = nullptr;
   int va_cap = 0;
   // device calls on this engine (counted by DeviceCall) and the one whose evaluation

@@ -825,7 +825,8 @@ __device__ __forceinline__ void tersoff_atom(const ForceArgs<R> &a, int i, int i
 // below 6e-14 for |x| < 700 and below 4e-15 for |x| < 40), e^x = 2^(n>>8)
 // 2^((n&255)/256) (1 + p(r)), p the degree-4 Taylor polynomial of e^r - 1 (truncation
 // below 4e-17 relative: the 256-entry table keeps |r| small enough for degree 4, two FP64
-// FMAs fewer than degree 6 over 64 entries).  Outside |x| < 700 the library exp.
+// FMAs fewer than degree 6 over 64 entries).  Outside |x| < 700 the library exp.  FULL: a
+// second FMA takes ln2/256's rounding out as well, for sums whose own error is that small.
 constexpr int EXP2_F64_N = 256;
 __device__ double g_exp2_f64[EXP2_F64_N];
 
@@ -834,13 +835,15 @@ __global__ void k_fill_exp2_f64() {
   if (j < EXP2_F64_N) g_exp2_f64[j] = exp2((double)j / EXP2_F64_N);
 }
 
+template <bool FULL = false>
 __device__ __forceinline__ double exp_t64(double x) {
   if (!(fabs(x) < 700.0)) return exp(x);
   const double magic = 6755399441055744.0;   // 1.5 * 2^52
   const double tn = __dadd_rn(x * 369.3299304675746, magic);   // 256 / ln2
   const int n = __double2loint(tn);
   const double nd = __dsub_rn(tn, magic);
-  const double r = fma(-nd, 0.0027076061740622863, x);          // ln2 / 256
+  double r = fma(-nd, 0.0027076061740622863, x);                // ln2 / 256
+  if constexpr (FULL) r = fma(-nd, 9.058776616587108e-20, r);   // its rounding
   double p = fma(r, 1.0 / 24.0, 1.0 / 6.0);
   p = fma(p, r, 0.5);
   p = fma(p, r, 1.0);
@@ -878,7 +881,7 @@ __device__ __forceinline__ double rsqrt3(double x) {
 // e = x exp(-L) - 1 of ~1e-6
 __device__ __forceinline__ double ln_t64(double x) {
   const double L = (double)__log2f((float)x) * 0.693147180559945309417;
-  const double e = fma(x, exp_t64(-L), -1.0);
+  const double e = fma(x, exp_t64<true>(-L), -1.0);
   return L + e * fma(e, fma(e, 1.0 / 3.0, -0.5), 1.0);
 }
 
@@ -953,7 +956,7 @@ __device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int i
   for (int s = 0; s < 3; s++) {
     if (s < cnt) {
       const TersP<R> &p = c_pot.ters[(ie * MAXELEM + el[s]) * MAXELEM + el[s]];
-      const double e1 = exp_t64(-p.lam1_64 * r[s]);
+      const double e1 = exp_t64<true>(-p.lam1_64 * r[s]);
       double rep = p.Al1_64 * e1 * ri[s], on = 1.0;
       if constexpr (GH) {
         int j, sx, sy, sz;
@@ -967,10 +970,10 @@ __device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int i
       if (iown) {
         const double tmp = p.beta * zeta[s];
         if (!(tmp > p.c3 && tmp <= p.c2t)) return false;
-        const double T = exp_t64(p.powern * ln_t64(tmp)), W = 1.0 + T;
-        const double bij = exp_t64(-p.inv2n * ln_t64(W));
+        const double T = exp_t64<true>(p.powern * ln_t64(tmp)), W = 1.0 + T;
+        const double bij = exp_t64<true>(-p.inv2n * ln_t64(W));
         const double bd = -0.5 * (bij * T) * rcp3(W * zeta[s]);
-        const double e2 = exp_t64(-p.lam2_64 * r[s]), fa = -p.B64 * e2;
+        const double e2 = exp_t64<true>(-p.lam2_64 * r[s]), fa = -p.B64 * e2;
         fp2[s] = 0.5 * bij * (p.Bl2_64 * e2) * ri[s];
         eb[s] = 0.5 * bij * fa;
         pref[s] = -0.5 * fa * bd;
@@ -2268,6 +2271,19 @@ __global__ void k_fill_df_tables(int ne) {
   g_dfTE[k] = make_float2(te[0], te[1]);
 }
 
+// the FP64 tables of the per-atom virial pass
+__device__ double g_va64[MAXELEM * MAXELEM * df::TAB64_N * 24];   // A, M, TE: 8 each per interval
+
+__global__ void k_fill_va_tables(int ne) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= ne * ne * df::TAB64_N) return;
+  const int p = k / df::TAB64_N, a = p / ne, b = p % ne;
+  const IlpP<R> &q = c_pot.ilp[a * MAXELEM + b];
+  const df::TabP t = {q.z0, q.lambda, 2.0 * q.eps_half, q.d, q.seff, q.C6, 1.0 / c_pot.i_inv_rcut, c_pot.tap};
+  double *o = g_va64 + 24 * (size_t)k;
+  df::tab64_fill(t, k % df::TAB64_N, o, o + 8, o + 16);
+}
+
 __global__ void k_fill_exp2_df() {
   const int j = threadIdx.x;
   if (j < df::EXP2_TAB) g_exp2_df[j] = df::exp2_entry(j);
@@ -2622,6 +2638,7 @@ static void upload_pair_df(const PotConst<R> &p, cudaStream_t s) {
   cudaMemcpyToSymbolAsync(g_dfk, rows, sizeof rows, 0, cudaMemcpyHostToDevice, s);
   k_fill_exp2_df<<<1, df::EXP2_TAB, 0, s>>>();
   k_fill_df_tables<<<(ne * ne * df::TAB_N + 63) / 64, 64, 0, s>>>(ne);
+  k_fill_va_tables<<<(ne * ne * df::TAB64_N + 63) / 64, 64, 0, s>>>(ne);
 }
 
 template <bool ONE, bool GH>
@@ -3296,17 +3313,36 @@ __global__ void __launch_bounds__(128) k_va_ilp(ForceArgs<R> a) {
   va_write_slots(a, i, ie >= 0 && iown, fri, gx, gy, gz, G);
 }
 
-// ---- the same shares in double-float arithmetic (k_ilp_df's pair terms), where that
-// kernel takes the potential.  As in the mixed pass, the own share is half of del (x) f_ij
-// and the partner's normal-derivative share comes from the 27 numbers of the partner's
-// frame, here as double-floats.  VA_LANES lanes per atom share its list; the atom's g_i and
-// G_i go to its slot storage, from which k_va_slots forms the slots with full warps.
-// k_va_ilp's ~500 FP64 instructions per pair at 1/75 of the FP32 rate become ~1,100 FP32
-// ones (36,800-atom slab: 30 -> 1.5 ms for the pass's pair kernel).
+// ---- the same shares where the double-float pair kernel takes the potential.  As in the
+// mixed pass, the own share is half of del (x) f_ij and the partner's normal-derivative share
+// comes from the 27 numbers of the partner's frame.  Two kernels split the list at
+// VA_NEARSQ: k_va_near evaluates the pairs below it in FP64, k_va_far the others (nine of
+// ten) in double-float arithmetic.  The near pairs are the ones whose terms are large; past
+// 7 A a term is below 1e-2 of theirs and the double-float error of 1e-13 of a term adds
+// less than the near terms' rounding.  The result's error against 80-bit arithmetic
+// (graphite stack, twisted hBN bilayer): k_va_ilp 4.2e-15, 1.9e-15; split at 6 A 4.6e-15,
+// 1.6e-15; at 7 A 2.9e-15, 1.5e-15; at 8 A 2.2e-15, 1.4e-15; everything in double-float
+// 1.6e-13, 5e-14, which would be less than k_va_ilp gave.  VA_LANES lanes per atom share its
+// list; the atom's g_i and G_i go to its slot storage, from which k_va_slots forms the slots
+// with full warps.  36,800-atom slab: k_va_ilp 30 ms (one thread per atom, ~500 FP64
+// instructions a pair); k_va_near 1.67 ms, FP64 pipe (~190 instructions for ~85 pairs an
+// atom), k_va_far 1.22 ms, FP32 issue.
 constexpr int VA_LANES = 8;
+constexpr float VA_NEARSQ = 49.f;
+static_assert(VA_NEARSQ <= df::Q64_MAX, "the FP64 tables end at Q64_MAX");
 
-// per atom: A (18, row-major k, a) then B (9, row-major a, b) of k_va_ilp_df as (hi, lo)
-// pairs, 14 float4
+// whether entry e of atom i's list is a pair inside the cutoff, and its q = r^2 as both
+// kernels' split tests it
+__device__ __forceinline__ bool va_pair_q(const DfAtom &I, const DfAtom &A, const SysDesc &sd, int sx, int sy, int sz,
+                                          df::D<float> d[3], df::D<float> &q) {
+  df_del<true>(I, A, sd, sx, sy, sz, d);
+  q = df::dot3(d, d);
+  return __fadd_rn(__fsub_rn(q.h, c_dfcut.h), __fsub_rn(q.l, c_dfcut.l)) < 0.f;
+}
+
+// per atom: A (18, row-major k, a) then B (9, row-major a, b) in 28 doubles, the last 1 where
+// B is not zero (atoms without exactly three intralayer neighbours); then, after those of
+// all atoms, as (hi, lo) pairs, 14 float4
 __global__ void __launch_bounds__(128) k_va_tens_df(ForceArgs<R> a) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
@@ -3327,7 +3363,11 @@ __global__ void __launch_bounds__(128) k_va_tens_df(ForceArgs<R> a) {
       for (int b = 0; b < 3; b++) t[18 + 3 * e + b] = o.c[0][b] + o.c[1][b] + o.c[2][b];
     }
   }
-  float4 *q = a.va_tens + 14 * (size_t)i;
+  t[27] = fr.ok && fr.cont != 3 ? 1.0 : 0.0;
+  double *t64 = reinterpret_cast<double *>(a.va_tens) + 28 * (size_t)i;
+#pragma unroll
+  for (int k = 0; k < 28; k++) t64[k] = t[k];
+  float4 *q = a.va_tens + 14 * ((size_t)a.n + i);
 #pragma unroll
   for (int k = 0; k < 14; k++) {
     const float h0 = (float)t[2 * k], h1 = (float)t[2 * k + 1];
@@ -3353,15 +3393,157 @@ __device__ __noinline__ void va_close_pairs(const ForceArgs<R> &a, int i, int la
     decode_entry(e, a.lc, j, sx, sy, sz);
     DfAtom A;
     A.load(a.jrec, a.jstride, j);
-    df::D<float> d[3];
-    df_del<true>(I, A, sd, sx, sy, sz, d);
-    if (!all && !(df::dot3(d, d).h < DF_CLOSE)) continue;
+    df::D<float> d[3], s;
+    if (!all && !(va_pair_q(I, A, sd, sx, sy, sz, d, s) && s.h < DF_CLOSE)) continue;
     va_pair64<GH, false>(a, i, e, ie, mi, itag, iown, ni.x, ni.y, ni.z, v, v[6], v[7], v[8], v + 9);
   }
 }
 
+template <bool GH>
+__global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
+  const unsigned FULL = 0xffffffffu;
+  __shared__ uint32_t s_queue[128 * 4];
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) / VA_LANES;
+  const bool valid = i0 < a.n;
+  const int i = valid ? i0 : a.n - 1;
+  const int lane = threadIdx.x & (VA_LANES - 1);
+  const unsigned gmask = ((1u << VA_LANES) - 1) << ((threadIdx.x & 31) & ~(VA_LANES - 1));
+  const unsigned below = gmask & ((1u << (threadIdx.x & 31)) - 1u);
+  uint32_t *const queue = s_queue + 4 * (threadIdx.x & ~(VA_LANES - 1));
+  const SysDesc &sd = a.A.sys[a.A.sysid[i]];
+  const d4 xi = a.A.xq[i], ni = a.nrm64[i];
+  const int ie = c_pot.i_map[info_type(__double_as_longlong(xi.w))];
+  const long long itag = GH ? a.tag[i] : 0;
+  const bool iown = !GH || owned(a, i);
+  DfAtom I;
+  I.load(a.jrec, a.jstride, i);
+  const bool out = fabsf(I.h[0]) > sd.dfmax || fabsf(I.h[1]) > sd.dfmax || fabsf(I.h[2]) > sd.dfmax;
+  double s[15];   // w[6], g[3], G[6]
+#pragma unroll
+  for (int c = 0; c < 15; c++) s[c] = 0.0;
+  const int64_t b = a.list_off[i];
+  const int cnt = valid && ie >= 0 && !out ? (int)(a.list_off[i + 1] - b) : 0;
+  const int most = __reduce_max_sync(FULL, cnt);
+  bool close = valid && ie >= 0 && out;
+  auto pair_of = [&](uint32_t e, int &j, int &je, double d[3]) {
+    int sx, sy, sz;
+    decode_entry(e, a.lc, j, sx, sy, sz);
+    const d4 xj = a.A.xq[j];
+    d[0] = xi.x - xj.x; d[1] = xi.y - xj.y; d[2] = xi.z - xj.z;
+    if ((sx | sy | sz) != 0) {
+      d[0] = __dsub_rn(xi.x, __dadd_rn(xj.x, sx * sd.L[0]));
+      d[1] = __dsub_rn(xi.y, __dadd_rn(xj.y, sy * sd.L[1]));
+      d[2] = __dsub_rn(xi.z, __dadd_rn(xj.z, sz * sd.L[2]));
+    }
+    je = c_pot.i_map[info_type(__double_as_longlong(xj.w))];
+  };
+  // weights of the subdomain mode: the vdW pair, the terms with n_i and with n_j
+  auto weights = [&](int j, const double d[3], double &wv, double &wi, double &wj) {
+    if constexpr (GH) {
+      const bool jown = owned(a, j);
+      wv = (keep_half_r(itag, (long long)a.tag[j], -d[0], -d[1], -d[2]) ? iown : jown) ? 1.0 : 0.0;
+      wi = iown ? 1.0 : 0.0;
+      wj = jown ? 1.0 : 0.0;
+    }
+  };
+  auto virial = [&](const double d[3], const double t[3]) {
+    s[0] = fma(d[0], t[0], s[0]); s[1] = fma(d[1], t[1], s[1]); s[2] = fma(d[2], t[2], s[2]);
+    s[3] = fma(d[0], t[1], s[3]); s[4] = fma(d[0], t[2], s[4]); s[5] = fma(d[1], t[2], s[5]);
+  };
+  int qh = 0, qn = 0;
+  auto near_batch = [&](bool on) {
+    __syncwarp();
+    if (on && qh + lane < qn) {
+      int j, je;
+      double d[3], wv = 1.0, wi = 1.0, wj = 1.0, t;
+      pair_of(queue[(qh + lane) & (4 * VA_LANES - 1)], j, je, d);
+      weights(j, d, wv, wi, wj);
+      const double q = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+      const IlpP<R> &p = c_pot.ilp[ie * MAXELEM + je];
+      const double *c = g_va64 + 24 * (size_t)((ie * ne + je) * df::TAB64_N + df::tab64_at(q, t));
+      const double M = df::tab64_poly<6>(c + 8, t), TE = df::tab64_poly<7>(c + 16, t);
+      double cr = df::tab64_poly<6>(c, t);
+      if constexpr (GH) cr = fma(M * (2.0 * p.eps_half), 0.5 * (wi + wj) - wv, cr * wv);
+      const d4 nj = a.nrm64[j];
+      const double pn = ni.x * d[0] + ni.y * d[1] + ni.z * d[2], qn_ = nj.x * d[0] + nj.y * d[1] + nj.z * d[2];
+      const double G1 = wi * exp_t64<true>(-p.delta2inv * (q - pn * pn)), G2 = wj * exp_t64<true>(-p.delta2inv * (q - qn_ * qn_));
+      const double B = TE * (2.0 * p.C * p.delta2inv);
+      const double tp = pn * B * G1, tq = qn_ * B * G2;
+      cr = fma(G1 + G2, fma(M, p.C, B), cr);
+      // the force on i (the n_i part of it after the loop)
+      const double f[3] = {fma(cr, d[0], -tq * nj.x), fma(cr, d[1], -tq * nj.y), fma(cr, d[2], -tq * nj.z)};
+      virial(d, f);
+      const double h[3] = {tp * d[0], tp * d[1], tp * d[2]};
+      s[6] += h[0]; s[7] += h[1]; s[8] += h[2];
+      s[9] = fma(h[0], d[0], s[9]); s[10] = fma(h[1], d[1], s[10]); s[11] = fma(h[2], d[2], s[11]);
+      s[12] = fma(h[0], d[1], s[12]); s[13] = fma(h[0], d[2], s[13]); s[14] = fma(h[1], d[2], s[14]);
+      // the partner's normal-derivative share, g = tq del
+      const double g[3] = {tq * d[0], tq * d[1], tq * d[2]};
+      const double *T = reinterpret_cast<const double *>(a.va_tens) + 28 * (size_t)j;
+#pragma unroll
+      for (int x = 0; x < 6; x++)
+        s[x] = fma(__ldg(T + 3 * x), g[0], fma(__ldg(T + 3 * x + 1), g[1], fma(__ldg(T + 3 * x + 2), g[2], s[x])));
+      if (__ldg(T + 27) != 0.0) {
+        double r[3];
+#pragma unroll
+        for (int x = 0; x < 3; x++)
+          r[x] = -(__ldg(T + 18 + x) * g[0] + __ldg(T + 21 + x) * g[1] + __ldg(T + 24 + x) * g[2]);
+        virial(d, r);
+      }
+    }
+    if (on) qh = min(qh + VA_LANES, qn);
+    __syncwarp();
+  };
+  for (int k0 = 0, it = 1; k0 < most; k0 += VA_LANES, it++) {
+    bool near = false;
+    uint32_t e = 0;
+    if (k0 + lane < cnt) {
+      e = __ldg(&a.list[b + k0 + lane]);
+      int j, sx, sy, sz;
+      decode_entry(e, a.lc, j, sx, sy, sz);
+      DfAtom A;
+      A.load(a.jrec, a.jstride, j);
+      df::D<float> d[3], q;
+      near = va_pair_q(I, A, sd, sx, sy, sz, d, q) && q.h < VA_NEARSQ;
+      if (near && q.h < DF_CLOSE) {   // rare
+        near = false;
+        close = true;
+      }
+    }
+    const unsigned bits = __ballot_sync(FULL, near);
+    if (near) queue[(qn + __popc(bits & below)) & (4 * VA_LANES - 1)] = e;
+    qn += __popc(bits & gmask);
+    if (it % 3 == 0)
+      while (__any_sync(FULL, qn - qh >= VA_LANES)) near_batch(qn - qh >= VA_LANES);
+  }
+  while (__any_sync(FULL, qh < qn)) near_batch(true);
+#pragma unroll
+  for (int c = 0; c < 15; c++)
+    for (int o = VA_LANES / 2; o > 0; o >>= 1) s[c] += __shfl_xor_sync(FULL, s[c], o);
+  // the n_i part of the pair forces, and the halves
+  s[0] = 0.5 * fma(-s[6], ni.x, s[0]); s[1] = 0.5 * fma(-s[7], ni.y, s[1]); s[2] = 0.5 * fma(-s[8], ni.z, s[2]);
+  s[3] = 0.5 * fma(-s[6], ni.y, s[3]); s[4] = 0.5 * fma(-s[6], ni.z, s[4]); s[5] = 0.5 * fma(-s[7], ni.z, s[5]);
+  if (__any_sync(FULL, close)) {
+    double x[15];
+#pragma unroll
+    for (int c = 0; c < 15; c++) x[c] = 0.0;
+    if (close) va_close_pairs<GH>(a, i, lane, ie, iown, out, x);
+#pragma unroll
+    for (int c = 0; c < 15; c++) {
+      for (int o = VA_LANES / 2; o > 0; o >>= 1) x[c] += __shfl_xor_sync(FULL, x[c], o);
+      s[c] += x[c];
+    }
+  }
+  if (!valid || lane != 0) return;
+#pragma unroll
+  for (int c = 0; c < 6; c++) a.va_i[6 * (size_t)i + c] = s[c];
+  double *q = a.va_is + 6 * MAXILP * (size_t)i;
+#pragma unroll
+  for (int c = 0; c < 9; c++) q[c] = s[6 + c];
+}
+
 template <bool ONE, bool GH>
-__global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
+__global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
   using namespace df;
   typedef float V;
   __shared__ float2 s_tab[EXP2_TAB];
@@ -3381,7 +3563,6 @@ __global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
 #pragma unroll
   for (int c = 0; c < 15; c++) s[c] = mk(0.f, 0.f);
   const bool out = fabsf(I.h[0]) > sd.dfmax || fabsf(I.h[1]) > sd.dfmax || fabsf(I.h[2]) > sd.dfmax;
-  bool close = ie >= 0 && out;
   if (ie >= 0 && !out) {
     D<V> ni[3];
 #pragma unroll
@@ -3394,13 +3575,8 @@ __global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
       DfAtom A;
       A.load(a.jrec, a.jstride, j);
       D<V> d[3], nj[3];
-      df_del<true>(I, A, sd, sx, sy, sz, d);
-      const D<V> q = dot3(d, d);
-      if (!(__fadd_rn(__fsub_rn(q.h, c_dfcut.h), __fsub_rn(q.l, c_dfcut.l)) < 0.f)) continue;
-      if (q.h < DF_CLOSE) {
-        close = true;
-        continue;
-      }
+      D<V> q;
+      if (!va_pair_q(I, A, sd, sx, sy, sz, d, q) || q.h < VA_NEARSQ) continue;
 #pragma unroll
       for (int c = 0; c < 3; c++) nj[c] = mk(A.nh[c], A.nl[c]);
       float wv = 1.f, wi = 1.f, wj = 1.f;
@@ -3457,7 +3633,7 @@ __global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
         D<V> g[3], b[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) g[c] = mul(tq, d[c]);
-        const float4 *tt = a.va_tens + 14 * (size_t)j;
+        const float4 *tt = a.va_tens + 14 * ((size_t)a.n + j);
         float4 T[14];
 #pragma unroll
         for (int c = 0; c < 14; c++) T[c] = __ldg(tt + c);
@@ -3498,23 +3674,12 @@ __global__ void __launch_bounds__(128, 4) k_va_ilp_df(ForceArgs<R> a, int ne) {
   // the n_i part of the pair forces, and the halves
   v[0] = 0.5 * fma(-v[6], n[0], v[0]); v[1] = 0.5 * fma(-v[7], n[1], v[1]); v[2] = 0.5 * fma(-v[8], n[2], v[2]);
   v[3] = 0.5 * fma(-v[6], n[1], v[3]); v[4] = 0.5 * fma(-v[6], n[2], v[4]); v[5] = 0.5 * fma(-v[7], n[2], v[5]);
-  if (__any_sync(gmask, close)) {
-    double x[15];
-#pragma unroll
-    for (int c = 0; c < 15; c++) x[c] = 0.0;
-    if (close) va_close_pairs<GH>(a, i, lane, ie, iown, out, x);
-#pragma unroll
-    for (int c = 0; c < 15; c++) {
-      for (int o = VA_LANES / 2; o > 0; o >>= 1) x[c] += __shfl_xor_sync(gmask, x[c], o);
-      v[c] += x[c];
-    }
-  }
   if (lane != 0) return;
 #pragma unroll
-  for (int c = 0; c < 6; c++) a.va_i[6 * (size_t)i + c] = v[c];
+  for (int c = 0; c < 6; c++) a.va_i[6 * (size_t)i + c] += v[c];
   double *q = a.va_is + 6 * MAXILP * (size_t)i;
 #pragma unroll
-  for (int c = 0; c < 9; c++) q[c] = v[6 + c];
+  for (int c = 0; c < 9; c++) q[c] += v[6 + c];
 }
 
 // the intralayer slots of the atoms from the sums g_i, G_i left in their slot storage
@@ -3998,10 +4163,12 @@ void launch_vatom_terms(const ForceArgs<R> &a, bool ilp, bool one_element, cudaS
     if (a.pair_df && !a.list_full) {
       const int gl = (int)(((long long)a.n * VA_LANES + 127) / 128);
       k_va_tens_df<<<g, 128, 0, s>>>(a);
-      if (gh && one_element) k_va_ilp_df<true, true><<<gl, 128, 0, s>>>(a, a.pair_df);
-      else if (gh) k_va_ilp_df<false, true><<<gl, 128, 0, s>>>(a, a.pair_df);
-      else if (one_element) k_va_ilp_df<true, false><<<gl, 128, 0, s>>>(a, a.pair_df);
-      else k_va_ilp_df<false, false><<<gl, 128, 0, s>>>(a, a.pair_df);
+      if (gh) k_va_near<true><<<gl, 128, 0, s>>>(a, a.pair_df);
+      else k_va_near<false><<<gl, 128, 0, s>>>(a, a.pair_df);
+      if (gh && one_element) k_va_far<true, true><<<gl, 128, 0, s>>>(a, a.pair_df);
+      else if (gh) k_va_far<false, true><<<gl, 128, 0, s>>>(a, a.pair_df);
+      else if (one_element) k_va_far<true, false><<<gl, 128, 0, s>>>(a, a.pair_df);
+      else k_va_far<false, false><<<gl, 128, 0, s>>>(a, a.pair_df);
       k_va_slots<<<g, 128, 0, s>>>(a);
     } else if (gh && a.kc) k_va_ilp<true, true><<<g, 128, 0, s>>>(a);
     else if (gh) k_va_ilp<true, false><<<g, 128, 0, s>>>(a);

@@ -101,6 +101,53 @@ static __device__ inline void tab_fill(const TabP &p, int k, float ca[8], float 
   te[1] = (float)(TE - (double)te[0]);
 }
 
+// The same functions in FP64 (the per-atom virial's near pairs): 2^TAB64_BITS intervals
+// per factor of two, A and M of degree 6 and TE of degree 7 (M's integral), 8 doubles each
+constexpr int TAB64_BITS = 7;
+constexpr int TAB64_SHIFT = 23 - TAB64_BITS;
+constexpr int TAB64_BASE = (127 - 2) << TAB64_BITS;
+constexpr float Q64_MAX = 64.f;         // their range, [Q_MIN, Q64_MAX)
+constexpr int TAB64_N = 8 << TAB64_BITS;
+static __device__ inline void tab64_fill(const TabP &p, int k, double *ca, double *cm, double *ct) {
+  const double lo = ldexp(1.0 + (k & ((1 << TAB64_BITS) - 1)) / (double)(1 << TAB64_BITS), (k >> TAB64_BITS) - 2);
+  const double half = 0.5 * ldexp(1.0, (k >> TAB64_BITS) - 2 - TAB64_BITS), mid = lo + half;
+  double v[2][7], U, TE;
+  for (int j = 0; j < 7; j++) tab_functions(p, mid + half * cos(M_PI * (2 * j + 1) / 14.0), v[0][j], v[1][j], U, TE);
+  for (int f = 0; f < 2; f++) {
+    double a[7];
+    for (int m = 0; m < 7; m++) {
+      double s = 0.0;
+      for (int j = 0; j < 7; j++) s += v[f][j] * cos(M_PI * (m * (2 * j + 1)) / 14.0);
+      a[m] = s * (m ? 2.0 : 1.0) / 7.0;
+    }
+    const double c[7] = {a[0] - a[2] + a[4] - a[6], a[1] - 3.0 * a[3] + 5.0 * a[5], 2.0 * a[2] - 8.0 * a[4] + 18.0 * a[6],
+                         4.0 * a[3] - 20.0 * a[5], 8.0 * a[4] - 48.0 * a[6], 16.0 * a[5], 32.0 * a[6]};
+    double w = 1.0;
+    for (int m = 0; m < 7; m++, w /= half) (f ? cm : ca)[m] = c[m] * w;
+  }
+  double a, m;
+  tab_functions(p, mid, a, m, U, TE);
+  ca[7] = cm[7] = 0.0;
+  ct[0] = TE;
+  for (int k2 = 0; k2 < 7; k2++) ct[k2 + 1] = -0.5 * cm[k2] / (k2 + 1);
+}
+// interval of q and q minus its centre.  The interval is the FP32 neighbour's, at most one
+// rounding outside which its polynomial serves; the clamps are for a q whose FP32 sum is
+// inside the range while q itself rounds to its end
+static __device__ __forceinline__ int tab64_at(double q, double &t) {
+  const int u = min(max(__float_as_int((float)q), TAB64_BASE << TAB64_SHIFT),
+                    ((TAB64_BASE + TAB64_N) << TAB64_SHIFT) - 1);
+  t = q - (double)__int_as_float((u & ~((1 << TAB64_SHIFT) - 1)) | (1 << (TAB64_SHIFT - 1)));
+  return (u >> TAB64_SHIFT) - TAB64_BASE;
+}
+template <int N>
+static __device__ __forceinline__ double tab64_poly(const double *c, double t) {
+  double s = __ldg(c + N);
+#pragma unroll
+  for (int k = N - 1; k >= 0; k--) s = fma(s, t, __ldg(c + k));
+  return s;
+}
+
 // interval of q.h (in [Q_MIN, Q_MAX)) and q.h minus its centre (exact)
 static __device__ __forceinline__ int tab_at(float qh, float &t) {
   const int u = __float_as_int(qh);

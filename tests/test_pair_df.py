@@ -111,6 +111,20 @@ def test_per_atom_virial():
         assert np.abs(a["vatom_ilp"] - b["vatom_ilp"]).max() <= TOL * np.abs(b["vatom_ilp"]).max()
 
 
+@pytest.mark.parametrize("cut", [5.0, 7.0, 8.0, 16.0])
+def test_per_atom_virial_near_and_far_pairs(cut):
+    """Cutoffs below, at and above the distance that splits the pass's pairs, and a pair of
+    layers about that distance apart."""
+    for s in (S.displace(S.graphite_slab(4, 6, 4, mol_mode="unique"), 0.03, seed=9),
+              S.displace(S.twisted_bilayer(11, 7, 3.0, top="hbn", spacing=7.0), 1e-6, seed=5)):
+        r = []
+        for full in (0, 1):
+            eng = capi.Engine(TERSOFF, ILP, cut_global=cut)
+            eng.set_option("list_full", full)
+            r.append(eng.compute_system(s, which=capi.ILP, vatom=True)["vatom_ilp"])
+        assert np.abs(r[0] - r[1]).max() <= TOL * np.abs(r[1]).max()
+
+
 @pytest.mark.parametrize("ev", [False, True])
 def test_subdomain_form(ev):
     s = S.displace(S.twisted_bilayer(14, 8, 2.0, top="hbn", spacing=3.3), 0.03, seed=7)
