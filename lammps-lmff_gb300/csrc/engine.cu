@@ -197,22 +197,61 @@ __global__ void k_unpermute_state(int n, const int *perm, const d4 *xq, const do
   }
 }
 
-// deterministic per-system reduction of the per-atom stat arrays: block (s, q) sums
-// quantity q of system s in a fixed order
-__global__ void k_reduce(int n, int nq, const double *const *arrs, const SysDesc *sys, double *out) {
-  int s = blockIdx.x / nq, q = blockIdx.x % nq;
-  const double *a = arrs[q / 8] + (size_t)(q % 8) * n;
-  int b = sys[s].atom_begin, e = sys[s].atom_end;
-  double acc = 0.0;
-  for (int p = b + threadIdx.x; p < e; p += blockDim.x) acc += a[p];
-  __shared__ double sh[256];
+// Deterministic per-system reduction of the per-atom stat arrays: block (s, q, c) sums chunk
+// c of quantity q of system s in a fixed order, and the last of a quantity's blocks its
+// chunks' sums.  A system of one chunk (and, without part, any system) is one block's work.
+// Chunks are counted from the system's first atom, so a system's sums do not depend on what
+// else is in its batch.  One block per quantity took 70 us for 36,800 atoms (a chain of
+// ~0.5 us loads) and grew with n; REDUCE_MEASURED.
+constexpr int RED_THREADS = 256, RED_CHUNK = 8 * RED_THREADS;
+__device__ __forceinline__ double block_sum(double acc, double *sh) {
   sh[threadIdx.x] = acc;
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+  for (int o = RED_THREADS / 2; o > 0; o >>= 1) {
     if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[blockIdx.x] = sh[0];
+  return sh[0];
+}
+__global__ void __launch_bounds__(RED_THREADS) k_reduce(int n, int nq, const double *const *arrs, const SysDesc *sys,
+                                                        double *out, int cmax, double *part, int *count) {
+  __shared__ double sh[RED_THREADS];
+  __shared__ bool last;
+  const int c = blockIdx.x % cmax, sq = blockIdx.x / cmax, s = sq / nq, q = sq % nq;
+  const double *a = arrs[q / 8] + (size_t)(q % 8) * n;
+  const int b = sys[s].atom_begin, e = sys[s].atom_end;
+  const int m = part ? (e - b + RED_CHUNK - 1) / RED_CHUNK : 1;   // chunks
+  if (c > 0 && c >= m) return;
+  const int p0 = b + c * RED_CHUNK, p1 = m > 1 ? min(e, p0 + RED_CHUNK) : e;
+  double acc = 0.0;
+  for (int p = p0 + threadIdx.x; p < p1; p += RED_CHUNK) {
+    double x[RED_CHUNK / RED_THREADS];
+#pragma unroll
+    for (int k = 0; k < RED_CHUNK / RED_THREADS; k++) x[k] = p + k * RED_THREADS < p1 ? a[p + k * RED_THREADS] : 0.0;
+#pragma unroll
+    for (int k = 0; k < RED_CHUNK / RED_THREADS; k++) acc += x[k];
+  }
+  const double v = block_sum(acc, sh);
+  if (m <= 1) {
+    if (threadIdx.x == 0) out[sq] = v;
+    return;
+  }
+  double *ps = part + ((size_t)(b / RED_CHUNK) + s) * nq;   // the systems before s have fewer chunks than that
+  if (threadIdx.x == 0) {
+    ps[(size_t)c * nq + q] = v;
+    __threadfence();
+    last = atomicAdd(&count[sq], 1) == m - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  acc = 0.0;
+  for (int k = threadIdx.x; k < m; k += RED_THREADS) acc += __ldcg(&ps[(size_t)k * nq + q]);
+  const double sum = block_sum(acc, sh);
+  if (threadIdx.x == 0) {
+    out[sq] = sum;
+    count[sq] = 0;
+  }
 }
 
 // interlayer pairs of the list within the ILP cutoff (same test as the pair kernel)
@@ -705,7 +744,7 @@ struct Engine {
     void *ptrs[] = {d.xq, d.xh, d.xl, d.v, d.f, d.xhold, d.tag, d.perm, d.sysid, d.mass, d.nrm64, d.nrm32, d.jrec, d.ilp_cnt,
                     d.ilp_nb, d.ters_cnt, d.ters_nb, d.ters_g, d.ters_f, d.ilp_f, d.ilp_c, d.ilp_g, d.nframe, d.list_off, d.list,
                     d.short_cnt, d.short_nb, d.list_img, d.nin_tmp, d.list_tmp, d.bin_key, d.bin_key2, d.idx, d.idx2, d.bin_start, d.bin_end, d.rowocc, d.cub_tmp,
-                    d.cnt_tmp, d.sys, d.red_out, d.status, d.maxdisp, d_xin, d_fin, d_fo, d_vin, d_ein, d_tin, d_sysin,
+                    d.cnt_tmp, d.sys, d.red_out, d.partials, d.red_count, d.status, d.maxdisp, d_xin, d_fin, d_fo, d_vin, d_ein, d_tin, d_sysin,
                     d_min, d_gin, d_massT, xq2, v2, mass2, tag2, perm2, sysid2, stat_ilp, stat_ters, eatom_ilp,
                     eatom_ters, ke, d_arrs, d_karrs, d_kout, d_cutILPsq, d_maxpred, d_va};
     for (void *p : ptrs)
@@ -1620,6 +1659,25 @@ struct Engine {
     timed(3, [&] { ff(a, eatom, kick_on ? &kick_args : nullptr, stream); });
   }
 
+  // the reduction's chunk sums (of every system) and counters (zero between launches)
+  int ensure_partials() {
+    red_cmax = 1;
+    for (const SysDesc &s : hsys) red_cmax = std::max(red_cmax, (s.atom_end - s.atom_begin + RED_CHUNK - 1) / RED_CHUNK);
+    const int need = (int)(16 * (n / RED_CHUNK + hsys.size() + 1));
+    if (red_cmax > 1 && need > d.partials_cap) {
+      CK(cudaStreamSynchronize(stream));
+      CK(dalloc(d.partials, need));
+      CK(dalloc(d.red_count, need));
+      CK(cudaMemsetAsync(d.red_count, 0, sizeof(int) * (size_t)need, stream));
+      d.partials_cap = need;
+    }
+    return LMFF_OK;
+  }
+  int red_cmax = 1;
+  void reduce(int nq, double *const *arrs, int nsys, double *out) {
+    k_reduce<<<nsys * nq * red_cmax, RED_THREADS, 0, stream>>>(n, nq, arrs, d.sys, out, red_cmax, d.partials, d.red_count);
+  }
+
   // forces (+ energies/virials per system into hres when ev) on the resident state
   // wait = false (force-only evaluations): the status word comes back into a pinned word
   // and the caller waits once for everything it queued, then calls forces_done
@@ -1637,6 +1695,7 @@ struct Engine {
     cudaEventRecord(e0, stream);
     if (n > 0) {
       if (!hilo_fresh) hilo_all();
+      if (ev && ensure_partials() != LMFF_OK) return LMFF_ECUDA;   // before any capture
       const bool cap = use_graphs && !ktiming && !kick_on;
       std::vector<unsigned char> key;
       if (cap) {
@@ -1657,7 +1716,7 @@ struct Engine {
           run_kernels(args<float>(), which, ev, eatom, f32::launch_short, f32::launch_tersoff, f32::launch_ilp,
                       f32::launch_nframe, f32::launch_nderiv, f32::launch_finish);
         }
-        if (ev) k_reduce<<<(int)hsys.size() * 16, 256, 0, stream>>>(n, 16, (const double *const *)d_arrs, d.sys, d.red_out);
+        if (ev) reduce(16, d_arrs, (int)hsys.size(), d.red_out);
         if (cap) {
           cudaGraph_t g = nullptr;
           cudaError_t e = cudaStreamEndCapture(stream, &g);
@@ -2260,9 +2319,10 @@ struct Engine {
     std::vector<unsigned char> k;
     if (precision == LMFF_FP64) key_put(k, args<double>());
     else key_put(k, args<float>());
-    const int ints[] = {precision, which, (int)ev, (int)eatom, tpa, block, (int)ters_concurrent, (int)hsys.size()};
+    const int ints[] = {precision, which, (int)ev, (int)eatom, tpa, block, (int)ters_concurrent, (int)hsys.size(),
+                        red_cmax};
     key_put(k, ints);
-    const void *ptrs[] = {d_arrs, d.sys, d.red_out, stat_ilp, stat_ters, eatom_ters};
+    const void *ptrs[] = {d_arrs, d.sys, d.red_out, d.partials, d.red_count, stat_ilp, stat_ters, eatom_ters};
     key_put(k, ptrs);
     return k;
   }
@@ -2514,7 +2574,8 @@ struct Engine {
     auto sample = [&](int64_t step, const std::vector<lmff_result> &r) -> int {
       double kes = 0.0;
       if (n > 0) {
-        k_reduce<<<1, 256, 0, stream>>>(n, 1, (const double *const *)d_karrs, d.sys, d_kout);
+        if (ensure_partials() != LMFF_OK) return LMFF_ECUDA;
+        reduce(1, d_karrs, 1, d_kout);
         CK(cudaMemcpyAsync(&kes, d_kout, sizeof(double), cudaMemcpyDeviceToHost, stream));
         CK(cudaStreamSynchronize(stream));
       }
@@ -3260,7 +3321,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     }
     f32::launch_finish(a, false, nullptr, st);
   }
-  k_reduce<<<16, 256, 0, st>>>(nn, 16, (const double *const *)arrs, dsys, red);
+  k_reduce<<<16, RED_THREADS, 0, st>>>(nn, 16, (const double *const *)arrs, dsys, red, 1, nullptr, nullptr);
   k_scatter_add<<<gb, 256, 0, st>>>(nn, perm2, fs, df, 1);
   CK2(cudaGetLastError());
   double hred[16];

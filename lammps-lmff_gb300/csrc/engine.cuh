@@ -189,7 +189,8 @@ struct DevState {
   // systems
   SysDesc *sys = nullptr;
   // reductions
-  double *partials = nullptr; // blocks * NSTAT * 2
+  double *partials = nullptr; // NSTAT * 2 per chunk of a system
+  int *red_count = nullptr;   // NSTAT * 2 * nsys: chunks summed so far
   int partials_cap = 0;
   double *red_out = nullptr;  // NSTAT * 2 * nsys
   int *status = nullptr;      // device status word
