@@ -9,16 +9,19 @@
 //   k_tersoff (bonds centred at each atom)   k_ilp (interlayer pairs, normal derivatives)
 //   k_finish (gather) -> [k_reduce energies/virials]
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <array>
 #include <atomic>
 #include <mutex>
+#include <functional>
 #include <shared_mutex>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -1681,7 +1684,9 @@ struct Engine {
   // forces (+ energies/virials per system into hres when ev) on the resident state
   // wait = false (force-only evaluations): the status word comes back into a pinned word
   // and the caller waits once for everything it queued, then calls forces_done
-  int forces(int which, bool ev, bool eatom, std::vector<lmff_result> *hres, bool wait = true) {
+  // while_waiting: host work of the call, done when the kernels are queued
+  int forces(int which, bool ev, bool eatom, std::vector<lmff_result> *hres, bool wait = true,
+             const std::function<void()> &while_waiting = nullptr) {
     int rc = push_consts();
     if (rc) return rc;
     if (!built) {
@@ -1746,6 +1751,7 @@ struct Engine {
       red.resize(hsys.size() * 16);
       CK(cudaMemcpyAsync(red.data(), d.red_out, sizeof(double) * red.size(), cudaMemcpyDeviceToHost, stream));
     }
+    if (while_waiting) while_waiting();
     CK(cudaStreamSynchronize(stream));
     harvest();
     float ms = 0;
@@ -1888,7 +1894,10 @@ struct Engine {
     if (rc) return rc;
     std::vector<lmff_result> hr;
     bool ev = eflag || vflag || eatom;
-    rc = forces(which, ev, eatom != nullptr, &hr);
+    rc = forces(which, ev, eatom != nullptr, &hr, true, [&] {
+      map_pages(f, sizeof(double) * 3 * (size_t)nn);
+      map_pages(eatom, sizeof(double) * (size_t)nn);
+    });
     if (rc) return rc;
     if (res) *res = hr.empty() ? lmff_result() : hr[0];
     bool overwrite = (which & LMFF_OVERWRITE) != 0;
@@ -1920,6 +1929,7 @@ struct Engine {
     const bool overwrite = (which & LMFF_OVERWRITE) != 0;
     if (!overwrite) CK(cudaMemcpyAsync(d_fin, f, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, stream));
     k_scatter_sum<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, d.f, overwrite ? nullptr : d_fin, d_fo);
+    map_pages(f, sizeof(double) * 3 * (size_t)nn);
     CK(cudaMemcpyAsync(f, d_fo, sizeof(double) * 3 * nn, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     double d2;
@@ -2170,6 +2180,7 @@ struct Engine {
     const bool overwrite = (which & LMFF_OVERWRITE) != 0;
     if (!overwrite) CK(cudaMemcpyAsync(inorder, out, sizeof(double) * 6 * (size_t)nn, cudaMemcpyHostToDevice, stream));
     k_scatter_add6<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, sorted, inorder, overwrite);
+    map_pages(out, sizeof(double) * 6 * (size_t)nn);
     CK(cudaMemcpyAsync(out, inorder, sizeof(double) * 6 * (size_t)nn, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     return LMFF_OK;
@@ -2887,6 +2898,7 @@ struct Engine {
     double *xo = d_xin, *vo = d_vin, *fo = d_fin;
     k_unpermute_state<<<(n + 255) / 256, 256, 0, stream>>>(n, d.perm, d.xq, d.v, d.f, xo, vo, fo);
     CK(cudaGetLastError());
+    for (double *p : {x, v, f}) map_pages(p, sizeof(double) * 3 * (size_t)n);
     if (x) CK(cudaMemcpyAsync(x, xo, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, stream));
     if (v) CK(cudaMemcpyAsync(v, vo, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, stream));
     if (f) CK(cudaMemcpyAsync(f, fo, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, stream));
@@ -3020,20 +3032,46 @@ struct Engine {
 
   // memcpy on up to 8 host threads, in 64-byte aligned pieces
   static void parallel_copy(void *dst, const void *src, size_t bytes) {
+    in_pieces(bytes, [=](size_t b, size_t e) { memcpy((char *)dst + b, (const char *)src + b, e - b); });
+  }
+  // f(begin, end) over [0, bytes): from 4 MiB on in up to 8 pieces, each on its host thread.
+  // A piece whose thread cannot be had is done here.
+  template <class F>
+  static void in_pieces(size_t bytes, const F &f) {
     const int nth = (int)std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency()));
     if (nth <= 1 || bytes < ((size_t)4 << 20)) {
-      memcpy(dst, src, bytes);
+      f((size_t)0, bytes);
       return;
     }
     const size_t piece = ((bytes / nth) + 63) & ~(size_t)63;
     std::vector<std::thread> pool;
+    pool.reserve(nth);
     for (int k = 0; k < nth; k++) {
       const size_t b = (size_t)k * piece;
       if (b >= bytes) break;
       const size_t e = std::min(bytes, b + piece);
-      pool.emplace_back([=] { memcpy((char *)dst + b, (const char *)src + b, e - b); });
+      try {
+        pool.emplace_back([=, &f] { f(b, e); });
+      } catch (const std::system_error &) {
+        f(b, e);
+      }
     }
     for (auto &t : pool) t.join();
+  }
+  // Maps the pages of a caller's output array, each byte keeping its value.  An array the
+  // program has just allocated has no pages yet; the GPU's copy into it then takes a fault of
+  // ~40 us for every 64 KB (490k atoms, lmff_download: 20-30 ms, with its pages there 0.9 ms),
+  // where a write by the host takes 5-10 us, on several threads at once and, where a call's
+  // kernels are already queued, while they run.
+  static void map_pages(void *p, size_t bytes) {
+    if (!p || !bytes) return;
+    static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
+    in_pieces(bytes, [=](size_t b, size_t e) {
+      for (size_t q = b; q < e; q = ((uintptr_t)p + q) / page * page + page - (uintptr_t)p) {
+        volatile char *c = (volatile char *)p + q;
+        *c = *c;
+      }
+    });
   }
 
   // ---------------------------------------------------------------- lists export

@@ -247,8 +247,9 @@ class Engine:
         t = np.ascontiguousarray(type_, dtype=np.int32)
         m = None if mol is None else np.ascontiguousarray(mol, dtype=np.int64)
         g = None if tag is None else np.ascontiguousarray(tag, dtype=np.int64)
-        out_f = np.zeros((n, 3)) if f is None else f
-        ea = np.zeros(n) if eatom else None
+        overwrite = overwrite or f is None   # nothing to add to: no copy of zeros to the device
+        out_f = np.empty((n, 3)) if f is None else f
+        ea = (np.empty(n) if overwrite else np.zeros(n)) if eatom else None
         r = Result()
         flags = which | (SAME_ATOMS if same_atoms else 0) | (OVERWRITE if overwrite else 0)
         self._ck(_lib.lmff_compute(self._h, n, _p(x), _p(t), _p(m), _p(g), flags, int(eflag), int(vflag),
@@ -267,8 +268,8 @@ class Engine:
         engine made: [n, 6], rows xx yy zz xy xz yz in that call's atom order (nall rows
         after compute_ghost), the styles selected by `which`."""
         n = getattr(self, "_last_n", 0) if natoms is None else int(natoms)
-        v = np.zeros((n, 6))
-        self._ck(_lib.lmff_compute_vatom(self._h, which, n, _p(v)))
+        v = np.empty((n, 6))
+        self._ck(_lib.lmff_compute_vatom(self._h, which | OVERWRITE, n, _p(v)))
         return v
 
     def _add_vatom(self, out: Dict, which: int):
@@ -291,10 +292,10 @@ class Engine:
         t = np.ascontiguousarray(type_, dtype=np.int32)
         m = np.ascontiguousarray(mol, dtype=np.int64)
         g = np.ascontiguousarray(tag, dtype=np.int64)
-        f = np.zeros((nall, 3))
-        ea = np.zeros(nall) if eatom else None
+        f = np.empty((nall, 3))
+        ea = np.empty(nall) if eatom else None
         r = Result()
-        flags = which | (SAME_ATOMS if same_atoms else 0)
+        flags = which | (SAME_ATOMS if same_atoms else 0) | OVERWRITE
         self._ck(_lib.lmff_compute_ghost(self._h, int(nlocal), nall, _p(x), _p(t), _p(m), _p(g), flags, int(eflag),
                                          int(vflag), _p(f), _p(ea), C.byref(r)))
         self._last_n = nall
