@@ -51,6 +51,8 @@ LMFF_FORCE_API(f32, float)
 namespace f64 {
 void launch_vatom_terms(const ForceArgs<double> &a, bool ilp, bool one_element, cudaStream_t s);
 void launch_vatom_gather(const ForceArgs<double> &a, double *out, cudaStream_t s);
+void fill_df_tables(int ne, float4 *A, float4 *M, float2 *U, float2 *TE, cudaStream_t s);
+void fill_va_tables(int ne, double *tab, cudaStream_t s);
 }
 namespace f32 {
 void launch_vatom_ilp(const ForceArgs<float> &a, cudaStream_t s);
@@ -749,7 +751,7 @@ struct Engine {
                     d.short_cnt, d.short_nb, d.list_img, d.nin_tmp, d.list_tmp, d.bin_key, d.bin_key2, d.idx, d.idx2, d.bin_start, d.bin_end, d.rowocc, d.cub_tmp,
                     d.cnt_tmp, d.sys, d.red_out, d.partials, d.red_count, d.status, d.maxdisp, d_xin, d_fin, d_fo, d_vin, d_ein, d_tin, d_sysin,
                     d_min, d_gin, d_massT, xq2, v2, mass2, tag2, perm2, sysid2, stat_ilp, stat_ters, eatom_ilp,
-                    eatom_ters, ke, d_arrs, d_karrs, d_kout, d_cutILPsq, d_maxpred, d_va};
+                    eatom_ters, ke, d_arrs, d_karrs, d_kout, d_cutILPsq, d_maxpred, d_va, d_dfA, d_dfM, d_dfU, d_dfTE, d_va64};
     for (void *p : ptrs)
       if (p) cudaFree(p);
     d = DevState();
@@ -770,6 +772,10 @@ struct Engine {
     d_cutILPsq = nullptr;
     d_maxpred = nullptr;
     d_va = nullptr;
+    d_dfA = d_dfM = nullptr;
+    d_dfU = d_dfTE = nullptr;
+    d_va64 = nullptr;
+    df_filled = va64_filled = false;
     va_cap = 0;
     if (h_pinned) cudaFreeHost(h_pinned);
     h_pinned = nullptr;
@@ -1014,6 +1020,14 @@ struct Engine {
     return pot64.i_ne;
   }
   int pair_df = 0;
+  // the double-float kernel's tables (491 KB per element pair, allocated with the engine) and
+  // the per-atom virial's (197 KB, with its first pass), filled once: engines of different
+  // potentials on one device do not refill them at each change of the device's constants
+  float4 *d_dfA = nullptr, *d_dfM = nullptr;
+  float2 *d_dfU = nullptr, *d_dfTE = nullptr;
+  double *d_va64 = nullptr;
+  bool df_filled = false, va64_filled = false;
+  size_t df_intervals() const { return (size_t)pair_df * pair_df * df::TAB_N; }
 
   // the square of the smallest R - D where every Tersoff entry has lambda3 = 0, symmetric
   // repulsion and constants whose functions stay in the FP32 exponent range (the estimates
@@ -1064,6 +1078,7 @@ struct Engine {
     nbc.innersq_f = (float)(cut_global * cut_global);
     hash_tables();
     pot_dirty = true;
+    df_filled = va64_filled = false;
     built = false;
     return LMFF_OK;
   }
@@ -1111,6 +1126,10 @@ struct Engine {
     CK(cudaMalloc(&d_arrs, sizeof(double *) * 2));
     CK(cudaMalloc(&d_karrs, sizeof(double *) * 2));
     CK(cudaMalloc(&d_kout, sizeof(double)));
+    if (pair_df) {
+      CK(dalloc(d_dfA, 2 * df_intervals())); CK(dalloc(d_dfM, 2 * df_intervals()));
+      CK(dalloc(d_dfU, df_intervals())); CK(dalloc(d_dfTE, df_intervals()));
+    }
     CK(cudaMemsetAsync(d.status, 0, sizeof(int), stream));
     return LMFF_OK;
   }
@@ -1118,6 +1137,10 @@ struct Engine {
   // The device's constant tables are this engine's (guaranteed by DeviceCall); only the
   // engine-owned copy of the intralayer cutoffs may still need refreshing.
   int push_consts() {
+    if (precision == LMFF_FP64 && pair_df && !df_filled) {
+      f64::fill_df_tables(pair_df, d_dfA, d_dfM, d_dfU, d_dfTE, stream);
+      df_filled = true;
+    }
     if (!pot_dirty) return LMFF_OK;
     double c[MAXELEM * MAXELEM] = {0};
     if (i_on) {
@@ -1213,7 +1236,7 @@ struct Engine {
   }
   double device_bytes() const {
     return (double)cap_n * per_atom_bytes() + (double)(d.list_cap + d.tmp_cap) * sizeof(uint32_t) +
-           (double)d.cub_tmp_bytes + (double)d.nbins_cap * 3 * sizeof(int) + (double)va_cap * VA_DOUBLES * sizeof(double);
+           (double)df_intervals() * 80.0 * (d_dfA != nullptr) + (double)d.cub_tmp_bytes + (double)d.nbins_cap * 3 * sizeof(int) + (double)va_cap * VA_DOUBLES * sizeof(double);
   }
   // device bytes per atom a batch like the current one needs: the per-atom arrays with
   // their growth margin, the pair list at the current density with the step graph's
@@ -1613,6 +1636,10 @@ struct Engine {
     a.no_small = !small_variants;
     a.kc = i_on && hi.model == LMFF_INTERLAYER_KC;
     a.pair_df = pair_df;
+    a.df_A = d_dfA;
+    a.df_M = d_dfM;
+    a.df_U = d_dfU;
+    a.df_TE = d_dfTE;
     a.jstride = cap_n;
     a.ters_rlosq = ters_rlosq;
     // not while kernels are timed one by one (events between the launches)
@@ -2149,7 +2176,14 @@ struct Engine {
       CK(cudaMalloc(&d_va, sizeof(double) * VA_DOUBLES * (size_t)cap_n));
       va_cap = cap_n;
     }
+    if (pair_df && precision == LMFF_FP64 && !va64_filled) {
+      const size_t per = (size_t)pair_df * pair_df * df::TAB64_N * 24;
+      if (!d_va64) CK(cudaMalloc(&d_va64, sizeof(double) * per));
+      f64::fill_va_tables(pair_df, d_va64, stream);
+      va64_filled = true;
+    }
     ForceArgs<double> a = args<double>();
+    a.va64 = d_va64;
     a.do_ters = t_on && (which & LMFF_TERSOFF);
     a.do_ilp = i_on && (which & LMFF_ILP);
     const size_t c6 = 6 * (size_t)va_cap;
@@ -3327,6 +3361,10 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     a.list_full = g.list_full;
     a.kc = g.i_on && g.hi.model == LMFF_INTERLAYER_KC;
     a.pair_df = g.pair_df;
+    a.df_A = g.d_dfA;
+    a.df_M = g.d_dfM;
+    a.df_U = g.d_dfU;
+    a.df_TE = g.d_dfTE;
     a.jstride = c;
     a.ters_rlosq = g.ters_rlosq;
   };

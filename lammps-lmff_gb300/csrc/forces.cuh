@@ -331,6 +331,12 @@ struct ForceArgs {
   // potential (Engine::pair_df), 0: k_ilp.  jrec then holds its records
   int pair_df;
   int jstride;         // atoms per array of the records
+  // the engine's tables of the radial functions (ilp_df.cuh): A and M in two float4 per
+  // interval of element pair a * pair_df + b, U and TE at its centre; in FP64 for the
+  // per-atom virial pass
+  const float4 *df_A, *df_M;
+  const float2 *df_U, *df_TE;
+  const double *va64;
   // FP64 mode: the square of the smallest R - D of the Tersoff triplets where tersoff_fast
   // takes the potential (Engine::ters_rlosq), else 0
   double ters_rlosq;

@@ -2248,14 +2248,9 @@ __constant__ DfCut c_dfcut;
 __constant__ float c_dfk[df::K_N];                    // element pair (0, 0)'s constants
 __device__ float g_dfk[MAXELEM * MAXELEM * df::K_N];  // element pair (a, b)'s at (a * ne + b) * K_N
 __device__ float2 g_exp2_df[df::EXP2_TAB];
-// tables (ilp_df.cuh), per interval of element pair a * ne + b: the coefficients of A and of
-// M in two float4 each, U and TE at the centre
-__device__ float4 g_dfA[MAXELEM * MAXELEM * df::TAB_N * 2];
-__device__ float4 g_dfM[MAXELEM * MAXELEM * df::TAB_N * 2];
-__device__ float2 g_dfU[MAXELEM * MAXELEM * df::TAB_N];
-__device__ float2 g_dfTE[MAXELEM * MAXELEM * df::TAB_N];
 
-__global__ void k_fill_df_tables(int ne) {
+// the engine's tables (ilp_df.cuh), per interval of element pair a * ne + b
+__global__ void k_fill_df_tables(int ne, float4 *A, float4 *M, float2 *U, float2 *TE) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= ne * ne * df::TAB_N) return;
   const int p = k / df::TAB_N, a = p / ne, b = p % ne;
@@ -2264,23 +2259,20 @@ __global__ void k_fill_df_tables(int ne) {
   float ca[8], cm[8], u[2], te[2];
   df::tab_fill(t, k % df::TAB_N, ca, cm, u, te);
   for (int m = 0; m < 2; m++) {
-    g_dfA[2 * (size_t)k + m] = make_float4(ca[4 * m], ca[4 * m + 1], ca[4 * m + 2], ca[4 * m + 3]);
-    g_dfM[2 * (size_t)k + m] = make_float4(cm[4 * m], cm[4 * m + 1], cm[4 * m + 2], cm[4 * m + 3]);
+    A[2 * (size_t)k + m] = make_float4(ca[4 * m], ca[4 * m + 1], ca[4 * m + 2], ca[4 * m + 3]);
+    M[2 * (size_t)k + m] = make_float4(cm[4 * m], cm[4 * m + 1], cm[4 * m + 2], cm[4 * m + 3]);
   }
-  g_dfU[k] = make_float2(u[0], u[1]);
-  g_dfTE[k] = make_float2(te[0], te[1]);
+  U[k] = make_float2(u[0], u[1]);
+  TE[k] = make_float2(te[0], te[1]);
 }
-
-// the FP64 tables of the per-atom virial pass
-__device__ double g_va64[MAXELEM * MAXELEM * df::TAB64_N * 24];   // A, M, TE: 8 each per interval
-
-__global__ void k_fill_va_tables(int ne) {
+// the FP64 tables of the per-atom virial pass: A, M and TE, 8 doubles each per interval
+__global__ void k_fill_va_tables(int ne, double *tab) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= ne * ne * df::TAB64_N) return;
   const int p = k / df::TAB64_N, a = p / ne, b = p % ne;
   const IlpP<R> &q = c_pot.ilp[a * MAXELEM + b];
   const df::TabP t = {q.z0, q.lambda, 2.0 * q.eps_half, q.d, q.seff, q.C6, 1.0 / c_pot.i_inv_rcut, c_pot.tap};
-  double *o = g_va64 + 24 * (size_t)k;
+  double *o = tab + 24 * (size_t)k;
   df::tab64_fill(t, k % df::TAB64_N, o, o + 8, o + 16);
 }
 
@@ -2449,8 +2441,8 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
         if constexpr (!ONE) k += (ie * ne + A.el) * TAB_N;
         const D<V> off = fast_two_sum(th, q.l);
         Coef<V> c;
-        coef_set(c, g_dfM + 2 * k);
-        const float2 f0 = __ldg(g_dfTE + k);
+        coef_set(c, a.df_M + 2 * k);
+        const float2 f0 = __ldg(a.df_TE + k);
         weights(j, d, wv, wi, wj);
 #pragma unroll
         for (int x = 0; x < 3; x++) {
@@ -2498,7 +2490,7 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
           if constexpr (!ONE) k += (ie * ne + A.el) * TAB_N;
           const D<V> off = fast_two_sum(th, q.l);
           Coef<V> c;
-          coef_set(c, g_dfA + 2 * k);
+          coef_set(c, a.df_A + 2 * k);
           D<V> crad = tab_poly(c, off);
           const auto K = consts(A.el);
           if constexpr (EV || GH) {
@@ -2507,11 +2499,11 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
             const float wm = 0.5f * (wi + wj);
             const D<V> eps = mk(K(K_EPS), K(K_EPS + 1));
             Coef<V> cM;
-            coef_set(cM, g_dfM + 2 * k);
+            coef_set(cM, a.df_M + 2 * k);
             // A = vdW part + eps M: weights wv and (wi + wj) / 2
             if constexpr (GH) crad = add(scale(crad, wv), scale(mul(tab_poly(cM, off), eps), wm - wv));
             if constexpr (EV) {
-              const float2 u0 = __ldg(g_dfU + k), f0 = __ldg(g_dfTE + k);
+              const float2 u0 = __ldg(a.df_U + k), f0 = __ldg(a.df_TE + k);
               const D<V> te = mul(tab_integral(cM, f0.x, f0.y, off), eps);
               D<V> vdw = add(tab_integral(c, u0.x, u0.y, off), neg(te));
               if constexpr (GH) {
@@ -2615,8 +2607,7 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
   }
 }
 
-// constants and tables of the double-float kernel from the FP64 ones (c_pot's copy is queued
-// on s before this)
+// constants of the double-float kernel from the FP64 ones
 static void upload_pair_df(const PotConst<R> &p, cudaStream_t s) {
   static float rows[MAXELEM * MAXELEM * df::K_N];   // static: the asynchronous copies read them after return
   static DfCut cut;
@@ -2637,8 +2628,14 @@ static void upload_pair_df(const PotConst<R> &p, cudaStream_t s) {
   cudaMemcpyToSymbolAsync(c_dfcut, &cut, sizeof cut, 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(g_dfk, rows, sizeof rows, 0, cudaMemcpyHostToDevice, s);
   k_fill_exp2_df<<<1, df::EXP2_TAB, 0, s>>>();
-  k_fill_df_tables<<<(ne * ne * df::TAB_N + 63) / 64, 64, 0, s>>>(ne);
-  k_fill_va_tables<<<(ne * ne * df::TAB64_N + 63) / 64, 64, 0, s>>>(ne);
+}
+
+// the engine's tables from c_pot
+void fill_df_tables(int ne, float4 *A, float4 *M, float2 *U, float2 *TE, cudaStream_t s) {
+  k_fill_df_tables<<<(ne * ne * df::TAB_N + 63) / 64, 64, 0, s>>>(ne, A, M, U, TE);
+}
+void fill_va_tables(int ne, double *tab, cudaStream_t s) {
+  k_fill_va_tables<<<(ne * ne * df::TAB64_N + 31) / 32, 32, 0, s>>>(ne, tab);
 }
 
 template <bool ONE, bool GH>
@@ -3460,7 +3457,7 @@ __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
       weights(j, d, wv, wi, wj);
       const double q = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
       const IlpP<R> &p = c_pot.ilp[ie * MAXELEM + je];
-      const double *c = g_va64 + 24 * (size_t)((ie * ne + je) * df::TAB64_N + df::tab64_at(q, t));
+      const double *c = a.va64 + 24 * (size_t)((ie * ne + je) * df::TAB64_N + df::tab64_at(q, t));
       const double M = df::tab64_poly<6>(c + 8, t), TE = df::tab64_poly<7>(c + 16, t);
       double cr = df::tab64_poly<6>(c, t);
       if constexpr (GH) cr = fma(M * (2.0 * p.eps_half), 0.5 * (wi + wj) - wv, cr * wv);
@@ -3597,19 +3594,19 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
       if constexpr (!ONE) ki += (ie * ne + A.el) * TAB_N;
       const D<V> off = fast_two_sum(th, q.l);
       Coef<V> cc;
-      coef_set(cc, g_dfA + 2 * ki);
+      coef_set(cc, a.df_A + 2 * ki);
       D<V> crad = tab_poly(cc, off);
       const bool near = near_one(K(K_ND2), q.h, I.nh[0] * d[0].h + I.nh[1] * d[1].h + I.nh[2] * d[2].h,
                                  A.nh[0] * d[0].h + A.nh[1] * d[1].h + A.nh[2] * d[2].h);
       D<V> M, tp = mk(0.f, 0.f), tq = tp;
       if (GH || near) {
-        coef_set(cc, g_dfM + 2 * ki);
+        coef_set(cc, a.df_M + 2 * ki);
         M = tab_poly(cc, off);
       }
       if constexpr (GH)
         crad = add(scale(crad, wv), scale(mul(M, mk(K(K_EPS), K(K_EPS + 1))), 0.5f * (wi + wj) - wv));
       if (near) {
-        const float2 f0 = __ldg(g_dfTE + ki);
+        const float2 f0 = __ldg(a.df_TE + ki);
         D<V> S;
         pair_near<GH>(K, s_tab, q, tab_integral(cc, f0.x, f0.y, off), M, dot3(ni, d), dot3(nj, d), wi, wj, crad, tp,
                       tq, S);
