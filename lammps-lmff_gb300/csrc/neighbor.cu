@@ -117,6 +117,43 @@ __device__ __forceinline__ bool le_exact(float rsq, float thr, double thr64, con
   return r2 <= thr64;
 }
 
+// The part of a stencil row that can hold partners of an atom.  Bins are at least half the
+// list cutoff wide, so the +-2 stencil's square has twice the area of the cutoff's circle.
+// A bin other than the atom's own is at least its nearer edge away (also where atoms outside
+// the box in a non-periodic dimension were put into an edge bin: they lie beyond its far
+// edge).  Positions are hi parts, exact to 2^-23 of base; STENCIL_SLACK covers their rounding and
+// the bin index's.
+constexpr float STENCIL_SLACK = 0.02f;
+struct Stencil {
+  float r[3], bs[3], cutsq;
+  int b[3], reach;
+  __device__ __forceinline__ void set(const SysDesc &sd, const float4 &h, int bx, int by, int bz) {
+    const float off = (float)sd.base + 32.f;
+    r[0] = h.x - off;
+    r[1] = h.y - off;
+    r[2] = h.z - off;
+    for (int c = 0; c < 3; c++) bs[c] = (float)(1.0 / sd.binv[c]);
+    b[0] = bx;
+    b[1] = by;
+    b[2] = bz;
+    reach = sd.reach[0];
+    cutsq = sd.prefilt_sq;
+  }
+  // distance to bin u of dimension c
+  __device__ __forceinline__ float gap(int c, int u) const {
+    const float g = u > b[c] ? (float)u * bs[c] - r[c] : u < b[c] ? r[c] - (float)(u + 1) * bs[c] : 0.f;
+    return fmaxf(g - STENCIL_SLACK, 0.f);
+  }
+  // x bins [x0, x1] of row (y, z) (not wrapped into the box); empty where the row is out of reach
+  __device__ __forceinline__ void row(int y, int z, int &x0, int &x1) const {
+    const float gy = gap(1, y), gz = gap(2, z), left = cutsq - gy * gy - gz * gz;
+    const float w = sqrtf(fmaxf(left, 0.f)) + 2.f * STENCIL_SLACK;
+    x0 = max(b[0] - reach, min(b[0], (int)floorf((r[0] - w) / bs[0])));
+    x1 = min(b[0] + reach, max(b[0], (int)floorf((r[0] + w) / bs[0])));
+    if (left < 0.f) x1 = x0 - 1;
+  }
+};
+
 // One warp per 32 consecutive atoms of the sorted order, one lane per atom.  Atoms are
 // sorted by bin and bins are numbered x fastest, so the lanes of a warp almost always
 // share one bin row (same system, y and z bin) and sit in one or two neighbouring x
@@ -305,107 +342,166 @@ __global__ void __launch_bounds__(32 * LW) k_list(NbArgs a) {
 }
 
 
-// One warp per atom, for small systems: the lanes take 32 consecutive candidates of the
-// atom's stencil at a time (the bins and the order of k_list's walk for that atom), and
-// ballots give every accepted entry its place -- inner entries from the front, the skin
-// shell from the back, short candidates in order -- so the lists equal k_list's entry for
-// entry.  k_list's warp walks its 32 atoms' stencils one candidate at a time, a serial
-// chain that the few warps of a small system cannot hide (7,200 atoms: 225 warps, about
-// 0.5 ms per build).  Per build, this kernel against k_list: 7,200-atom bilayer 0.26 vs
-// 0.62 ms, 36,800-atom graphite 1.61 vs 1.94 ms, 331,200-atom graphite 12.8 vs 5.2 ms
-// (there k_list's shared tiles save most candidate loads).
-constexpr int LIST_ATOM_MAX_ATOMS = 40000;
+// One warp per atom, for small systems: the atom's stencil in k_list's order, so that the
+// lists equal k_list's entry for entry.  A bin row's atoms are contiguous (bins are numbered
+// x fastest), so the stencil is a few runs of atoms, one per row and image; the lanes look up
+// 32 of them at once.  A run is tested 32 candidates at a time on the hi parts and the
+// molecule alone, ~25 instructions; what passes (one in five) is queued in order, and whole
+// warps of queued candidates take the exact tests and get their places by ballots -- inner
+// entries from the front, the skin shell from the back, short candidates in order.
+// Testing each bin's candidates exactly in place cost ~190 instructions per 32 of them.
+// k_list's warp walks its 32 atoms' stencils one candidate at a time, a serial chain that the
+// few warps of a small system cannot hide; its shared tiles pay in large ones.  A rebuild
+// (with the sort and the copy to the list; in place / here / k_list): 1,152 atoms 0.19 / 0.16 /
+// 0.89 ms, 5,040-atom bilayer 0.25 / 0.20 / 0.62, 36,800-atom slab 1.90 / 1.04 / 2.28,
+// 60,480-atom bilayer - / 0.66 / 0.78, 81,200-atom slab - / 2.04 / 2.52, 300,240-atom bilayer
+// - / 2.58 / 1.98.  Bound by instruction issue (occupancy of 20 to 40 warps made no
+// difference).
+constexpr int LIST_ATOM_MAX_ATOMS = 65536;
+constexpr int LIST_QUEUE = 64;
+__device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+
 template <int MODE>
 __global__ void __launch_bounds__(128) k_list_atom(NbArgs a) {
   constexpr bool FILL = MODE != 0;
+  __shared__ uint32_t s_queue[4][LIST_QUEUE];
   const int i = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= a.n) return;   // whole warps
+  uint32_t *const queue = s_queue[threadIdx.x >> 5];
   const unsigned FULL = 0xffffffffu, below = (1u << lane) - 1u;
   const SysDesc &sd = a.sys[a.sysid[i]];
-  const int lb = (int)(a.bin_key[i] >> KEY_MOL_BITS) - sd.bin_begin;
-  const int bx = lb % sd.nb[0], by = (lb / sd.nb[0]) % sd.nb[1], bz = lb / (sd.nb[0] * sd.nb[1]);
   const float4 hi = a.xh[i], lo = a.xl[i];
   const int infoi = __float_as_int(hi.w);
   const int ti = infoi & 255;
   const int mi = infoi >> 8;
   const int ilp_i = c_nb.ilp_mapped[ti];
   const float prefilt = sd.prefilt_sq;
+  // the short cutoff with prefilt_sq's allowance for the hi parts (2^-19 base), and another
+  // for this sum
+  const float rs = sqrtf(c_nb.rshortsq_f) + (float)sd.base * 0x1p-18f;
+  const float preshort = rs * rs * 1.0001f;
   int nlong = 0, nin = 0, nsh = 0, nshort = 0;
   bool img = false;
   const int64_t base = MODE == 1 ? a.list_off[i] : MODE == 2 ? (int64_t)i * a.stride : 0;
   const int64_t lend = MODE == 1 ? a.list_off[i + 1] : MODE == 2 ? base + a.stride : 0;
   uint32_t *const dst = MODE == 2 ? a.tmp : a.list;
   const int64_t dcap = MODE == 2 ? (int64_t)a.n * a.stride : a.list_cap;
-  for (int dz = -sd.reach[2]; dz <= sd.reach[2]; dz++) {
-    int jz = bz + dz, sz = 0;
-    if (sd.per[2]) {
-      sz = jz >= 0 ? jz / sd.nb[2] : -((-jz + sd.nb[2] - 1) / sd.nb[2]);
-      jz -= sz * sd.nb[2];
-    } else if (jz < 0 || jz >= sd.nb[2]) continue;
-    for (int dy = -sd.reach[1]; dy <= sd.reach[1]; dy++) {
-      int jy = by + dy, sy = 0;
-      if (sd.per[1]) {
-        sy = jy >= 0 ? jy / sd.nb[1] : -((-jy + sd.nb[1] - 1) / sd.nb[1]);
-        jy -= sy * sd.nb[1];
-      } else if (jy < 0 || jy >= sd.nb[1]) continue;
-      if (a.rowocc && !a.rowocc[sd.bin_begin + (jz * sd.nb[1] + jy) * sd.nb[0]]) continue;   // empty row
-      for (int xu = bx - sd.reach[0]; xu <= bx + sd.reach[0]; xu++) {
-        int jx = xu, sx = 0;
-        if (sd.per[0]) {
-          sx = jx >= 0 ? jx / sd.nb[0] : -((-jx + sd.nb[0] - 1) / sd.nb[0]);
-          jx -= sx * sd.nb[0];
-        } else if (jx < 0 || jx >= sd.nb[0]) continue;
-        const int gbj = sd.bin_begin + (jz * sd.nb[1] + jy) * sd.nb[0] + jx;
-        const int jstart = a.bin_start[gbj], jend = a.bin_end[gbj];
-        const float shx = (float)sx * sd.Lhi[0], shy = (float)sy * sd.Lhi[1], shz = (float)sz * sd.Lhi[2];
-        const float slx = (float)sx * sd.Llo[0], sly = (float)sy * sd.Llo[1], slz = (float)sz * sd.Llo[2];
-        const bool self_image = (sx | sy | sz) == 0;
-        for (int j0 = jstart; j0 < jend; j0 += 32) {
-          const int j = j0 + lane;
-          bool take_long = false, inner = false, take_short = false;
-          if (j < jend) {
-            const float4 hj = a.xh[j];
-            const float hx = (hi.x - hj.x) - shx, hy = (hi.y - hj.y) - shy, hz = (hi.z - hj.z) - shz;
-            if (!(hx * hx + hy * hy + hz * hz > prefilt)) {
-              const float4 lj = a.xl[j];
-              float ddx = hx + ((lo.x - lj.x) - slx);
-              float ddy = hy + ((lo.y - lj.y) - sly);
-              float ddz = hz + ((lo.z - lj.z) - slz);
-              float rsq = ddx * ddx + ddy * ddy + ddz * ddz;
-              const int infoj = __float_as_int(hj.w);
-              const int tj = infoj & 255;
-              const int mj = infoj >> 8;
-              const int tt = ti * (MAXTYPE + 1) + tj;
-              if ((a.full || (mj != mi && ilp_i && c_nb.ilp_mapped[tj])) && !(self_image && j == i))
-                take_long = le_exact(rsq, c_nb.cutnsq_f[tt], c_nb.cutnsq_d[tt], a.xq, sd, i, j, sx, sy, sz);
-              inner = rsq < c_nb.innersq_f;
-              if (MODE != 1 && !(self_image && j == i))
-                take_short = le_exact(rsq, c_nb.rshortsq_f, c_nb.rshortsq_d, a.xq, sd, i, j, sx, sy, sz);
+  int qh = 0, qn = 0;
+  // the next (up to) 32 queued candidates
+  auto batch = [&]() {
+    __syncwarp();
+    bool take_long = false, inner = false, take_short = false, image = false;
+    uint32_t e = 0;
+    if (qh + lane < qn) {
+      e = queue[(qh + lane) & (LIST_QUEUE - 1)];
+      int j, sx, sy, sz;
+      decode_entry(e, a.lc, j, sx, sy, sz);
+      const float4 hj = a.xh[j], lj = a.xl[j];
+      const float shx = (float)sx * sd.Lhi[0], shy = (float)sy * sd.Lhi[1], shz = (float)sz * sd.Lhi[2];
+      const float slx = (float)sx * sd.Llo[0], sly = (float)sy * sd.Llo[1], slz = (float)sz * sd.Llo[2];
+      const bool self_image = (sx | sy | sz) == 0;
+      const float hx = (hi.x - hj.x) - shx, hy = (hi.y - hj.y) - shy, hz = (hi.z - hj.z) - shz;
+      float ddx = hx + ((lo.x - lj.x) - slx);
+      float ddy = hy + ((lo.y - lj.y) - sly);
+      float ddz = hz + ((lo.z - lj.z) - slz);
+      float rsq = ddx * ddx + ddy * ddy + ddz * ddz;
+      const int infoj = __float_as_int(hj.w);
+      const int tj = infoj & 255;
+      const int mj = infoj >> 8;
+      const int tt = ti * (MAXTYPE + 1) + tj;
+      if ((a.full || (mj != mi && ilp_i && c_nb.ilp_mapped[tj])) && !(self_image && j == i))
+        take_long = le_exact(rsq, c_nb.cutnsq_f[tt], c_nb.cutnsq_d[tt], a.xq, sd, i, j, sx, sy, sz);
+      inner = rsq < c_nb.innersq_f;
+      image = !self_image;
+      if (MODE != 1 && !(self_image && j == i))
+        take_short = le_exact(rsq, c_nb.rshortsq_f, c_nb.rshortsq_d, a.xq, sd, i, j, sx, sy, sz);
+    }
+    qh = min(qh + 32, qn);
+    const unsigned bin_ = __ballot_sync(FULL, take_long && inner);
+    const unsigned bsh_ = __ballot_sync(FULL, take_long && !inner);
+    if (FILL && take_long) {
+      const int64_t pos = inner ? base + nin + __popc(bin_ & below) : lend - 1 - (nsh + __popc(bsh_ & below));
+      if (pos >= base && pos < lend && pos < dcap) dst[pos] = e;
+    }
+    if (MODE != 1) {
+      const unsigned bs = __ballot_sync(FULL, take_short);
+      if (take_short) {
+        const int q = nshort + __popc(bs & below);
+        if (q < MAXSHORT) a.short_nb[(size_t)i * MAXSHORT + q] = e;
+      }
+      nshort += __popc(bs);
+    }
+    nin += __popc(bin_);
+    nsh += __popc(bsh_);
+    nlong += __popc(bin_ | bsh_);
+    if (FILL) img |= __any_sync(FULL, take_long && image);
+    __syncwarp();
+  };
+  // the stencil's runs: (dz, dy) rows, each in as many x images as its bins span
+  const int nbx = sd.nb[0], nby = sd.nb[1], nbz = sd.nb[2], rx = sd.reach[0], ry = sd.reach[1], rz = sd.reach[2];
+  const int lb = (int)(a.bin_key[i] >> KEY_MOL_BITS) - sd.bin_begin;
+  const int bx = lb % nbx, by = (lb / nbx) % nby, bz = lb / (nbx * nby);
+  Stencil st;
+  st.set(sd, hi, bx, by, bz);
+  const int s0 = sd.per[0] ? floor_div(bx - rx, nbx) : 0;
+  const int ns = sd.per[0] ? floor_div(bx + rx, nbx) - s0 + 1 : 1;
+  const int ny = 2 * ry + 1, nruns = (2 * rz + 1) * ny * ns;
+  for (int t0 = 0; t0 < nruns; t0 += 32) {
+    const int t = t0 + lane;
+    int js = INT_MAX, je = 0;   // this lane's run of the 32
+    uint32_t image = 0;
+    if (t < nruns) {
+      const int sx = s0 + t % ns;
+      int jy = by + (t / ns) % ny - ry, jz = bz + t / (ns * ny) - rz, x0, x1;
+      st.row(jy, jz, x0, x1);
+      x0 = max(x0 - sx * nbx, 0);
+      x1 = min(x1 - sx * nbx, nbx - 1);
+      const int sy = sd.per[1] ? floor_div(jy, nby) : 0, sz = sd.per[2] ? floor_div(jz, nbz) : 0;
+      jy -= sy * nby;
+      jz -= sz * nbz;
+      image = encode_entry(0, sx, sy, sz, a.lc);
+      if (x0 <= x1 && jz >= 0 && jz < nbz && jy >= 0 && jy < nby) {
+        const int row = sd.bin_begin + (jz * nby + jy) * nbx;
+        if (!a.rowocc || a.rowocc[row]) {
+          for (int x = x0; x <= x1; x++) {
+            const int b0 = a.bin_start[row + x], b1 = a.bin_end[row + x];
+            if (b1 > b0) {
+              js = min(js, b0);
+              je = max(je, b1);
             }
           }
-          const unsigned bin_ = __ballot_sync(FULL, take_long && inner);
-          const unsigned bsh_ = __ballot_sync(FULL, take_long && !inner);
-          if (FILL && take_long) {
-            const int64_t pos = inner ? base + nin + __popc(bin_ & below) : lend - 1 - (nsh + __popc(bsh_ & below));
-            if (pos >= base && pos < lend && pos < dcap) dst[pos] = encode_entry(j, sx, sy, sz, a.lc);
-          }
-          if (MODE != 1) {
-            const unsigned bs = __ballot_sync(FULL, take_short);
-            if (take_short) {
-              const int q = nshort + __popc(bs & below);
-              if (q < MAXSHORT) a.short_nb[(size_t)i * MAXSHORT + q] = encode_entry(j, sx, sy, sz, a.lc);
-            }
-            nshort += __popc(bs);
-          }
-          nin += __popc(bin_);
-          nsh += __popc(bsh_);
-          nlong += __popc(bin_ | bsh_);
-          if ((bin_ | bsh_) && !self_image) img = true;
         }
       }
     }
+    unsigned runs = __ballot_sync(FULL, js < je);
+    while (runs) {
+      const int l = __ffs(runs) - 1;
+      runs &= runs - 1u;
+      const int j0 = __shfl_sync(FULL, js, l), j1 = __shfl_sync(FULL, je, l);
+      const uint32_t shift = __shfl_sync(FULL, image, l);
+      int j, sx, sy, sz;
+      decode_entry(shift, a.lc, j, sx, sy, sz);
+      const float shx = (float)sx * sd.Lhi[0], shy = (float)sy * sd.Lhi[1], shz = (float)sz * sd.Lhi[2];
+      float4 next = a.xh[min(j0 + lane, j1 - 1)];
+      for (int jt = j0; jt < j1; jt += 32) {
+        j = jt + lane;
+        const float4 hj = next;
+        if (jt + 32 < j1) next = a.xh[min(j + 32, j1 - 1)];
+        bool pass = false;
+        if (j < j1) {
+          const float hx = (hi.x - hj.x) - shx, hy = (hi.y - hj.y) - shy, hz = (hi.z - hj.z) - shz;
+          const float d2 = hx * hx + hy * hy + hz * hz;
+          pass = !(d2 > prefilt) && (a.full || (__float_as_int(hj.w) >> 8) != mi || (MODE != 1 && !(d2 > preshort)));
+        }
+        const unsigned m = __ballot_sync(FULL, pass);
+        if (pass) queue[(qn + __popc(m & below)) & (LIST_QUEUE - 1)] = (uint32_t)j | shift;
+        qn += __popc(m);
+        if (qn - qh >= 32) batch();
+      }
+    }
   }
+  if (qh < qn) batch();
   if (lane != 0) return;
   if (MODE != 1) {
     a.cnt[i] = nlong;
