@@ -2218,7 +2218,7 @@ __global__ void __launch_bounds__(256, (ilp_min_blocks<TPA, EV, EATOM, ONE, GH, 
 // and there is no FP64 instruction in the loop; displacements come from three-part
 // positions whose leading parts subtract exactly.
 // (Pair kernel against the FP64 form: 331,200-atom slab with energies and virial 79.3 ->
-// 8.0 ms, 7,200-atom bilayer, forces, 786 -> 68 us, 5,016 atoms in six layers 2,010 -> 149 us.)
+// 7.85 ms, 7,200-atom bilayer, forces, 786 -> 66 us, 5,016 atoms in six layers 2,010 -> 146 us.)
 // The error of a pair's force against 64-bit arithmetic is below the FP64 form's, whose
 // 1/sqrt and 1/x are one FP64 Newton step from an FP32 estimate (CPU emulation against
 // 113-bit arithmetic, rms over 200,000 pairs of BNCH.ILP's element pairs: 2-5e-14 of the
@@ -2469,11 +2469,13 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
       if (on) qh = min(qh + tpa, qn);
       __syncwarp();
     };
+    // the list is read a round ahead, so that an entry's record does not wait for it
+    uint32_t ahead = lane < cnt ? __ldg(&lst[lane]) : 0;
     for (int k0 = 0, it = 1; k0 < most; k0 += tpa, it++) {
       bool near = false;
-      uint32_t e = 0;
+      const uint32_t e = ahead;
+      if (k0 + tpa + lane < cnt) ahead = __ldg(&lst[k0 + tpa + lane]);
       if (k0 + lane < cnt) {
-        e = __ldg(&lst[k0 + lane]);
         DfAtom A;
         int j;
         D<V> d[3];
@@ -3322,8 +3324,8 @@ __global__ void __launch_bounds__(128) k_va_ilp(ForceArgs<R> a) {
 // 1.6e-13, 5e-14, which would be less than k_va_ilp gave.  VA_LANES lanes per atom share its
 // list; the atom's g_i and G_i go to its slot storage, from which k_va_slots forms the slots
 // with full warps.  36,800-atom slab: k_va_ilp 30 ms (one thread per atom, ~500 FP64
-// instructions a pair); k_va_near 1.67 ms, FP64 pipe (~190 instructions for ~85 pairs an
-// atom), k_va_far 1.22 ms, FP32 issue.
+// instructions a pair); k_va_near 1.60 ms, FP64 pipe (~190 instructions for ~85 pairs an
+// atom), k_va_far 1.15 ms, FP32 issue.
 constexpr int VA_LANES = 8;
 constexpr float VA_NEARSQ = 49.f;
 static_assert(VA_NEARSQ <= df::Q64_MAX, "the FP64 tables end at Q64_MAX");
@@ -3491,11 +3493,12 @@ __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
     if (on) qh = min(qh + VA_LANES, qn);
     __syncwarp();
   };
+  uint32_t ahead = lane < cnt ? __ldg(&a.list[b + lane]) : 0;   // the list a round ahead
   for (int k0 = 0, it = 1; k0 < most; k0 += VA_LANES, it++) {
     bool near = false;
-    uint32_t e = 0;
+    const uint32_t e = ahead;
+    if (k0 + VA_LANES + lane < cnt) ahead = __ldg(&a.list[b + k0 + VA_LANES + lane]);
     if (k0 + lane < cnt) {
-      e = __ldg(&a.list[b + k0 + lane]);
       int j, sx, sy, sz;
       decode_entry(e, a.lc, j, sx, sy, sz);
       DfAtom A;
@@ -3565,8 +3568,11 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
 #pragma unroll
     for (int c = 0; c < 3; c++) ni[c] = mk(I.nh[c], I.nl[c]);
     const int64_t q1 = a.list_off[i + 1];
-    for (int64_t k = a.list_off[i] + lane; k < q1; k += VA_LANES) {
-      const uint32_t e = __ldg(&a.list[k]);
+    int64_t k = a.list_off[i] + lane;
+    uint32_t ahead = k < q1 ? __ldg(&a.list[k]) : 0;   // the list a round ahead
+    for (; k < q1; k += VA_LANES) {
+      const uint32_t e = ahead;
+      if (k + VA_LANES < q1) ahead = __ldg(&a.list[k + VA_LANES]);
       int j, sx, sy, sz;
       decode_entry(e, a.lc, j, sx, sy, sz);
       DfAtom A;
@@ -3805,9 +3811,12 @@ __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
     const long long itag = a.tag[i];
     const float4 ni = a.nrm32[i];
     const int64_t q1 = a.list_off[i + 1];
-    for (int64_t q = a.list_off[i] + lane; q < q1; q += VA_LANES) {
+    int64_t q = a.list_off[i] + lane;
+    uint32_t ahead = q < q1 ? __ldg(&a.list[q]) : 0;   // the list a round ahead
+    for (; q < q1; q += VA_LANES) {
       int j, sx, sy, sz;
-      decode_entry(a.list[q], a.lc, j, sx, sy, sz);
+      decode_entry(ahead, a.lc, j, sx, sy, sz);
+      if (q + VA_LANES < q1) ahead = __ldg(&a.list[q + VA_LANES]);
       R dx, dy, dz;
       long long jinfo;
       ai.disp(a.A, sd, j, sx, sy, sz, dx, dy, dz, jinfo);
