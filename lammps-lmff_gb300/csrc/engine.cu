@@ -209,14 +209,18 @@ __global__ void k_unpermute_state(int n, const int *perm, const d4 *xq, const do
 // else is in its batch.  One block per quantity took 70 us for 36,800 atoms (a chain of
 // ~0.5 us loads) and grew with n; REDUCE_MEASURED.
 constexpr int RED_THREADS = 256, RED_CHUNK = 8 * RED_THREADS;
+// sum over the block, in thread 0
 __device__ __forceinline__ double block_sum(double acc, double *sh) {
   sh[threadIdx.x] = acc;
   __syncthreads();
-  for (int o = RED_THREADS / 2; o > 0; o >>= 1) {
+  for (int o = RED_THREADS / 2; o >= 32; o >>= 1) {
     if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
     __syncthreads();
   }
-  return sh[0];
+  double v = sh[threadIdx.x];
+  if (threadIdx.x < 32)
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
 }
 __global__ void __launch_bounds__(RED_THREADS) k_reduce(int n, int nq, const double *const *arrs, const SysDesc *sys,
                                                         double *out, int cmax, double *part, int *count) {
@@ -1131,7 +1135,7 @@ struct Engine {
       CK(dalloc(d_dfU, df_intervals())); CK(dalloc(d_dfTE, df_intervals()));
     }
     CK(cudaMemsetAsync(d.status, 0, sizeof(int), stream));
-    return LMFF_OK;
+    return ensure_stream2();   // here: lmff_compute_device_noalloc uses it and may not create it
   }
 
   // The device's constant tables are this engine's (guaranteed by DeviceCall); only the
@@ -3268,7 +3272,8 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
   SysDesc *dsys = cv.take<SysDesc>(1);
   double *red = cv.take<double>(16);
   double **arrs = cv.take<double *>(2);
-  int *status = cv.take<int>(1);
+  cv.take<int>(1);
+  int *status = reinterpret_cast<int *>(list_off + nn + 1);   // beside the list's total (the piece is padded)
   size_t tmp_bytes = nb_sort_tmp_bytes(c, 32);
   void *tmp = cv.take<unsigned char>(tmp_bytes);
   if (!tmp) return g.fail(LMFF_EOVERFLOW, "lmff_compute_device_noalloc: scratch layout does not fit");
@@ -3277,11 +3282,16 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
   // what must start at zero: status word, bin ranges, the count past the last atom
   const double *host_arrs[2] = {stat_ilp, stat_ters};
   CK2(cudaMemsetAsync(status, 0, sizeof(int), st));
-  CK2(cudaMemsetAsync(bin_start, 0, sizeof(int) * nbins, st));
-  CK2(cudaMemsetAsync(bin_end, 0, sizeof(int) * nbins, st));
+  CK2(cudaMemsetAsync(bin_start, 0, sizeof(int) * (size_t)(bin_end - bin_start + nbins), st));   // both: neighbours
   CK2(cudaMemsetAsync(cnt + nn, 0, sizeof(int64_t), st));
-  CK2(cudaMemcpyAsync(dsys, &sd, sizeof sd, cudaMemcpyHostToDevice, st));
-  CK2(cudaMemcpyAsync(arrs, host_arrs, sizeof host_arrs, cudaMemcpyHostToDevice, st));
+  // the system and the table of arrays lie close together: one copy
+  unsigned char head[2048];
+  const size_t arrs_at = (size_t)(reinterpret_cast<unsigned char *>(arrs) - reinterpret_cast<unsigned char *>(dsys));
+  static_assert(sizeof(SysDesc) + 16 * sizeof(double) + 512 + sizeof host_arrs <= sizeof head, "head of the scratch");
+  memset(head, 0, sizeof head);
+  memcpy(head, &sd, sizeof sd);
+  memcpy(head + arrs_at, host_arrs, sizeof host_arrs);
+  CK2(cudaMemcpyAsync(dsys, head, arrs_at + sizeof host_arrs, cudaMemcpyHostToDevice, st));
   int gb = (nn + 255) / 256;
   k_load<<<gb, 256, 0, st>>>(nn, dx, dtype, dmol, nullptr, nullptr, nullptr, nullptr, xq, tag, perm, sysid, v, mass);
   nb_wrap_bin(nn, xq, dsys, sysid, key, idx, st);
@@ -3311,15 +3321,32 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
   na.lc = lc;
   na.full = g.list_full;
   na.status = status;
-  nb_list(na, 0, st);
+  // one walk over the candidates: entries and counts together, into equal shares of the
+  // list space's upper half, from where they are copied to the list in the lower one.  A list
+  // that does not fit that way is walked a second time instead, into the whole space.
+  const size_t half = list_cap / 2;
+  na.tmp = list + (list_cap - half);
+  na.stride = (int)std::min<size_t>(half / nn, 1 << 20);
+  na.nin = reinterpret_cast<int *>(eat_t);   // not used before the Tersoff kernel
+  nb_list(na, 2, st);
   CK2(nb_scan(tmp, tmp_bytes, cnt, list_off, nn, st));
-  int64_t total = 0;
-  CK2(cudaMemcpyAsync(&total, list_off + nn, sizeof total, cudaMemcpyDeviceToHost, st));
+  struct {
+    int64_t total;
+    int status, pad;
+  } built = {0, 0, 0};
+  CK2(cudaMemcpyAsync(&built, list_off + nn, sizeof built, cudaMemcpyDeviceToHost, st));
   CK2(cudaStreamSynchronize(st));
+  const int64_t total = built.total;
   if (total < 0 || (size_t)total > list_cap)
     return g.fail(LMFF_EOVERFLOW, "lmff_compute_device_noalloc: pair list of " + std::to_string(total) +
                                       " entries exceeds the scratch capacity of " + std::to_string(list_cap));
-  nb_list(na, 1, st);
+  if ((built.status & ST_STRIDE_OVERFLOW) || (size_t)total > list_cap - half) {
+    built.status &= ~(ST_STRIDE_OVERFLOW | ST_LIST_OVERFLOW);
+    CK2(cudaMemcpyAsync(status, &built.status, sizeof built.status, cudaMemcpyHostToDevice, st));
+    nb_list(na, 1, st);
+  } else {
+    nb_compact(na, (int64_t)(list_cap - half), st);
+  }
   auto fill = [&](auto &a) {
     memset(&a, 0, sizeof a);
     a.A.xq = xq2;
@@ -3369,11 +3396,25 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     a.ters_rlosq = g.ters_rlosq;
   };
   const bool ev = true;
+  // the Tersoff kernel beside the interlayer ones, as in the resident path (1,152 atoms: 27
+  // of ~190 us of kernels, on a few warps)
+  auto beside = [&](const auto &a) { return a.do_ters && a.do_ilp && g.ters_concurrent && g.stream2; };
+  auto fork = [&](const auto &a) {
+    if (!beside(a)) return st;
+    cudaEventRecord(g.ev_fork, st);
+    cudaStreamWaitEvent(g.stream2, g.ev_fork, 0);
+    return g.stream2;
+  };
+  auto join = [&](const auto &a) {
+    if (!beside(a)) return;
+    cudaEventRecord(g.ev_join, g.stream2);
+    cudaStreamWaitEvent(st, g.ev_join, 0);
+  };
   if (g.precision == LMFF_FP64) {
     ForceArgs<double> a;
     fill(a);
     f64::launch_short(a, g.d_cutILPsq, g.ht.cutmax * g.ht.cutmax, st);
-    if (a.do_ters) f64::launch_tersoff(a, ev, false, st);
+    if (a.do_ters) f64::launch_tersoff(a, ev, false, fork(a));
     else CK2(cudaMemsetAsync(stat_ters, 0, sizeof(double) * 8 * (size_t)nn, st));
     if (a.do_ilp) {
       f64::launch_nframe(a, st);
@@ -3382,12 +3423,13 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     } else {
       CK2(cudaMemsetAsync(stat_ilp, 0, sizeof(double) * 8 * (size_t)nn, st));
     }
+    join(a);
     f64::launch_finish(a, false, nullptr, st);
   } else {
     ForceArgs<float> a;
     fill(a);
     f32::launch_short(a, g.d_cutILPsq, g.ht.cutmax * g.ht.cutmax, st);
-    if (a.do_ters) f32::launch_tersoff(a, ev, false, st);
+    if (a.do_ters) f32::launch_tersoff(a, ev, false, fork(a));
     else CK2(cudaMemsetAsync(stat_ters, 0, sizeof(double) * 8 * (size_t)nn, st));
     if (a.do_ilp) {
       f32::launch_ilp(a, ev, false, g.tpa, g.block, g.i_one, st);
@@ -3395,6 +3437,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     } else {
       CK2(cudaMemsetAsync(stat_ilp, 0, sizeof(double) * 8 * (size_t)nn, st));
     }
+    join(a);
     f32::launch_finish(a, false, nullptr, st);
   }
   k_reduce<<<16, RED_THREADS, 0, st>>>(nn, 16, (const double *const *)arrs, dsys, red, 1, nullptr, nullptr);
