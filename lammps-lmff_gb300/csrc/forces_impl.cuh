@@ -3324,8 +3324,9 @@ __global__ void __launch_bounds__(128) k_va_ilp(ForceArgs<R> a) {
 // 1.6e-13, 5e-14, which would be less than k_va_ilp gave.  VA_LANES lanes per atom share its
 // list; the atom's g_i and G_i go to its slot storage, from which k_va_slots forms the slots
 // with full warps.  36,800-atom slab: k_va_ilp 30 ms (one thread per atom, ~500 FP64
-// instructions a pair); k_va_near 1.60 ms, FP64 pipe (~190 instructions for ~85 pairs an
-// atom), k_va_far 1.15 ms, FP32 issue.
+// instructions a pair); k_va_near 1.07 ms, FP64 pipe (~190 instructions for ~85 pairs an
+// atom; 1.60 ms with batches every third round, when few of the warp's atoms had one), k_va_far
+// 1.15 ms, FP32 issue.
 constexpr int VA_LANES = 8;
 constexpr float VA_NEARSQ = 49.f;
 static_assert(VA_NEARSQ <= df::Q64_MAX, "the FP64 tables end at Q64_MAX");
@@ -3401,14 +3402,15 @@ __device__ __noinline__ void va_close_pairs(const ForceArgs<R> &a, int i, int la
 template <bool GH>
 __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
   const unsigned FULL = 0xffffffffu;
-  __shared__ uint32_t s_queue[128 * 4];
+  constexpr int QUEUE = 8 * VA_LANES;   // entries per atom
+  __shared__ uint32_t s_queue[128 * 8];
   const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) / VA_LANES;
   const bool valid = i0 < a.n;
   const int i = valid ? i0 : a.n - 1;
   const int lane = threadIdx.x & (VA_LANES - 1);
   const unsigned gmask = ((1u << VA_LANES) - 1) << ((threadIdx.x & 31) & ~(VA_LANES - 1));
   const unsigned below = gmask & ((1u << (threadIdx.x & 31)) - 1u);
-  uint32_t *const queue = s_queue + 4 * (threadIdx.x & ~(VA_LANES - 1));
+  uint32_t *const queue = s_queue + 8 * (threadIdx.x & ~(VA_LANES - 1));
   const SysDesc &sd = a.A.sys[a.A.sysid[i]];
   const d4 xi = a.A.xq[i], ni = a.nrm64[i];
   const int ie = c_pot.i_map[info_type(__double_as_longlong(xi.w))];
@@ -3455,7 +3457,7 @@ __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
     if (on && qh + lane < qn) {
       int j, je;
       double d[3], wv = 1.0, wi = 1.0, wj = 1.0, t;
-      pair_of(queue[(qh + lane) & (4 * VA_LANES - 1)], j, je, d);
+      pair_of(queue[(qh + lane) & (QUEUE - 1)], j, je, d);
       weights(j, d, wv, wi, wj);
       const double q = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
       const IlpP<R> &p = c_pot.ilp[ie * MAXELEM + je];
@@ -3494,7 +3496,7 @@ __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
     __syncwarp();
   };
   uint32_t ahead = lane < cnt ? __ldg(&a.list[b + lane]) : 0;   // the list a round ahead
-  for (int k0 = 0, it = 1; k0 < most; k0 += VA_LANES, it++) {
+  for (int k0 = 0; k0 < most; k0 += VA_LANES) {
     bool near = false;
     const uint32_t e = ahead;
     if (k0 + VA_LANES + lane < cnt) ahead = __ldg(&a.list[b + k0 + VA_LANES + lane]);
@@ -3511,10 +3513,12 @@ __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
       }
     }
     const unsigned bits = __ballot_sync(FULL, near);
-    if (near) queue[(qn + __popc(bits & below)) & (4 * VA_LANES - 1)] = e;
+    if (near) queue[(qn + __popc(bits & below)) & (QUEUE - 1)] = e;
     qn += __popc(bits & gmask);
-    if (it % 3 == 0)
-      while (__any_sync(FULL, qn - qh >= VA_LANES)) near_batch(qn - qh >= VA_LANES);
+    // whole batches once an atom's queue could overflow: by then the warp's other atoms have
+    // theirs too.  A batch is VA_LANES entries of the list in order, whenever it is taken
+    if (__any_sync(FULL, qn - qh > QUEUE - VA_LANES))
+      for (int k = 0; k < 6; k++) near_batch(qn - qh >= VA_LANES);
   }
   while (__any_sync(FULL, qh < qn)) near_batch(true);
 #pragma unroll
