@@ -894,10 +894,11 @@ __device__ __forceinline__ double ln_t64(double x) {
 // the two is the term's own bond, and on s along e_k - cos e_s), and g(theta) without the
 // cancellation of two ~1e8 terms (c^2/d^2 - c^2/(d^2 + u^2) = c^2 u^2/(d^2 (d^2 + u^2))).
 // Bound by the FP64 pipe: with energies and virial 1,267 -> 377 us on 331k atoms, 26 us of
-// latency at 5k.  Against 80-bit arithmetic the forces' error is 0.9e-14 where the general
-// routine's is 1.2e-14.
+// latency at 5k; the per-atom virial's pass 160 -> 58 us on 36,800.  Against 80-bit arithmetic
+// the forces' error is 0.9e-14 where the general routine's is 1.2e-14, the per-atom virial's
+// 1.0e-14 where it is 1.5e-14.
 // Returns false, nothing written, for an atom it does not take.
-template <bool EV, bool GH>
+template <bool EV, bool GH, bool VA>
 __device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int ie, int cnt) {
   if (cnt < 2 || cnt > 3 || !(a.ters_rlosq > 0.0)) return false;
   const SysDesc &sd = a.A.sys[a.A.sysid[i]];
@@ -983,17 +984,43 @@ __device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int i
     }
   }
   // ---- forces on the partners: radial, then three-body
-  double t[3][3];
+  double t[3][3], vo[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, vs[VA ? 3 : 1][6];   // VA: tersoff_atom's shares
 #pragma unroll
-  for (int s = 0; s < 3; s++)
+  for (int s = 0; s < 3; s++) {
 #pragma unroll
     for (int c = 0; c < 3; c++) t[s][c] = 0.0;
+    if constexpr (VA) {
+      // half of the repulsion's and of the bond term's del (x) f here, of the latter at the partner
+      constexpr int P[6] = {0, 1, 2, 0, 0, 1}, Q[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+      for (int c = 0; c < 6; c++) {
+        vs[s][c] = s < cnt ? -0.5 * fp2[s] * (d[s][P[c]] * d[s][Q[c]]) : 0.0;
+        if (s < cnt) vo[c] += fma(hw[s], d[s][P[c]] * d[s][Q[c]], vs[s][c]);
+      }
+    }
+  }
 #pragma unroll
   for (int s = 0; s < 3; s++) {
 #pragma unroll
     for (int k = s + 1; k < 3; k++) {
       if (k < cnt) {
         const double q = fma(pref[s], gd[s][k], pref[k] * gd[k][s]), qs = q * ri[s], qk = q * ri[k], c = cs[s][k];
+        if constexpr (VA) {   // of both terms of the angle a third to each of the three
+          double fk[3], fs[3];
+#pragma unroll
+          for (int x = 0; x < 3; x++) {
+            fk[x] = qk * fma(-c, e[k][x], e[s][x]);
+            fs[x] = qs * fma(-c, e[s][x], e[k][x]);
+          }
+          constexpr int P[6] = {0, 1, 2, 0, 0, 1}, Q[6] = {0, 1, 2, 1, 2, 2};
+#pragma unroll
+          for (int x = 0; x < 6; x++) {
+            const double w = (1.0 / 3.0) * fma(d[s][P[x]], fs[Q[x]], d[k][P[x]] * fk[Q[x]]);
+            vo[x] += w;
+            vs[s][x] += w;
+            vs[k][x] += w;
+          }
+        }
 #pragma unroll
         for (int x = 0; x < 3; x++) {
           t[k][x] = fma(qk, fma(-c, e[k][x], e[s][x]), t[k][x]);
@@ -1026,6 +1053,15 @@ __device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int i
   a.ters_f[i] = f[0];
   a.ters_f[a.n + i] = f[1];
   a.ters_f[2 * a.n + i] = f[2];
+  if constexpr (VA) {
+#pragma unroll
+    for (int c = 0; c < 6; c++) a.va_t[6 * (size_t)i + c] = vo[c];
+#pragma unroll
+    for (int s = 0; s < 3; s++)
+      if (s < cnt)
+#pragma unroll
+        for (int c = 0; c < 6; c++) a.va_ts[((size_t)i * MAXTERS + s) * 6 + c] = vs[s][c];
+  }
   if (EV) {
     double *st = a.stat_ters;
     st[i] = eng;
@@ -1046,8 +1082,7 @@ __global__ void __launch_bounds__(128) k_tersoff(ForceArgs<R> a) {
   const int ie = c_pot.t_map[info_type(iinfo)];
   const int cnt = ie < 0 ? 0 : a.ters_cnt[i];
 #ifndef LMFF_PACKED_X2
-  if constexpr (!VA)
-    if (tersoff_fast<EV, GH>(a, i, ie, cnt)) return;
+  if (tersoff_fast<EV, GH, VA>(a, i, ie, cnt)) return;
 #endif
   if (cnt <= 3) tersoff_atom<3, EV, GH, VA>(a, i, ie, cnt);
   else tersoff_atom<MAXTERS, EV, GH, VA>(a, i, ie, cnt);

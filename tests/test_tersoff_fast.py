@@ -77,3 +77,14 @@ def test_subdomain_form(ev):
     assert rel_max(f, ref["f"]) <= TOL
     if ev:
         assert abs(got["e_tersoff"] - ref["e_tersoff"]) <= TOL * abs(ref["e_tersoff"])
+
+
+@pytest.mark.parametrize("name", sorted(SYSTEMS))
+def test_per_atom_virial(name):
+    from oracle import Oracle
+    s = SYSTEMS[name]()
+    o = Oracle(TERSOFF, None, nthreads=4)
+    o.set_system(s)
+    ref = o.forces(which=1, vatom=True)["vatom_tersoff"]
+    got = capi.Engine(TERSOFF).compute_system(s, which=capi.TERSOFF, vatom=True)["vatom_tersoff"]
+    assert rel_max(got, ref) <= TOL
