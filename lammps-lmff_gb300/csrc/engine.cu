@@ -9,6 +9,7 @@
 //   k_tersoff (bonds centred at each atom)   k_ilp (interlayer pairs, normal derivatives)
 //   k_finish (gather) -> [k_reduce energies/virials]
 #include <cuda_runtime.h>
+#include <sys/mman.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -1925,13 +1926,14 @@ struct Engine {
     if (rc) return rc;
     std::vector<lmff_result> hr;
     bool ev = eflag || vflag || eatom;
+    const bool overwrite = (which & LMFF_OVERWRITE) != 0;
     rc = forces(which, ev, eatom != nullptr, &hr, true, [&] {
+      if (!overwrite) return;
       map_pages(f, sizeof(double) * 3 * (size_t)nn);
       map_pages(eatom, sizeof(double) * (size_t)nn);
     });
     if (rc) return rc;
     if (res) *res = hr.empty() ? lmff_result() : hr[0];
-    bool overwrite = (which & LMFF_OVERWRITE) != 0;
     if (nn > 0 && f) {
       if (!overwrite) CK(cudaMemcpyAsync(d_fin, f, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, stream));
       k_scatter_add<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, d.f, d_fin, overwrite);
@@ -1960,7 +1962,7 @@ struct Engine {
     const bool overwrite = (which & LMFF_OVERWRITE) != 0;
     if (!overwrite) CK(cudaMemcpyAsync(d_fin, f, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, stream));
     k_scatter_sum<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, d.f, overwrite ? nullptr : d_fin, d_fo);
-    map_pages(f, sizeof(double) * 3 * (size_t)nn);
+    if (overwrite) map_pages(f, sizeof(double) * 3 * (size_t)nn);
     CK(cudaMemcpyAsync(f, d_fo, sizeof(double) * 3 * nn, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     double d2;
@@ -2218,7 +2220,7 @@ struct Engine {
     const bool overwrite = (which & LMFF_OVERWRITE) != 0;
     if (!overwrite) CK(cudaMemcpyAsync(inorder, out, sizeof(double) * 6 * (size_t)nn, cudaMemcpyHostToDevice, stream));
     k_scatter_add6<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, sorted, inorder, overwrite);
-    map_pages(out, sizeof(double) * 6 * (size_t)nn);
+    if (overwrite) map_pages(out, sizeof(double) * 6 * (size_t)nn);
     CK(cudaMemcpyAsync(out, inorder, sizeof(double) * 6 * (size_t)nn, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     return LMFF_OK;
@@ -3096,19 +3098,24 @@ struct Engine {
     }
     for (auto &t : pool) t.join();
   }
-  // Maps the pages of a caller's output array, each byte keeping its value.  An array the
-  // program has just allocated has no pages yet; the GPU's copy into it then takes a fault of
-  // ~40 us for every 64 KB (490k atoms, lmff_download: 20-30 ms, with its pages there 0.9 ms),
-  // where a write by the host takes 5-10 us, on several threads at once and, where a call's
-  // kernels are already queued, while they run.
+  // Maps the pages of a caller's output array that the call overwrites as a whole.  An array
+  // the program has just allocated has no pages yet; the GPU's copy into it then takes a fault
+  // of ~40 us for every 64 KB (490k atoms, lmff_download: 20-30 ms, with its pages there 0.9
+  // ms), where a write by the host takes a few us, on several threads at once and, where a
+  // call's kernels are already queued, while they run.  (Only written: reading a byte first
+  // maps the zero page, and replacing that is a second fault with a flush of every thread's
+  // translations, 70 ms for 2.7M atoms.)
   static void map_pages(void *p, size_t bytes) {
     if (!p || !bytes) return;
     static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
+    const uintptr_t p0 = (uintptr_t)p / page * page, p1 = (uintptr_t)p + bytes;
+    std::vector<unsigned char> in((p1 - p0 + page - 1) / page);
+    if (mincore((void *)p0, p1 - p0, in.data()) != 0) return;
+    if (std::all_of(in.begin(), in.end(), [](unsigned char c) { return c & 1; })) return;
+    const unsigned char *there = in.data();
     in_pieces(bytes, [=](size_t b, size_t e) {
-      for (size_t q = b; q < e; q = ((uintptr_t)p + q) / page * page + page - (uintptr_t)p) {
-        volatile char *c = (volatile char *)p + q;
-        *c = *c;
-      }
+      for (size_t q = b; q < e; q = ((uintptr_t)p + q) / page * page + page - (uintptr_t)p)
+        if (!(there[((uintptr_t)p + q - p0) / page] & 1)) *((volatile char *)p + q) = 0;
     });
   }
 
