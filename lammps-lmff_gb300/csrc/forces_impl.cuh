@@ -3850,12 +3850,9 @@ __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
     const long long itag = a.tag[i];
     const float4 ni = a.nrm32[i];
     const int64_t q1 = a.list_off[i + 1];
-    int64_t q = a.list_off[i] + lane;
-    uint32_t ahead = q < q1 ? __ldg(&a.list[q]) : 0;   // the list a round ahead
-    for (; q < q1; q += VA_LANES) {
+    for (int64_t q = a.list_off[i] + lane; q < q1; q += VA_LANES) {
       int j, sx, sy, sz;
-      decode_entry(ahead, a.lc, j, sx, sy, sz);
-      if (q + VA_LANES < q1) ahead = __ldg(&a.list[q + VA_LANES]);
+      decode_entry(a.list[q], a.lc, j, sx, sy, sz);
       R dx, dy, dz;
       long long jinfo;
       ai.disp(a.A, sd, j, sx, sy, sz, dx, dy, dz, jinfo);
