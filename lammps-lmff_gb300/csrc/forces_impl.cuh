@@ -3361,7 +3361,7 @@ __global__ void __launch_bounds__(128) k_va_ilp(ForceArgs<R> a) {
 // with full warps.  36,800-atom slab: k_va_ilp 30 ms (one thread per atom, ~500 FP64
 // instructions a pair); k_va_near 1.07 ms, FP64 pipe (~190 instructions for ~85 pairs an
 // atom; 1.60 ms with batches every third round, when few of the warp's atoms had one), k_va_far
-// 1.15 ms, FP32 issue.
+// 0.90 ms, FP32 issue (1.15 with each lane's normal terms evaluated in place).
 constexpr int VA_LANES = 8;
 constexpr float VA_NEARSQ = 49.f;
 static_assert(VA_NEARSQ <= df::Q64_MAX, "the FP64 tables end at Q64_MAX");
@@ -3585,13 +3585,19 @@ template <bool ONE, bool GH>
 __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
   using namespace df;
   typedef float V;
+  constexpr int QUEUE = 8 * VA_LANES;   // entries per atom
+  const unsigned FULL = 0xffffffffu;
   __shared__ float2 s_tab[EXP2_TAB];
+  __shared__ uint32_t s_queue[128 * 8];
   for (int w = threadIdx.x; w < EXP2_TAB; w += blockDim.x) s_tab[w] = g_exp2_df[w];
   __syncthreads();
-  const int i = (blockIdx.x * blockDim.x + threadIdx.x) / VA_LANES;
+  const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) / VA_LANES;
+  const bool valid = i0 < a.n;
+  const int i = valid ? i0 : a.n - 1;
   const int lane = threadIdx.x & (VA_LANES - 1);
-  if (i >= a.n) return;   // whole groups
   const unsigned gmask = ((1u << VA_LANES) - 1) << ((threadIdx.x & 31) & ~(VA_LANES - 1));
+  const unsigned below = gmask & ((1u << (threadIdx.x & 31)) - 1u);
+  uint32_t *const queue = s_queue + 8 * (threadIdx.x & ~(VA_LANES - 1));
   const SysDesc &sd = a.A.sys[a.A.sysid[i]];
   DfAtom I;
   I.load(a.jrec, a.jstride, i);
@@ -3602,121 +3608,157 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
 #pragma unroll
   for (int c = 0; c < 15; c++) s[c] = mk(0.f, 0.f);
   const bool out = fabsf(I.h[0]) > sd.dfmax || fabsf(I.h[1]) > sd.dfmax || fabsf(I.h[2]) > sd.dfmax;
-  if (ie >= 0 && !out) {
-    D<V> ni[3];
+  const int64_t b = a.list_off[i];
+  const int cnt = valid && ie >= 0 && !out ? (int)(a.list_off[i + 1] - b) : 0;
+  const int most = __reduce_max_sync(FULL, cnt);
+  constexpr int P[6] = {0, 1, 2, 0, 0, 1}, Q[6] = {0, 1, 2, 1, 2, 2};
+  // weights of the subdomain mode: the vdW pair, the terms with n_i and with n_j
+  auto weights = [&](int j, const D<V> d[3], float &wv, float &wi, float &wj) {
+    if constexpr (GH) {
+      const bool jown = owned(a, j);
+      const bool keep = keep_half_r(itag, (long long)a.tag[j], -(d[0].h + d[0].l), -(d[1].h + d[1].l), -(d[2].h + d[2].l));
+      wv = (keep ? iown : jown) ? 1.f : 0.f;
+      wi = iown ? 1.f : 0.f;
+      wj = jown ? 1.f : 0.f;
+    }
+  };
+  auto virial = [&](const D<V> d[3], const D<V> t[3]) {
 #pragma unroll
-    for (int c = 0; c < 3; c++) ni[c] = mk(I.nh[c], I.nl[c]);
-    const int64_t q1 = a.list_off[i + 1];
-    int64_t k = a.list_off[i] + lane;
-    uint32_t ahead = k < q1 ? __ldg(&a.list[k]) : 0;   // the list a round ahead
-    for (; k < q1; k += VA_LANES) {
-      const uint32_t e = ahead;
-      if (k + VA_LANES < q1) ahead = __ldg(&a.list[k + VA_LANES]);
+    for (int c = 0; c < 6; c++) acc_mul(s[c], d[P[c]], t[Q[c]]);
+  };
+  int qh = 0, qn = 0;
+  // the parts the normals enter, of the first entries in the queue
+  auto near_batch = [&](bool on) {
+    __syncwarp();
+    if (on && qh + lane < qn) {
       int j, sx, sy, sz;
-      decode_entry(e, a.lc, j, sx, sy, sz);
+      decode_entry(queue[(qh + lane) & (QUEUE - 1)], a.lc, j, sx, sy, sz);
       DfAtom A;
       A.load(a.jrec, a.jstride, j);
-      D<V> d[3], nj[3];
-      D<V> q;
-      if (!va_pair_q(I, A, sd, sx, sy, sz, d, q) || q.h < VA_NEARSQ) continue;
+      D<V> d[3], ni[3], nj[3], q, tp, tq, S, crad = mk(0.f, 0.f);
+      va_pair_q(I, A, sd, sx, sy, sz, d, q);
+      float th, wv = 1.f, wi = 1.f, wj = 1.f;
+      weights(j, d, wv, wi, wj);
+      int ki = tab_at(q.h, th);
+      if constexpr (!ONE) ki += (ie * ne + A.el) * TAB_N;
+      const D<V> off = fast_two_sum(th, q.l);
+      Coef<V> cc;
+      coef_set(cc, a.df_M + 2 * ki);
+      const float2 f0 = __ldg(a.df_TE + ki);
 #pragma unroll
-      for (int c = 0; c < 3; c++) nj[c] = mk(A.nh[c], A.nl[c]);
-      float wv = 1.f, wi = 1.f, wj = 1.f;
-      if constexpr (GH) {
-        const bool jown = owned(a, j);
-        const bool keep = keep_half_r(itag, (long long)a.tag[j], -(d[0].h + d[0].l), -(d[1].h + d[1].l), -(d[2].h + d[2].l));
-        wv = (keep ? iown : jown) ? 1.f : 0.f;
-        wi = iown ? 1.f : 0.f;
-        wj = jown ? 1.f : 0.f;
+      for (int c = 0; c < 3; c++) {
+        ni[c] = mk(I.nh[c], I.nl[c]);
+        nj[c] = mk(A.nh[c], A.nl[c]);
       }
       const float *row = ONE ? nullptr : g_dfk + (ie * ne + A.el) * K_N;
       auto K = [&](int k2) {
         if constexpr (ONE) return c_dfk[k2];
         else return __ldg(&row[k2]);
       };
-      float th;
-      int ki = tab_at(q.h, th);
-      if constexpr (!ONE) ki += (ie * ne + A.el) * TAB_N;
-      const D<V> off = fast_two_sum(th, q.l);
-      Coef<V> cc;
-      coef_set(cc, a.df_A + 2 * ki);
-      D<V> crad = tab_poly(cc, off);
-      const bool near = near_one(K(K_ND2), q.h, I.nh[0] * d[0].h + I.nh[1] * d[1].h + I.nh[2] * d[2].h,
-                                 A.nh[0] * d[0].h + A.nh[1] * d[1].h + A.nh[2] * d[2].h);
-      D<V> M, tp = mk(0.f, 0.f), tq = tp;
-      if (GH || near) {
-        coef_set(cc, a.df_M + 2 * ki);
-        M = tab_poly(cc, off);
-      }
-      if constexpr (GH)
-        crad = add(scale(crad, wv), scale(mul(M, mk(K(K_EPS), K(K_EPS + 1))), 0.5f * (wi + wj) - wv));
-      if (near) {
-        const float2 f0 = __ldg(a.df_TE + ki);
-        D<V> S;
-        pair_near<GH>(K, s_tab, q, tab_integral(cc, f0.x, f0.y, off), M, dot3(ni, d), dot3(nj, d), wi, wj, crad, tp,
-                      tq, S);
-      }
+      pair_near<GH>(K, s_tab, q, tab_integral(cc, f0.x, f0.y, off), tab_poly(cc, off), dot3(ni, d), dot3(nj, d), wi, wj,
+                    crad, tp, tq, S);
       const D<V> ntq = neg(tq);
-      D<V> t[3], h[3];
+      D<V> t[3], h[3], g[3];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         t[c] = add(mul(crad, d[c]), mul(ntq, nj[c]));
         h[c] = mul(tp, d[c]);
+        g[c] = mul(tq, d[c]);   // the partner's normal-derivative share is linear in it
         acc(s[6 + c], h[c]);
       }
-      constexpr int P[6] = {0, 1, 2, 0, 0, 1}, Q[6] = {0, 1, 2, 1, 2, 2};
+      virial(d, t);
+#pragma unroll
+      for (int c = 0; c < 6; c++) acc_mul(s[9 + c], h[P[c]], d[Q[c]]);
+      const float4 *tt = a.va_tens + 14 * ((size_t)a.n + j);
+      float4 T[14];
+#pragma unroll
+      for (int c = 0; c < 14; c++) T[c] = __ldg(tt + c);
+      auto num = [&](int c) { return (c & 1) ? mk(T[c / 2].z, T[c / 2].w) : mk(T[c / 2].x, T[c / 2].y); };
+      bool any = false;   // B = 0 for atoms with three intralayer neighbours
+#pragma unroll
+      for (int c = 18; c < 27; c++) any = any || num(c).h != 0.f;
+      if (any) {
+        D<V> r[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) {   // - sum_e B[e][c] g_e
+          r[c] = mul(num(18 + c), g[0]);
+          acc_mul(r[c], num(21 + c), g[1]);
+          acc_mul(r[c], num(24 + c), g[2]);
+          r[c] = neg(renorm(r[c]));
+        }
+        virial(d, r);
+      }
 #pragma unroll
       for (int c = 0; c < 6; c++) {
-        acc_mul(s[c], d[P[c]], t[Q[c]]);
-        acc_mul(s[9 + c], h[P[c]], d[Q[c]]);
-      }
-      if (tq.h != 0.f) {
-        // the partner's normal-derivative share, g = tq del
-        D<V> g[3], b[3];
-#pragma unroll
-        for (int c = 0; c < 3; c++) g[c] = mul(tq, d[c]);
-        const float4 *tt = a.va_tens + 14 * ((size_t)a.n + j);
-        float4 T[14];
-#pragma unroll
-        for (int c = 0; c < 14; c++) T[c] = __ldg(tt + c);
-        auto num = [&](int c) { return (c & 1) ? mk(T[c / 2].z, T[c / 2].w) : mk(T[c / 2].x, T[c / 2].y); };
-        bool any = false;   // B = 0 for atoms with three intralayer neighbours
-#pragma unroll
-        for (int c = 18; c < 27; c++) any = any || num(c).h != 0.f;
-        if (any) {
-#pragma unroll
-          for (int c = 0; c < 3; c++) {   // - sum_e B[e][c] g_e
-            b[c] = mul(num(18 + c), g[0]);
-            acc_mul(b[c], num(21 + c), g[1]);
-            acc_mul(b[c], num(24 + c), g[2]);
-            b[c] = neg(renorm(b[c]));
-          }
-#pragma unroll
-          for (int c = 0; c < 6; c++) acc_mul(s[c], d[P[c]], b[Q[c]]);
-        }
-#pragma unroll
-        for (int c = 0; c < 6; c++) {
-          acc_mul(s[c], num(3 * c), g[0]);
-          acc_mul(s[c], num(3 * c + 1), g[1]);
-          acc_mul(s[c], num(3 * c + 2), g[2]);
-        }
+        acc_mul(s[c], num(3 * c), g[0]);
+        acc_mul(s[c], num(3 * c + 1), g[1]);
+        acc_mul(s[c], num(3 * c + 2), g[2]);
       }
     }
+    if (on) qh = min(qh + VA_LANES, qn);
+    __syncwarp();
+  };
+  uint32_t ahead = lane < cnt ? __ldg(&a.list[b + lane]) : 0;   // the list a round ahead
+  for (int k0 = 0; k0 < most; k0 += VA_LANES) {
+    bool near = false;
+    const uint32_t e = ahead;
+    if (k0 + VA_LANES + lane < cnt) ahead = __ldg(&a.list[b + k0 + VA_LANES + lane]);
+    if (k0 + lane < cnt) {
+      int j, sx, sy, sz;
+      decode_entry(e, a.lc, j, sx, sy, sz);
+      DfAtom A;
+      A.load(a.jrec, a.jstride, j);
+      D<V> d[3], q;
+      if (va_pair_q(I, A, sd, sx, sy, sz, d, q) && !(q.h < VA_NEARSQ)) {
+        const float *row = ONE ? nullptr : g_dfk + (ie * ne + A.el) * K_N;
+        auto K = [&](int k2) {
+          if constexpr (ONE) return c_dfk[k2];
+          else return __ldg(&row[k2]);
+        };
+        float th;
+        int ki = tab_at(q.h, th);
+        if constexpr (!ONE) ki += (ie * ne + A.el) * TAB_N;
+        const D<V> off = fast_two_sum(th, q.l);
+        Coef<V> cc;
+        coef_set(cc, a.df_A + 2 * ki);
+        D<V> crad = tab_poly(cc, off);
+        if constexpr (GH) {
+          float wv, wi, wj;
+          weights(j, d, wv, wi, wj);
+          coef_set(cc, a.df_M + 2 * ki);
+          crad = add(scale(crad, wv), scale(mul(tab_poly(cc, off), mk(K(K_EPS), K(K_EPS + 1))), 0.5f * (wi + wj) - wv));
+        }
+        D<V> t[3];
+#pragma unroll
+        for (int c = 0; c < 3; c++) t[c] = mul(crad, d[c]);
+        virial(d, t);
+        near = near_one(K(K_ND2), q.h, I.nh[0] * d[0].h + I.nh[1] * d[1].h + I.nh[2] * d[2].h,
+                        A.nh[0] * d[0].h + A.nh[1] * d[1].h + A.nh[2] * d[2].h);
+      }
+    }
+    const unsigned bits = __ballot_sync(FULL, near);
+    if (near) queue[(qn + __popc(bits & below)) & (QUEUE - 1)] = e;
+    qn += __popc(bits & gmask);
+    // every seventh round (before the queue can overflow), for the atoms that have a batch:
+    // an atom's sums depend on its own list alone
+    if (k0 / VA_LANES % 7 == 6)
+      while (__any_sync(FULL, qn - qh >= VA_LANES)) near_batch(qn - qh >= VA_LANES);
   }
+  while (__any_sync(FULL, qh < qn)) near_batch(true);
   double v[15];
 #pragma unroll
   for (int c = 0; c < 15; c++) {
     D<V> x = renorm(s[c]);
     for (int o = VA_LANES / 2; o > 0; o >>= 1)
-      x = renorm(add(x, mk(__shfl_xor_sync(gmask, x.h, o), __shfl_xor_sync(gmask, x.l, o))));
+      x = renorm(add(x, mk(__shfl_xor_sync(FULL, x.h, o), __shfl_xor_sync(FULL, x.l, o))));
     v[c] = (double)x.h + (double)x.l;
   }
+  if (!valid || lane != 0) return;
   const double n[3] = {(double)I.nh[0] + (double)I.nl[0], (double)I.nh[1] + (double)I.nl[1],
                        (double)I.nh[2] + (double)I.nl[2]};
   // the n_i part of the pair forces, and the halves
   v[0] = 0.5 * fma(-v[6], n[0], v[0]); v[1] = 0.5 * fma(-v[7], n[1], v[1]); v[2] = 0.5 * fma(-v[8], n[2], v[2]);
   v[3] = 0.5 * fma(-v[6], n[1], v[3]); v[4] = 0.5 * fma(-v[6], n[2], v[4]); v[5] = 0.5 * fma(-v[7], n[2], v[5]);
-  if (lane != 0) return;
 #pragma unroll
   for (int c = 0; c < 6; c++) a.va_i[6 * (size_t)i + c] += v[c];
   double *q = a.va_is + 6 * MAXILP * (size_t)i;
