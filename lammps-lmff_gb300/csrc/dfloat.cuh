@@ -5,10 +5,9 @@
 // here several times faster than on the FP64 pipe.
 //
 // Everything is built from error-free transformations (T. J. Dekker, Numer. Math. 18, 1971;
-// D. E. Knuth, TAOCP vol. 2): two_sum and the FMA product error.  The types are templates
-// over V = float or V = float2; float2 holds two independent values and uses the packed
-// FP32x2 instructions, which take half the issue slots at the same arithmetic rate (the
-// negation of an operand is free in both).
+// D. E. Knuth, TAOCP vol. 2): two_sum and the FMA product error.  (Two values at a time with
+// the packed FP32x2 instructions took half the issue slots at the same arithmetic rate, and
+// twice the registers: the pair kernel was 10 % slower.)
 //
 // Results are left unnormalised (|l| of a few ulp of h): products and sums accept that, and
 // renorm is called where a chain would let it grow.
@@ -20,29 +19,15 @@ namespace lmff {
 namespace df {
 
 #define LMFF_DF static __device__ __forceinline__
-LMFF_DF float vset(float a, float) { return a; }
 LMFF_DF float vneg(float a) { return -a; }
 LMFF_DF float vadd(float a, float b) { return __fadd_rn(a, b); }
 LMFF_DF float vsub(float a, float b) { return __fsub_rn(a, b); }
 LMFF_DF float vmul(float a, float b) { return __fmul_rn(a, b); }
 LMFF_DF float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-LMFF_DF float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
-LMFF_DF float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
-LMFF_DF float2 vsub(float2 a, float2 b) { return __fadd2_rn(a, vneg(b)); }
-LMFF_DF float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
-LMFF_DF float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 template <class V>
-LMFF_DF V vall(float a);   // the same value in every component
+LMFF_DF V vall(float a);   // a constant
 template <>
 __device__ __forceinline__ float vall<float>(float a) { return a; }
-template <>
-__device__ __forceinline__ float2 vall<float2>(float a) { return make_float2(a, a); }
-// f applied to each component (MUFU estimates, table addresses)
-template <class F>
-LMFF_DF float vmap(F f, float a) { return f(a); }
-template <class F>
-LMFF_DF float2 vmap(F f, float2 a) { return make_float2(f(a.x), f(a.y)); }
-
 template <class V>
 struct D {
   V h, l;
@@ -102,13 +87,6 @@ LMFF_DF D<V> add1(D<V> a, V b) {
   const D<V> s = two_sum(a.h, b);
   return mk(s.h, vadd(s.l, a.l));
 }
-// c + a, c a constant that is a multiple of ulp(a.h) (an integer, |a| < 2^23): fast_two_sum
-// is exact for that too, whichever of the two is larger
-template <class V>
-LMFF_DF D<V> addc(float c, D<V> a) {
-  const D<V> s = fast_two_sum(vall<V>(c), a.h);
-  return mk(s.h, vadd(s.l, a.l));
-}
 template <class V>
 LMFF_DF D<V> scale(D<V> a, V m) { return mk(vmul(a.h, m), vmul(a.l, m)); }   // m a power of two or zero
 // running sum: acc += a
@@ -125,40 +103,6 @@ LMFF_DF D<V> dot3(const D<V> *a, const D<V> *b) {
   const D<V> s = two_sum(x.h, y.h), t = two_sum(s.h, z.h);
   const V lo = vadd(vadd(vadd(x.l, y.l), z.l), vadd(s.l, t.l));
   return fast_two_sum(t.h, lo);
-}
-
-LMFF_DF float rsqrt_est(float x) {
-  float y;
-  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-LMFF_DF float rcp_est(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// r = sqrt(q) and ri = 1 / sqrt(q), q > 0: the FP32 estimate y (relative error 2^-22.9) is
-// brought to FP32 rounding by one Newton step, so that the final Newton corrections, whose
-// error is the square of y's, stay below 2^-47
-template <class V>
-LMFF_DF void sqrt_rsqrt(D<V> q, D<V> &r, D<V> &ri) {
-  V y = vmap([](float x) { return rsqrt_est(x); }, q.h);
-  const V half = vall<V>(0.5f), one = vall<V>(1.f);
-  y = vfma(vmul(half, y), vfma(vneg(vmul(q.h, y)), y, one), y);
-  const V r0 = vmul(q.h, y), hy = vmul(half, y);
-  const V res = vadd(vfma(vneg(r0), r0, q.h), q.l);
-  r = fast_two_sum(r0, vmul(res, hy));
-  const V t = vfma(vneg(r.l), y, vfma(vneg(r.h), y, one));
-  ri = mk(y, vmul(y, vfma(t, t, t)));
-}
-
-// 1 / a
-template <class V>
-LMFF_DF D<V> rcp(D<V> a) {
-  const V y = vmap([](float x) { return rcp_est(x); }, a.h);
-  const V t = vfma(vneg(a.l), y, vfma(vneg(a.h), y, vall<V>(1.f)));
-  return mk(y, vmul(y, vfma(t, t, t)));   // 1/(1 - t) = 1 + t + t^2, |t| < 2^-22
 }
 
 // 2^a by Tang's table-driven method (P. T. P. Tang, ACM TOMS 15, 1989): a = k/64 + f,
@@ -180,14 +124,10 @@ LMFF_DF void exp2_parts(float t, const float2 *tab, float &th, float &tl, float 
   tl = T.y;
   sc = __int_as_float(((k >> 6) + 127) << 23);
 }
-LMFF_DF void exp2_parts(float2 t, const float2 *tab, float2 &th, float2 &tl, float2 &sc) {
-  exp2_parts(t.x, tab, th.x, tl.x, sc.x);
-  exp2_parts(t.y, tab, th.y, tl.y, sc.y);
-}
 template <class V>
 LMFF_DF D<V> exp2(D<V> a, const float2 *tab) {
   const V magic = vall<V>(12582912.f);   // 1.5 2^23
-  const V ah = vmap([](float x) { return clamp_exp(x); }, a.h);
+  const V ah = clamp_exp(a.h);
   const V t = vfma(ah, vall<V>((float)EXP2_TAB), magic);
   const V k = vsub(t, magic);
   // ah - k/64 is exact and a multiple of ulp(ah), so zero or larger than a.l

@@ -44,12 +44,6 @@ __device__ __forceinline__ R cR(double v) { return (R)v; }
 
 __device__ __forceinline__ void raise_status(int *status, int bit) { atomicOr(status, bit); }
 
-// squared distance in R; for FP64 in the reference's rounding
-__device__ __forceinline__ R rsqR(R dx, R dy, R dz) {
-  if constexpr (sizeof(R) == 8) return rsq_rn(dx, dy, dz);
-  else return dx * dx + dy * dy + dz * dz;
-}
-
 // rsq < thr decided exactly as FP64 would (FP32 first, FP64 when within 1e-5)
 __device__ __forceinline__ bool lt_exact(float rsq, float thr, const d4 *xq, const SysDesc &sd, int i, int j, int sx,
                                          int sy, int sz, double thr64) {
@@ -2701,10 +2695,11 @@ struct NDeriv {
 };
 // The normal frame of atom i: the part of the assembly that does not depend on g_i -- the
 // bond vectors to its intralayer neighbours, the unit normal and 1/|n1|.  With a frame
-// array (ForceArgs::nframe) k_nframe computes it beside the pair kernel, on the Tersoff
-// stream, and k_nderiv only applies g_i to it: about half of the assembly's FP64 work
-// leaves the step's critical path.  The arithmetic is that of the assembly done in one
-// piece, so the results are the same to the bit.
+// array (ForceArgs::nframe) k_nframe computes it beside the pair kernel, on a stream of its
+// own (FP64 mode: k_frame ahead of the pair kernel, whose normals it makes), and k_nderiv
+// only applies g_i to it: about half of the assembly's FP64 work leaves the step's critical
+// path.  The arithmetic is that of the assembly done in one piece, so the results are the
+// same to the bit.
 struct NFrame {
   int cont;   // intralayer neighbours (0 when i is not ILP-mapped)
   bool ok;    // cont >= 2 and |n1| > 0
@@ -3188,7 +3183,7 @@ __device__ __forceinline__ void va_write_slots(const ForceArgs<R> &a, int i, boo
 // Subdomain mode: vdW when the end the tag-parity half keeps is owned, each repulsion
 // term when its normal's atom is owned.
 
-// the frame k_nframe left for atom i and the normal it carries: the reference's (0,0,1)
+// the frame k_frame or k_nframe left for atom i and the normal it carries: the reference's (0,0,1)
 // for fewer than two intralayer neighbours (calc_normal, pair_ilp_graphene_hbn.cpp:800-806)
 __device__ __forceinline__ void va_frame(const ForceArgs<R> &a, int i, NFrame &fr, double &nx, double &ny,
                                          double &nz) {

@@ -1,6 +1,5 @@
 // The FP64 mode's interlayer pair terms in double-float arithmetic (dfloat.cuh): what
-// calc_FvdW and calc_FRep (pair_ilp_graphene_hbn.cpp:449-675) form per pair, for two pairs
-// at a time (V = float2) or one (V = float).
+// calc_FvdW and calc_FRep (pair_ilp_graphene_hbn.cpp:449-675) form per pair.
 //
 // With q = r^2, Tap and dTap of r, E0 = e^{-lambda (r - z0)}, E = e^{-d (r/seff - 1)},
 // X = 1/(r^6 (1 + E)), G_n = e^{-rho_n^2/delta^2} of the two normals n, S = G_i + G_j:
