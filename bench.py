@@ -597,7 +597,7 @@ def rooflines(m, s, prec, pk, peaks) -> dict:
     st = m["stats"]
     ka = m["kernel_ms_avg"]
     pairs, cands = st["pairs_in_cutoff"], st["list_entries"]
-    name = "fp32" if prec == capi.MIXED else "fp64"
+    name = "fp32"   # the plain FP64 form's pair kernel too: double-float arithmetic in FP32 instructions
     k_s = ka["pair_ilp"] / 1e3
     achieved = alg_flops_pair_kernel(pairs, cands) / k_s / 1e12
     out = {"k_ilp": {
@@ -606,7 +606,9 @@ def rooflines(m, s, prec, pk, peaks) -> dict:
         "traffic": K_ILP_DRAM_BYTES_PER_ENTRY * cands if prec == capi.MIXED else None,
         "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one k_ilp launch on the "
                           "331,200-atom slab (1.317 GB for 310.3 M list entries), scaled by list entries",
-        "kernel": "k_ilp (pair kernel)", "kernel_ms_avg": ka["pair_ilp"],
+        "kernel": "k_ilp (pair kernel)" if prec == capi.MIXED
+        else "k_ilp_df (pair kernel, ~48-bit double-float values in FP32 instructions)",
+        "kernel_ms_avg": ka["pair_ilp"],
         "peak_source": f"cuBLAS {name.upper()} GEMM measured in this run (SIMT; MEASURED_PEAKS.json has HBM "
                        f"{peaks.get('hbm_gbs')} GB/s and bf16 tensor only)",
         "pairs_in_cutoff": pairs, "list_entries": cands,
