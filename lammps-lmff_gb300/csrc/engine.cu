@@ -15,8 +15,8 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <memory>
 #include <mutex>
-#include <functional>
 #include <shared_mutex>
 #include <cmath>
 #include <cstdio>
@@ -1136,7 +1136,9 @@ struct Engine {
       CK(dalloc(d_dfU, df_intervals())); CK(dalloc(d_dfTE, df_intervals()));
     }
     CK(cudaMemsetAsync(d.status, 0, sizeof(int), stream));
-    return ensure_stream2();   // here: lmff_compute_device_noalloc uses it and may not create it
+    // here: lmff_compute_device_noalloc uses it and may not create it (without it, one stream)
+    if (ensure_stream2() != LMFF_OK) cudaGetLastError();
+    return LMFF_OK;
   }
 
   // The device's constant tables are this engine's (guaranteed by DeviceCall); only the
@@ -1281,12 +1283,11 @@ struct Engine {
   }
 
   int ensure_stream2() {
-    if (stream2) return LMFF_OK;
-    CK(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithFlags(&stream3, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&ev_frame, cudaEventDisableTiming));
+    if (!stream2) CK(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
+    if (!stream3) CK(cudaStreamCreateWithFlags(&stream3, cudaStreamNonBlocking));
+    if (!ev_fork) CK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+    if (!ev_join) CK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+    if (!ev_frame) CK(cudaEventCreateWithFlags(&ev_frame, cudaEventDisableTiming));
     return LMFF_OK;
   }
 
@@ -1694,6 +1695,11 @@ struct Engine {
     timed(3, [&] { ff(a, eatom, kick_on ? &kick_args : nullptr, stream); });
   }
 
+  // host arrays a call overwrites (either may be null)
+  struct HostOut {
+    double *f, *eatom;
+  };
+
   // the reduction's chunk sums (of every system) and counters (zero between launches)
   int ensure_partials() {
     red_cmax = 1;
@@ -1716,9 +1722,9 @@ struct Engine {
   // forces (+ energies/virials per system into hres when ev) on the resident state
   // wait = false (force-only evaluations): the status word comes back into a pinned word
   // and the caller waits once for everything it queued, then calls forces_done
-  // while_waiting: host work of the call, done when the kernels are queued
+  // out: the call's output arrays, mapped once the kernels are queued
   int forces(int which, bool ev, bool eatom, std::vector<lmff_result> *hres, bool wait = true,
-             const std::function<void()> &while_waiting = nullptr) {
+             const HostOut *out = nullptr) {
     int rc = push_consts();
     if (rc) return rc;
     if (!built) {
@@ -1783,7 +1789,10 @@ struct Engine {
       red.resize(hsys.size() * 16);
       CK(cudaMemcpyAsync(red.data(), d.red_out, sizeof(double) * red.size(), cudaMemcpyDeviceToHost, stream));
     }
-    if (while_waiting) while_waiting();
+    if (out) {
+      map_pages(out->f, sizeof(double) * 3 * (size_t)n);
+      map_pages(out->eatom, sizeof(double) * (size_t)n);
+    }
     CK(cudaStreamSynchronize(stream));
     harvest();
     float ms = 0;
@@ -1927,11 +1936,8 @@ struct Engine {
     std::vector<lmff_result> hr;
     bool ev = eflag || vflag || eatom;
     const bool overwrite = (which & LMFF_OVERWRITE) != 0;
-    rc = forces(which, ev, eatom != nullptr, &hr, true, [&] {
-      if (!overwrite) return;
-      map_pages(f, sizeof(double) * 3 * (size_t)nn);
-      map_pages(eatom, sizeof(double) * (size_t)nn);
-    });
+    const HostOut out = {f, eatom};
+    rc = forces(which, ev, eatom != nullptr, &hr, true, overwrite ? &out : nullptr);
     if (rc) return rc;
     if (res) *res = hr.empty() ? lmff_result() : hr[0];
     if (nn > 0 && f) {
@@ -2182,6 +2188,7 @@ struct Engine {
       CK(cudaMalloc(&d_va, sizeof(double) * VA_DOUBLES * (size_t)cap_n));
       va_cap = cap_n;
     }
+    if (int rc = push_consts()) return rc;   // the tables: the evaluation may have been a mixed one
     if (pair_df && precision == LMFF_FP64 && !va64_filled) {
       const size_t per = (size_t)pair_df * pair_df * df::TAB64_N * 24;
       if (!d_va64) CK(cudaMalloc(&d_va64, sizeof(double) * per));
@@ -3084,19 +3091,19 @@ struct Engine {
       return;
     }
     const size_t piece = ((bytes / nth) + 63) & ~(size_t)63;
-    std::vector<std::thread> pool;
-    pool.reserve(nth);
+    std::thread pool[8];
     for (int k = 0; k < nth; k++) {
       const size_t b = (size_t)k * piece;
       if (b >= bytes) break;
       const size_t e = std::min(bytes, b + piece);
       try {
-        pool.emplace_back([=, &f] { f(b, e); });
-      } catch (const std::system_error &) {
+        pool[k] = std::thread([=, &f] { f(b, e); });
+      } catch (const std::exception &) {
         f(b, e);
       }
     }
-    for (auto &t : pool) t.join();
+    for (auto &t : pool)
+      if (t.joinable()) t.join();
   }
   // Maps the pages of a caller's output array that the call overwrites as a whole.  An array
   // the program has just allocated has no pages yet; the GPU's copy into it then takes a fault
@@ -3109,10 +3116,11 @@ struct Engine {
     if (!p || !bytes) return;
     static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
     const uintptr_t p0 = (uintptr_t)p / page * page, p1 = (uintptr_t)p + bytes;
-    std::vector<unsigned char> in((p1 - p0 + page - 1) / page);
-    if (mincore((void *)p0, p1 - p0, in.data()) != 0) return;
-    if (std::all_of(in.begin(), in.end(), [](unsigned char c) { return c & 1; })) return;
-    const unsigned char *there = in.data();
+    const size_t pages = (p1 - p0 + page - 1) / page;
+    const std::unique_ptr<unsigned char[]> in(new (std::nothrow) unsigned char[pages]);
+    const unsigned char *there = in.get();
+    if (!in || mincore((void *)p0, p1 - p0, in.get()) != 0) return;
+    if (std::all_of(there, there + pages, [](unsigned char c) { return c & 1; })) return;
     in_pieces(bytes, [=](size_t b, size_t e) {
       for (size_t q = b; q < e; q = ((uintptr_t)p + q) / page * page + page - (uintptr_t)p)
         if (!(there[((uintptr_t)p + q - p0) / page] & 1)) *((volatile char *)p + q) = 0;
@@ -3405,7 +3413,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
   const bool ev = true;
   // the Tersoff kernel beside the interlayer ones, as in the resident path (1,152 atoms: 27
   // of ~190 us of kernels, on a few warps)
-  auto beside = [&](const auto &a) { return a.do_ters && a.do_ilp && g.ters_concurrent && g.stream2; };
+  auto beside = [&](const auto &a) { return a.do_ters && a.do_ilp && g.ters_concurrent && g.ev_frame; };
   auto fork = [&](const auto &a) {
     if (!beside(a)) return st;
     cudaEventRecord(g.ev_fork, st);

@@ -125,6 +125,18 @@ def test_per_atom_virial_near_and_far_pairs(cut):
         assert np.abs(r[0] - r[1]).max() <= TOL * np.abs(r[1]).max()
 
 
+def test_per_atom_virial_after_a_change_of_precision():
+    """The per-atom virial of a mixed evaluation asked for in FP64: an engine that has not
+    evaluated in FP64 before."""
+    s = S.displace(S.twisted_bilayer(11, 7, 3.0, top="hbn", spacing=3.3), 0.05, seed=5)
+    eng = capi.Engine(TERSOFF, ILP, precision=capi.MIXED)
+    eng.compute_system(s)
+    eng.set_precision(capi.FP64)
+    got = eng.vatom(capi.ILP)
+    ref = capi.Engine(TERSOFF, ILP).compute_system(s, vatom=True)["vatom_ilp"]
+    assert np.abs(got - ref).max() <= TOL * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("ev", [False, True])
 def test_subdomain_form(ev):
     s = S.displace(S.twisted_bilayer(14, 8, 2.0, top="hbn", spacing=3.3), 0.03, seed=7)
