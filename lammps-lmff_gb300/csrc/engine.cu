@@ -1379,13 +1379,8 @@ struct Engine {
 
   // the sorted copies back into the primary arrays, so device pointers stay fixed
   // across rebuilds (a captured step graph holds them)
-  cudaError_t copy_back_permuted(cudaStream_t s) {
-    cudaMemcpyAsync(d.xq, xq2, sizeof(d4) * n, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.v, v2, sizeof(double) * 3 * n, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.tag, tag2, sizeof(int64_t) * n, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.perm, perm2, sizeof(int) * n, cudaMemcpyDeviceToDevice, s);
-    cudaMemcpyAsync(d.sysid, sysid2, sizeof(int) * n, cudaMemcpyDeviceToDevice, s);
-    return cudaMemcpyAsync(d.mass, mass2, sizeof(double) * n, cudaMemcpyDeviceToDevice, s);
+  Permuted permuted() const {
+    return {xq2, v2, tag2, perm2, sysid2, mass2, d.xq, d.v, d.tag, d.perm, d.sysid, d.mass};
   }
 
   int rebuild() {
@@ -1400,17 +1395,12 @@ struct Engine {
       return LMFF_OK;
     }
     int g = (n + 255) / 256;
-    nb_wrap_bin(n, d.xq, d.sys, d.sysid, d.bin_key, d.idx, stream);
+    nb_wrap_bin(n, d.xq, d.sys, d.sysid, d.bin_key, d.idx, d.bin_start, d.bin_end, d.rowocc, d.nbins, stream);
     CK(nb_sort(d.cub_tmp, d.cub_tmp_bytes, d.bin_key, d.bin_key2, d.idx, d.idx2, n, (int)nbit_bins, stream));
     nb_permute(n, d.idx2, d.xq, xq2, d.v, v2, d.tag, tag2, d.perm, perm2, d.sysid, sysid2, d.mass, mass2, stream);
-    CK(copy_back_permuted(stream));
-    CK(cudaMemsetAsync(d.bin_start, 0, sizeof(int) * d.nbins, stream));
-    CK(cudaMemsetAsync(d.bin_end, 0, sizeof(int) * d.nbins, stream));
-    CK(cudaMemsetAsync(d.rowocc, 0, sizeof(int) * d.nbins, stream));
-    nb_bin_ranges(n, d.bin_key2, d.bin_start, d.bin_end, stream, d.sys, d.sysid, d.rowocc);
+    nb_place(n, permuted(), d.bin_key2, d.bin_start, d.bin_end, d.rowocc, d.sys, d.xh, d.xl, stream);
     // atoms' systems are contiguous after the sort: atom ranges per system
     CK(cudaGetLastError());
-    hilo_all();
     NbArgs a;
     memset(&a, 0, sizeof a);
     a.n = n;
@@ -2297,16 +2287,11 @@ struct Engine {
   int64_t graph_cap_limit = 0;     // > 0: lower it to this (exercises the overflow redo)
 
   cudaError_t enqueue_rebuild_fixed(cudaStream_t s) {
-    nb_wrap_bin(n, d.xq, d.sys, d.sysid, d.bin_key, d.idx, s);
+    nb_wrap_bin(n, d.xq, d.sys, d.sysid, d.bin_key, d.idx, d.bin_start, d.bin_end, d.rowocc, d.nbins, s);
     cudaError_t e = nb_sort(d.cub_tmp, d.cub_tmp_bytes, d.bin_key, d.bin_key2, d.idx, d.idx2, n, (int)nbit_bins, s);
     if (e != cudaSuccess) return e;
     nb_permute(n, d.idx2, d.xq, xq2, d.v, v2, d.tag, tag2, d.perm, perm2, d.sysid, sysid2, d.mass, mass2, s);
-    copy_back_permuted(s);
-    cudaMemsetAsync(d.bin_start, 0, sizeof(int) * d.nbins, s);
-    cudaMemsetAsync(d.bin_end, 0, sizeof(int) * d.nbins, s);
-    cudaMemsetAsync(d.rowocc, 0, sizeof(int) * d.nbins, s);
-    nb_bin_ranges(n, d.bin_key2, d.bin_start, d.bin_end, s, d.sys, d.sysid, d.rowocc);
-    hilo_all(s);
+    nb_place(n, permuted(), d.bin_key2, d.bin_start, d.bin_end, d.rowocc, d.sys, d.xh, d.xl, s);
     NbArgs a;
     memset(&a, 0, sizeof a);
     a.n = n;
@@ -3294,10 +3279,9 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
   if (!tmp) return g.fail(LMFF_EOVERFLOW, "lmff_compute_device_noalloc: scratch layout does not fit");
   size_t list_cap = (size_t)(cv.end - cv.p) / sizeof(uint32_t);
   uint32_t *list = cv.take<uint32_t>(list_cap);
-  // what must start at zero: status word, bin ranges, the count past the last atom
+  // what must start at zero: status word, the count past the last atom
   const double *host_arrs[2] = {stat_ilp, stat_ters};
   CK2(cudaMemsetAsync(status, 0, sizeof(int), st));
-  CK2(cudaMemsetAsync(bin_start, 0, sizeof(int) * (size_t)(bin_end - bin_start + nbins), st));   // both: neighbours
   CK2(cudaMemsetAsync(cnt + nn, 0, sizeof(int64_t), st));
   // the system and the table of arrays lie close together: one copy
   unsigned char head[2048];
@@ -3309,11 +3293,13 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
   CK2(cudaMemcpyAsync(dsys, head, arrs_at + sizeof host_arrs, cudaMemcpyHostToDevice, st));
   int gb = (nn + 255) / 256;
   k_load<<<gb, 256, 0, st>>>(nn, dx, dtype, dmol, nullptr, nullptr, nullptr, nullptr, xq, tag, perm, sysid, v, mass);
-  nb_wrap_bin(nn, xq, dsys, sysid, key, idx, st);
+  nb_wrap_bin(nn, xq, dsys, sysid, key, idx, bin_start, bin_end, nullptr, (int)nbins, st);
   CK2(nb_sort(tmp, tmp_bytes, key, key2, idx, idx2, nn, nbits, st));
   nb_permute(nn, idx2, xq, xq2, v, v2, tag, tag2, perm, perm2, sysid, sysid2, mass, mass2, st);
-  nb_bin_ranges(nn, key2, bin_start, bin_end, st);
-  nb_hilo(nn, xq2, dsys, sysid2, xh, xl, st);
+  Permuted sorted = {};
+  sorted.xq2 = xq2;
+  sorted.sysid2 = sysid2;
+  nb_place(nn, sorted, key2, bin_start, bin_end, nullptr, dsys, xh, xl, st);
   NbArgs na;
   memset(&na, 0, sizeof na);
   na.n = nn;

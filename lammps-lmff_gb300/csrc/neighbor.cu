@@ -26,9 +26,15 @@ __device__ __forceinline__ int bin_coord(double x, double lo, double binv, int n
 }
 
 // Wrap periodic coordinates into the box (LAMMPS Domain::pbc at reneighbouring) and
-// compute each atom's global bin.
-__global__ void k_wrap_bin(int n, d4 *xq, const SysDesc *sys, const int *sysid, uint32_t *key, int *idx) {
+// compute each atom's global bin; the bin arrays are set to zero (empty) on the way.
+__global__ void k_wrap_bin(int n, d4 *xq, const SysDesc *sys, const int *sysid, uint32_t *key, int *idx, int *bin_start,
+                           int *bin_end, int *rowocc, int nbins) {
   int p = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int b = p; b < nbins; b += gridDim.x * blockDim.x) {
+    bin_start[b] = 0;
+    bin_end[b] = 0;
+    if (rowocc) rowocc[b] = 0;
+  }
   if (p >= n) return;
   const SysDesc &sd = sys[sysid[p]];
   d4 q = xq[p];
@@ -66,40 +72,56 @@ __global__ void k_permute(int n, const int *idx2, const d4 *xq, d4 *xq2, const d
   mass2[q] = mass[o];
 }
 
-// Atom range of every occupied bin, and (rowocc) a flag at the first bin of every bin
-// row that holds atoms: the list build skips empty rows of its stencil whole (a bilayer
-// in a box with vacuum leaves most of them empty).
-__global__ void k_bin_ranges(int n, const uint32_t *key, int *bin_start, int *bin_end, const SysDesc *sys,
-                             const int *sysid, int *rowocc) {
-  int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const uint32_t k = key[q] >> KEY_MOL_BITS;
-  if (q == 0 || (key[q - 1] >> KEY_MOL_BITS) != k) {
-    bin_start[k] = q;
-    if (rowocc) {
-      const SysDesc &sd = sys[sysid[q]];
-      rowocc[k - (uint32_t)((int)k - sd.bin_begin) % (uint32_t)sd.nb[0]] = 1;
-    }
-  }
-  if (q == n - 1 || (key[q + 1] >> KEY_MOL_BITS) != k) bin_end[k] = q + 1;
-}
-
-// double-float split of each position: X = x - lo + 32 + base lies in [base, 2 base) for
+// double-float split of a position: X = x - lo + 32 + base lies in [base, 2 base) for
 // every position within 32 A of the box (base = 2^ceil(log2(Lmax + 64))), so
 // the hi parts of any two atoms of a system share one binade and their difference is
 // exact in FP32; lo = X - hi carries the remaining bits.
-__global__ void k_hilo(int n, const d4 *xq, const SysDesc *sys, const int *sysid, float4 *xh, float4 *xl) {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  const SysDesc &sd = sys[sysid[p]];
-  d4 q = xq[p];
+__device__ __forceinline__ void hilo_of(const d4 &q, const SysDesc &sd, float4 &xh, float4 &xl) {
   double X = q.x - sd.lo[0] + 32.0 + sd.base;
   double Y = q.y - sd.lo[1] + 32.0 + sd.base;
   double Z = q.z - sd.lo[2] + 32.0 + sd.base;
   float hx = (float)X, hy = (float)Y, hz = (float)Z;
   int info = (int)__double_as_longlong(q.w);
-  xh[p] = make_float4(hx, hy, hz, __int_as_float(info));
-  xl[p] = make_float4((float)(X - (double)hx), (float)(Y - (double)hy), (float)(Z - (double)hz), 0.f);
+  xh = make_float4(hx, hy, hz, __int_as_float(info));
+  xl = make_float4((float)(X - (double)hx), (float)(Y - (double)hy), (float)(Z - (double)hz), 0.f);
+}
+__global__ void k_hilo(int n, const d4 *xq, const SysDesc *sys, const int *sysid, float4 *xh, float4 *xl) {
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  hilo_of(xq[p], sys[sysid[p]], xh[p], xl[p]);
+}
+
+// What follows the permutation, in one pass over the sorted atoms: the arrays back to their
+// resident place (where there is one), the double-float positions, the atom range of every
+// occupied bin, and (rowocc) a flag at the first bin of every bin row that holds atoms: the
+// list build skips empty rows of its stencil whole (a bilayer in a box with vacuum leaves
+// most of them empty).  As six copies, three fills (k_wrap_bin's now) and two kernels these
+// took two to four us each: a rebuild of 1,152 atoms 163 -> 126 us, of 5,040 203 -> 173 us, of
+// a 300,240-atom bilayer 1.98 -> 1.92 ms.
+__global__ void k_place(int n, Permuted a, const uint32_t *key, int *bin_start, int *bin_end, int *rowocc,
+                        const SysDesc *sys, float4 *xh, float4 *xl) {
+  int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= n) return;
+  const d4 x = a.xq2[q];
+  const int sid = a.sysid2[q];
+  const SysDesc &sd = sys[sid];
+  if (a.xq) {
+    a.xq[q] = x;
+    a.v[q] = a.v2[q];
+    a.v[n + q] = a.v2[n + q];
+    a.v[2 * n + q] = a.v2[2 * n + q];
+    a.tag[q] = a.tag2[q];
+    a.perm[q] = a.perm2[q];
+    a.sysid[q] = sid;
+    a.mass[q] = a.mass2[q];
+  }
+  hilo_of(x, sd, xh[q], xl[q]);
+  const uint32_t k = key[q] >> KEY_MOL_BITS;
+  if (q == 0 || (key[q - 1] >> KEY_MOL_BITS) != k) {
+    bin_start[k] = q;
+    if (rowocc) rowocc[k - (uint32_t)((int)k - sd.bin_begin) % (uint32_t)sd.nb[0]] = 1;
+  }
+  if (q == n - 1 || (key[q + 1] >> KEY_MOL_BITS) != k) bin_end[k] = q + 1;
 }
 
 __device__ __forceinline__ bool le_exact(float rsq, float thr, double thr64, const d4 *xq, const SysDesc &sd,
@@ -355,8 +377,8 @@ __global__ void __launch_bounds__(32 * LW) k_list(NbArgs a) {
 // (with the sort and the copy to the list; in place / here / k_list): 1,152 atoms 0.19 / 0.16 /
 // 0.89 ms, 5,040-atom bilayer 0.25 / 0.20 / 0.62, 36,800-atom slab 1.90 / 1.04 / 2.28,
 // 60,480-atom bilayer - / 0.66 / 0.78, 81,200-atom slab - / 2.04 / 2.52, 300,240-atom bilayer
-// - / 2.58 / 1.98.  Bound by instruction issue (occupancy of 20 to 40 warps made no
-// difference).
+// - / 2.58 / 1.98 (all three before k_place took ~40 us off a rebuild).  Bound by instruction
+// issue (occupancy of 20 to 40 warps made no difference).
 constexpr int LIST_ATOM_MAX_ATOMS = 65536;
 constexpr int LIST_QUEUE = 64;
 __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
@@ -559,8 +581,9 @@ void nb_upload_const(const NbConst &c, cudaStream_t s) {
   cudaMemcpyToSymbolAsync(c_nb, &c, sizeof(c), 0, cudaMemcpyHostToDevice, s);
 }
 
-void nb_wrap_bin(int n, d4 *xq, const SysDesc *sys, const int *sysid, uint32_t *key, int *idx, cudaStream_t s) {
-  if (n) k_wrap_bin<<<(n + 255) / 256, 256, 0, s>>>(n, xq, sys, sysid, key, idx);
+void nb_wrap_bin(int n, d4 *xq, const SysDesc *sys, const int *sysid, uint32_t *key, int *idx, int *bs, int *be, int *rowocc,
+                 int nbins, cudaStream_t s) {
+  if (n) k_wrap_bin<<<(n + 255) / 256, 256, 0, s>>>(n, xq, sys, sysid, key, idx, bs, be, rowocc, nbins);
 }
 
 size_t nb_sort_tmp_bytes(int n, int nbits) {
@@ -587,9 +610,9 @@ void nb_permute(int n, const int *idx2, const d4 *xq, d4 *xq2, const double *v, 
   if (n) k_permute<<<(n + 255) / 256, 256, 0, s>>>(n, idx2, xq, xq2, v, v2, tag, tag2, perm, perm2, sysid, sysid2, mass, mass2);
 }
 
-void nb_bin_ranges(int n, const uint32_t *key, int *bs, int *be, cudaStream_t s, const SysDesc *sys, const int *sysid,
-                   int *rowocc) {
-  if (n) k_bin_ranges<<<(n + 255) / 256, 256, 0, s>>>(n, key, bs, be, sys, sysid, rowocc);
+void nb_place(int n, const Permuted &a, const uint32_t *key, int *bs, int *be, int *rowocc, const SysDesc *sys, float4 *xh,
+              float4 *xl, cudaStream_t s) {
+  if (n) k_place<<<(n + 255) / 256, 256, 0, s>>>(n, a, key, bs, be, rowocc, sys, xh, xl);
 }
 
 void nb_hilo(int n, const d4 *xq, const SysDesc *sys, const int *sysid, float4 *xh, float4 *xl, cudaStream_t s) {

@@ -52,7 +52,9 @@ struct NbArgs {
 };
 
 void nb_upload_const(const NbConst &c, cudaStream_t s);
-void nb_wrap_bin(int n, d4 *xq, const SysDesc *sys, const int *sysid, uint32_t *key, int *idx, cudaStream_t s);
+// bs, be and (or null) rowocc: the bin arrays, nbins each, set to zero
+void nb_wrap_bin(int n, d4 *xq, const SysDesc *sys, const int *sysid, uint32_t *key, int *idx, int *bs, int *be, int *rowocc,
+                 int nbins, cudaStream_t s);
 size_t nb_sort_tmp_bytes(int n, int nbits);
 cudaError_t nb_sort(void *tmp, size_t tmp_bytes, const uint32_t *k, uint32_t *k2, const int *v, int *v2, int n, int nbits,
                     cudaStream_t s);
@@ -60,8 +62,22 @@ cudaError_t nb_scan(void *tmp, size_t tmp_bytes, const int64_t *cnt, int64_t *of
 void nb_permute(int n, const int *idx2, const d4 *xq, d4 *xq2, const double *v, double *v2, const int64_t *tag,
                 int64_t *tag2, const int *perm, int *perm2, const int *sysid, int *sysid2, const double *mass,
                 double *mass2, cudaStream_t s);
-void nb_bin_ranges(int n, const uint32_t *key, int *bs, int *be, cudaStream_t s, const SysDesc *sys = nullptr,
-                   const int *sysid = nullptr, int *rowocc = nullptr);
+// after nb_permute: the permuted arrays (the names with 2) to their resident place unless
+// xq is null, the double-float positions and the bins' atom ranges
+struct Permuted {
+  const d4 *xq2;
+  const double *v2;
+  const int64_t *tag2;
+  const int *perm2, *sysid2;
+  const double *mass2;
+  d4 *xq;
+  double *v;
+  int64_t *tag;
+  int *perm, *sysid;
+  double *mass;
+};
+void nb_place(int n, const Permuted &a, const uint32_t *key, int *bs, int *be, int *rowocc, const SysDesc *sys, float4 *xh,
+              float4 *xl, cudaStream_t s);
 void nb_hilo(int n, const d4 *xq, const SysDesc *sys, const int *sysid, float4 *xh, float4 *xl, cudaStream_t s);
 // mode 0: count (+ short lists); 1: fill the CSR list; 2: count and write each atom's
 // entries into the strided buffer, for nb_compact after the scan
