@@ -2560,24 +2560,28 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
       const unsigned bits = __ballot_sync(FULL, near);
       if (near) queue[(qn + __popc(bits & below)) & (4 * tpa - 1)] = e;
       qn += __popc(bits & gmask);
-      // whole batches every third round (fewer than 4 tpa entries wait), so that when and on
-      // which lane an entry is evaluated depends on its atom's list alone: results are
-      // the same whatever atoms share the warp
+      // whole batches every third round (fewer than 4 tpa entries wait) of the atom's own
+      // list, not of the warp's longest: when and on which lane an entry is evaluated, and
+      // which sums have been brought to h + l before it is added, depends on the atom's list
+      // alone, so that its results are the same whatever atoms share the warp
       if (it % 3 == 0) {
-        while (__any_sync(FULL, qn - qh >= tpa)) near_batch(qn - qh >= tpa);
+        const bool own = k0 < cnt;
+        while (__any_sync(FULL, own && qn - qh >= tpa)) near_batch(own && qn - qh >= tpa);
         // the sums' lo parts gather one rounding of the hi part per term: brought back below
         // it before their own rounding shows
+        if (own) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          f[c] = renorm(f[c]);
-          g[c] = renorm(g[c]);
-        }
-        tpi = renorm(tpi);
-        if constexpr (EV) {
-          ev = renorm(ev);
-          er = renorm(er);
+          for (int c = 0; c < 3; c++) {
+            f[c] = renorm(f[c]);
+            g[c] = renorm(g[c]);
+          }
+          tpi = renorm(tpi);
+          if constexpr (EV) {
+            ev = renorm(ev);
+            er = renorm(er);
 #pragma unroll
-          for (int c = 0; c < 6; c++) w[c] = renorm(w[c]);
+            for (int c = 0; c < 6; c++) w[c] = renorm(w[c]);
+          }
         }
       }
     }
