@@ -2255,9 +2255,9 @@ __global__ void __launch_bounds__(256, (ilp_min_blocks<TPA, EV, EATOM, ONE, GH, 
 // The virial: half of del (x) f_ij at each end of a pair, which sums to the whole of the
 // pair's; the n_i part of f_ij is applied to the sums after the loop (f -= tpi n_i,
 // W -= g (x) n_i).
-// Pairs closer than 0.5 A (below the tables) are left to ilp_pair (FP64) in a second walk
-// over the lane's entries; so is every pair of an atom so far outside its box that the
-// position grids do not hold it (SysDesc::dfmax).
+// Pairs closer than 0.5 A (below the tables) or at the cutoff to the last bits of r^2 are left
+// to ilp_pair (FP64) in a second walk over the lane's entries; so is every pair of an atom so
+// far outside its box that the position grids do not hold it (SysDesc::dfmax).
 //
 // An atom's lanes walk its list tpa entries at a time.  The parts the normals enter are
 // ~350 instructions for a third of the pairs (carbon), scattered through the list: entries
@@ -2274,6 +2274,19 @@ struct DfCut {
   float h, l;   // r_cut^2
 };
 __constant__ DfCut c_dfcut;
+// r^2 - r_cut^2 of a pair (double-float q).  Within DF_EDGE of the cutoff, 30 times q's error
+// at the tables' end, the FP64 form decides, as it does for every pair of the general kernel:
+// without the taper a pair's force ends in a step there
+constexpr float DF_EDGE = 0x1p-31f;   // A^2
+__device__ __forceinline__ float df_past_cut(const df::D<float> &q) {
+  return __fadd_rn(__fsub_rn(q.h, c_dfcut.h), __fsub_rn(q.l, c_dfcut.l));
+}
+__device__ __forceinline__ bool df_inside(const df::D<float> &q, float past) {
+  return past <= -DF_EDGE && q.h >= DF_CLOSE;
+}
+__device__ __forceinline__ bool df_apart(const df::D<float> &q, float past) {   // left to the FP64 form
+  return !df_inside(q, past) && past < DF_EDGE;
+}
 __constant__ float c_dfk[df::K_N];                    // element pair (0, 0)'s constants
 __device__ float g_dfk[MAXELEM * MAXELEM * df::K_N];  // element pair (a, b)'s at (a * ne + b) * K_N
 __device__ float2 g_exp2_df[df::EXP2_TAB];
@@ -2354,7 +2367,8 @@ __device__ __forceinline__ void df_del(const DfAtom &I, const DfAtom &A, const S
   }
 }
 
-// the pairs closer than DF_CLOSE (with all, every pair) of one lane's entries, in FP64
+// the pairs closer than DF_CLOSE or at the cutoff (with all, every pair) of one lane's
+// entries, in FP64
 template <bool EV, bool ONE, bool GH>
 __device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int lane, int tpa, int ie, bool iown,
                                             bool all, IlpAcc &acc) {
@@ -2375,7 +2389,8 @@ __device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int la
     A.load(a.jrec, a.jstride, j);
     df::D<float> d[3];
     df_del<true>(I, A, sd, sx, sy, sz, d);
-    if (!all && !(df::dot3(d, d).h < DF_CLOSE)) continue;
+    const df::D<float> q = df::dot3(d, d);
+    if (!all && !df_apart(q, df_past_cut(q))) continue;
     ilp_pair<EV, ONE, false, true, GH>(a, ai, sd, e, ai.fetch(a.A, j), NrmJ<R>::load(a, j), ni.x, ni.y, ni.z, ie,
                                        info_mol(ai.info), itag, false, iown, acc);
   }
@@ -2510,11 +2525,9 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
         D<V> d[3];
         pair_of(e, A, j, d);
         const D<V> q = dot3(d, d);
-        bool in = __fadd_rn(__fsub_rn(q.h, c_dfcut.h), __fsub_rn(q.l, c_dfcut.l)) < 0.f;
-        if (in && q.h < DF_CLOSE) {   // rare
-          close = true;
-          in = false;
-        }
+        const float past = df_past_cut(q);
+        const bool in = df_inside(q, past);
+        close = close || df_apart(q, past);   // rare
         if (in) {
           float th;
           int k = tab_at(q.h, th);
@@ -3365,13 +3378,12 @@ constexpr int VA_LANES = 8;
 constexpr float VA_NEARSQ = 49.f;
 static_assert(VA_NEARSQ <= df::Q64_MAX, "the FP64 tables end at Q64_MAX");
 
-// whether entry e of atom i's list is a pair inside the cutoff, and its q = r^2 as both
-// kernels' split tests it
-__device__ __forceinline__ bool va_pair_q(const DfAtom &I, const DfAtom &A, const SysDesc &sd, int sx, int sy, int sz,
-                                          df::D<float> d[3], df::D<float> &q) {
+// r^2 - r_cut^2 of an entry of atom i's list, and its q = r^2 as both kernels' split tests it
+__device__ __forceinline__ float va_pair_q(const DfAtom &I, const DfAtom &A, const SysDesc &sd, int sx, int sy, int sz,
+                                           df::D<float> d[3], df::D<float> &q) {
   df_del<true>(I, A, sd, sx, sy, sz, d);
   q = df::dot3(d, d);
-  return __fadd_rn(__fsub_rn(q.h, c_dfcut.h), __fsub_rn(q.l, c_dfcut.l)) < 0.f;
+  return df_past_cut(q);
 }
 
 // per atom: A (18, row-major k, a) then B (9, row-major a, b) in 28 doubles, the last 1 where
@@ -3409,8 +3421,8 @@ __global__ void __launch_bounds__(128) k_va_tens_df(ForceArgs<R> a) {
   }
 }
 
-// the pairs closer than DF_CLOSE (with all, every pair) of one lane's entries, in FP64:
-// v = w[6], g[3], G[6]
+// the pairs closer than DF_CLOSE or at the cutoff (with all, every pair) of one lane's
+// entries, in FP64: v = w[6], g[3], G[6]
 template <bool GH>
 __device__ __noinline__ void va_close_pairs(const ForceArgs<R> &a, int i, int lane, int ie, bool iown, bool all,
                                             double *v) {
@@ -3428,7 +3440,8 @@ __device__ __noinline__ void va_close_pairs(const ForceArgs<R> &a, int i, int la
     DfAtom A;
     A.load(a.jrec, a.jstride, j);
     df::D<float> d[3], s;
-    if (!all && !(va_pair_q(I, A, sd, sx, sy, sz, d, s) && s.h < DF_CLOSE)) continue;
+    const float past = va_pair_q(I, A, sd, sx, sy, sz, d, s);
+    if (!all && !df_apart(s, past)) continue;
     va_pair64<GH, false>(a, i, e, ie, mi, itag, iown, ni.x, ni.y, ni.z, v, v[6], v[7], v[8], v + 9);
   }
 }
@@ -3540,11 +3553,9 @@ __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
       DfAtom A;
       A.load(a.jrec, a.jstride, j);
       df::D<float> d[3], q;
-      near = va_pair_q(I, A, sd, sx, sy, sz, d, q) && q.h < VA_NEARSQ;
-      if (near && q.h < DF_CLOSE) {   // rare
-        near = false;
-        close = true;
-      }
+      const float past = va_pair_q(I, A, sd, sx, sy, sz, d, q);
+      near = df_inside(q, past) && q.h < VA_NEARSQ;
+      close = close || df_apart(q, past);   // rare
     }
     const unsigned bits = __ballot_sync(FULL, near);
     if (near) queue[(qn + __popc(bits & below)) & (QUEUE - 1)] = e;
@@ -3708,7 +3719,7 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
       DfAtom A;
       A.load(a.jrec, a.jstride, j);
       D<V> d[3], q;
-      if (va_pair_q(I, A, sd, sx, sy, sz, d, q) && !(q.h < VA_NEARSQ)) {
+      if (va_pair_q(I, A, sd, sx, sy, sz, d, q) <= -DF_EDGE && !(q.h < VA_NEARSQ)) {   // k_va_near has the pairs at the cutoff
         const float *row = ONE ? nullptr : g_dfk + (ie * ne + A.el) * K_N;
         auto K = [&](int k2) {
           if constexpr (ONE) return c_dfk[k2];
