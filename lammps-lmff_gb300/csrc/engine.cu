@@ -1679,7 +1679,12 @@ struct Engine {
       if (fork && !FRAME_FIRST) cudaStreamWaitEvent(stream, ev_frame, 0);
       timed(6, [&] { fn(a, ev, stream); });
     }
-    else if (ev) cudaMemsetAsync(stat_ilp, 0, sizeof(double) * 8 * (size_t)n, stream);
+    else {
+      // an atom without a normal is an error for every style: the mixed k_short says so, in
+      // FP64 the frames do (4 us for 7,200 atoms)
+      if (FRAME_FIRST && i_on) timed(6, [&] { fr(a, stream); });
+      if (ev) cudaMemsetAsync(stat_ilp, 0, sizeof(double) * 8 * (size_t)n, stream);
+    }
     if (eatom && !a.do_ters) cudaMemsetAsync(eatom_ters, 0, sizeof(double) * (size_t)n, stream);
     if (fork) cudaStreamWaitEvent(stream, ev_join, 0);
     timed(3, [&] { ff(a, eatom, kick_on ? &kick_args : nullptr, stream); });
@@ -3417,8 +3422,8 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     f64::launch_short(a, g.d_cutILPsq, g.ht.cutmax * g.ht.cutmax, st);
     if (a.do_ters) f64::launch_tersoff(a, ev, false, fork(a));
     else CK2(cudaMemsetAsync(stat_ters, 0, sizeof(double) * 8 * (size_t)nn, st));
+    if (g.i_on) f64::launch_nframe(a, st);   // also without ILP: it finds atoms without a normal
     if (a.do_ilp) {
-      f64::launch_nframe(a, st);
       f64::launch_ilp(a, ev, false, g.tpa, g.block, g.i_one, st);
       f64::launch_nderiv(a, ev, st);
     } else {
