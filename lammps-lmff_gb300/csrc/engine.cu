@@ -2192,6 +2192,7 @@ struct Engine {
     }
     ForceArgs<double> a = args<double>();
     a.va64 = d_va64;
+    a.status = nullptr;   // the evaluation has reported; the next one's word stays clear
     a.do_ters = t_on && (which & LMFF_TERSOFF);
     a.do_ilp = i_on && (which & LMFF_ILP);
     const size_t c6 = 6 * (size_t)va_cap;

@@ -305,7 +305,7 @@ struct ForceArgs {
   // MAXTERS per atom, by short-list slot) and intralayer neighbours (va_is: MAXILP per atom)
   double *va_t, *va_i, *va_ts, *va_is;
   float4 *va_tens;     // the frames' partner-share tensors (k_va_tens: 7 per atom; k_va_tens_df: 14 + 14)
-  int *status;
+  int *status;         // null in the per-atom virial pass
   int do_ters, do_ilp;
   int list_full;       // the pair list also holds same-molecule / non-ILP pairs
   // subdomain (ghost-atom) mode: non-null when the caller passes owned atoms followed by

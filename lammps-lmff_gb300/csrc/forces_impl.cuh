@@ -2855,7 +2855,7 @@ __global__ void __launch_bounds__(128) k_frame(ForceArgs<R> a) {
   if (i >= a.n) return;
   NFrame fr;
   nframe_eval(a, i, fr);
-  if (fr.cont >= 2 && !fr.ok) raise_status(a.status, ST_ZERO_NORMAL);
+  if (fr.cont >= 2 && !fr.ok && a.status) raise_status(a.status, ST_ZERO_NORMAL);
   if (a.nframe) {
     d4 *q = a.nframe + 4 * (size_t)i;
     q[0] = make_d4(fr.nx, fr.ny, fr.nz, fr.inn);

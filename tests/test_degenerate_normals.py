@@ -56,3 +56,18 @@ def test_refused_without_allocation(which, precision):
         eng.compute_device_noalloc(torch.tensor(x, device="cuda"), *args, f, which=which)
     x[-1, 1] += 0.3
     eng.compute_device_noalloc(torch.tensor(x, device="cuda"), *args, f, which=which)
+
+
+def test_per_atom_virial_leaves_no_error_behind():
+    """Three atoms on a line whose cross product is zero in FP64 and a rounding in FP32: the
+    mixed evaluation goes through, and so does the next one after the per-atom virial, which
+    makes the normals in FP64."""
+    x, t, m, g, s = _line()
+    v = np.array([943718, 838861, 734003]) * 2.0 ** -20   # products exact in FP64, not in FP32
+    x[-3:] = np.round(x[-2]) + np.array([-1.0, 0.0, 1.0])[:, None] * v
+    eng = _engine(s, capi.MIXED)
+    eng.compute(x, t, m, g)
+    eng.set_precision(capi.FP64)
+    eng.vatom(capi.ILP)
+    x[-1, 1] += 0.3
+    eng.compute(x, t, m, g, same_atoms=True)
