@@ -203,12 +203,13 @@ __global__ void k_unpermute_state(int n, const int *perm, const d4 *xq, const do
   }
 }
 
-// Deterministic per-system reduction of the per-atom stat arrays: block (s, q, c) sums chunk
-// c of quantity q of system s in a fixed order, and the last of a quantity's blocks its
-// chunks' sums.  A system of one chunk (and, without part, any system) is one block's work.
+// Deterministic per-system reduction of the per-atom stat arrays: a block sums quantity q of
+// one chunk of a system in a fixed order, and the last of the quantity's blocks in the system
+// its chunks' sums.  map: each chunk's system and place in it, so that a batch has as many
+// blocks as chunks whatever its systems' sizes; without map a block per system and quantity.
 // Chunks are counted from the system's first atom, so a system's sums do not depend on what
 // else is in its batch.  One block per quantity took 70 us for 36,800 atoms (a chain of
-// ~0.5 us loads) and grew with n; REDUCE_MEASURED.
+// ~0.5 us loads) and grew with n; in chunks 8.4 us, for 331,200 atoms 21.7 us (caches cold).
 constexpr int RED_THREADS = 256, RED_CHUNK = 8 * RED_THREADS;
 // sum over the block, in thread 0
 __device__ __forceinline__ double block_sum(double acc, double *sh) {
@@ -224,14 +225,14 @@ __device__ __forceinline__ double block_sum(double acc, double *sh) {
   return v;
 }
 __global__ void __launch_bounds__(RED_THREADS) k_reduce(int n, int nq, const double *const *arrs, const SysDesc *sys,
-                                                        double *out, int cmax, double *part, int *count) {
+                                                        double *out, const int2 *map, double *part, int *count) {
   __shared__ double sh[RED_THREADS];
   __shared__ bool last;
-  const int c = blockIdx.x % cmax, sq = blockIdx.x / cmax, s = sq / nq, q = sq % nq;
+  const int g = blockIdx.x / nq, q = blockIdx.x % nq;
+  const int s = map ? map[g].x : g, c = map ? map[g].y : 0, sq = s * nq + q;
   const double *a = arrs[q / 8] + (size_t)(q % 8) * n;
   const int b = sys[s].atom_begin, e = sys[s].atom_end;
-  const int m = part ? (e - b + RED_CHUNK - 1) / RED_CHUNK : 1;   // chunks
-  if (c > 0 && c >= m) return;
+  const int m = map ? (e - b + RED_CHUNK - 1) / RED_CHUNK : 1;   // chunks
   const int p0 = b + c * RED_CHUNK, p1 = m > 1 ? min(e, p0 + RED_CHUNK) : e;
   double acc = 0.0;
   for (int p = p0 + threadIdx.x; p < p1; p += RED_CHUNK) {
@@ -246,7 +247,7 @@ __global__ void __launch_bounds__(RED_THREADS) k_reduce(int n, int nq, const dou
     if (threadIdx.x == 0) out[sq] = v;
     return;
   }
-  double *ps = part + ((size_t)(b / RED_CHUNK) + s) * nq;   // the systems before s have fewer chunks than that
+  double *ps = part + (size_t)(g - c) * nq;
   if (threadIdx.x == 0) {
     ps[(size_t)c * nq + q] = v;
     __threadfence();
@@ -754,12 +755,13 @@ struct Engine {
     void *ptrs[] = {d.xq, d.xh, d.xl, d.v, d.f, d.xhold, d.tag, d.perm, d.sysid, d.mass, d.nrm64, d.nrm32, d.jrec, d.ilp_cnt,
                     d.ilp_nb, d.ters_cnt, d.ters_nb, d.ters_g, d.ters_f, d.ilp_f, d.ilp_c, d.ilp_g, d.nframe, d.list_off, d.list,
                     d.short_cnt, d.short_nb, d.list_img, d.nin_tmp, d.list_tmp, d.bin_key, d.bin_key2, d.idx, d.idx2, d.bin_start, d.bin_end, d.rowocc, d.cub_tmp,
-                    d.cnt_tmp, d.sys, d.red_out, d.partials, d.red_count, d.status, d.maxdisp, d_xin, d_fin, d_fo, d_vin, d_ein, d_tin, d_sysin,
+                    d.cnt_tmp, d.sys, d.red_out, d.red_map, d.partials, d.red_count, d.status, d.maxdisp, d_xin, d_fin, d_fo, d_vin, d_ein, d_tin, d_sysin,
                     d_min, d_gin, d_massT, xq2, v2, mass2, tag2, perm2, sysid2, stat_ilp, stat_ters, eatom_ilp,
                     eatom_ters, ke, d_arrs, d_karrs, d_kout, d_cutILPsq, d_maxpred, d_va, d_dfA, d_dfM, d_dfU, d_dfTE, d_va64};
     for (void *p : ptrs)
       if (p) cudaFree(p);
     d = DevState();
+    red_layout.clear();
     d_xin = d_fin = d_fo = d_vin = d_ein = nullptr;
     if (h_words) cudaFreeHost(h_words);
     h_words = nullptr;
@@ -1695,23 +1697,45 @@ struct Engine {
     double *f, *eatom;
   };
 
-  // the reduction's chunk sums (of every system) and counters (zero between launches)
+  // the reduction's chunks (a table of them where a system has more than one), their sums,
+  // and counters (zero between launches), for the resident systems' atom counts
   int ensure_partials() {
-    red_cmax = 1;
-    for (const SysDesc &s : hsys) red_cmax = std::max(red_cmax, (s.atom_end - s.atom_begin + RED_CHUNK - 1) / RED_CHUNK);
-    const int need = (int)(16 * (n / RED_CHUNK + hsys.size() + 1));
-    if (red_cmax > 1 && need > d.partials_cap) {
-      CK(cudaStreamSynchronize(stream));
-      CK(dalloc(d.partials, need));
-      CK(dalloc(d.red_count, need));
-      CK(cudaMemsetAsync(d.red_count, 0, sizeof(int) * (size_t)need, stream));
-      d.partials_cap = need;
+    const std::vector<int> one = {0, n};
+    const std::vector<int> &lay = batch_offsets.size() == hsys.size() + 1 ? batch_offsets : one;
+    if (lay == red_layout) return LMFF_OK;
+    red_layout.clear();
+    CK(cudaStreamSynchronize(stream));   // an earlier copy out of red_map is done
+    red_map.clear();
+    const int nsys = (int)lay.size() - 1;
+    for (int s = 0; s < nsys; s++) {
+      const int m = std::max(1, (lay[s + 1] - lay[s] + RED_CHUNK - 1) / RED_CHUNK);
+      for (int c = 0; c < m; c++) red_map.push_back(make_int2(s, c));
+      if (s == 0) red_first = m;
     }
+    red_split = (int)red_map.size() > nsys;
+    if (red_split) {
+      const int need = (int)red_map.size();
+      if (need > d.partials_cap) {
+        CK(dalloc(d.red_map, need));
+        CK(dalloc(d.partials, 16 * (size_t)need));
+        CK(dalloc(d.red_count, 16 * (size_t)need));
+        CK(cudaMemsetAsync(d.red_count, 0, sizeof(int) * 16 * (size_t)need, stream));
+        d.partials_cap = need;
+      }
+      CK(cudaMemcpyAsync(d.red_map, red_map.data(), sizeof(int2) * (size_t)need, cudaMemcpyHostToDevice, stream));
+    }
+    red_layout = lay;
     return LMFF_OK;
   }
-  int red_cmax = 1;
+  std::vector<int> red_layout;   // the systems' offsets that red_map is for
+  std::vector<int2> red_map;
+  int red_first = 1;             // chunks of the first system
+  bool red_split = false;
+  int red_blocks(int nsys) const { return !red_split ? nsys : nsys == 1 ? red_first : (int)red_map.size(); }
+  // the first system (nsys 1) or all
   void reduce(int nq, double *const *arrs, int nsys, double *out) {
-    k_reduce<<<nsys * nq * red_cmax, RED_THREADS, 0, stream>>>(n, nq, arrs, d.sys, out, red_cmax, d.partials, d.red_count);
+    k_reduce<<<red_blocks(nsys) * nq, RED_THREADS, 0, stream>>>(n, nq, arrs, d.sys, out, red_split ? d.red_map : nullptr,
+                                                                d.partials, d.red_count);
   }
 
   // forces (+ energies/virials per system into hres when ev) on the resident state
@@ -2369,9 +2393,9 @@ struct Engine {
     if (precision == LMFF_FP64) key_put(k, args<double>());
     else key_put(k, args<float>());
     const int ints[] = {precision, which, (int)ev, (int)eatom, tpa, block, (int)ters_concurrent, (int)hsys.size(),
-                        red_cmax};
+                        red_blocks((int)hsys.size()), (int)red_split};
     key_put(k, ints);
-    const void *ptrs[] = {d_arrs, d.sys, d.red_out, d.partials, d.red_count, stat_ilp, stat_ters, eatom_ters};
+    const void *ptrs[] = {d_arrs, d.sys, d.red_out, d.red_map, d.partials, d.red_count, stat_ilp, stat_ters, eatom_ters};
     key_put(k, ptrs);
     return k;
   }
@@ -3447,7 +3471,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     join(a);
     f32::launch_finish(a, false, nullptr, st);
   }
-  k_reduce<<<16, RED_THREADS, 0, st>>>(nn, 16, (const double *const *)arrs, dsys, red, 1, nullptr, nullptr);
+  k_reduce<<<16, RED_THREADS, 0, st>>>(nn, 16, (const double *const *)arrs, dsys, red, nullptr, nullptr, nullptr);
   k_scatter_add<<<gb, 256, 0, st>>>(nn, perm2, fs, df, 1);
   CK2(cudaGetLastError());
   double hred[16];

@@ -189,8 +189,9 @@ struct DevState {
   // systems
   SysDesc *sys = nullptr;
   // reductions
-  double *partials = nullptr; // NSTAT * 2 per chunk of a system
-  int *red_count = nullptr;   // NSTAT * 2 * nsys: chunks summed so far
+  int2 *red_map = nullptr;    // each chunk's system and place in it
+  double *partials = nullptr; // NSTAT * 2 per chunk
+  int *red_count = nullptr;   // NSTAT * 2 per system: chunks summed so far
   int partials_cap = 0;
   double *red_out = nullptr;  // NSTAT * 2 * nsys
   int *status = nullptr;      // device status word
