@@ -1055,10 +1055,12 @@ struct Engine {
     return lo < 1e30 ? lo * lo : 0.0;
   }
   double ters_rlosq = 0.0;
+  int two_pair = 0;
 
   int build_consts() {
     fill_pot(pot64);
     fill_pot(pot32);
+    two_pair = two_pair_forms(pot32);
     pair_df = pair_df_elements();
     ters_rlosq = ters_fast_rlosq();
     memset(&nbc, 0, sizeof nbc);
@@ -1164,7 +1166,8 @@ struct Engine {
   }
 
   // Upload the constant tables to the device (caller holds the device lock exclusively
-  // and the device is idle); synchronous so that other streams see them complete.
+  // and the device is idle); synchronous so that other streams see them complete.  Threads
+  // may be here at the same time for other devices: nothing of it is process-wide.
   int upload_tables() {
     f64::upload_pot(pot64, stream);
     f32::upload_pot(pot32, stream);
@@ -1633,6 +1636,7 @@ struct Engine {
     a.pair_tile = pair_tile;
     a.no_small = !small_variants;
     a.kc = i_on && hi.model == LMFF_INTERLAYER_KC;
+    a.two_pair = two_pair;
     a.pair_df = pair_df;
     a.df_A = d_dfA;
     a.df_M = d_dfM;
@@ -3418,6 +3422,7 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
     a.do_ilp = g.i_on && (which & LMFF_ILP);
     a.list_full = g.list_full;
     a.kc = g.i_on && g.hi.model == LMFF_INTERLAYER_KC;
+    a.two_pair = g.two_pair;
     a.pair_df = g.pair_df;
     a.df_A = g.d_dfA;
     a.df_M = g.d_dfM;

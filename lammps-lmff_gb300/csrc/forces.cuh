@@ -337,6 +337,7 @@ struct ForceArgs {
   const float4 *df_A, *df_M;
   const float2 *df_U, *df_TE;
   const double *va64;
+  int two_pair;        // mixed mode: two_pair_forms of the potential
   // FP64 mode: the square of the smallest R - D of the Tersoff triplets where tersoff_fast
   // takes the potential (Engine::ters_rlosq), else 0
   double ters_rlosq;
@@ -348,6 +349,21 @@ struct ForceArgs {
   // their blocks exit
   int pdl;
 };
+
+// whether the mixed mode's two-pair loop takes the potential: bit 0, with one element (C >= 0);
+// bit 1, with several (symmetric element-pair constants with C >= 0).  Not in PotConst:
+// growing c_pot changes the single-element pair kernel's register allocation (measured: a
+// spill and -2 %)
+inline int two_pair_forms(const PotConst<float> &p) {
+  if (!p.i_enabled || p.kc) return 0;
+  bool multi = p.vdw_sym;
+  for (int a = 0; a < p.i_ne; a++)
+    for (int b = 0; b < p.i_ne; b++) {
+      const IlpP<float> &o = p.ilp[a * MAXELEM + b];
+      multi = multi && o.same_as_swapped && o.C >= 0.f;
+    }
+  return (p.ilp[0].C >= 0.f ? 1 : 0) | (multi ? 2 : 0);
+}
 
 enum : int { PDL_ILP = 1, PDL_NDERIV = 2, PDL_FINISH = 4, PDL_SHORT = 8, PDL_TRIGGER = 16 };
 

@@ -35,11 +35,6 @@ constexpr bool TWO_PAIR_BODY = true;
 constexpr bool TWO_PAIR_BODY = false;
 #endif
 
-// whether the two-pair loop applies (set with the constants by upload_pot, read by the
-// launch): element 0's C >= 0 (single element); symmetric element-pair constants with
-// C >= 0 (several elements)
-static int h_two_one = 0, h_two_multi = 0;
-
 __device__ __forceinline__ R cR(double v) { return (R)v; }
 
 __device__ __forceinline__ void raise_status(int *status, int bit) { atomicOr(status, bit); }
@@ -1743,7 +1738,7 @@ __constant__ PairX2Const c_x2;
 // neighbours of one iteration, the parameter pairs (X[a][b], X[a][c]) of every per-pair
 // constant, one 64-bit shared-memory read each.  Valid when every element pair's
 // parameters equal those of the swapped pair (then both repulsion terms and vdW use
-// X[a][b]) and C >= 0 (h_two_multi, set by upload_pot).
+// X[a][b]) and C >= 0 (two_pair_forms).
 constexpr int X2M_N = 11;   // nd2_l2e, log2C, eps, 2/delta^2, lambda, -lam log2e, lam z0 log2e,
                             // -ts_a, ts_a seff, C6, d/seff
 constexpr int X2M_ROWS = MAXELEM * MAXELEM * MAXELEM;
@@ -2655,10 +2650,15 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
   }
 }
 
-// constants of the double-float kernel from the FP64 ones
-static void upload_pair_df(const PotConst<R> &p, cudaStream_t s) {
-  static float rows[MAXELEM * MAXELEM * df::K_N];   // static: the asynchronous copies read them after return
-  static DfCut cut;
+// constants of the double-float kernel from the FP64 ones, in storage of this call: threads
+// with engines on several devices upload at the same time
+struct PairDfConst {
+  float rows[MAXELEM * MAXELEM * df::K_N];
+  DfCut cut;
+};
+static void upload_pair_df(const PotConst<R> &p, PairDfConst &c, cudaStream_t s) {
+  float *const rows = c.rows;
+  DfCut &cut = c.cut;
   auto split = [](double v, float &h, float &l) {
     h = (float)v;
     l = (float)(v - (double)h);
@@ -2674,7 +2674,7 @@ static void upload_pair_df(const PotConst<R> &p, cudaStream_t s) {
     }
   cudaMemcpyToSymbolAsync(c_dfk, rows, sizeof c_dfk, 0, cudaMemcpyHostToDevice, s);
   cudaMemcpyToSymbolAsync(c_dfcut, &cut, sizeof cut, 0, cudaMemcpyHostToDevice, s);
-  cudaMemcpyToSymbolAsync(g_dfk, rows, sizeof rows, 0, cudaMemcpyHostToDevice, s);
+  cudaMemcpyToSymbolAsync(g_dfk, rows, sizeof c.rows, 0, cudaMemcpyHostToDevice, s);
   k_fill_exp2_df<<<1, df::EXP2_TAB, 0, s>>>();
 }
 
@@ -4015,15 +4015,18 @@ __global__ void __launch_bounds__(128) k_va_slots(ForceArgs<R> a) {
 
 // ============================================================ host launchers ======
 
+// Returns when the copies have been made: they read storage of this call.
 void upload_pot(const PotConst<R> &p, cudaStream_t s) {
   cudaMemcpyToSymbolAsync(c_pot, &p, sizeof(p), 0, cudaMemcpyHostToDevice, s);
 #ifndef LMFF_PACKED_X2
   k_fill_exp2_f64<<<1, EXP2_F64_N, 0, s>>>();
-  if (p.i_enabled && !p.kc) upload_pair_df(p, s);
+  PairDfConst dfc = {};
+  if (p.i_enabled && !p.kc) upload_pair_df(p, dfc, s);
 #endif
 #ifdef LMFF_PACKED_X2
+  PairX2Const x2;
+  float2 tab[X2M_ROWS * X2M_N];
   {
-    static PairX2Const x2;   // static: the asynchronous copy reads it after return
     const IlpP<float> &q = p.ilp[0];
     x2.tap0 = make_float2(20.f, 140.f);
     x2.tap1 = make_float2(-70.f, -420.f);
@@ -4057,19 +4060,7 @@ void upload_pot(const PotConst<R> &p, cudaStream_t s) {
     x2.log2C = make_float2(l2c, l2c);
     x2.eps = make_float2(2.f * q.eps_half, 2.f * q.eps_half);
     cudaMemcpyToSymbolAsync(c_x2, &x2, sizeof(x2), 0, cudaMemcpyHostToDevice, s);
-    // kept out of PotConst: growing c_pot changes the single-element pair kernel's
-    // register allocation (measured: a spill and -2 %)
-    static int p2m;
-    p2m = (p.i_enabled && !p.kc && p.vdw_sym) ? 1 : 0;
-    for (int ea = 0; ea < p.i_ne; ea++)
-      for (int eb = 0; eb < p.i_ne; eb++) {
-        const IlpP<float> &o = p.ilp[ea * MAXELEM + eb];
-        if (!o.same_as_swapped || !(o.C >= 0.f)) p2m = 0;
-      }
-    h_two_multi = p2m;
-    h_two_one = (p.i_enabled && !p.kc && p.ilp[0].C >= 0.f) ? 1 : 0;
-    if (p2m) {
-      static float2 tab[X2M_ROWS * X2M_N];
+    if (two_pair_forms(p) & 2) {
       for (int ea = 0; ea < MAXELEM; ea++)
         for (int eb = 0; eb < MAXELEM; eb++)
           for (int ec = 0; ec < MAXELEM; ec++) {
@@ -4094,6 +4085,7 @@ void upload_pot(const PotConst<R> &p, cudaStream_t s) {
   }
 #endif
   if (sizeof(R) == 4) k_fill_exptab<<<EXP_TAB_N / 256, 256, 0, s>>>();
+  cudaStreamSynchronize(s);
 }
 
 void launch_short(const ForceArgs<R> &a, const double *cutILPsq64, double tcutmaxsq64, cudaStream_t s) {
@@ -4138,7 +4130,7 @@ static void launch_ilp_t(const ForceArgs<R> &a, bool ev, bool eatom, int block, 
   }
   if (ev && eatom) launch_pdl(p, k_ilp<TPA, true, true, ONE, false, false, false>, g, block, s, a);
   else if (ev) launch_pdl(p, k_ilp<TPA, true, false, ONE, false, false, false>, g, block, s, a);
-  else if (TWO_PAIR_BODY && !a.list_full && a.pair_tile != 1 && (ONE ? h_two_one : h_two_multi))
+  else if (TWO_PAIR_BODY && !a.list_full && a.pair_tile != 1 && (a.two_pair & (ONE ? 1 : 2)))
     launch_pdl(p, k_ilp<TPA, false, false, ONE, false, false, TWO_PAIR_BODY>, g, block, s, a);
   else launch_pdl(p, k_ilp<TPA, false, false, ONE, false, false, false>, g, block, s, a);
 }
