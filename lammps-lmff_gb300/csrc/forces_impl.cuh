@@ -886,35 +886,49 @@ __device__ __forceinline__ double ln_t64(double x) {
 // latency at 5k; the per-atom virial's pass 160 -> 58 us on 36,800.  Against 80-bit arithmetic
 // the forces' error is 0.9e-14 where the general routine's is 1.2e-14, the per-atom virial's
 // 1.0e-14 where it is 1.5e-14.
-// Returns false, nothing written, for an atom it does not take.
-template <bool EV, bool GH, bool VA>
-__device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int ie, int cnt) {
-  if (cnt < 2 || cnt > 3 || !(a.ters_rlosq > 0.0)) return false;
-  const SysDesc &sd = a.A.sys[a.A.sysid[i]];
-  double d[3][3], r[3], ri[3], e[3][3];
+// tersoff_bonds: the bonds of an atom, and whether its form is the short one; tersoff_fast
+// returns false, nothing written, where that shows only later (b_ij's limits).
+struct TersBonds {
+  double d[3][3], rs[3];   // x_j - x_i, r^2
   int el[3];
   uint32_t en[3];
+};
+__device__ __forceinline__ bool tersoff_bonds(const ForceArgs<R> &a, int i, int cnt, TersBonds &o) {
+  if (cnt < 2 || cnt > 3) return false;
+  const SysDesc &sd = a.A.sys[a.A.sysid[i]];
   bool ok = true;
 #pragma unroll
   for (int s = 0; s < 3; s++) {
-    el[s] = 0;
-    en[s] = 0;
+    o.el[s] = 0;
+    o.en[s] = 0;
     if (s < cnt) {
-      en[s] = a.ters_nb[(size_t)i * MAXTERS + s];
+      o.en[s] = a.ters_nb[(size_t)i * MAXTERS + s];
       int j, sx, sy, sz;
-      decode_entry(en[s], a.lc, j, sx, sy, sz);
+      decode_entry(o.en[s], a.lc, j, sx, sy, sz);
       double x, y, z;
       disp64(a.A.xq, sd, i, j, sx, sy, sz, x, y, z);
-      d[s][0] = -x; d[s][1] = -y; d[s][2] = -z;   // x_j - x_i
-      const double rs = x * x + y * y + z * z;
-      ok = ok && rs < a.ters_rlosq && rs > 1e-12;
-      ri[s] = rsqrt3(rs);
-      r[s] = rs * ri[s];
-      e[s][0] = d[s][0] * ri[s]; e[s][1] = d[s][1] * ri[s]; e[s][2] = d[s][2] * ri[s];
-      el[s] = c_pot.t_map[info_type(__double_as_longlong(a.A.xq[j].w))];
+      o.d[s][0] = -x; o.d[s][1] = -y; o.d[s][2] = -z;
+      o.rs[s] = x * x + y * y + z * z;
+      ok = ok && o.rs[s] < a.ters_rlosq && o.rs[s] > 1e-12;
+      o.el[s] = c_pot.t_map[info_type(__double_as_longlong(a.A.xq[j].w))];
     }
   }
-  if (!ok) return false;
+  return ok;
+}
+template <bool EV, bool GH, bool VA>
+__device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int ie, int cnt, const TersBonds &o) {
+  const auto &d = o.d;
+  const auto &el = o.el;
+  const auto &en = o.en;
+  double r[3], ri[3], e[3][3];
+#pragma unroll
+  for (int s = 0; s < 3; s++) {
+    if (s < cnt) {
+      ri[s] = rsqrt3(o.rs[s]);
+      r[s] = o.rs[s] * ri[s];
+      e[s][0] = d[s][0] * ri[s]; e[s][1] = d[s][1] * ri[s]; e[s][2] = d[s][2] * ri[s];
+    }
+  }
   const bool iown = !GH || owned(a, i);
   // ---- angles: cos(theta), g and dg/dcos of each ordered bond pair, zeta
   double cs[3][3], gd[3][3], zeta[3] = {0.0, 0.0, 0.0};
@@ -1062,17 +1076,59 @@ __device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int i
 }
 #endif
 
-// sp2 layers give 3 bonds per atom: those atoms run with their bonds in registers
+__device__ __forceinline__ void ters_centre(const ForceArgs<R> &a, int i, int &ie, int &cnt) {
+  ie = c_pot.t_map[info_type(__double_as_longlong(a.A.xq[i].w))];
+  cnt = ie < 0 ? 0 : a.ters_cnt[i];
+}
+
+// sp2 layers give 3 bonds per atom: those atoms run with their bonds in registers.
+// FP64 mode (ters_rlosq > 0): a block's atoms that tersoff_fast does not take are gathered,
+// so that they fill warps of their own: in a warp of both kinds every lane waits for both
+// forms, ~500 and ~1,800 FP64 instructions (forces, atoms displaced by 0.15 A: 331,200 atoms
+// 5.19 -> 3.00 ms, 36,800 730 -> 534 us; intact sheets the same).  split (small systems alone,
+// whose time is one atom's chain): twice as many threads as atoms, the second half for the
+// gathered ones, and the two forms run beside each other (7,200 atoms, 0.10 A, with energies:
+// 334 -> 320 us).  Three blocks of 128 threads per SM (168 registers): at two, 58,800 atoms
+// with free edges took 108 us instead of 81.
 template <bool EV, bool EATOM, bool GH, bool VA = false>
-__global__ void __launch_bounds__(128) k_tersoff(ForceArgs<R> a) {
+#ifdef LMFF_PACKED_X2
+__global__ void __launch_bounds__(128) k_tersoff(ForceArgs<R> a, int split) {
+#else
+__global__ void __launch_bounds__(128, VA ? 2 : 3) k_tersoff(ForceArgs<R> a, int split) {
+#endif
+  int ie, cnt;
+#ifndef LMFF_PACKED_X2
+  if (a.ters_rlosq > 0.0) {
+    __shared__ int s_rest[128], s_n[2];   // refused by tersoff_bonds from the front, by tersoff_fast from the back
+    const int tid = threadIdx.x, atoms = split ? blockDim.x / 2 : blockDim.x;
+    if (tid < 2) s_n[tid] = 0;
+    __syncthreads();
+    const int i = blockIdx.x * atoms + tid;
+    TersBonds bonds;
+    bool takes = false;
+    if (tid < atoms && i < a.n) {
+      ters_centre(a, i, ie, cnt);
+      takes = tersoff_bonds(a, i, cnt, bonds);
+      if (!takes) s_rest[atomicAdd(&s_n[0], 1)] = i;
+    }
+    __syncthreads();
+    if (takes && !tersoff_fast<EV, GH, VA>(a, i, ie, cnt, bonds)) s_rest[atoms - 1 - atomicAdd(&s_n[1], 1)] = i;
+    for (int pass = 0; pass < 2; pass++) {
+      if (pass) __syncthreads();
+      const int t = split && !pass ? tid - atoms : tid;
+      if (t >= 0 && t < s_n[pass]) {
+        const int k = s_rest[pass ? atoms - 1 - t : t];
+        ters_centre(a, k, ie, cnt);
+        if (cnt <= 3) tersoff_atom<3, EV, GH, VA>(a, k, ie, cnt);
+        else tersoff_atom<MAXTERS, EV, GH, VA>(a, k, ie, cnt);
+      }
+    }
+    return;
+  }
+#endif
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= a.n) return;
-  const long long iinfo = __double_as_longlong(a.A.xq[i].w);
-  const int ie = c_pot.t_map[info_type(iinfo)];
-  const int cnt = ie < 0 ? 0 : a.ters_cnt[i];
-#ifndef LMFF_PACKED_X2
-  if (tersoff_fast<EV, GH, VA>(a, i, ie, cnt)) return;
-#endif
+  ters_centre(a, i, ie, cnt);
   if (cnt <= 3) tersoff_atom<3, EV, GH, VA>(a, i, ie, cnt);
   else tersoff_atom<MAXTERS, EV, GH, VA>(a, i, ie, cnt);
 }
@@ -1089,17 +1145,43 @@ __global__ void __launch_bounds__(128) k_tersoff(ForceArgs<R> a) {
 // atoms, per NVE step: Tersoff alone 30.3 -> 26.8 us, the two styles one after the other
 // 56.1 -> 52.5 us, side by side 41.2 -> 43.1 us).  Force-only evaluations in periodic
 // mode (the energy/virial and subdomain evaluations run k_tersoff).
+// FP64 mode (ters_rlosq > 0): a fifth warp evaluates the block's atoms that tersoff_fast takes,
+// one thread each, beside the lanes of the others (1,152 atoms displaced by 0.15 A: k_tersoff
+// 394 us, here 305; intact 26 us either way), up to one wave of its blocks, two per SM: beyond,
+// k_tersoff's gathered warps are faster (12,000 atoms, 0.10 A: 276 us, the lanes alone 289;
+// 36,800: 334, 458).
 constexpr int TERS_LANES = 4;
-constexpr int TERS_LANES_MAX_ATOMS = 65536;
-__global__ void __launch_bounds__(128) k_tersoff_lanes(ForceArgs<R> a) {
+constexpr int TERS_LANES_MAX_ATOMS = 65536, TERS_LANES_MAX_ATOMS_FP64 = 8192;
+__global__ void __launch_bounds__(sizeof(R) == 8 ? 160 : 128) k_tersoff_lanes(ForceArgs<R> a) {
   constexpr int NB = TERS_LANES;
-  const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = gtid / NB;
-  if (i >= a.n) return;   // whole groups: blockDim is a multiple of NB
+  int i = blockIdx.x * 32 + (threadIdx.x & 127) / NB, ie, cnt;
+#ifndef LMFF_PACKED_X2
+  if (a.ters_rlosq > 0.0) {
+    __shared__ unsigned s_takes;
+    const bool fast_warp = threadIdx.x >= 128;
+    TersBonds bonds;
+    bool takes = false;
+    if (fast_warp) {
+      i = blockIdx.x * 32 + (threadIdx.x & 31);
+      if (i < a.n) {
+        ters_centre(a, i, ie, cnt);
+        takes = tersoff_bonds(a, i, cnt, bonds);
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, takes);
+      if ((threadIdx.x & 31) == 0) s_takes = m;
+    }
+    __syncthreads();
+    if (fast_warp) {
+      if (takes && !tersoff_fast<false, false, false>(a, i, ie, cnt, bonds)) tersoff_atom<3, false, false>(a, i, ie, cnt);
+      return;
+    }
+    if (s_takes >> (i & 31) & 1u) return;
+  }
+#endif
+  if (i >= a.n) return;   // whole groups
   const int wl = threadIdx.x & 31, l = wl & (NB - 1), gbase = wl & ~(NB - 1);
   const unsigned gmask = ((1u << NB) - 1) << gbase;
-  const int ie = c_pot.t_map[info_type(__double_as_longlong(a.A.xq[i].w))];
-  const int cnt = ie < 0 ? 0 : a.ters_cnt[i];
+  ters_centre(a, i, ie, cnt);
   if (cnt > NB) {   // the same in every lane of the group
     if (l == 0) tersoff_atom<MAXTERS, false, false>(a, i, ie, cnt);
     return;
@@ -4104,15 +4186,17 @@ void launch_tersoff(const ForceArgs<R> &a, bool ev, bool eatom, cudaStream_t s) 
   if (a.n == 0) return;
   const int b = per_atom_block(a.n);
   const int g = (a.n + b - 1) / b;
+  const bool fast = sizeof(R) == 8 && a.ters_rlosq > 0.0;
+  const int split = fast && b <= 32 && a.ters_alone, bs = split ? 2 * b : b;
   if (a.own_perm) {
-    if (ev) k_tersoff<true, false, true><<<g, b, 0, s>>>(a);
-    else k_tersoff<false, false, true><<<g, b, 0, s>>>(a);
+    if (ev) k_tersoff<true, false, true><<<g, bs, 0, s>>>(a, split);
+    else k_tersoff<false, false, true><<<g, bs, 0, s>>>(a, split);
   } else if (ev) {
-    k_tersoff<true, false, false><<<g, b, 0, s>>>(a);
-  } else if (a.ters_alone && a.n <= TERS_LANES_MAX_ATOMS && !a.no_small && !(sizeof(R) == 8 && a.ters_rlosq > 0.0)) {
-    k_tersoff_lanes<<<(int)(((long long)a.n * TERS_LANES + 127) / 128), 128, 0, s>>>(a);
+    k_tersoff<true, false, false><<<g, bs, 0, s>>>(a, split);
+  } else if (a.ters_alone && a.n <= (fast ? TERS_LANES_MAX_ATOMS_FP64 : TERS_LANES_MAX_ATOMS) && !a.no_small) {
+    k_tersoff_lanes<<<(a.n + 31) / 32, fast ? 160 : 128, 0, s>>>(a);
   } else {
-    k_tersoff<false, false, false><<<g, b, 0, s>>>(a);
+    k_tersoff<false, false, false><<<g, bs, 0, s>>>(a, split);
   }
   if (ev && eatom) k_ters_eatom_own<<<g, b, 0, s>>>(a);
 }
@@ -4241,8 +4325,8 @@ void launch_vatom_terms(const ForceArgs<R> &a, bool ilp, bool one_element, cudaS
   const int g = (a.n + 127) / 128;
   const bool gh = a.own_perm != nullptr;
   if (a.do_ters) {
-    if (gh) k_tersoff<false, false, true, true><<<g, 128, 0, s>>>(a);
-    else k_tersoff<false, false, false, true><<<g, 128, 0, s>>>(a);
+    if (gh) k_tersoff<false, false, true, true><<<g, 128, 0, s>>>(a, 0);
+    else k_tersoff<false, false, false, true><<<g, 128, 0, s>>>(a, 0);
   }
   if (a.do_ilp && ilp) {
     k_frame<<<g, 128, 0, s>>>(a);
