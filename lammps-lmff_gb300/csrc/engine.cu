@@ -9,9 +9,6 @@
 //   k_tersoff (bonds centred at each atom)   k_ilp (interlayer pairs, normal derivatives)
 //   k_finish (gather) -> [k_reduce energies/virials]
 #include <cuda_runtime.h>
-#include <sys/mman.h>
-#include <unistd.h>
-
 #include <algorithm>
 #include <array>
 #include <atomic>
@@ -22,13 +19,13 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
 
 #include "engine.cuh"
 #include "forces.cuh"
+#include "host_pages.h"
 #include "ilp_df.cuh"
 #include "lmff_gb300.h"
 #include "neighbor.cuh"
@@ -1813,8 +1810,8 @@ struct Engine {
       CK(cudaMemcpyAsync(red.data(), d.red_out, sizeof(double) * red.size(), cudaMemcpyDeviceToHost, stream));
     }
     if (out) {
-      map_pages(out->f, sizeof(double) * 3 * (size_t)n);
-      map_pages(out->eatom, sizeof(double) * (size_t)n);
+      map_pages(out->f, sizeof(double) * 3 * (size_t)n, true);
+      map_pages(out->eatom, sizeof(double) * (size_t)n, true);
     }
     CK(cudaStreamSynchronize(stream));
     harvest();
@@ -1991,7 +1988,7 @@ struct Engine {
     const bool overwrite = (which & LMFF_OVERWRITE) != 0;
     if (!overwrite) CK(cudaMemcpyAsync(d_fin, f, sizeof(double) * 3 * nn, cudaMemcpyHostToDevice, stream));
     k_scatter_sum<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, d.f, overwrite ? nullptr : d_fin, d_fo);
-    if (overwrite) map_pages(f, sizeof(double) * 3 * (size_t)nn);
+    if (overwrite) map_pages(f, sizeof(double) * 3 * (size_t)nn, false);
     CK(cudaMemcpyAsync(f, d_fo, sizeof(double) * 3 * nn, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     double d2;
@@ -2251,7 +2248,7 @@ struct Engine {
     const bool overwrite = (which & LMFF_OVERWRITE) != 0;
     if (!overwrite) CK(cudaMemcpyAsync(inorder, out, sizeof(double) * 6 * (size_t)nn, cudaMemcpyHostToDevice, stream));
     k_scatter_add6<<<(nn + 255) / 256, 256, 0, stream>>>(nn, d.perm, sorted, inorder, overwrite);
-    if (overwrite) map_pages(out, sizeof(double) * 6 * (size_t)nn);
+    if (overwrite) map_pages(out, sizeof(double) * 6 * (size_t)nn, false);
     CK(cudaMemcpyAsync(out, inorder, sizeof(double) * 6 * (size_t)nn, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
     return LMFF_OK;
@@ -2964,7 +2961,7 @@ struct Engine {
     double *xo = d_xin, *vo = d_vin, *fo = d_fin;
     k_unpermute_state<<<(n + 255) / 256, 256, 0, stream>>>(n, d.perm, d.xq, d.v, d.f, xo, vo, fo);
     CK(cudaGetLastError());
-    for (double *p : {x, v, f}) map_pages(p, sizeof(double) * 3 * (size_t)n);
+    for (double *p : {x, v, f}) map_pages(p, sizeof(double) * 3 * (size_t)n, false);
     if (x) CK(cudaMemcpyAsync(x, xo, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, stream));
     if (v) CK(cudaMemcpyAsync(v, vo, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, stream));
     if (f) CK(cudaMemcpyAsync(f, fo, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, stream));
@@ -3094,56 +3091,6 @@ struct Engine {
     }
     CK(cudaStreamSynchronize(stream));
     return LMFF_OK;
-  }
-
-  // memcpy on up to 8 host threads, in 64-byte aligned pieces
-  static void parallel_copy(void *dst, const void *src, size_t bytes) {
-    in_pieces(bytes, [=](size_t b, size_t e) { memcpy((char *)dst + b, (const char *)src + b, e - b); });
-  }
-  // f(begin, end) over [0, bytes): from 4 MiB on in up to 8 pieces, each on its host thread.
-  // A piece whose thread cannot be had is done here.
-  template <class F>
-  static void in_pieces(size_t bytes, const F &f) {
-    const int nth = (int)std::min<size_t>(8, std::max(1u, std::thread::hardware_concurrency()));
-    if (nth <= 1 || bytes < ((size_t)4 << 20)) {
-      f((size_t)0, bytes);
-      return;
-    }
-    const size_t piece = ((bytes / nth) + 63) & ~(size_t)63;
-    std::thread pool[8];
-    for (int k = 0; k < nth; k++) {
-      const size_t b = (size_t)k * piece;
-      if (b >= bytes) break;
-      const size_t e = std::min(bytes, b + piece);
-      try {
-        pool[k] = std::thread([=, &f] { f(b, e); });
-      } catch (const std::exception &) {
-        f(b, e);
-      }
-    }
-    for (auto &t : pool)
-      if (t.joinable()) t.join();
-  }
-  // Maps the pages of a caller's output array that the call overwrites as a whole.  An array
-  // the program has just allocated has no pages yet; the GPU's copy into it then takes a fault
-  // of ~40 us for every 64 KB (490k atoms, lmff_download: 20-30 ms, with its pages there 0.9
-  // ms), where a write by the host takes a few us, on several threads at once and, where a
-  // call's kernels are already queued, while they run.  (Only written: reading a byte first
-  // maps the zero page, and replacing that is a second fault with a flush of every thread's
-  // translations, 70 ms for 2.7M atoms.)
-  static void map_pages(void *p, size_t bytes) {
-    if (!p || !bytes) return;
-    static const size_t page = (size_t)std::max(4096L, sysconf(_SC_PAGESIZE));
-    const uintptr_t p0 = (uintptr_t)p / page * page, p1 = (uintptr_t)p + bytes;
-    const size_t pages = (p1 - p0 + page - 1) / page;
-    const std::unique_ptr<unsigned char[]> in(new (std::nothrow) unsigned char[pages]);
-    const unsigned char *there = in.get();
-    if (!in || mincore((void *)p0, p1 - p0, in.get()) != 0) return;
-    if (std::all_of(there, there + pages, [](unsigned char c) { return c & 1; })) return;
-    in_pieces(bytes, [=](size_t b, size_t e) {
-      for (size_t q = b; q < e; q = ((uintptr_t)p + q) / page * page + page - (uintptr_t)p)
-        if (!(there[((uintptr_t)p + q - p0) / page] & 1)) *((volatile char *)p + q) = 0;
-    });
   }
 
   // ---------------------------------------------------------------- lists export
