@@ -24,84 +24,65 @@ LMFF_DF float vadd(float a, float b) { return __fadd_rn(a, b); }
 LMFF_DF float vsub(float a, float b) { return __fsub_rn(a, b); }
 LMFF_DF float vmul(float a, float b) { return __fmul_rn(a, b); }
 LMFF_DF float vfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-template <class V>
-LMFF_DF V vall(float a);   // a constant
-template <>
-__device__ __forceinline__ float vall<float>(float a) { return a; }
-template <class V>
 struct D {
-  V h, l;
+  float h, l;
 };
-template <class V>
-LMFF_DF D<V> mk(V h, V l) {
-  D<V> r;
+LMFF_DF D mk(float h, float l) {
+  D r;
   r.h = h;
   r.l = l;
   return r;
 }
-template <class V>
-LMFF_DF D<V> neg(D<V> a) { return mk(vneg(a.h), vneg(a.l)); }
+LMFF_DF D neg(D a) { return mk(vneg(a.h), vneg(a.l)); }
 
 // s + e = a + b exactly
-template <class V>
-LMFF_DF D<V> two_sum(V a, V b) {
-  const V s = vadd(a, b), bb = vsub(s, a);
+LMFF_DF D two_sum(float a, float b) {
+  const float s = vadd(a, b), bb = vsub(s, a);
   return mk(s, vadd(vsub(a, vsub(s, bb)), vsub(b, bb)));
 }
 // the same for |a| >= |b| or a = 0
-template <class V>
-LMFF_DF D<V> fast_two_sum(V a, V b) {
-  const V s = vadd(a, b);
+LMFF_DF D fast_two_sum(float a, float b) {
+  const float s = vadd(a, b);
   return mk(s, vsub(b, vsub(s, a)));
 }
-template <class V>
-LMFF_DF D<V> renorm(D<V> a) { return fast_two_sum(a.h, a.l); }
+LMFF_DF D renorm(D a) { return fast_two_sum(a.h, a.l); }
 
-template <class V>
-LMFF_DF D<V> mul(D<V> a, D<V> b) {
-  const V p = vmul(a.h, b.h);
-  V e = vfma(a.h, b.h, vneg(p));
+LMFF_DF D mul(D a, D b) {
+  const float p = vmul(a.h, b.h);
+  float e = vfma(a.h, b.h, vneg(p));
   e = vfma(a.h, b.l, e);
   return mk(p, vfma(a.l, b.h, e));
 }
-template <class V>
-LMFF_DF D<V> sqr(D<V> a) {
-  const V p = vmul(a.h, a.h);
-  const V e = vfma(a.h, a.h, vneg(p));
+LMFF_DF D sqr(D a) {
+  const float p = vmul(a.h, a.h);
+  const float e = vfma(a.h, a.h, vneg(p));
   return mk(p, vfma(vadd(a.h, a.h), a.l, e));
 }
-template <class V>
-LMFF_DF D<V> add(D<V> a, D<V> b) {
-  const D<V> s = two_sum(a.h, b.h);
+LMFF_DF D add(D a, D b) {
+  const D s = two_sum(a.h, b.h);
   return mk(s.h, vadd(s.l, vadd(a.l, b.l)));
 }
 // |a| >= |b|
-template <class V>
-LMFF_DF D<V> add_ordered(D<V> a, D<V> b) {
-  const D<V> s = fast_two_sum(a.h, b.h);
+LMFF_DF D add_ordered(D a, D b) {
+  const D s = fast_two_sum(a.h, b.h);
   return mk(s.h, vadd(s.l, vadd(a.l, b.l)));
 }
 // a + b, b in single precision
-template <class V>
-LMFF_DF D<V> add1(D<V> a, V b) {
-  const D<V> s = two_sum(a.h, b);
+LMFF_DF D add1(D a, float b) {
+  const D s = two_sum(a.h, b);
   return mk(s.h, vadd(s.l, a.l));
 }
-template <class V>
-LMFF_DF D<V> scale(D<V> a, V m) { return mk(vmul(a.h, m), vmul(a.l, m)); }   // m a power of two or zero
+LMFF_DF D scale(D a, float m) { return mk(vmul(a.h, m), vmul(a.l, m)); }   // m a power of two or zero
 // running sum: acc += a
-template <class V>
-LMFF_DF void acc(D<V> &s, D<V> a) { s = add(s, a); }
+LMFF_DF void acc(D &s, D a) { s = add(s, a); }
 // running sum of products: s += a b, s -= a b
-template <class V>
-LMFF_DF void acc_mul(D<V> &s, D<V> a, D<V> b) { acc(s, mul(a, b)); }
+LMFF_DF void acc_mul(D &s, D a, D b) { acc(s, mul(a, b)); }
 
 // a . b of three-vectors
-template <class V>
-LMFF_DF D<V> dot3(const D<V> *a, const D<V> *b) {
-  const D<V> x = mul(a[0], b[0]), y = mul(a[1], b[1]), z = mul(a[2], b[2]);
-  const D<V> s = two_sum(x.h, y.h), t = two_sum(s.h, z.h);
-  const V lo = vadd(vadd(vadd(x.l, y.l), z.l), vadd(s.l, t.l));
+LMFF_DF D dot3(const D *a, const D *b) {
+  const D x = mul(a[0], b[0]), y = mul(a[1], b[1]), z = mul(a[2], b[2]);
+  const D s = two_sum(x.h, y.h), t = two_sum(s.h, z.h);
+  const float lo = vadd(vadd(vadd(x.l, y.l), z.l), vadd(s.l, t.l));
   return fast_two_sum(t.h, lo);
 }
 
@@ -124,34 +105,33 @@ LMFF_DF void exp2_parts(float t, const float2 *tab, float &th, float &tl, float 
   tl = T.y;
   sc = __int_as_float(((k >> 6) + 127) << 23);
 }
-template <class V>
-LMFF_DF D<V> exp2(D<V> a, const float2 *tab) {
-  const V magic = vall<V>(12582912.f);   // 1.5 2^23
-  const V ah = clamp_exp(a.h);
-  const V t = vfma(ah, vall<V>((float)EXP2_TAB), magic);
-  const V k = vsub(t, magic);
+LMFF_DF D exp2(D a, const float2 *tab) {
+  const float magic = 12582912.f;   // 1.5 2^23
+  const float ah = clamp_exp(a.h);
+  const float t = vfma(ah, (float)EXP2_TAB, magic);
+  const float k = vsub(t, magic);
   // ah - k/64 is exact and a multiple of ulp(ah), so zero or larger than a.l
-  const D<V> f = fast_two_sum(vfma(vneg(k), vall<V>(1.f / EXP2_TAB), ah), a.l);
-  const V L = vall<V>(0.693147182464599609375f), Ll = vall<V>(-1.90465429995776804525e-9f);   // ln 2
-  const V p = vmul(f.h, L);
-  V e = vfma(f.h, L, vneg(p));
+  const D f = fast_two_sum(vfma(vneg(k), 1.f / EXP2_TAB, ah), a.l);
+  const float L = 0.693147182464599609375f, Ll = -1.90465429995776804525e-9f;   // ln 2
+  const float p = vmul(f.h, L);
+  float e = vfma(f.h, L, vneg(p));
   e = vfma(f.h, Ll, e);
   e = vfma(f.l, L, e);
-  const V c = vfma(vfma(p, vall<V>(1.f / 60.f), vall<V>(1.f / 12.f)), p, vall<V>(1.f / 3.f));
-  const V hp = vmul(vall<V>(0.5f), p);
-  const V q = vmul(hp, p);
-  V qe = vfma(hp, p, vneg(q));
+  const float c = vfma(vfma(p, 1.f / 60.f, 1.f / 12.f), p, 1.f / 3.f);
+  const float hp = vmul(0.5f, p);
+  const float q = vmul(hp, p);
+  float qe = vfma(hp, p, vneg(q));
   qe = vfma(p, e, qe);
   qe = vfma(vmul(q, p), c, qe);
-  const D<V> s = fast_two_sum(p, q);
-  const V sl = vadd(s.l, vadd(e, qe));
-  V th, tl, sc;
+  const D s = fast_two_sum(p, q);
+  const float sl = vadd(s.l, vadd(e, qe));
+  float th, tl, sc;
   exp2_parts(t, tab, th, tl, sc);
-  const V m = vmul(th, s.h);
-  V me = vfma(th, s.h, vneg(m));
+  const float m = vmul(th, s.h);
+  float me = vfma(th, s.h, vneg(m));
   me = vfma(th, sl, me);
   me = vfma(tl, s.h, me);
-  const D<V> r = fast_two_sum(th, m);
+  const D r = fast_two_sum(th, m);
   return mk(vmul(r.h, sc), vmul(vadd(r.l, vadd(me, tl)), sc));
 }
 #undef LMFF_DF

@@ -2341,7 +2341,9 @@ __global__ void __launch_bounds__(256, (ilp_min_blocks<TPA, EV, EATOM, ONE, GH, 
 // that need them go to a queue per atom, and the lanes take tpa queued entries at once
 // (331,200-atom slab, forces: 23 of 32 lanes active and 6.5 ms when each lane evaluated
 // its own in place with direct radial functions; 31 of 32 and 5.2 ms with queue and
-// tables).  What bounds it now is the gathers: L1 wavefronts 75 %, issue 51 %.
+// tables).  What bounds it is the latency of the record and table gathers at 4.6 warps per
+// scheduler: issue 68 %, L1 wavefronts 55 %, FMA pipe 48 % (36,800-atom slab, forces; with
+// energies 3.7 warps, issue 56 %, L1 43 %, FMA 43 %, a fifth of the waits for instructions).
 // Blocks of up to 128 threads, 5 per SM (96 registers), with energies and virial 4 (128):
 // one block more or less per SM measured 3-10 % slower on the 331,200-atom slab.
 constexpr int DF_THREADS = 128;
@@ -2355,13 +2357,13 @@ __constant__ DfCut c_dfcut;
 // at the tables' end, the FP64 form decides, as it does for every pair of the general kernel:
 // without the taper a pair's force ends in a step there
 constexpr float DF_EDGE = 0x1p-31f;   // A^2
-__device__ __forceinline__ float df_past_cut(const df::D<float> &q) {
+__device__ __forceinline__ float df_past_cut(const df::D &q) {
   return __fadd_rn(__fsub_rn(q.h, c_dfcut.h), __fsub_rn(q.l, c_dfcut.l));
 }
-__device__ __forceinline__ bool df_inside(const df::D<float> &q, float past) {
+__device__ __forceinline__ bool df_inside(const df::D &q, float past) {
   return past <= -DF_EDGE && q.h >= DF_CLOSE;
 }
-__device__ __forceinline__ bool df_apart(const df::D<float> &q, float past) {   // left to the FP64 form
+__device__ __forceinline__ bool df_apart(const df::D &q, float past) {   // left to the FP64 form
   return !df_inside(q, past) && past < DF_EDGE;
 }
 __constant__ float c_dfk[df::K_N];                    // element pair (0, 0)'s constants
@@ -2434,7 +2436,7 @@ __device__ __forceinline__ void df_disp(const DfAtom &I, const DfAtom &A, const 
 
 template <bool IMG>
 __device__ __forceinline__ void df_del(const DfAtom &I, const DfAtom &A, const SysDesc &sd, int sx, int sy, int sz,
-                                       df::D<float> d[3]) {
+                                       df::D d[3]) {
 #pragma unroll
   for (int c = 0; c < 3; c++) {
     float dh, dm, dl;
@@ -2464,9 +2466,9 @@ __device__ __noinline__ void df_close_pairs(const ForceArgs<R> &a, int i, int la
     decode_entry(e, a.lc, j, sx, sy, sz);
     DfAtom A;
     A.load(a.jrec, a.jstride, j);
-    df::D<float> d[3];
+    df::D d[3];
     df_del<true>(I, A, sd, sx, sy, sz, d);
-    const df::D<float> q = df::dot3(d, d);
+    const df::D q = df::dot3(d, d);
     if (!all && !df_apart(q, df_past_cut(q))) continue;
     ilp_pair<EV, ONE, false, true, GH>(a, ai, sd, e, ai.fetch(a.A, j), NrmJ<R>::load(a, j), ni.x, ni.y, ni.z, ie,
                                        info_mol(ai.info), itag, false, iown, acc);
@@ -2477,7 +2479,6 @@ template <bool EV, bool ONE, bool GH>
 __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_ilp_df(ForceArgs<R> a, int tpa, int eatom, int ne) {
   pdl_enter(a.pdl);
   using namespace df;
-  typedef float V;
   __shared__ float2 s_tab[EXP2_TAB];
   __shared__ float s_dfk[ONE ? 1 : MAXELEM * MAXELEM * K_N];
   __shared__ uint32_t s_queue[DF_THREADS * 4];   // 4 tpa entries per atom
@@ -2505,7 +2506,7 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
   const int ie = I.el;
   const long long itag = GH ? a.tag[ii] : 0;
   const bool iown = !GH || owned(a, ii);
-  D<V> f[3], g[3], tpi, ev, er, w[6];
+  D f[3], g[3], tpi, ev, er, w[6];
 #pragma unroll
   for (int c = 0; c < 3; c++) f[c] = g[c] = mk(0.f, 0.f);
   tpi = ev = er = mk(0.f, 0.f);
@@ -2519,7 +2520,7 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
   const int most = __reduce_max_sync(FULL, cnt);
   auto run = [&](auto img_t) {
     constexpr bool IMG = decltype(img_t)::value;
-    auto pair_of = [&](uint32_t e, DfAtom &A, int &j, D<V> d[3]) {
+    auto pair_of = [&](uint32_t e, DfAtom &A, int &j, D d[3]) {
       int sx = 0, sy = 0, sz = 0;
       if constexpr (IMG) decode_entry(e, a.lc, j, sx, sy, sz);
       else j = (int)(e & a.lc.imask);
@@ -2527,7 +2528,7 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
       df_del<IMG>(I, A, sd, sx, sy, sz, d);
     };
     // weights of the subdomain mode: the vdW pair, the terms with n_i and with n_j
-    auto weights = [&](int j, const D<V> d[3], float &wv, float &wi, float &wj) {
+    auto weights = [&](int j, const D d[3], float &wv, float &wi, float &wj) {
       if constexpr (GH) {
         const bool jown = owned(a, j);
         const bool keep =
@@ -2543,7 +2544,7 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
         else return s_dfk[(ie * ne + je) * K_N + k];
       };
     };
-    auto virial = [&](const D<V> d[3], const D<V> t[3]) {
+    auto virial = [&](const D d[3], const D t[3]) {
       acc_mul(w[0], d[0], t[0]); acc_mul(w[1], d[1], t[1]); acc_mul(w[2], d[2], t[2]);
       acc_mul(w[3], d[0], t[1]); acc_mul(w[4], d[0], t[2]); acc_mul(w[5], d[1], t[2]);
     };
@@ -2554,14 +2555,14 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
       if (on && qh + lane < qn) {
         DfAtom A;
         int j;
-        D<V> d[3], ni[3], nj[3], tp, tq, S, crad = mk(0.f, 0.f);
+        D d[3], ni[3], nj[3], tp, tq, S, crad = mk(0.f, 0.f);
         pair_of(queue[(qh + lane) & (4 * tpa - 1)], A, j, d);
-        const D<V> q = dot3(d, d);
+        const D q = dot3(d, d);
         float th, wv = 1.f, wi = 1.f, wj = 1.f;
         int k = tab_at(q.h, th);
         if constexpr (!ONE) k += (ie * ne + A.el) * TAB_N;
-        const D<V> off = fast_two_sum(th, q.l);
-        Coef<V> c;
+        const D off = fast_two_sum(th, q.l);
+        Coef c;
         coef_set(c, a.df_M + 2 * k);
         const float2 f0 = __ldg(a.df_TE + k);
         weights(j, d, wv, wi, wj);
@@ -2571,11 +2572,11 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
           nj[x] = mk(A.nh[x], A.nl[x]);
         }
         const auto K = consts(A.el);
-        const D<V> TE = tab_integral(c, f0.x, f0.y, off);
+        const D TE = tab_integral(c, f0.x, f0.y, off);
         pair_near<GH>(K, s_tab, q, TE, tab_poly(c, off), dot3(ni, d), dot3(nj, d), wi, wj, crad, tp, tq, S);
         acc(tpi, tp);
-        const D<V> ntq = neg(tq);
-        D<V> t[3];
+        const D ntq = neg(tq);
+        D t[3];
 #pragma unroll
         for (int x = 0; x < 3; x++) {
           acc_mul(g[x], tp, d[x]);
@@ -2599,9 +2600,9 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
       if (k0 + lane < cnt) {
         DfAtom A;
         int j;
-        D<V> d[3];
+        D d[3];
         pair_of(e, A, j, d);
-        const D<V> q = dot3(d, d);
+        const D q = dot3(d, d);
         const float past = df_past_cut(q);
         const bool in = df_inside(q, past);
         close = close || df_apart(q, past);   // rare
@@ -2609,24 +2610,24 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
           float th;
           int k = tab_at(q.h, th);
           if constexpr (!ONE) k += (ie * ne + A.el) * TAB_N;
-          const D<V> off = fast_two_sum(th, q.l);
-          Coef<V> c;
+          const D off = fast_two_sum(th, q.l);
+          Coef c;
           coef_set(c, a.df_A + 2 * k);
-          D<V> crad = tab_poly(c, off);
+          D crad = tab_poly(c, off);
           const auto K = consts(A.el);
           if constexpr (EV || GH) {
             float wv = 1.f, wi = 1.f, wj = 1.f;
             weights(j, d, wv, wi, wj);
             const float wm = 0.5f * (wi + wj);
-            const D<V> eps = mk(K(K_EPS), K(K_EPS + 1));
-            Coef<V> cM;
+            const D eps = mk(K(K_EPS), K(K_EPS + 1));
+            Coef cM;
             coef_set(cM, a.df_M + 2 * k);
             // A = vdW part + eps M: weights wv and (wi + wj) / 2
             if constexpr (GH) crad = add(scale(crad, wv), scale(mul(tab_poly(cM, off), eps), wm - wv));
             if constexpr (EV) {
               const float2 u0 = __ldg(a.df_U + k), f0 = __ldg(a.df_TE + k);
-              const D<V> te = mul(tab_integral(cM, f0.x, f0.y, off), eps);
-              D<V> vdw = add(tab_integral(c, u0.x, u0.y, off), neg(te));
+              const D te = mul(tab_integral(cM, f0.x, f0.y, off), eps);
+              D vdw = add(tab_integral(c, u0.x, u0.y, off), neg(te));
               if constexpr (GH) {
                 vdw = scale(vdw, wv);
                 acc(er, scale(te, wm));
@@ -2638,7 +2639,7 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
           }
           near = near_one(K(K_ND2), q.h, I.nh[0] * d[0].h + I.nh[1] * d[1].h + I.nh[2] * d[2].h,
                           A.nh[0] * d[0].h + A.nh[1] * d[1].h + A.nh[2] * d[2].h);
-          D<V> t[3];
+          D t[3];
 #pragma unroll
           for (int x = 0; x < 3; x++) {
             t[x] = mul(crad, d[x]);
@@ -2680,10 +2681,10 @@ __global__ void __launch_bounds__(DF_THREADS, EV ? DF_BLOCKS_EV : DF_BLOCKS) k_i
   if (__any_sync(FULL, cnt > 0 && a.list_img[ii] != 0)) run(std::true_type{});
   else run(std::false_type{});
   // ---- the atom's lanes in double-float; FP64 from there
-  auto total = [&](const D<V> &v) {
-    D<float> s = renorm(v);
+  auto total = [&](const D &v) {
+    D s = renorm(v);
     for (int o = tpa / 2; o > 0; o >>= 1) {
-      const D<float> p = mk(__shfl_xor_sync(FULL, s.h, o), __shfl_xor_sync(FULL, s.l, o));
+      const D p = mk(__shfl_xor_sync(FULL, s.h, o), __shfl_xor_sync(FULL, s.l, o));
       s = renorm(add(s, p));
     }
     return (double)s.h + (double)s.l;
@@ -3462,7 +3463,7 @@ static_assert(VA_NEARSQ <= df::Q64_MAX, "the FP64 tables end at Q64_MAX");
 
 // r^2 - r_cut^2 of an entry of atom i's list, and its q = r^2 as both kernels' split tests it
 __device__ __forceinline__ float va_pair_q(const DfAtom &I, const DfAtom &A, const SysDesc &sd, int sx, int sy, int sz,
-                                           df::D<float> d[3], df::D<float> &q) {
+                                           df::D d[3], df::D &q) {
   df_del<true>(I, A, sd, sx, sy, sz, d);
   q = df::dot3(d, d);
   return df_past_cut(q);
@@ -3521,7 +3522,7 @@ __device__ __noinline__ void va_close_pairs(const ForceArgs<R> &a, int i, int la
     decode_entry(e, a.lc, j, sx, sy, sz);
     DfAtom A;
     A.load(a.jrec, a.jstride, j);
-    df::D<float> d[3], s;
+    df::D d[3], s;
     const float past = va_pair_q(I, A, sd, sx, sy, sz, d, s);
     if (!all && !df_apart(s, past)) continue;
     va_pair64<GH, false>(a, i, e, ie, mi, itag, iown, ni.x, ni.y, ni.z, v, v[6], v[7], v[8], v + 9);
@@ -3634,7 +3635,7 @@ __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
       decode_entry(e, a.lc, j, sx, sy, sz);
       DfAtom A;
       A.load(a.jrec, a.jstride, j);
-      df::D<float> d[3], q;
+      df::D d[3], q;
       const float past = va_pair_q(I, A, sd, sx, sy, sz, d, q);
       near = df_inside(q, past) && q.h < VA_NEARSQ;
       close = close || df_apart(q, past);   // rare
@@ -3676,7 +3677,6 @@ __global__ void __launch_bounds__(128) k_va_near(ForceArgs<R> a, int ne) {
 template <bool ONE, bool GH>
 __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
   using namespace df;
-  typedef float V;
   constexpr int QUEUE = 8 * VA_LANES;   // entries per atom
   const unsigned FULL = 0xffffffffu;
   __shared__ float2 s_tab[EXP2_TAB];
@@ -3696,7 +3696,7 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
   const int ie = I.el;
   const long long itag = GH ? a.tag[i] : 0;
   const bool iown = !GH || owned(a, i);
-  D<V> s[15];   // w[6], g[3], G[6]
+  D s[15];   // w[6], g[3], G[6]
 #pragma unroll
   for (int c = 0; c < 15; c++) s[c] = mk(0.f, 0.f);
   const bool out = fabsf(I.h[0]) > sd.dfmax || fabsf(I.h[1]) > sd.dfmax || fabsf(I.h[2]) > sd.dfmax;
@@ -3705,7 +3705,7 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
   const int most = __reduce_max_sync(FULL, cnt);
   constexpr int P[6] = {0, 1, 2, 0, 0, 1}, Q[6] = {0, 1, 2, 1, 2, 2};
   // weights of the subdomain mode: the vdW pair, the terms with n_i and with n_j
-  auto weights = [&](int j, const D<V> d[3], float &wv, float &wi, float &wj) {
+  auto weights = [&](int j, const D d[3], float &wv, float &wi, float &wj) {
     if constexpr (GH) {
       const bool jown = owned(a, j);
       const bool keep = keep_half_r(itag, (long long)a.tag[j], -(d[0].h + d[0].l), -(d[1].h + d[1].l), -(d[2].h + d[2].l));
@@ -3714,7 +3714,7 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
       wj = jown ? 1.f : 0.f;
     }
   };
-  auto virial = [&](const D<V> d[3], const D<V> t[3]) {
+  auto virial = [&](const D d[3], const D t[3]) {
 #pragma unroll
     for (int c = 0; c < 6; c++) acc_mul(s[c], d[P[c]], t[Q[c]]);
   };
@@ -3727,14 +3727,14 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
       decode_entry(queue[(qh + lane) & (QUEUE - 1)], a.lc, j, sx, sy, sz);
       DfAtom A;
       A.load(a.jrec, a.jstride, j);
-      D<V> d[3], ni[3], nj[3], q, tp, tq, S, crad = mk(0.f, 0.f);
+      D d[3], ni[3], nj[3], q, tp, tq, S, crad = mk(0.f, 0.f);
       va_pair_q(I, A, sd, sx, sy, sz, d, q);
       float th, wv = 1.f, wi = 1.f, wj = 1.f;
       weights(j, d, wv, wi, wj);
       int ki = tab_at(q.h, th);
       if constexpr (!ONE) ki += (ie * ne + A.el) * TAB_N;
-      const D<V> off = fast_two_sum(th, q.l);
-      Coef<V> cc;
+      const D off = fast_two_sum(th, q.l);
+      Coef cc;
       coef_set(cc, a.df_M + 2 * ki);
       const float2 f0 = __ldg(a.df_TE + ki);
 #pragma unroll
@@ -3749,8 +3749,8 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
       };
       pair_near<GH>(K, s_tab, q, tab_integral(cc, f0.x, f0.y, off), tab_poly(cc, off), dot3(ni, d), dot3(nj, d), wi, wj,
                     crad, tp, tq, S);
-      const D<V> ntq = neg(tq);
-      D<V> t[3], h[3], g[3];
+      const D ntq = neg(tq);
+      D t[3], h[3], g[3];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         t[c] = add(mul(crad, d[c]), mul(ntq, nj[c]));
@@ -3770,7 +3770,7 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
 #pragma unroll
       for (int c = 18; c < 27; c++) any = any || num(c).h != 0.f;
       if (any) {
-        D<V> r[3];
+        D r[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) {   // - sum_e B[e][c] g_e
           r[c] = mul(num(18 + c), g[0]);
@@ -3800,7 +3800,7 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
       decode_entry(e, a.lc, j, sx, sy, sz);
       DfAtom A;
       A.load(a.jrec, a.jstride, j);
-      D<V> d[3], q;
+      D d[3], q;
       if (va_pair_q(I, A, sd, sx, sy, sz, d, q) <= -DF_EDGE && !(q.h < VA_NEARSQ)) {   // k_va_near has the pairs at the cutoff
         const float *row = ONE ? nullptr : g_dfk + (ie * ne + A.el) * K_N;
         auto K = [&](int k2) {
@@ -3810,17 +3810,17 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
         float th;
         int ki = tab_at(q.h, th);
         if constexpr (!ONE) ki += (ie * ne + A.el) * TAB_N;
-        const D<V> off = fast_two_sum(th, q.l);
-        Coef<V> cc;
+        const D off = fast_two_sum(th, q.l);
+        Coef cc;
         coef_set(cc, a.df_A + 2 * ki);
-        D<V> crad = tab_poly(cc, off);
+        D crad = tab_poly(cc, off);
         if constexpr (GH) {
           float wv, wi, wj;
           weights(j, d, wv, wi, wj);
           coef_set(cc, a.df_M + 2 * ki);
           crad = add(scale(crad, wv), scale(mul(tab_poly(cc, off), mk(K(K_EPS), K(K_EPS + 1))), 0.5f * (wi + wj) - wv));
         }
-        D<V> t[3];
+        D t[3];
 #pragma unroll
         for (int c = 0; c < 3; c++) t[c] = mul(crad, d[c]);
         virial(d, t);
@@ -3840,7 +3840,7 @@ __global__ void __launch_bounds__(128, 4) k_va_far(ForceArgs<R> a, int ne) {
   double v[15];
 #pragma unroll
   for (int c = 0; c < 15; c++) {
-    D<V> x = renorm(s[c]);
+    D x = renorm(s[c]);
     for (int o = VA_LANES / 2; o > 0; o >>= 1)
       x = renorm(add(x, mk(__shfl_xor_sync(FULL, x.h, o), __shfl_xor_sync(FULL, x.l, o))));
     v[c] = (double)x.h + (double)x.l;
@@ -3971,7 +3971,7 @@ __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
   const int lane = threadIdx.x & (VA_LANES - 1);
   if (i >= a.n) return;   // whole groups
   const unsigned gmask = ((1u << VA_LANES) - 1) << ((threadIdx.x & 31) & ~(VA_LANES - 1));
-  df::D<float> s[15];   // w[6] (without the halves), g[3], G[6] (xx yy zz xy xz yz)
+  df::D s[15];   // w[6] (without the halves), g[3], G[6] (xx yy zz xy xz yz)
 #pragma unroll
   for (int k = 0; k < 15; k++) s[k] = df::mk(0.f, 0.f);
   AtomI<R> ai;
@@ -4067,7 +4067,7 @@ __global__ void __launch_bounds__(128) k_va_ilp32(ForceArgs<R> a) {
   double v[15];
 #pragma unroll
   for (int k = 0; k < 15; k++) {
-    df::D<float> x = df::renorm(s[k]);
+    df::D x = df::renorm(s[k]);
     for (int o = VA_LANES / 2; o > 0; o >>= 1)
       x = df::renorm(df::add(x, df::mk(__shfl_xor_sync(gmask, x.h, o), __shfl_xor_sync(gmask, x.l, o))));
     v[k] = (double)x.h + (double)x.l;

@@ -154,35 +154,32 @@ static __device__ __forceinline__ int tab_at(float qh, float &t) {
   return (u >> TAB_SHIFT) - TAB_BASE;
 }
 // one interval's coefficients
-template <class V>
 struct Coef {
-  V c0h, c0l, c1h, c1l, c2h, c2l, c3, c4;
+  float c0h, c0l, c1h, c1l, c2h, c2l, c3, c4;
 };
-static __device__ __forceinline__ void coef_set(Coef<float> &o, const float4 *a) {
+static __device__ __forceinline__ void coef_set(Coef &o, const float4 *a) {
   const float4 x = __ldg(a), y = __ldg(a + 1);
   o.c0h = x.x; o.c0l = x.y; o.c1h = x.z; o.c1l = x.w;
   o.c2h = y.x; o.c2l = y.y; o.c3 = y.z; o.c4 = y.w;
 }
 // the polynomial at t (normalised).  |t| is below 2^-TAB_BITS-1 of q, so the terms fall off
 // by ~2^-7 each and FP32 serves from the third power on
-template <class V>
-static __device__ __forceinline__ D<V> tab_poly(const Coef<V> &c, D<V> t) {
-  D<V> s = mul(mk(c.c2h, vfma(vfma(c.c4, t.h, c.c3), t.h, c.c2l)), t);
-  const D<V> s1 = two_sum(c.c1h, s.h);
+static __device__ __forceinline__ D tab_poly(const Coef &c, D t) {
+  D s = mul(mk(c.c2h, vfma(vfma(c.c4, t.h, c.c3), t.h, c.c2l)), t);
+  const D s1 = two_sum(c.c1h, s.h);
   s = mul(mk(s1.h, vadd(s1.l, vadd(s.l, c.c1l))), t);
-  const D<V> s0 = two_sum(c.c0h, s.h);
+  const D s0 = two_sum(c.c0h, s.h);
   return mk(s0.h, vadd(s0.l, vadd(s.l, c.c0l)));
 }
 // f0 - 1/2 the integral of the polynomial from 0 to t
-template <class V>
-static __device__ __forceinline__ D<V> tab_integral(const Coef<V> &c, V f0h, V f0l, D<V> t) {
-  const V half = vall<V>(0.5f);
-  V u = vfma(vmul(c.c4, vall<V>(0.2f)), t.h, vmul(c.c3, vall<V>(0.25f)));
-  u = vfma(u, t.h, vmul(c.c2h, vall<V>(1.f / 3.f)));
-  D<V> s = mul(mk(vmul(half, c.c1h), vfma(u, t.h, vmul(half, c.c1l))), t);
-  const D<V> s1 = two_sum(c.c0h, s.h);
-  s = scale(mul(mk(s1.h, vadd(s1.l, vadd(s.l, c.c0l))), t), vall<V>(-0.5f));
-  const D<V> s0 = two_sum(f0h, s.h);
+static __device__ __forceinline__ D tab_integral(const Coef &c, float f0h, float f0l, D t) {
+  const float half = 0.5f;
+  float u = vfma(vmul(c.c4, 0.2f), t.h, vmul(c.c3, 0.25f));
+  u = vfma(u, t.h, vmul(c.c2h, 1.f / 3.f));
+  D s = mul(mk(vmul(half, c.c1h), vfma(u, t.h, vmul(half, c.c1l))), t);
+  const D s1 = two_sum(c.c0h, s.h);
+  s = scale(mul(mk(s1.h, vadd(s1.l, vadd(s.l, c.c0l))), t), -0.5f);
+  const D s0 = two_sum(f0h, s.h);
   return mk(s0.h, vadd(s0.l, vadd(s.l, f0l)));
 }
 
@@ -195,19 +192,19 @@ static __device__ __forceinline__ bool near_one(float nd2, float q, float p1, fl
 // The parts the normals enter: crad += (C M + B) S, tp, tq, and S (weighted).  pn = n_i .
 // del, qn = n_j . del; K(k): constant k; tab: the exp2 table.  W (subdomain mode): weights
 // wi and wj of the repulsion terms with n_i and n_j.
-template <bool W, class V, class KF>
-static __device__ __forceinline__ void pair_near(KF K, const float2 *tab, D<V> q, D<V> TE, D<V> M, D<V> pn, D<V> qn, V wi,
-                                                 V wj, D<V> &crad, D<V> &tp, D<V> &tq, D<V> &S) {
-  auto KD = [&](int k) { return mk<V>(K(k), K(k + 1)); };
-  const D<V> rho1 = add_ordered(q, neg(sqr(pn))), rho2 = add_ordered(q, neg(sqr(qn)));
-  D<V> G1 = exp2(mul(renorm(rho1), KD(K_ND2)), tab);
-  D<V> G2 = exp2(mul(renorm(rho2), KD(K_ND2)), tab);
+template <bool W, class KF>
+static __device__ __forceinline__ void pair_near(KF K, const float2 *tab, D q, D TE, D M, D pn, D qn, float wi,
+                                                 float wj, D &crad, D &tp, D &tq, D &S) {
+  auto KD = [&](int k) { return mk(K(k), K(k + 1)); };
+  const D rho1 = add_ordered(q, neg(sqr(pn))), rho2 = add_ordered(q, neg(sqr(qn)));
+  D G1 = exp2(mul(renorm(rho1), KD(K_ND2)), tab);
+  D G2 = exp2(mul(renorm(rho2), KD(K_ND2)), tab);
   if constexpr (W) {
     G1 = scale(G1, wi);
     G2 = scale(G2, wj);
   }
   S = renorm(add(G1, G2));
-  const D<V> B = renorm(mul(TE, KD(K_C2D)));
+  const D B = renorm(mul(TE, KD(K_C2D)));
   tp = mul(mul(pn, B), G1);
   tq = mul(mul(qn, B), G2);
   crad = add(crad, mul(S, renorm(add(mul(M, KD(K_C)), B))));
