@@ -558,7 +558,7 @@ static void sys_geometry(SysDesc &sd, const double lo[3], const double L[3], con
   // three-part positions: the coarse grid leaves 24 bits for four times the largest
   // coordinate in or near the box (differences of h are then exact in FP32), the fine grid
   // is 2^-21 of it (differences of m, up to several image shifts included, stay within 24
-  // bits); beyond dfmax, four times what the coarse grid holds, m would need more
+  // bits); beyond dfmax, twice what the coarse grid holds in 24 bits, m would need more
   double big = 0.0;
   for (int k = 0; k < 3; k++)
     big = std::max(big, std::max(std::fabs(sd.lo[k]), std::fabs(sd.lo[k] + sd.L[k])) + sd.L[k] + 64.0);
@@ -1651,6 +1651,9 @@ struct Engine {
                    NS_ND fn, NS_FIN ff) {
     a.do_ters = t_on && (which & LMFF_TERSOFF);
     a.do_ilp = i_on && (which & LMFF_ILP);
+    // the sums of a style that does not run; ahead of the kernels that may be launched early
+    if (ev && !a.do_ters) cudaMemsetAsync(stat_ters, 0, sizeof(double) * 8 * (size_t)n, stream);
+    if (ev && !a.do_ilp) cudaMemsetAsync(stat_ilp, 0, sizeof(double) * 8 * (size_t)n, stream);
     timed(2, [&] { fs(a, d_cutILPsq, ht.cutmax * ht.cutmax, stream); });
     // Tersoff (FP64-pipe bound) on a second stream beside the pair kernel (FP32 bound):
     // the two share the SMs and overlap; joined before the gather.  Serial when the
@@ -1673,8 +1676,6 @@ struct Engine {
       cudaEventRecord(ev_join, stream2);
     } else if (a.do_ters) {
       timed(1, [&] { ft(a, ev, eatom, stream); });
-    } else if (ev) {
-      cudaMemsetAsync(stat_ters, 0, sizeof(double) * 8 * (size_t)n, stream);
     }
     if (a.do_ilp) {
       if (!fork || FRAME_FIRST) timed(6, [&] { fr(a, stream); });
@@ -1682,11 +1683,10 @@ struct Engine {
       if (fork && !FRAME_FIRST) cudaStreamWaitEvent(stream, ev_frame, 0);
       timed(6, [&] { fn(a, ev, stream); });
     }
-    else {
+    else if (FRAME_FIRST && i_on) {
       // an atom without a normal is an error for every style: the mixed k_short says so, in
       // FP64 the frames do (4 us for 7,200 atoms)
-      if (FRAME_FIRST && i_on) timed(6, [&] { fr(a, stream); });
-      if (ev) cudaMemsetAsync(stat_ilp, 0, sizeof(double) * 8 * (size_t)n, stream);
+      timed(6, [&] { fr(a, stream); });
     }
     if (eatom && !a.do_ters) cudaMemsetAsync(eatom_ters, 0, sizeof(double) * (size_t)n, stream);
     if (fork) cudaStreamWaitEvent(stream, ev_join, 0);
@@ -3246,15 +3246,15 @@ int noalloc_compute(Engine &g, int nn, const double *dx, const int *dtype, const
   double *ters_f = cv.take<double>(3 * c), *ilp_f = cv.take<double>(3 * c), *fs = cv.take<double>(3 * c);
   double *stat_ilp = cv.take<double>(8 * c), *stat_ters = cv.take<double>(8 * c);
   double *eat_i = cv.take<double>(c), *eat_t = cv.take<double>(c);
-  int64_t *list_off = cv.take<int64_t>(c + 1), *cnt = cv.take<int64_t>(c + 1);
+  // list_off's piece also holds the status word, beside the list's total: one copy brings both
+  int64_t *list_off = cv.take<int64_t>(c + 1 + 32), *cnt = cv.take<int64_t>(c + 1);
   uint32_t *key = cv.take<uint32_t>(c), *key2 = cv.take<uint32_t>(c);
   int *idx = cv.take<int>(c), *idx2 = cv.take<int>(c);
   int *bin_start = cv.take<int>(NOALLOC_MAX_BINS), *bin_end = cv.take<int>(NOALLOC_MAX_BINS);
   SysDesc *dsys = cv.take<SysDesc>(1);
   double *red = cv.take<double>(16);
   double **arrs = cv.take<double *>(2);
-  cv.take<int>(1);
-  int *status = reinterpret_cast<int *>(list_off + nn + 1);   // beside the list's total (the piece is padded)
+  int *status = reinterpret_cast<int *>(list_off + nn + 1);
   size_t tmp_bytes = nb_sort_tmp_bytes(c, 32);
   void *tmp = cv.take<unsigned char>(tmp_bytes);
   if (!tmp) return g.fail(LMFF_EOVERFLOW, "lmff_compute_device_noalloc: scratch layout does not fit");
