@@ -376,9 +376,12 @@ __global__ void __launch_bounds__(32 * LW) k_list(NbArgs a) {
 // few warps of a small system cannot hide; its shared tiles pay in large ones.  A rebuild
 // (with the sort and the copy to the list; in place / here / k_list): 1,152 atoms 0.19 / 0.16 /
 // 0.89 ms, 5,040-atom bilayer 0.25 / 0.20 / 0.62, 36,800-atom slab 1.90 / 1.04 / 2.28,
-// 60,480-atom bilayer - / 0.66 / 0.78, 81,200-atom slab - / 2.04 / 2.52, 300,240-atom bilayer
-// - / 2.58 / 1.98 (all three before k_place took ~40 us off a rebuild).  Bound by instruction
-// issue (occupancy of 20 to 40 warps made no difference).
+// 60,480-atom bilayer - / 0.66 / 0.78 (all three before k_place took ~40 us off a rebuild).
+// The line lies below the first size at which k_list is as fast.  A system's first build
+// (two walks; here / k_list): bilayers of 65,688 atoms 1.10 / 1.15 ms, 81,312 1.30 / 1.30,
+// 119,784 1.78 / 1.54; ten-layer slabs of 65,720 2.73 / 3.47, 80,240 3.23 / 3.61, 120,960
+// 4.82 / 4.70; 64 bilayers of 500 to 20,000 atoms, 363,498 together, 3.07 / 2.34.
+// Issue 69 %, ALU pipe 51 % (36,800-atom slab); occupancy of 20 to 40 warps made no difference.
 constexpr int LIST_ATOM_MAX_ATOMS = 65536;
 constexpr int LIST_QUEUE = 64;
 __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
