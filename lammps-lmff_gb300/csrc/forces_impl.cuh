@@ -961,7 +961,7 @@ __device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int i
     if (s < cnt) {
       const TersP<R> &p = c_pot.ters[(ie * MAXELEM + el[s]) * MAXELEM + el[s]];
       const double e1 = exp_t64<true>(-p.lam1_64 * r[s]);
-      double rep = p.Al1_64 * e1 * ri[s], on = 1.0;
+      double rep = p.A64 * e1 * p.lam1_64 * ri[s], on = 1.0;   // (A lam1 rounded beforehand would bias every bond alike)
       if constexpr (GH) {
         int j, sx, sy, sz;
         decode_entry(en[s], a.lc, j, sx, sy, sz);
@@ -978,7 +978,7 @@ __device__ __forceinline__ bool tersoff_fast(const ForceArgs<R> &a, int i, int i
         const double bij = exp_t64<true>(-p.inv2n * ln_t64(W));
         const double bd = -0.5 * (bij * T) * rcp3(W * zeta[s]);
         const double e2 = exp_t64<true>(-p.lam2_64 * r[s]), fa = -p.B64 * e2;
-        fp2[s] = 0.5 * bij * (p.Bl2_64 * e2) * ri[s];
+        fp2[s] = 0.5 * bij * (p.B64 * e2 * p.lam2_64) * ri[s];
         eb[s] = 0.5 * bij * fa;
         pref[s] = -0.5 * fa * bd;
         if (EV) eng += eb[s];
