@@ -1025,8 +1025,9 @@ struct Engine {
   }
   int pair_df = 0;
   // the double-float kernel's tables (491 KB per element pair, allocated with the engine) and
-  // the per-atom virial's (197 KB, with its first pass), filled once: engines of different
-  // potentials on one device do not refill them at each change of the device's constants
+  // the per-atom virial's (197 KB, with its first pass), filled once, in the first FP64
+  // evaluation and pass: they depend on the potential and the cutoff alone, which an engine
+  // keeps
   float4 *d_dfA = nullptr, *d_dfM = nullptr;
   float2 *d_dfU = nullptr, *d_dfTE = nullptr;
   double *d_va64 = nullptr;
@@ -1084,7 +1085,6 @@ struct Engine {
     nbc.innersq_f = (float)(cut_global * cut_global);
     hash_tables();
     pot_dirty = true;
-    df_filled = va64_filled = false;
     built = false;
     return LMFF_OK;
   }
