@@ -63,7 +63,12 @@ extern "C" {
 #define LMFF_PENDING 1                /* lmff_server_wait: the request has not finished yet */
 
 /* ---- precision modes ------------------------------------------------------------ */
-#define LMFF_FP64 0   /* all-FP64 drop-in */
+#define LMFF_FP64 0   /* the drop-in: results to 1e-10 of the reference's.  All of it FP64
+                         but the pairs of ilp/graphene/hbn with element-symmetric
+                         constants, which run in double-float arithmetic (two FP32
+                         numbers, ~48 bits, per-atom sums included; FP64 below 0.5 A and
+                         at the cutoff): errors against 80-bit arithmetic at or below
+                         those of the general FP64 kernel, which "list_full" 1 selects */
 #define LMFF_MIXED 1  /* FP32 pair / three-body arithmetic on FP64 displacements;
                          FP64 integration, per-atom accumulation, reductions and
                          normal-derivative assembly */
@@ -291,8 +296,9 @@ int lmff_compute_ghost(lmff_engine *e, int nlocal, int nall, const double *x, co
  * order, energy units, not divided by a volume); natoms = that call's natoms (nall in
  * subdomain mode, where ghost rows carry the shares LAMMPS's reverse communication
  * folds into their owners).  A separate pass on the evaluated positions: Tersoff's
- * shares in FP64, the interlayer shares in the evaluation's precision (LMFF_MIXED: FP32
- * pair terms, FP64 sums); not for batches (LMFF_EUNSUPPORTED). */
+ * shares in FP64, the interlayer shares in the evaluation's precision (LMFF_FP64: FP64
+ * below 7 A, double-float beyond; LMFF_MIXED: FP32 pair terms, double-float sums); not for
+ * batches (LMFF_EUNSUPPORTED). */
 int lmff_compute_vatom(lmff_engine *e, int which, int natoms, double *vatom);
 
 /* Same on device pointers (d_x[natoms*3] double, d_type int32, d_mol int64, d_tag int64
