@@ -57,9 +57,11 @@ ILP_FILE = os.path.join(ROOT, "lammps-lmff_gb300", "potentials", "BNCH.ILP")
 # 331,200-atom graphite slab (k_ilp<16,0,0,1,0,0,1>: 1.297 GB read + 20.1 MB written for
 # 310,301,280 entries; the list is larger than L2, so traffic grows with the entries)
 K_ILP_DRAM_BYTES_PER_ENTRY = (1.297430e9 + 20.068096e6) / 310301280
-# FP64-pipe activity of the two FP64-bound per-atom kernels of the mixed step (ncu
-# sm__pipe_fp64_cycles_active on the 331,200-atom slab, profiles/)
-FP64_PIPE_ACTIVE_NCU = {"k_tersoff": 0.624, "k_nderiv": 0.824}
+# FP64-pipe activity of the two FP64-bound per-atom kernels, forces only (ncu
+# sm__pipe_fp64_cycles_active on the 331,200-atom slab, profiles/); normal_deriv times the
+# frames and the derivative assembly together, in FP64 84.4 us at 0.832 and 32.6 at 0.732
+FP64_PIPE_ACTIVE_NCU = {"mixed": {"k_tersoff": 0.624, "k_nderiv": 0.824},
+                        "fp64": {"k_tersoff": 0.855, "k_nderiv": 0.804}}
 L2_BYTES = 129e6   # GB300 L2
 FLOPS_H = os.path.join(ROOT, "bench", "flops.h")
 
@@ -625,16 +627,12 @@ def rooflines(m, s, prec, pk, peaks) -> dict:
         a = flops / (t / 1e3) / 1e12
         e = {"bound": "fp64", "kernel_ms_avg": t, "alg_flops": flops, "achieved_alg": a, "unit": "TFLOP/s",
              "peak_fp64": pk["fp64"], "peak_fp32": pk["fp32"]}
-        if prec == capi.FP64:
-            e["frac"] = a / pk["fp64"] if pk["fp64"] else None
-            e["frac_source"] = "algorithmic flops over the measured DGEMM peak"
-        else:
-            # the mixed kernels do the reference's FP64 arithmetic partly in FP32 and in
-            # fewer FP64 operations, so their position on the FP64 roofline is the
-            # measured FP64-pipe activity
-            e["frac"] = FP64_PIPE_ACTIVE_NCU[kern]
-            e["frac_source"] = "ncu sm__pipe_fp64_cycles_active, 331,200-atom slab (profiles/)"
-            e["alg_frac_of_fp32_peak"] = a / pk["fp32"] if pk["fp32"] else None
+        # the kernels do the reference's arithmetic in fewer FP64 operations (the mixed ones
+        # partly in FP32), so their position on the FP64 roofline is the measured FP64-pipe
+        # activity, not the algorithmic flops over the DGEMM peak
+        e["frac"] = FP64_PIPE_ACTIVE_NCU["fp64" if prec == capi.FP64 else "mixed"][kern]
+        e["frac_source"] = "ncu sm__pipe_fp64_cycles_active, 331,200-atom slab (profiles/)"
+        e["alg_frac_of_fp32_peak"] = a / pk["fp32"] if pk["fp32"] else None
         out[kern] = e
     return out
 
