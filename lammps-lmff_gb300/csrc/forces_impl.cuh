@@ -2343,7 +2343,7 @@ __global__ void __launch_bounds__(256, (ilp_min_blocks<TPA, EV, EATOM, ONE, GH, 
 // its own in place with direct radial functions; 31 of 32 and 5.2 ms with queue and
 // tables).  What bounds it is the latency of the record and table gathers at 4.6 warps per
 // scheduler: issue 68 %, L1 wavefronts 55 %, FMA pipe 48 % (36,800-atom slab, forces; with
-// energies 3.7 warps, issue 56 %, L1 43 %, FMA 43 %, a fifth of the waits for instructions).
+// energies 3.7 warps, issue 56 %, L1 43 %, FMA 43 %, a quarter of the waits for instructions).
 // Blocks of up to 128 threads, 5 per SM (96 registers), with energies and virial 4 (128):
 // one block more or less per SM measured 3-10 % slower on the 331,200-atom slab.
 constexpr int DF_THREADS = 128;
